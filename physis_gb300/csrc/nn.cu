@@ -5,16 +5,20 @@
 //
 // Tensors are channels-last, [batch, z, y, x, 16] BF16 (16 channels: 32
 // bytes per voxel).  A convolution is an implicit GEMM per tap: rows are
-// voxels, K the 16 input channels, N the 16 output channels.  Tensor cores
-// via mma.sync.m16n8k16 (BF16 in, FP32 accumulate): each warp owns 16
-// voxels and accumulates 27 taps x 2 n-tiles; the layer's weights sit in
-// shared memory in the fragment-friendly [tap][out][in] order.  The
-// backward-data pass is the same kernel with the weights flipped in space
-// and transposed in channels; the weight gradient is a K = voxels GEMM per
-// tap, split over CTAs and reduced in a fixed order (deterministic).
+// voxels, K the 16 input channels, N the 16 output channels.  Three forms:
+// conv_pad_kernel (tcgen05 over zero-padded slabs) wherever a padded plane has
+// at most 1024 voxels, conv_tc_kernel (tcgen05, gathered tiles) for larger
+// planes, and conv_kernel (mma.sync.m16n8k16: each warp owns 16 voxels and
+// accumulates 27 taps x 2 n-tiles) when PS_WARMSTART_TC=0 asks for it.  The
+// backward-data pass is the same kernel with the weights flipped in space and
+// transposed in channels; the weight gradient is a K = voxels GEMM per tap
+// (wgrad_pad_kernel; wgrad_kernel where a slab does not fit), split over CTAs
+// and reduced in a fixed order (deterministic).
 // Pooling (fine grids -> coarse network input), the MSE gradient, Adam and
 // cubic upsampling (coarse prediction -> fine warm start) complete the
 // set.  Every kernel is checked against oracle/nn_oracle.py.
+#include <cooperative_groups.h>
+#include <cuda.h>
 #include <cuda_bf16.h>
 #include <stdlib.h>
 #include <cuda_runtime.h>
@@ -297,6 +301,406 @@ conv_tc_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restr
   }
 }
 
+// ---- padded slabs ---------------------------------------------------------------
+//
+// The kernels below stage a slab of z planes of one instance as zero-padded
+// planes: rows of X + 1 voxels, Y + 1 rows, the last column and row zero, so
+// that the neighbour of padded voxel m at tap (dz, dy, dx) is voxel
+// m + dz P + dy (X + 1) + dx (P = (Y + 1)(X + 1)) whatever m is: one voxel's
+// left pad is the previous row's last column.  A slab arrives as one TMA box
+// per 8-channel half of [batch, z, y, x, channel]; TMA fills what lies
+// outside the tensor with zeros, which is the padding.  A half plane holds 16
+// bytes per voxel, so a tap of 8 or 128 consecutive voxels is contiguous
+// shared memory at a shifted start address: nothing is gathered per tap.
+struct PadGeom {
+  int px, P;       // row and plane pitch in padded voxels
+  int zs, nslab;   // planes per slab, slabs per instance
+  int pre;         // bytes in front of a half plane (zeros: the first row's upper-left taps)
+};
+
+// Planes per slab: at most zmax, fewer while there are not `want` slabs,
+// then evened out over the slabs of an instance.
+PadGeom pad_geom(const Dims &d, int zmax, long long want) {
+  PadGeom g;
+  g.px = d.X + 1;
+  g.P = (d.Y + 1) * g.px;
+  g.pre = ((g.px + 1) * 16 + 127) / 128 * 128;
+  const long long spread = ((long long)d.B * d.Z + want - 1) / want;
+  int zs = zmax < d.Z ? zmax : d.Z;
+  if (spread < zs) zs = (int)spread;
+  g.nslab = (d.Z + zs - 1) / zs;
+  g.zs = (d.Z + g.nslab - 1) / g.nslab;
+  g.nslab = (d.Z + g.zs - 1) / g.zs;
+  return g;
+}
+
+__device__ __forceinline__ void tma_load_5d(uint32_t dst, const CUtensorMap *map, int c, int x,
+                                            int y, int z, int b, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%2, %3, %4, %5, %6}], [%7];" ::"r"(dst),
+      "l"(reinterpret_cast<unsigned long long>(map)), "r"(c), "r"(x), "r"(y), "r"(z), "r"(b),
+      "r"(bar)
+      : "memory");
+}
+
+// ---- tcgen05 convolution over padded slabs --------------------------------------
+//
+// As conv_tc_kernel (M = 128, N = 16, 27 taps of K = 16 in the same order, so
+// the same bits), with the A operand of every tap read straight from the
+// padded half planes: tap t of 128 consecutive padded voxels is the no-swizzle
+// K-major matrix whose 8-voxel core matrices lie 128 bytes apart and whose two
+// 8-channel halves one half plane apart, at a start address shifted by the
+// tap.  Rows that are padding compute values nobody stores (19 % of 9 x 9
+// planes).  Warp 4 issues the TMA boxes and all MMAs, one commit per tile of
+// 128; warps 0-3 read each finished tile's 16 accumulator columns and apply
+// the epilogue while later tiles are still running.
+// Bound: every MMA reads its 4 KB A tile from shared memory, 27 * 32 cycles
+// per 128 voxels (46 us of the case below).  Measured on 1024 x 17 x 9 x 9
+// voxels: 73 us (267 TFLOP/s, tensor pipe 86 % active) against 187 us of
+// conv_tc_kernel, which gathers every tap's tile through registers; on 32
+// instances 9.6 against 12.5 us.
+constexpr int kPcThreads = 160;
+constexpr int kPcMaxTiles = 8;                     // 8 x 16 accumulator columns
+constexpr int kPcCols = kPcMaxTiles * kC;          // tensor memory columns
+constexpr int kPcHead = 256;                       // barriers, tensor memory address, bias
+constexpr int kPcB = kTaps * kTcBTile;             // weights
+constexpr size_t kPcMinSmem = 46 * 1024;           // at most 4 CTAs x 128 columns per SM
+
+__host__ __device__ constexpr int pc_tiles(int zs, int P) { return (zs * P + kTcM - 1) / kTcM; }
+// Bytes of one half plane: the zeros in front, then every row a tile's taps read.
+__host__ __device__ constexpr int pc_half(int zs, int P, int px, int pre) {
+  return pre + ((pc_tiles(zs, P) * kTcM + 2 * P + px + 1) * 16 + 127) / 128 * 128;
+}
+size_t pc_smem(const PadGeom &g) {
+  const size_t n = 128 + kPcHead + kPcB + 2 * (size_t)pc_half(g.zs, g.P, g.px, g.pre);
+  return n < kPcMinSmem ? kPcMinSmem : n;
+}
+
+__global__ void __launch_bounds__(kPcThreads)
+conv_pad_kernel(const __grid_constant__ CUtensorMap tmx, const __nv_bfloat16 *__restrict__ w,
+                const float *__restrict__ bias, const __nv_bfloat16 *__restrict__ mask, int relu,
+                __nv_bfloat16 *__restrict__ y, float *__restrict__ yf, Dims d, PadGeom g,
+                int *err) {
+  extern __shared__ __align__(128) unsigned char pc_raw[];
+  unsigned char *smem = pc_raw + ((128u - (smem_u32(pc_raw) & 127u)) & 127u);
+  unsigned long long *bars = reinterpret_cast<unsigned long long *>(smem);  // load, tiles
+  uint32_t *tslot = reinterpret_cast<uint32_t *>(smem + 128);
+  float *sbias = reinterpret_cast<float *>(smem + 192);
+  unsigned char *sb = smem + kPcHead;
+  unsigned char *sx = sb + kPcB;
+  const int half = pc_half(g.zs, g.P, g.px, g.pre);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int b = blockIdx.x / g.nslab;
+  const int z0 = (blockIdx.x - b * g.nslab) * g.zs;
+  const int nz = min(g.zs, d.Z - z0);
+  const int rows = nz * g.P;
+  const int ntiles = (rows + kTcM - 1) / kTcM;
+
+  if (warp == 4) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     smem_u32(tslot)),
+                 "r"(kPcCols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    if (lane == 0) {
+      for (int i = 0; i <= kPcMaxTiles; ++i) mbar_init(&bars[i], 1);
+      fence_barrier_init();
+      // planes z0 - 1 .. z0 + zs of both halves
+      mbar_arrive_expect_tx(&bars[0], 2u * (unsigned)((g.zs + 2) * g.P * 16));
+      for (int h = 0; h < 2; ++h)
+        tma_load_5d(smem_u32(sx + h * half + g.pre), &tmx, 8 * h, 0, 0, z0 - 1, b,
+                    smem_u32(&bars[0]));
+    }
+  } else {
+    // weights: out channel n's 16 in-channels as two 16-byte halves
+    for (int i = tid; i < kTaps * kC * 2; i += 128) {
+      const int t = i / (kC * 2), n = (i / 2) % kC, c = i & 1;
+      const uint4 v = *reinterpret_cast<const uint4 *>(w + (t * kC + n) * kC + c * 8);
+      *reinterpret_cast<uint4 *>(sb + t * kTcBTile + (n >> 3) * 256 + c * 128 + (n & 7) * 16) = v;
+    }
+    for (int i = tid; i < g.pre / 8; i += 128)
+      *reinterpret_cast<uint4 *>(sx + (i >= g.pre / 16 ? half - g.pre : 0) + i * 16) =
+          make_uint4(0u, 0u, 0u, 0u);
+    if (tid < kC) sbias[tid] = bias ? bias[tid] : 0.f;
+    // generic-proxy writes visible to the tensor core (async proxy)
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tslot;
+
+  if (warp == 4) {
+    if (lane == 0) {
+      const bool ok = mbar_wait(&bars[0], 0, err);
+      const uint32_t a0 = smem_u32(sx) + g.pre, b0 = smem_u32(sb);
+      for (int i = 0; i < ntiles && ok; ++i) {
+        // row m of the tile is padded voxel m of the slab's first own plane,
+        // one plane into the staged ones
+        const uint32_t base = a0 + i * kTcM * 16;
+#pragma unroll
+        for (int t = 0; t < kTaps; ++t) {
+          const int dz = t / 9, dy = (t / 3) % 3 - 1, dx = t % 3 - 1;
+          const uint64_t ad = umma_desc(base + (dz * g.P + dy * g.px + dx) * 16, half, 128);
+          const uint64_t bd = umma_desc(b0 + t * kTcBTile, 128, 256);
+          asm volatile(
+              "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %4, 0;\n\t"
+              "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem + i * kC),
+              "l"(ad), "l"(bd), "r"(kTcIdesc), "r"((uint32_t)(t > 0))
+              : "memory");
+        }
+        asm volatile(
+            "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                smem_u32(&bars[1 + i]))
+            : "memory");
+      }
+    }
+    __syncwarp();
+  } else {
+    const long long vox0 = ((long long)b * d.Z + z0) * d.Y * d.X;
+    // padded voxel of this thread's row: coordinates advanced by 128 per tile
+    int m = tid;
+    int zz = m / g.P, r = m - zz * g.P;
+    int yy = r / g.px, xx = r - yy * g.px;
+    const int sz = kTcM / g.P, sr = kTcM - sz * g.P, sy = sr / g.px, sxx = sr - sy * g.px;
+    for (int i = 0; i < ntiles; ++i) {
+      if (!__all_sync(0xffffffffu, mbar_wait(&bars[1 + i], 0, err))) break;
+      tc_fence_after();
+      uint32_t a[16];
+      asm volatile(
+          "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+          "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+          : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3]), "=r"(a[4]), "=r"(a[5]), "=r"(a[6]),
+            "=r"(a[7]), "=r"(a[8]), "=r"(a[9]), "=r"(a[10]), "=r"(a[11]), "=r"(a[12]),
+            "=r"(a[13]), "=r"(a[14]), "=r"(a[15])
+          : "r"(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)(i * kC)));
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      if (zz < nz && yy < d.Y && xx < d.X) {
+        const long long v = vox0 + ((long long)zz * d.Y + yy) * d.X + xx;
+        float f[16];
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+          f[k] = __uint_as_float(a[k]);
+          if (bias) f[k] += sbias[k];
+          if (relu) f[k] = fmaxf(f[k], 0.f);
+        }
+        if (mask) {
+          uint4 mv[2];
+          mv[0] = *reinterpret_cast<const uint4 *>(mask + v * kC);
+          mv[1] = *reinterpret_cast<const uint4 *>(mask + v * kC + 8);
+          const __nv_bfloat16 *mb = reinterpret_cast<const __nv_bfloat16 *>(mv);
+#pragma unroll
+          for (int k = 0; k < 16; ++k)
+            if (!(__bfloat162float(mb[k]) > 0.f)) f[k] = 0.f;
+        }
+        uint4 o[2];
+        __nv_bfloat162 *ob = reinterpret_cast<__nv_bfloat162 *>(o);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) ob[k] = __floats2bfloat162_rn(f[2 * k], f[2 * k + 1]);
+        *reinterpret_cast<uint4 *>(y + v * kC) = o[0];
+        *reinterpret_cast<uint4 *>(y + v * kC + 8) = o[1];
+        if (yf) yf[v] = f[0];
+      }
+      xx += sxx;
+      yy += sy;
+      zz += sz;
+      if (xx >= g.px) {
+        xx -= g.px;
+        ++yy;
+      }
+      if (yy > d.Y) {
+        yy -= d.Y + 1;
+        ++zz;
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 4) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
+                 "r"(kPcCols)
+                 : "memory");
+  }
+}
+
+// ---- weight gradient over padded slabs -------------------------------------------
+//
+// dW[t][in][out] = sum over voxels v of X[v + d_t][in] * dY[v][out]: a GEMM
+// per tap with M = N = 16 and K = voxels.  M = 16 is below tcgen05's smallest
+// tile, so the products run on mma.sync.m16n8k16.  X and dY are staged as
+// padded slabs (two stages, so the next slab loads while this one is used);
+// padding contributes zeros.  Warp w owns the three x taps of its (z, y)
+// offset for every voxel of the CTA, so nothing is summed across warps: per 16
+// voxels it reads dY's fragment and three of X (ldmatrix.trans turns
+// [voxel][channel] rows into K = voxel fragments; eight 16-byte rows of a half
+// plane are 128 contiguous bytes, no bank conflicts) and issues six products.
+// The CTAs of a split form a cluster that adds its sums through distributed
+// shared memory in rank order, so the caller's work buffer holds nsplit
+// partials whatever the number of CTAs and results repeat bit for bit.
+// Bound: 54 products per 16 padded voxels on the mma.sync pipe (about 10
+// cycles each per sub-partition: 62 us of the case below); shared memory hands
+// out 36 ldmatrix tiles of 512 B for them (144 cycles, 54 us).  Measured on
+// 1024 x 17 x 9 x 9 voxels, nsplit 64: 137 us against 1760 us of wgrad_kernel
+// (2-byte gathers from L2 for each tap); on 32 instances 12.3 against 60 us.
+// What is left is balance: nine warps on four sub-partitions, 2.5 CTAs per SM.
+constexpr int kPwWarps = 9;   // one per (z, y) tap offset
+constexpr int kPwThreads = 32 * kPwWarps;
+constexpr int kPwMaxCluster = 8;
+constexpr size_t kPwSmem = 74 * 1024;   // three CTAs per SM
+constexpr size_t kPwMaxSmem = 200 * 1024;
+constexpr int kPwSums = kTaps * kC * kC + kPwWarps * kC;
+
+// Half planes of X (zs + 2 planes) and dY (zs planes); a last chunk of 16
+// voxels may read past the planes (zeroed once, never written again).
+__host__ __device__ constexpr int pw_half_x(int zs, int P, int px, int pre) {
+  return pre + (((zs + 2) * P + 16 + px + 1) * 16 + 127) / 128 * 128;
+}
+__host__ __device__ constexpr int pw_half_y(int zs, int P) {
+  return ((zs * P + 16) * 16 + 127) / 128 * 128;
+}
+__host__ __device__ constexpr int pw_stage(int zs, int P, int px, int pre) {
+  return 2 * (pw_half_x(zs, P, px, pre) + pw_half_y(zs, P));
+}
+size_t pw_smem(const PadGeom &g) {
+  const size_t n = 128 + 128 + 2 * (size_t)pw_stage(g.zs, g.P, g.px, g.pre);
+  const size_t sums = 128 + 128 + (size_t)kPwSums * 4;  // reuses the stages
+  return n < sums ? sums : n;
+}
+
+__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr)
+               : "memory");
+}
+
+__global__ void __launch_bounds__(kPwThreads, 3)
+wgrad_pad_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant__ CUtensorMap tmy,
+                 float *__restrict__ part, float *__restrict__ bpart, Dims d, PadGeom g, int items,
+                 int *err) {
+  namespace cg = cooperative_groups;
+  extern __shared__ __align__(128) unsigned char pw_raw[];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  // the same offset in every CTA of the cluster
+  unsigned char *smem = pw_raw + ((128u - (smem_u32(pw_raw) & 127u)) & 127u);
+  unsigned long long *bars = reinterpret_cast<unsigned long long *>(smem);
+  unsigned char *stage0 = smem + 128;
+  const int hx = pw_half_x(g.zs, g.P, g.px, g.pre), hy = pw_half_y(g.zs, g.P);
+  const int sbytes = 2 * (hx + hy);
+  const int rank = blockIdx.x, s = blockIdx.y, C = gridDim.x;
+  const int cta = s * C + rank, nctas = C * gridDim.y;
+
+  for (int i = tid; i < 2 * sbytes / 16; i += kPwThreads)
+    reinterpret_cast<uint4 *>(stage0)[i] = make_uint4(0u, 0u, 0u, 0u);
+  if (tid == 0) {
+    mbar_init(&bars[0], 1);
+    mbar_init(&bars[1], 1);
+    fence_barrier_init();
+  }
+  // the zeros before the TMA boxes that overwrite most of them
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  __syncthreads();
+
+  auto issue = [&](int item, int st) {
+    const int b = item / g.nslab, z0 = (item - b * g.nslab) * g.zs;
+    const uint32_t base = smem_u32(stage0) + st * sbytes, bar = smem_u32(&bars[st]);
+    mbar_arrive_expect_tx(&bars[st], 2u * (unsigned)((2 * g.zs + 2) * g.P * 16));
+    for (int h = 0; h < 2; ++h) {
+      tma_load_5d(base + h * hx + g.pre, &tmx, 8 * h, 0, 0, z0 - 1, b, bar);
+      tma_load_5d(base + 2 * hx + h * hy, &tmy, 8 * h, 0, 0, z0, b, bar);
+    }
+  };
+  if (tid == 0) {
+    if (cta < items) issue(cta, 0);
+    if (cta + nctas < items) issue(cta + nctas, 1);
+  }
+
+  float acc[3][2][4] = {};
+  float bacc[2][4] = {};  // ones x dY: this warp's share of the bias gradient
+  const uint32_t ones[4] = {0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u};
+  // this lane's row of an ldmatrix.x4: voxel lv of the chunk, channel half lh
+  const int lv = (lane & 7) + ((lane >> 4) << 3), lh = (lane >> 3) & 1;
+  const uint32_t xl = lh * hx + g.pre +
+                      (lv + (warp / 3) * g.P + (warp % 3 - 1) * g.px - 1) * 16;
+  const uint32_t yl = 2 * hx + lh * hy + lv * 16;
+  const int chunks = (g.zs * g.P + 15) / 16;
+
+  int st = 0;
+  uint32_t phase = 0;
+  bool ok = true;
+  for (int item = cta; item < items; item += nctas) {
+    if (!mbar_wait(&bars[st], phase, err)) ok = false;
+    uint32_t xa = smem_u32(stage0) + st * sbytes + xl;
+    uint32_t ya = smem_u32(stage0) + st * sbytes + yl;
+    int bias = warp + 1;
+#pragma unroll 4
+    for (int c = 0; c < chunks; ++c) {
+      uint32_t b[4], a[3][4];
+      ldmatrix_x4_trans(b, ya);
+#pragma unroll
+      for (int k = 0; k < 3; ++k) ldmatrix_x4_trans(a[k], xa + k * 16);
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        mma_16816(acc[k][0], a[k], b[0], b[2]);
+        mma_16816(acc[k][1], a[k], b[1], b[3]);
+      }
+      if (--bias == 0) {  // every ninth chunk: the warps share dY's sums evenly
+        bias = kPwWarps;
+        mma_16816(bacc[0], ones, b[0], b[2]);
+        mma_16816(bacc[1], ones, b[1], b[3]);
+      }
+      xa += 256;
+      ya += 256;
+    }
+    ok = __syncthreads_and(ok);  // every warp is done with the stage
+    if (!ok) break;
+    if (tid == 0 && item + 2 * nctas < items) issue(item + 2 * nctas, st);
+    if ((st ^= 1) == 0) phase ^= 1u;
+  }
+  if (!ok && tid == 0) {
+    // give copies still in flight a bounded chance to land
+    for (int i = 0; i < 2; ++i)
+      for (uint32_t q = 0; q < 2; ++q) mbar_wait(&bars[i], q, nullptr, 1024);
+  }
+  __syncthreads();
+
+  float *sums = reinterpret_cast<float *>(stage0);
+  const int gq = lane >> 2, q = lane & 3;
+#pragma unroll
+  for (int k = 0; k < 3; ++k)
+#pragma unroll
+    for (int n = 0; n < 2; ++n)
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+        *reinterpret_cast<float2 *>(sums + (warp * 3 + k) * kC * kC + (gq + i * 8) * kC + n * 8 +
+                                    2 * q) = make_float2(acc[k][n][2 * i], acc[k][n][2 * i + 1]);
+  if (gq == 0) {
+#pragma unroll
+    for (int n = 0; n < 2; ++n)
+      *reinterpret_cast<float2 *>(sums + kTaps * kC * kC + warp * kC + n * 8 + 2 * q) =
+          make_float2(bacc[n][0], bacc[n][1]);
+  }
+  cg::cluster_group cl = cg::this_cluster();
+  cl.sync();
+  const int n = kTaps * kC * kC;
+  for (int i = tid + rank * kPwThreads; i < n + kC; i += C * kPwThreads) {
+    float v = 0.f;
+    if (i < n) {
+      for (int r = 0; r < C; ++r) v += cl.map_shared_rank(sums, r)[i];
+      part[(long long)s * n + i] = v;
+    } else {
+      for (int r = 0; r < C; ++r) {
+        const float *p = cl.map_shared_rank(sums, r);
+        for (int k = 0; k < kPwWarps; ++k) v += p[i + k * kC];
+      }
+      bpart[s * kC + (i - n)] = v;
+    }
+  }
+  cl.sync();  // no CTA leaves while its sums are still being read
+}
+
 // Partial weight gradients: block (t, s) sums over the s-th share of the
 // 16-voxel chunks dW[t][in][out] = sum_v X[v + d_t][in] * dY[v][out] into
 // part[s][t][in][out]; blocks of the centre tap also sum dY into
@@ -371,19 +775,29 @@ wgrad_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restric
   }
 }
 
-__global__ void wgrad_reduce_kernel(const float *__restrict__ part,
-                                    const float *__restrict__ bpart, int S,
-                                    float *__restrict__ dw, float *__restrict__ db) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+// Sums the splits' partials in a fixed order: eight lanes per gradient, each
+// over every eighth split, then a shuffle tree (a thread per gradient walking
+// 64 partials one after the other took 5.1 us, latency-bound).
+__global__ void __launch_bounds__(256)
+wgrad_reduce_kernel(const float *__restrict__ part, const float *__restrict__ bpart, int S,
+                    float *__restrict__ dw, float *__restrict__ db) {
+  // a warp holds four gradients' worth of lanes: neighbouring lanes read
+  // neighbouring gradients of the same split
+  const int lane = threadIdx.x & 31;
+  const int i = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 4 + (lane & 3);
+  const int k = lane >> 2;
   const int n = kTaps * kC * kC;
+  float v = 0.f;
   if (i < n) {
-    float v = 0.f;
-    for (int s = 0; s < S; ++s) v += part[(long long)s * n + i];
-    dw[i] = v;
+    for (int s = k; s < S; s += 8) v += part[(long long)s * n + i];
   } else if (i < n + kC && db) {
-    float v = 0.f;
-    for (int s = 0; s < S; ++s) v += bpart[s * kC + (i - n)];
-    db[i - n] = v;
+    for (int s = k; s < S; s += 8) v += bpart[s * kC + (i - n)];
+  }
+#pragma unroll
+  for (int o = 4; o < 32; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if (k == 0) {
+    if (i < n) dw[i] = v;
+    else if (i < n + kC && db) db[i - n] = v;
   }
 }
 
@@ -711,11 +1125,85 @@ static bool use_tcgen05() {
   return !(e && e[0] == '0');
 }
 
+static bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
+
+static int sm_count() {
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+    cudaGetLastError();
+    return 1;
+  }
+  return n;
+}
+
+// Tensor map of x [batch, z, y, x, 16] BF16 with a box of 8 channels x bx x by
+// x bz voxels of one instance; false if the driver cannot encode it.
+static bool tmap_slab(CUtensorMap *m, const void *x, const Dims &d, int bx, int by, int bz) {
+  typedef CUresult (*Encode)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *,
+                             const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
+                             const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
+                             CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+  static const Encode encode = [] {
+    void *fn = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault,
+                                         &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess) {
+      cudaGetLastError();
+      fn = nullptr;
+    }
+    return reinterpret_cast<Encode>(fn);
+  }();
+  if (!encode) return false;
+  const cuuint64_t dims[5] = {(cuuint64_t)kC, (cuuint64_t)d.X, (cuuint64_t)d.Y, (cuuint64_t)d.Z,
+                              (cuuint64_t)d.B};
+  const cuuint64_t row = (cuuint64_t)kC * 2;
+  const cuuint64_t strides[4] = {row, row * d.X, row * d.X * d.Y,
+                                 row * d.X * d.Y * (cuuint64_t)d.Z};
+  const cuuint32_t box[5] = {8, (cuuint32_t)bx, (cuuint32_t)by, (cuuint32_t)bz, 1};
+  const cuuint32_t one[5] = {1, 1, 1, 1, 1};
+  return encode(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void *>(x), dims, strides, box,
+                one, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// conv_pad_kernel over slabs, or false if a slab of one plane does not fit
+// (more than 1024 padded voxels per plane), a pointer is not aligned for TMA
+// and 16-byte accesses, or the map cannot be encoded.
+static bool launch_conv_pad(const void *x, const void *w, const float *bias, const void *mask,
+                            int relu, void *y, float *yf, const Dims &d, cudaStream_t s,
+                            cudaError_t *e) {
+  const long long P = (long long)(d.X + 1) * (d.Y + 1);
+  if (d.X > 255 || d.Y > 255 || P > kPcMaxTiles * kTcM || !aligned16(x) || !aligned16(w) ||
+      !aligned16(mask) || !aligned16(y))
+    return false;
+  int zmax = (int)(kPcMaxTiles * kTcM / P);
+  if (zmax > 254) zmax = 254;
+  const PadGeom g = pad_geom(d, zmax, 4LL * sm_count());
+  const long long items = (long long)d.B * g.nslab;
+  if (items > 0x7fffffff) return false;
+  CUtensorMap tm;
+  if (!tmap_slab(&tm, x, d, g.px, d.Y + 1, g.zs + 2)) return false;
+  const size_t smem = pc_smem(g);
+  *e = cudaFuncSetAttribute(conv_pad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                            (int)smem);
+  if (*e != cudaSuccess) return true;
+  conv_pad_kernel<<<(unsigned)items, kPcThreads, smem, s>>>(
+      tm, static_cast<const __nv_bfloat16 *>(w), bias, static_cast<const __nv_bfloat16 *>(mask),
+      relu, static_cast<__nv_bfloat16 *>(y), yf, d, g, g_err);
+  *e = cudaGetLastError();
+  return true;
+}
+
 int nn_conv(const void *x, const void *w, const float *bias, const void *mask, int relu,
             void *y, float *yf, int B, int Z, int Y, int X, cudaStream_t s) {
   Dims d{B, Z, Y, X, (long long)B * Z * Y * X};
   if (d.nvox <= 0) return 0;
   if (use_tcgen05()) {
+    cudaError_t e = cudaSuccess;
+    if (launch_conv_pad(x, w, bias, mask, relu, y, yf, d, s, &e)) return (int)e;
     static bool attr = false;
     if (!attr) {
       const cudaError_t e = cudaFuncSetAttribute(
@@ -737,16 +1225,70 @@ int nn_conv(const void *x, const void *w, const float *bias, const void *mask, i
   return (int)cudaGetLastError();
 }
 
+// wgrad_pad_kernel over slabs, or false if the planes are too large to stage
+// or the tensors not aligned for TMA.
+static bool launch_wgrad_pad(const void *x, const void *dy, float *part, float *bpart, int S,
+                             const Dims &d, cudaStream_t s, cudaError_t *e) {
+  if (d.X > 255 || d.Y > 255 || !aligned16(x) || !aligned16(dy)) return false;
+  const int sms = sm_count();
+  PadGeom g = pad_geom(d, 1, 1);
+  int zmax = 0;  // most planes per slab with three CTAs per SM, else with one
+  for (size_t limit : {kPwSmem, kPwMaxSmem}) {
+    for (int z = 1; z <= d.Z && z <= 254; ++z) {
+      g.zs = z;
+      if (pw_smem(g) > limit) break;
+      zmax = z;
+    }
+    if (zmax) break;
+  }
+  if (!zmax) return false;
+  g = pad_geom(d, zmax, 3LL * sms);
+  const long long items = (long long)d.B * g.nslab;
+  if (items > 0x3fffffff) return false;
+  CUtensorMap tmx, tmy;
+  if (!tmap_slab(&tmx, x, d, g.px, d.Y + 1, g.zs + 2) ||
+      !tmap_slab(&tmy, dy, d, g.px, d.Y + 1, g.zs))
+    return false;
+  // CTAs per split: up to 2.6 per SM in all.  Three fit, but a cluster's CTAs
+  // stay within one GPC, and 64 clusters of 7 (2.95 per SM) did not all find
+  // room at once: the last few ran alone (147 us, against 137 us with 6).
+  long long c = 26LL * sms / (10LL * S);
+  if (c > (items + S - 1) / S) c = (items + S - 1) / S;
+  if (c > kPwMaxCluster) c = kPwMaxCluster;
+  if (c < 1) c = 1;
+  const size_t smem = pw_smem(g);
+  *e = cudaFuncSetAttribute(wgrad_pad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                            (int)smem);
+  if (*e != cudaSuccess) return true;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)c, (unsigned)S);
+  cfg.blockDim = dim3(kPwThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)c;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  *e = cudaLaunchKernelEx(&cfg, wgrad_pad_kernel, tmx, tmy, part, bpart, d, g, (int)items, g_err);
+  return true;
+}
+
 int nn_wgrad(const void *x, const void *dy, float *part, int S, float *dw, float *db, int B,
              int Z, int Y, int X, cudaStream_t s) {
   Dims d{B, Z, Y, X, (long long)B * Z * Y * X};
   if (S < 1) return -1;
   float *bpart = part + (long long)S * kTaps * kC * kC;
-  wgrad_kernel<<<dim3(kTaps, S), 32 * kConvWarps, 0, s>>>(
-      static_cast<const __nv_bfloat16 *>(x), static_cast<const __nv_bfloat16 *>(dy), part, bpart,
-      d);
+  cudaError_t e = cudaSuccess;
+  if (!launch_wgrad_pad(x, dy, part, bpart, S, d, s, &e))
+    wgrad_kernel<<<dim3(kTaps, S), 32 * kConvWarps, 0, s>>>(
+        static_cast<const __nv_bfloat16 *>(x), static_cast<const __nv_bfloat16 *>(dy), part, bpart,
+        d);
+  if (e != cudaSuccess) return (int)e;
   const int n = kTaps * kC * kC + kC;
-  wgrad_reduce_kernel<<<(n + 255) / 256, 256, 0, s>>>(part, bpart, S, dw, db);
+  wgrad_reduce_kernel<<<(n + 31) / 32, 256, 0, s>>>(part, bpart, S, dw, db);
   return (int)cudaGetLastError();
 }
 
