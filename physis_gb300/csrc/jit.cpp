@@ -971,27 +971,18 @@ const char *type_name(int type) {
   }
 }
 
-std::string key_string(const PtsJitKey &k) {
-  std::string s;
-  char buf[64];
-  snprintf(buf, sizeof(buf), "%d,%d,%d,%d,%d,%d,%d,%d;", k.type, k.ry, k.warps, k.n,
-           k.unit ? 1 : 0, k.w, k.nstage, k.pstride);
-  s += buf;
-  for (int i = 0; i < k.n; ++i) {
-    snprintf(buf, sizeof(buf), "%d:%d:%a;", k.off[i], k.lag[i], k.wt[i]);
-    s += buf;
-  }
-  return s;
-}
-
 std::string points_source(const PtsJitKey &k) {
   std::string s = "#include \"points_body.cuh\"\nstruct GenSpec {\n"
                   "  static constexpr bool kStatic = true;\n";
   char buf[96];
   snprintf(buf, sizeof(buf), "  static constexpr int kN = %d;\n", k.n);
   s += buf;
-  s += "  static constexpr int kOff[kN] = {";
-  for (int i = 0; i < k.n; ++i) s += (i ? ", " : "") + std::to_string(k.off[i]);
+  s += "  static constexpr int kW = " + std::to_string(k.w) + ", kPlanes = " +
+       std::to_string(k.planes) + ", kCentre = " + std::to_string(k.centre) + ";\n";
+  s += "  static constexpr int kDx[kN] = {";
+  for (int i = 0; i < k.n; ++i) s += (i ? ", " : "") + std::to_string(k.dx[i]);
+  s += "};\n  static constexpr int kDy[kN] = {";
+  for (int i = 0; i < k.n; ++i) s += (i ? ", " : "") + std::to_string(k.dy[i]);
   s += "};\n  static constexpr int kLag[kN] = {";
   for (int i = 0; i < k.n; ++i) s += (i ? ", " : "") + std::to_string(k.lag[i]);
   s += "};\n  static constexpr double kWt[kN] = {";
@@ -1008,8 +999,8 @@ std::string points_source(const PtsJitKey &k) {
   s += "  template <typename T> static __device__ __forceinline__ int pstride("
        "const psg::PtsParams<T> &) { return " + std::to_string(k.pstride) + "; }\n};\n";
   const std::string T = type_name(k.type);
-  s += "extern \"C\" __global__ void __launch_bounds__(" + std::to_string(32 * k.warps) +
-       ", 1) __ps_points(const __grid_constant__ psg::PtsParams<" + T + "> p, "
+  s += "extern \"C\" __global__ void __launch_bounds__(" + std::to_string(32 * (k.warps + 1)) +
+       ", " + std::to_string(k.min_ctas) + ") __ps_points(const __grid_constant__ psg::PtsParams<" + T + "> p, "
        "const __grid_constant__ psg::PtsTmap tm) {\n"
        "  extern __shared__ __align__(128) unsigned char smem[];\n"
        "  psg::pts_body<" + T + ", " + std::to_string(k.ry) + ", " +
@@ -1017,14 +1008,22 @@ std::string points_source(const PtsJitKey &k) {
   return s;
 }
 
-std::map<std::string, void *> g_points_jit;  // key -> CUfunction (nullptr: failed)
+struct PointsJit {
+  void *fn = nullptr;  // CUfunction (nullptr: failed)
+  int occ = 0;
+};
+std::map<std::string, PointsJit> g_points_jit;  // by the key's bytes and smem
 
 }  // namespace
 
-void *jit_points_function(const PtsJitKey &k) {
-  const std::string key = key_string(k);
+void *jit_points_function(const PtsJitKey &k, size_t smem, int *occ) {
+  std::string key(reinterpret_cast<const char *>(&k), sizeof(k));
+  key.append(reinterpret_cast<const char *>(&smem), sizeof(smem));
   auto hit = g_points_jit.find(key);
-  if (hit != g_points_jit.end()) return hit->second;
+  if (hit != g_points_jit.end()) {
+    *occ = hit->second.occ;
+    return hit->second.fn;
+  }
   std::string err;
   void *fn = nullptr;
   if (load_nvrtc(&err) && load_driver(&err)) {
@@ -1034,7 +1033,15 @@ void *jit_points_function(const PtsJitKey &k) {
     nvrtcProgram_t prog = nullptr;
     if (g_nvrtc.create(&prog, program.c_str(), "points.cu", 2, hdr_src, hdr_name) == 0) {
       const char *opts[] = {"--gpu-architecture=sm_103a", "--std=c++17", "--fmad=false"};
-      if (g_nvrtc.compile(prog, 3, opts) == 0) {
+      const int rc = g_nvrtc.compile(prog, 3, opts);
+      if (rc != 0 && getenv("PS_JIT_LOG")) {
+        size_t n = 0;
+        g_nvrtc.log_size(prog, &n);
+        std::string log(n, '\0');
+        if (n) g_nvrtc.log(prog, &log[0]);
+        fprintf(stderr, "%s\n", log.c_str());
+      }
+      if (rc == 0) {
         size_t n = 0;
         g_nvrtc.cubin_size(prog, &n);
         std::vector<char> image(n);
@@ -1049,16 +1056,16 @@ void *jit_points_function(const PtsJitKey &k) {
       g_nvrtc.destroy(&prog);
     }
   }
-  g_points_jit[key] = fn;
-  return fn;
-}
-
-bool jit_prepare(void *fn, int threads, size_t smem, int *occ) {
+  PointsJit e;
+  e.fn = fn;
   CUfunction f = static_cast<CUfunction>(fn);
-  if (g_drv.set_attr(f, CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, (int)smem) !=
-      CUDA_SUCCESS)
-    return false;
-  return g_drv.occupancy(occ, f, threads, smem) == CUDA_SUCCESS;
+  if (fn && (g_drv.set_attr(f, CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, (int)smem) !=
+                 CUDA_SUCCESS ||
+             g_drv.occupancy(&e.occ, f, 32 * (k.warps + 1), smem) != CUDA_SUCCESS))
+    e.occ = 0;
+  g_points_jit[key] = e;
+  *occ = e.occ;
+  return fn;
 }
 
 cudaError_t jit_launch_raw(void *fn, int grid, dim3 block, size_t smem, cudaStream_t s,

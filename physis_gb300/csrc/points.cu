@@ -11,21 +11,30 @@
 // neighbour sums of the reference's system tests (27-point, 9-point 2D,
 // 3-point 1D, asymmetric, hole, periodic variants, red/black).
 //
-// Design.  A tile is 128 cells wide in x (32 lanes x 4 columns, lane-strided
-// so that every shared-memory access of a warp is conflict-free) and
-// warps*RY rows high; work items are (z-chunk, tile) pairs in chunk-major
-// order taken round-robin by a persistent grid, as in the 7-point kernels.
+// Design.  A tile is 128 cells wide in x and warps*RY rows high; a lane owns
+// RY rows of 16 bytes of consecutive cells (two such groups for 8-byte types)
+// in the compiled form, RY rows of four lane-strided cells in the table form;
+// work items are (z-chunk, tile) pairs in chunk-major order taken round-robin
+// by a persistent grid, as in the 7-point kernels.
 // * Each z-plane of the tile plus its x/y halo arrives in a ring of
 //   shared-memory planes by one TMA 3D box load (mbarrier per stage, bounded
 //   waits).  A box cannot wrap and fills cells outside the grid with zeros,
 //   so on the edge tiles of periodic and clamped stencils those halo cells
-//   are then rewritten through the boundary map (periodic cells from the
-//   opposite face, clamped ones from the face); the compute loop is the same
-//   for every rule.  Grids without a tensor map are staged with cp.async
-//   through the boundary map instead (16-byte copies inside the grid,
-//   element copies across an edge).
+//   that the offsets reach are then rewritten through the boundary map
+//   (periodic cells from the opposite face, clamped ones from the face); the
+//   compute loop is the same for every rule.
 // * The ring holds rzl + rzh + 1 planes for the stencil's z extent plus
-//   planes in flight ahead of the newest one a step reads.
+//   planes in flight ahead of the newest one a step reads; loading runs on
+//   into a CTA's next item.  A producer warp issues the boxes and rewrites the
+//   halo cells (their values fetched a plane ahead); consumer warps release
+//   stages one by one, so no step ends in a CTA barrier.
+// Bound: issue slots where the stencil is wide (27 weighted points: 26 adds
+// and, products being shared by a lane's cells, 7 multiplies of 48
+// instructions a cell), HBM where it is narrow.  Measured, float, per sweep,
+// against lane-strided cells, halos rewritten by all threads between two CTA
+// barriers and no loading across items: 27 points periodic at 320 x 300 x 257
+// 63 against 198 us, 9 points periodic at 4099 x 3001 21 against 41 us, one
+// colour of the 7-point clamped stencil at 319 x 257 x 255 42 against 94 us.
 // * The sweep body (points_body.cuh) is compiled two ways: here with the
 //   point table (shared-memory offset, plane lag, weight) copied to shared
 //   memory once per CTA and walked in order, and by jit.cpp with NVRTC per
@@ -49,26 +58,16 @@ namespace psg {
 namespace {
 
 template <typename T, int RY, bool UNIT>
-__global__ void __launch_bounds__(512, 1)
+__global__ void __launch_bounds__(32 * 17, 1)
 pts_kernel(const __grid_constant__ PtsParams<T> p, const __grid_constant__ PtsTmap tm) {
   extern __shared__ __align__(128) unsigned char smem[];
   pts_body<T, RY, UNIT, PtsTableSpec>(p, &tm, smem);
 }
 
-// Planes in flight ahead of the newest plane a step reads: the cp.async ring
-// waits with wait_group<kPtsPrefetch>; a TMA plane lands in one copy, and one
-// plane ahead is enough (measured at 512^3: two or three planes ahead run the
-// 7-point stencil 4-15 % and the 27-point 1-2 % slower, whatever the tile).
-// PS_POINTS_PREFETCH=<1..4> overrides the TMA depth (a tuning knob).
-int points_prefetch(bool tma) {
-  if (!tma) return kPtsPrefetch;
-  static const int depth = [] {
-    const char *e = getenv("PS_POINTS_PREFETCH");
-    const int v = e ? atoi(e) : 0;
-    return (v >= 1 && v <= 4) ? v : 1;
-  }();
-  return depth;
-}
+// Planes in flight ahead of the newest plane a step reads: one, as a deeper
+// ring costs CTAs (at 512^3 two or three ran the 7-point stencil 4-15 % and the
+// 27-point one 1-2 % slower, measured when CTA barriers ended each step).
+constexpr int kPtsAhead = 1;
 
 // Offsets' extent per axis: lo <= 0 <= hi.
 void extents(const PointsArgs &a, int lo[3], int hi[3]) {
@@ -104,7 +103,10 @@ void fill_params(const PointsArgs &a, int warps, int ry, PtsParams<T> *pp) {
   p.n = a.n;
   int lo[3], hi[3];
   extents(a, lo, hi);
+  p.rxl = -lo[0];
+  p.rxh = hi[0];
   p.ryl = -lo[1];
+  p.ryh = hi[1];
   p.rzl = -lo[2];
   p.rzh = hi[2];
   p.lp = (-lo[0] + VEC - 1) / VEC * VEC;
@@ -112,10 +114,9 @@ void fill_params(const PointsArgs &a, int warps, int ry, PtsParams<T> *pp) {
   p.w = p.lp + kPtsTX + rp;
   const int TY = warps * ry;
   p.rows_h = TY + p.ryl + hi[1];
-  p.nstage = p.rzl + p.rzh + 1 + points_prefetch(a.has_tmap);
+  p.nstage = p.rzl + p.rzh + 1 + kPtsAhead;
   p.plane_elems = p.rows_h * p.w;
   p.pstride = (int)(((size_t)p.plane_elems * sizeof(T) + 127) / 128 * 128 / sizeof(T));
-  p.use_tma = a.has_tmap ? 1 : 0;
   p.err = a.err;
   for (int i = 0; i < a.n; ++i) {
     p.off[i] = (p.ryl + a.d[i][1]) * p.w + p.lp + a.d[i][0];
@@ -157,7 +158,7 @@ cudaError_t launch_t(const PointsArgs &a, int warps, int sm_count, cudaStream_t 
   PtsTmap tm;
   memset(&tm, 0, sizeof(tm));
   static_assert(sizeof(PtsTmap) == sizeof(CUtensorMap), "tensor map layout");
-  if (a.has_tmap) memcpy(&tm, &a.tmap, sizeof(tm));
+  memcpy(&tm, &a.tmap, sizeof(tm));
   if (jit_enabled()) {
     // The stencil compiled with its table as constants (cached per stencil,
     // type and tile shape); on any failure the table kernel below runs.
@@ -167,21 +168,29 @@ cudaError_t launch_t(const PointsArgs &a, int warps, int sm_count, cudaStream_t 
     key.ry = RY;
     key.warps = warps;
     key.n = a.n;
+    // Registers: four rows of four cells compile to 72 of 80 without spilling
+    // (4-byte types, 7 to 27 points); 8-byte types need about 120.
+    const int regs = a.in.esz == 4 ? 80 : 120;
+    key.min_ctas = 65536 / (regs * 32 * (warps + 1));
+    if (key.min_ctas < 1) key.min_ctas = 1;
     key.unit = UNIT;
     key.w = p.w;
     key.nstage = p.nstage;
     key.pstride = p.pstride;
+    key.planes = p.rzl + p.rzh + 1;
+    key.centre = p.rzl;
     for (int i = 0; i < a.n; ++i) {
-      key.off[i] = p.off[i];
+      key.dx[i] = a.d[i][0];
+      key.dy[i] = a.d[i][1];
       key.lag[i] = p.lag[i];
       key.wt[i] = UNIT ? 1.0 : a.w[i];
     }
-    void *fn = jit_points_function(key);
     int occ = 0;
-    if (fn && jit_prepare(fn, 32 * warps, smem, &occ) && occ >= 1) {
+    void *fn = jit_points_function(key, smem, &occ);
+    if (fn && occ >= 1) {
       const int grid = schedule(&p, occ, sm_count);
       void *args[2] = {&p, &tm};
-      return jit_launch_raw(fn, grid, dim3(32, warps, 1), smem, s, args);
+      return jit_launch_raw(fn, grid, dim3(32, warps + 1, 1), smem, s, args);
     }
   }
   auto kern = pts_kernel<T, RY, UNIT>;
@@ -189,11 +198,11 @@ cudaError_t launch_t(const PointsArgs &a, int warps, int sm_count, cudaStream_t 
                                        (int)smem);
   if (e != cudaSuccess) return e;
   int occ = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, 32 * warps, smem);
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, 32 * (warps + 1), smem);
   if (e != cudaSuccess) return e;
   if (occ < 1) return cudaErrorInvalidConfiguration;
   const int grid = schedule(&p, occ, sm_count);
-  kern<<<grid, dim3(32, warps, 1), smem, s>>>(p, tm);
+  kern<<<grid, dim3(32, warps + 1, 1), smem, s>>>(p, tm);
   return cudaGetLastError();
 }
 
@@ -227,7 +236,7 @@ size_t points_smem_bytes(const PointsArgs &a, const MarchConfig &cfg) {
   int lo[3], hi[3], w, h;
   extents(a, lo, hi);
   points_box(a, cfg, &w, &h);
-  const int nstage = -lo[2] + hi[2] + 1 + points_prefetch(a.has_tmap);
+  const int nstage = -lo[2] + hi[2] + 1 + kPtsAhead;
   const size_t stage = ((size_t)w * h * a.in.esz + 127) / 128 * 128;
   return 128 + (size_t)kPtsRingOffset + (size_t)nstage * stage;
 }

@@ -3,9 +3,8 @@
 //    kernel serves every registered stencil;
 //  * jit.cpp compiles it with NVRTC for one stencil at a time, with a
 //    generated spec whose offsets, plane lags, weights and tile geometry are
-//    compile-time constants (the point loop unrolls into shared-memory loads
-//    at immediate offsets, and loads that two rows of a thread share are
-//    issued once).
+//    compile-time constants (the point loop unrolls into 16-byte shared loads
+//    at immediate offsets, each issued once for all the cells that use it).
 // No header dependencies beyond ps_arith.cuh, so NVRTC can compile it from
 // memory.  See points.cu for the design.
 #pragma once
@@ -15,14 +14,14 @@
 namespace psg {
 
 constexpr int kPtsTX = 128;       // tile width in cells
-constexpr int kPtsVX = 4;         // columns per lane (lane + 32*j)
-constexpr int kPtsPrefetch = 2;   // cp.async ring: planes in flight ahead of the newest needed one
+constexpr int kPtsVX = 4;         // cells per lane and row
 constexpr int kPtsMaxPoints = 64;
 // Shared memory: point table (run-time spec only: offsets, lags, weights),
-// then the ring's mbarriers, then the ring (128-byte aligned stages).
+// then the ring's mbarriers (full, empty, raw), then the ring (128-byte
+// aligned stages).
 constexpr int kPtsTableBytes = kPtsMaxPoints * (4 + 4 + 8);
 constexpr int kPtsMaxStages = 16;
-constexpr int kPtsRingOffset = kPtsTableBytes + 8 * kPtsMaxStages;
+constexpr int kPtsRingOffset = kPtsTableBytes + 24 * kPtsMaxStages;
 // Opaque TMA descriptor (the layout of CUtensorMap: 128 bytes, 64-aligned).
 struct alignas(64) PtsTmap {
   unsigned long long opaque[16];
@@ -40,10 +39,9 @@ struct PtsParams {
   int boundary;      // kPtsNone / kPtsPeriodic / kPtsClamp
   int color;         // -1 every cell, 0 red, 1 black
   int n;             // points
-  int ryl, rzl, rzh;
+  int rxl, rxh, ryl, ryh, rzl, rzh;  // extent of the offsets per axis
   int lp, w, rows_h, nstage, plane_elems;
   int pstride;       // ring stage stride in elements (128-byte multiple)
-  int use_tma;       // 1: the tmap parameter maps `in` with box {w, rows_h, 1}
   int xbase, tiles_x, tiles, zlen;
   long long items;
   int *err;          // device error word (bounded waits that give up)
@@ -59,73 +57,63 @@ struct PtsParams {
 // Clamp, and the never-read halo of boundary "none": the nearest face.
 __device__ __forceinline__ int pts_map_axis(int i, int n, int boundary) {
   if (boundary == kPtsPeriodic) {
+    if ((unsigned)i < (unsigned)n) return i;
     const int m = i % n;
     return m < 0 ? m + n : m;
   }
   return min(max(i, 0), n - 1);
 }
 
-// Issues the copies of global plane zg (tile origin x0, y0) into `dst`:
-// 16-byte copies for aligned chunks inside the grid, element copies through
-// the boundary map for chunks that cross an edge.
+// The cells of a tile's TMA box that lie outside the grid and that some cell
+// of the tile can read (at most the offsets' extent beyond a face): whole rows
+// beyond a y face, then the columns beyond an x face of the other rows.  TMA
+// filled them with zeros; cell e is rewritten with the value the boundary rule
+// maps it to.  Only edge tiles of periodic and clamped stencils have any.
+struct PtsHalo {
+  int xs, ys;              // box origin
+  int c0, ncol, r0, rtop;  // outside rows: columns c0 .. c0 + ncol, rtop rows from r0, then from rin1
+  int rin0, rin1;          // rows inside the grid
+  int clow, cin1, nc;      // outside columns: clow from c0, then from cin1, nc in all
+  int rows, total;         // cells in outside rows, cells in all
+};
 template <typename T>
-__device__ __forceinline__ void pts_load_plane(const PtsParams<T> &p, T *dst, int zg, int x0,
-                                               int y0) {
-  constexpr int VEC = 16 / (int)sizeof(T);
-  const T *src_plane = p.in + (long long)pts_map_axis(zg, p.nz, p.boundary) * p.plane;
-  const int nchunk = p.w / VEC;
-  const int xs = x0 - p.lp;
-  for (int r = threadIdx.y; r < p.rows_h; r += blockDim.y) {
-    const T *src =
-        src_plane + (long long)pts_map_axis(y0 - p.ryl + r, p.ny, p.boundary) * p.row;
-    T *d = dst + r * p.w;
-    for (int c = threadIdx.x; c < nchunk; c += 32) {
-      const int x = xs + c * VEC;
-      if (x >= 0 && x + VEC <= p.nx) {
-        cp_async16(d + c * VEC, src + x);
-      } else {
-#pragma unroll
-        for (int i = 0; i < VEC; ++i)
-          cp_async_small<sizeof(T)>(d + c * VEC + i, src + pts_map_axis(x + i, p.nx, p.boundary));
-      }
-    }
-  }
+__device__ __forceinline__ PtsHalo pts_halo(const PtsParams<T> &p, int x0, int y0, int W) {
+  PtsHalo h;
+  h.xs = x0 - p.lp;
+  h.ys = y0 - p.ryl;
+  h.c0 = max(0, -p.rxl - h.xs);
+  const int c1 = min(W, p.nx + p.rxh - h.xs);
+  h.ncol = c1 - h.c0;
+  h.r0 = max(0, -p.ryl - h.ys);
+  const int r1 = min(p.rows_h, p.ny + p.ryh - h.ys);
+  h.rin0 = max(h.r0, -h.ys);
+  h.rin1 = min(r1, p.ny - h.ys);
+  h.rtop = h.rin0 - h.r0;
+  h.clow = max(h.c0, -h.xs) - h.c0;
+  h.cin1 = min(c1, p.nx - h.xs);
+  h.nc = h.clow + (c1 - h.cin1);
+  h.rows = (h.rtop + (r1 - h.rin1)) * h.ncol;
+  h.total = h.rows + h.nc * (h.rin1 - h.rin0);
+  return h;
 }
-
-// After a TMA box load of plane zg (tile origin x0, y0; zero-filled outside
-// the grid), rewrites the box cells that lie outside the grid with the
-// values the boundary rule maps them to.  Only edge tiles of periodic and
-// clamped stencils have such cells; all threads share the work.
+// Cell e of the halo: its offset in the box (return value) and in the grid
+// plane that its values come from.
 template <typename T>
-__device__ __forceinline__ void pts_fix_halo(const PtsParams<T> &p, T *dst, int zg, int x0,
-                                             int y0, int W) {
-  const int xs = x0 - p.lp, ys = y0 - p.ryl, H = p.rows_h;
-  const T *plane = p.in + (long long)pts_map_axis(zg, p.nz, p.boundary) * p.plane;
-  const int cl = min(max(0, -xs), W);
-  const int cr = min(max(0, xs + W - p.nx), W - cl);
-  const int rt = min(max(0, -ys), H);
-  const int rb = min(max(0, ys + H - p.ny), H - rt);
-  const int nfull = (rt + rb) * W;            // whole rows outside in y
-  const int side = cl + cr;                   // cells per inner row outside in x
-  const int total = nfull + (H - rt - rb) * side;
-  const int nthr = blockDim.x * blockDim.y;
-  for (int i = threadIdx.y * 32 + threadIdx.x; i < total; i += nthr) {
-    int r, c;
-    if (i < nfull) {
-      const int rr = i / W;
-      c = i - rr * W;
-      r = rr < rt ? rr : H - rb + (rr - rt);
-    } else {
-      const int k = i - nfull;
-      const int rr = k / side;
-      const int cc = k - rr * side;
-      r = rt + rr;
-      c = cc < cl ? cc : W - cr + (cc - cl);
-    }
-    const int x = pts_map_axis(xs + c, p.nx, p.boundary);
-    const int y = pts_map_axis(ys + r, p.ny, p.boundary);
-    dst[r * W + c] = plane[(long long)y * p.row + x];
+__device__ __forceinline__ int pts_halo_cell(const PtsParams<T> &p, const PtsHalo &h, int e, int W,
+                                             long long *src) {
+  int r, c;
+  if (e < h.rows) {
+    const int k = e / h.ncol;
+    c = h.c0 + (e - k * h.ncol);
+    r = k < h.rtop ? h.r0 + k : h.rin1 + (k - h.rtop);
+  } else {
+    const int k = (e - h.rows) / h.nc, m = (e - h.rows) - k * h.nc;
+    r = h.rin0 + k;
+    c = m < h.clow ? h.c0 + m : h.cin1 + (m - h.clow);
   }
+  *src = (long long)pts_map_axis(h.ys + r, p.ny, p.boundary) * p.row +
+         pts_map_axis(h.xs + c, p.nx, p.boundary);
+  return r * W + c;
 }
 
 // The run-time spec: the point table travels in the kernel parameters and is
@@ -140,7 +128,53 @@ struct PtsTableSpec {
   static __device__ __forceinline__ int pstride(const PtsParams<T> &p) { return p.pstride; }
 };
 
-// acc[r][j] (+)= w * src[r*W + 32*j]; `first` starts the sum.
+// 16 bytes of a shared row as VEC cells.
+template <typename T>
+struct PtsVec {
+  static constexpr int N = 16 / (int)sizeof(T);
+  T v[N];
+};
+template <typename T>
+__device__ __forceinline__ PtsVec<T> pts_ld16(const T *src) {
+  union { uint4 u; PtsVec<T> v; } c;
+  c.u = *reinterpret_cast<const uint4 *>(src);
+  return c.v;
+}
+
+// Compiled spec.  acc[r][c] (+)= w * the point's value for the cells of row r:
+// lane l owns the VEC = 16 / sizeof(T) consecutive cells from
+// 32 VEC j + VEC l of each of the 4 / VEC column groups j.  Every read is an
+// aligned 16-byte shared load (conflict-free); a point's row and x offset only
+// select cells of such vectors, and the compiler issues each vector once per
+// step however many points and rows use it (a 27-point stencil needs 3 planes
+// x 6 rows x 3 vectors for 16 cells, 3.4 loads a cell).
+template <typename T, int RY, bool UNIT, class S, int K>
+__device__ __forceinline__ void pts_point(T (&acc)[RY][kPtsVX], const T *const *pl, int cell0) {
+  typedef RN<T> R;
+  constexpr int VEC = 16 / (int)sizeof(T);
+  constexpr int DX = S::kDx[K], DY = S::kDy[K], LAG = S::kLag[K];
+  constexpr T wk = (T)S::kWt[K];
+#pragma unroll
+  for (int r = 0; r < RY; ++r)
+#pragma unroll
+    for (int c = 0; c < kPtsVX; ++c) {
+      const int j = c / VEC, i = c % VEC + DX;
+      const int vi = (i + 8 * VEC) / VEC - 8, e = i - vi * VEC;
+      const T v = pts_ld16<T>(pl[LAG] + cell0 + (r + DY) * S::kW + j * 32 * VEC + vi * VEC)
+                      .v[e];
+      const T t = UNIT ? v : R::mul(wk, v);
+      acc[r][c] = K == 0 ? t : R::add(acc[r][c], t);
+    }
+}
+template <typename T, int RY, bool UNIT, class S, int K>
+__device__ __forceinline__ void pts_points(T (&acc)[RY][kPtsVX], const T *const *pl, int cell0) {
+  if constexpr (K < S::kN) {
+    pts_point<T, RY, UNIT, S, K>(acc, pl, cell0);
+    pts_points<T, RY, UNIT, S, K + 1>(acc, pl, cell0);
+  }
+}
+
+// Table spec: acc[r][j] (+)= w * src[r*W + 32*j]; `first` starts the sum.
 template <typename T, int RY, bool UNIT>
 __device__ __forceinline__ void pts_term(T (&acc)[RY][kPtsVX], const T *src, int W, T wk,
                                          bool first) {
@@ -155,29 +189,70 @@ __device__ __forceinline__ void pts_term(T (&acc)[RY][kPtsVX], const T *src, int
     }
 }
 
+// Position of an item (tile column, tile row, z-chunk), advanced by a fixed
+// number of items without divisions.
+struct PtsPos {
+  int tx, ty, chunk;
+};
+__device__ __forceinline__ PtsPos pts_split(long long item, int tiles_x, int tiles) {
+  PtsPos q;
+  q.chunk = (int)(item / tiles);
+  const int tile = (int)(item - (long long)q.chunk * tiles);
+  q.ty = tile / tiles_x;
+  q.tx = tile - q.ty * tiles_x;
+  return q;
+}
+__device__ __forceinline__ void pts_advance(PtsPos &q, const PtsPos &step, int tiles_x,
+                                            int tiles_y) {
+  q.tx += step.tx;
+  q.ty += step.ty;
+  q.chunk += step.chunk;
+  if (q.tx >= tiles_x) {
+    q.tx -= tiles_x;
+    ++q.ty;
+  }
+  if (q.ty >= tiles_y) {
+    q.ty -= tiles_y;
+    ++q.chunk;
+  }
+}
+
 // The sweep: persistent (z-chunk, tile) items, a ring of planes, the points
-// summed in order, masked stores.  Each plane of a tile arrives by one TMA
-// box load (mbarrier per stage); on the edge tiles of periodic and clamped
-// stencils the out-of-grid cells of the box are then rewritten through the
-// boundary map (with boundary "none" they are never read).  Without a TMA
-// descriptor (p.use_tma == 0) planes are copied with cp.async through the
-// boundary map instead (one commit group per plane).  `smem_raw` is the
-// dynamic shared memory, `tmap` the TMA descriptor of `in`.
+// summed in order.  The last warp of the CTA is the producer, the others
+// consume.  Each plane of a tile arrives by one TMA box load on its stage's
+// "full" mbarrier; a consumer warp that is done with a stage arrives on its
+// "empty" mbarrier, so warps run up to a ring apart and no step ends in a CTA
+// barrier.  Planes are loaded in one sequence over all of the CTA's items: an
+// item's first planes arrive while the previous item is being computed (a 2D
+// grid is one plane per item).  On the edge tiles of periodic and clamped
+// stencils the out-of-grid cells of the box are rewritten through the boundary
+// map by the producer warp before it completes the stage's "full" barrier (the
+// box then lands on a barrier of its own, "raw"; with boundary "none" those
+// cells are never read).  A consumer whose bounded wait gives up computes and
+// stores nothing more, but keeps its arrivals going so that the CTA ends.
+// `smem_raw` is the dynamic shared memory, `tmap` the TMA descriptor of `in`.
 template <typename T, int RY, bool UNIT, class S>
 __device__ __forceinline__ void pts_body(const PtsParams<T> &p, const void *tmap,
                                          unsigned char *smem_raw) {
+  constexpr int VEC = 16 / (int)sizeof(T);
   unsigned char *smem = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);
   int *s_off = reinterpret_cast<int *>(smem);
   int *s_lag = s_off + kPtsMaxPoints;
   T *s_w = reinterpret_cast<T *>(smem + kPtsMaxPoints * 8);
-  unsigned long long *bars = reinterpret_cast<unsigned long long *>(smem + kPtsTableBytes);
+  unsigned long long *full = reinterpret_cast<unsigned long long *>(smem + kPtsTableBytes);
+  unsigned long long *empty = full + kPtsMaxStages, *raw = empty + kPtsMaxStages;
   T *ring = reinterpret_cast<T *>(smem + kPtsRingOffset);
   const int W = S::w(p), NST = S::nstage(p), PS = S::pstride(p);
 
   const int lane = threadIdx.x, warp = threadIdx.y;
+  const int consumers = blockDim.y - 1;  // warps
   const int tid = warp * 32 + lane;
   if (tid == 0) {
-    for (int s = 0; s < NST; ++s) mbar_init(&bars[s], 1);
+    for (int s = 0; s < NST; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], consumers);
+      mbar_init(&raw[s], 1);
+    }
     fence_barrier_init();
   }
   if (!S::kStatic) {
@@ -189,113 +264,221 @@ __device__ __forceinline__ void pts_body(const PtsParams<T> &p, const void *tmap
   }
   __syncthreads();
 
-  const int TY = blockDim.y * RY;
-  const int pre = NST - 1;  // planes issued before the first compute step
-  const int cell0 = warp * RY * W + lane;
-  const unsigned tma_bytes = (unsigned)(p.plane_elems * (int)sizeof(T));
-  unsigned phase = 0;  // bit s: parity of the next completion of stage s
-  bool ok = true;
+  const int TY = consumers * RY;
+  const int zext = p.rzl + p.rzh;
+  const int tiles_y = p.tiles / p.tiles_x;
+  PtsPos pos = pts_split(blockIdx.x, p.tiles_x, p.tiles);
+  const PtsPos step = pts_split(gridDim.x, p.tiles_x, p.tiles);
 
-  for (long long item = blockIdx.x; item < p.items && ok; item += gridDim.x) {
-    const int chunk = (int)(item / p.tiles);
-    const int tile = (int)(item - (long long)chunk * p.tiles);
-    const int zs = p.dmin2 + chunk * p.zlen;
+  if (warp == consumers) {
+    const unsigned bytes = (unsigned)(p.plane_elems * (int)sizeof(T));
+    int slot = 0, fslot = 0;    // next slot to fill, next slot whose halo is to be rewritten
+    unsigned phase = 0;         // bit s: parity of slot s's next fill
+    unsigned raws = 0;          // bit s: parity of the next box landing on raw[s]
+    bool used = false;          // every slot has been filled once
+    for (long long item = blockIdx.x; item < p.items; item += gridDim.x) {
+      const int zs = p.dmin2 + pos.chunk * p.zlen;
+      const int n = min(p.zlen, p.dmax2 - zs) + zext;
+      const int x0 = p.xbase + pos.tx * kPtsTX, y0 = p.dmin1 + pos.ty * TY;
+      pts_advance(pos, step, p.tiles_x, tiles_y);
+      PtsHalo h;
+      h.total = 0;
+      if (p.boundary != kPtsNone &&
+          !(x0 - p.rxl >= 0 && x0 + kPtsTX + p.rxh <= p.nx && y0 - p.ryl >= 0 &&
+            y0 - p.ryl + p.rows_h <= p.ny))
+        h = pts_halo(p, x0, y0, W);
+      const bool fix = h.total > 0;
+      // this lane's first halo cells, the same ones in every plane
+      constexpr int kBatch = 5;
+      int dst[kBatch];
+      long long src[kBatch];
+      if (fix) {
+#pragma unroll
+        for (int i = 0; i < kBatch; ++i) {
+          const int e = lane + 32 * i;
+          dst[i] = e < h.total ? pts_halo_cell(p, h, e, W, &src[i]) : -1;
+        }
+      }
+      // their values in plane q, fetched a plane ahead of the rewrite
+      T v[kBatch];
+      auto fetch = [&](int q) {
+        const T *plane = p.in + (long long)pts_map_axis(zs - p.rzl + q, p.nz, p.boundary) * p.plane;
+#pragma unroll
+        for (int i = 0; i < kBatch; ++i)
+          if (dst[i] >= 0) v[i] = plane[src[i]];
+      };
+      if (fix) fetch(0);
+      int filled = 0, done = 0;  // planes whose box was issued / whose stage is complete
+      while (done < n) {
+        // fill free stages; block for one only when there is nothing to rewrite
+        while (filled < n && filled - done < NST) {
+          bool free = !used;
+          if (used) {
+            void *e = &empty[slot];
+            const unsigned par = ((phase >> slot) & 1u) ^ 1u;  // the last fill's readers
+            if (fix && filled > done) {
+              free = __all_sync(0xffffffffu, mbar_test_wait(e, par));
+              if (!free) break;
+            } else if (!__all_sync(0xffffffffu, mbar_wait(e, par, p.err))) {
+              return;
+            }
+          }
+          if (lane == 0) {
+            void *bar = fix ? &raw[slot] : &full[slot];
+            mbar_arrive_expect_tx(bar, bytes);
+            tma_load_3d(ring + slot * PS, tmap, x0 - p.lp, y0 - p.ryl,
+                        pts_map_axis(zs - p.rzl + filled, p.nz, p.boundary), bar);
+          }
+          phase ^= 1u << slot;
+          if (++slot == NST) {
+            slot = 0;
+            used = true;
+          }
+          ++filled;
+          if (!fix) {
+            ++done;
+            if (++fslot == NST) fslot = 0;
+          }
+        }
+        if (!fix) continue;
+        // rewrite the halo of plane `done`
+        T *box = ring + fslot * PS;
+        if (!__all_sync(0xffffffffu, mbar_wait(&raw[fslot], (raws >> fslot) & 1u, p.err))) return;
+        raws ^= 1u << fslot;
+#pragma unroll
+        for (int i = 0; i < kBatch; ++i)
+          if (dst[i] >= 0) box[dst[i]] = v[i];
+        const T *plane =
+            p.in + (long long)pts_map_axis(zs - p.rzl + done, p.nz, p.boundary) * p.plane;
+        for (int e = lane + 32 * kBatch; e < h.total; e += 32) {
+          long long from;
+          const int to = pts_halo_cell(p, h, e, W, &from);
+          box[to] = plane[from];
+        }
+        // these writes precede the consumers' reads (the arrival below) and
+        // the box that reuses the stage (the proxy fence)
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&full[fslot]);
+        if (++fslot == NST) fslot = 0;
+        if (++done < n) fetch(done);
+      }
+    }
+    // the last copies land before the CTA may end (the consumers see to that
+    // themselves unless one of them gave up)
+    for (int s = 0; s < NST; ++s)
+      if (used || s < slot) mbar_wait(&full[s], ((phase >> s) & 1u) ^ 1u, nullptr, 1u << 16);
+    return;
+  }
+
+  // first cell of the lane's first row relative to a plane: its vector
+  // (compiled spec) or its first lane-strided cell (table spec)
+  const int cell0 = S::kStatic ? (warp * RY + p.ryl) * W + p.lp + lane * VEC : warp * RY * W + lane;
+  bool ok = true;
+  // Slot of plane z - rzl of the current step, the next slot to wait for, and
+  // the parity of each slot's next completion (bit s).
+  int cs = 0, wslot = 0;
+  unsigned phase = 0;
+  for (long long item = blockIdx.x; item < p.items; item += gridDim.x) {
+    const int zs = p.dmin2 + pos.chunk * p.zlen;
     const int ze = min(zs + p.zlen, p.dmax2);
-    const int x0 = p.xbase + (tile % p.tiles_x) * kPtsTX;
-    const int y0 = p.dmin1 + (tile / p.tiles_x) * TY;
-    const int nplanes = ze - zs + p.rzl + p.rzh;  // planes zs-rzl .. ze+rzh-1
-    const bool tma = p.use_tma != 0;
-    const bool fix = tma && p.boundary != kPtsNone &&
-                     !(x0 - p.lp >= 0 && x0 - p.lp + W <= p.nx && y0 - p.ryl >= 0 &&
-                       y0 - p.ryl + p.rows_h <= p.ny);
-    // store masks: columns j in the domain, rows r in the domain
+    const int x0 = p.xbase + pos.tx * kPtsTX;
+    const int y0 = p.dmin1 + pos.ty * TY;
+    pts_advance(pos, step, p.tiles_x, tiles_y);
+    // cells of the lane in the domain: bit c of colmask, bit r of rowmask
     unsigned colmask = 0, rowmask = 0;
 #pragma unroll
-    for (int j = 0; j < kPtsVX; ++j) {
-      const int x = x0 + lane + 32 * j;
-      if (x >= p.dmin0 && x < p.dmax0) colmask |= 1u << j;
+    for (int c = 0; c < kPtsVX; ++c) {
+      const int x = S::kStatic ? x0 + (c / VEC) * 32 * VEC + lane * VEC + c % VEC
+                               : x0 + lane + 32 * c;
+      if (x >= p.dmin0 && x < p.dmax0) colmask |= 1u << c;
     }
 #pragma unroll
     for (int r = 0; r < RY; ++r)
       if (y0 + warp * RY + r < p.dmax1) rowmask |= 1u << r;
-    const int xpar = (x0 + lane) & 1;  // parity of every column of this lane
-    T *out0 = p.out + (long long)(y0 + warp * RY) * p.row + x0 + lane;
+    const bool whole = colmask == (1u << kPtsVX) - 1u && rowmask == (1u << RY) - 1u;
+    T *dst = p.out + (long long)zs * p.plane + (long long)(y0 + warp * RY) * p.row + x0 +
+             lane * (S::kStatic ? VEC : 1);
 
-    int ld = 0, issued = 0, waited = 0, wslot = 0;
-    auto issue = [&](int q) {
-      if (tma) {
-        if (tid == 0) {
-          mbar_arrive_expect_tx(&bars[ld], tma_bytes);
-          tma_load_3d(ring + ld * PS, tmap, x0 - p.lp, y0 - p.ryl,
-                      pts_map_axis(zs - p.rzl + q, p.nz, p.boundary), &bars[ld]);
-        }
-        ++issued;
-      } else {
-        if (q < nplanes) pts_load_plane(p, ring + ld * PS, zs - p.rzl + q, x0, y0);
-        cp_async_commit();
-      }
-      if (++ld == NST) ld = 0;
-    };
-    for (int q = 0; q < pre; ++q)
-      if (q < nplanes || !tma) issue(q);
-    int cs = 0;  // ring slot of plane z - rzl
-    for (int z = zs; z < ze && ok; ++z) {
-      const int q = z - zs + pre;
-      if (q < nplanes || !tma) issue(q);
-      if (tma) {
-        const int need = z - zs + p.rzl + p.rzh;  // newest plane this step reads
-        while (waited <= need) {
-          if (!mbar_wait(&bars[wslot], (phase >> wslot) & 1u, p.err)) ok = false;
-          if (fix && ok) pts_fix_halo(p, ring + wslot * PS, zs - p.rzl + waited, x0, y0, W);
-          phase ^= 1u << wslot;
-          ++waited;
-          if (++wslot == NST) wslot = 0;
-        }
-      } else {
-        cp_async_wait<kPtsPrefetch>();  // planes up to z + rzh have landed
-      }
-      ok = __syncthreads_and(ok);
-      if (!ok) break;
-
-      T acc[RY][kPtsVX];
-      if constexpr (S::kStatic) {
-#pragma unroll
-        for (int k = 0; k < S::kN; ++k) {
-          int s = cs + S::kLag[k];
-          if (s >= NST) s -= NST;
-          pts_term<T, RY, UNIT>(acc, ring + s * PS + cell0 + S::kOff[k], W, (T)S::kWt[k],
-                                k == 0);
-        }
-      } else {
-        for (int k = 0; k < p.n; ++k) {
-          int s = cs + s_lag[k];
-          if (s >= NST) s -= NST;
-          pts_term<T, RY, UNIT>(acc, ring + s * PS + cell0 + s_off[k], W, s_w[k], k == 0);
-        }
-      }
-
-      T *dst = out0 + (long long)z * p.plane;
-#pragma unroll
-      for (int r = 0; r < RY; ++r) {
-        const int y = y0 + warp * RY + r;
-        const bool row_on = ((rowmask >> r) & 1u) &&
-                            (p.color < 0 || ((xpar + y + z + p.color) & 1) == 0);
-        if (row_on) {
-#pragma unroll
-          for (int j = 0; j < kPtsVX; ++j)
-            if ((colmask >> j) & 1u) dst[r * p.row + 32 * j] = acc[r][j];
-        }
-      }
-      if (++cs == NST) cs = 0;
-      __syncthreads();  // the slot of plane z - rzl is refilled next step
-    }
-    if (!tma) cp_async_wait<0>();  // only empty groups can remain
-    if (!ok && tma && tid == 0) {
-      // a wait gave up: let copies still in flight land (bounded) before exit
-      for (; waited < issued; ++waited) {
-        mbar_wait(&bars[wslot], (phase >> wslot) & 1u, nullptr, 1024);
+    int waited = 0;  // planes of this item that have landed
+    for (int z = zs; z < ze; ++z, dst += p.plane) {
+      const int need = z - zs + zext;  // newest plane this step reads
+      while (waited <= need) {
+        if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&full[wslot], (phase >> wslot) & 1u, p.err));
         phase ^= 1u << wslot;
+        ++waited;
         if (++wslot == NST) wslot = 0;
+      }
+
+      if (ok) {
+        T acc[RY][kPtsVX];
+        if constexpr (S::kStatic) {
+          const T *pl[S::kPlanes];
+#pragma unroll
+          for (int l = 0; l < S::kPlanes; ++l) {
+            int s = cs + l;
+            if (s >= NST) s -= NST;
+            pl[l] = ring + s * PS;
+          }
+          pts_points<T, RY, UNIT, S, 0>(acc, pl, cell0);
+          if (p.color >= 0) {
+            // the lane's other-colour cells keep their value: nothing writes
+            // them in this launch, so a whole vector can be stored
+#pragma unroll
+            for (int r = 0; r < RY; ++r)
+#pragma unroll
+              for (int c = 0; c < kPtsVX; ++c) {
+                const int x = x0 + (c / VEC) * 32 * VEC + lane * VEC + c % VEC;
+                const T own =
+                    pts_ld16<T>(pl[S::kCentre] + cell0 + r * S::kW + (c / VEC) * 32 * VEC)
+                        .v[c % VEC];
+                if ((x + y0 + warp * RY + r + z + p.color) & 1) acc[r][c] = own;
+              }
+          }
+#pragma unroll
+          for (int r = 0; r < RY; ++r) {
+            if (!whole && !((rowmask >> r) & 1u)) continue;
+#pragma unroll
+            for (int j = 0; j < kPtsVX / VEC; ++j) {
+              const unsigned m = (colmask >> (j * VEC)) & ((1u << VEC) - 1u);
+              T *d = dst + r * p.row + j * 32 * VEC;
+              if (whole || m == (1u << VEC) - 1u) {
+                union { uint4 u; T t[VEC]; } c;
+#pragma unroll
+                for (int i = 0; i < VEC; ++i) c.t[i] = acc[r][j * VEC + i];
+                *reinterpret_cast<uint4 *>(d) = c.u;
+              } else {
+#pragma unroll
+                for (int i = 0; i < VEC; ++i)
+                  if ((m >> i) & 1u) d[i] = acc[r][j * VEC + i];
+              }
+            }
+          }
+        } else {
+          for (int k = 0; k < p.n; ++k) {
+            int s = cs + s_lag[k];
+            if (s >= NST) s -= NST;
+            pts_term<T, RY, UNIT>(acc, ring + s * PS + cell0 + s_off[k], W, s_w[k], k == 0);
+          }
+#pragma unroll
+          for (int r = 0; r < RY; ++r) {
+            const int y = y0 + warp * RY + r;
+            const bool row_on = ((rowmask >> r) & 1u) &&
+                                (p.color < 0 || ((x0 + lane + y + z + p.color) & 1) == 0);
+            if (row_on) {
+#pragma unroll
+              for (int j = 0; j < kPtsVX; ++j)
+                if ((colmask >> j) & 1u) dst[r * p.row + 32 * j] = acc[r][j];
+            }
+          }
+        }
+      }
+      // plane z - rzl is done with; after the item's last step all its planes
+      __syncwarp();
+      const int freed = z + 1 < ze ? 1 : 1 + zext;
+      for (int f = 0; f < freed; ++f) {
+        if (lane == 0) mbar_arrive(&empty[cs]);
+        if (++cs == NST) cs = 0;
       }
     }
   }

@@ -131,8 +131,7 @@ struct PointsArgs {
   double w[kMaxPoints];
   bool unit;         // every weight is 1: terms are the point values
   int *err;          // device error word
-  bool has_tmap;     // tmap maps `in` with the box points_box() gives
-  CUtensorMap tmap;
+  CUtensorMap tmap;  // maps `in` with the box points_box() gives
 };
 // cfg.warps x points_rows(cfg) (1, 2 or 4) rows per tile; the other fields
 // are unused.
@@ -193,17 +192,19 @@ cudaError_t jit_launch(const JitKernel &k, const Box &dom, int color, const Grid
 // depends on; the kernel takes one PtsParams<T> by value.
 struct PtsJitKey {
   int type;                  // ElemType
-  int ry, warps, n;
+  int ry, warps, n;          // warps: consumers (the CTA has one more)
+  int min_ctas;              // per SM, for the register limit
   bool unit;
   int w, nstage, pstride;
-  int off[kMaxPoints], lag[kMaxPoints];
+  int planes, centre;        // z extent of the points, lag of the cell's own plane
+  int dx[kMaxPoints], dy[kMaxPoints], lag[kMaxPoints];
   double wt[kMaxPoints];
 };
 // The compiled kernel (cached; nullptr if NVRTC is missing or compiling
-// failed, after which the table kernel is used).
-void *jit_points_function(const PtsJitKey &k);
-// Sets the kernel's dynamic shared memory limit and returns its occupancy.
-bool jit_prepare(void *fn, int threads, size_t smem, int *occ);
+// failed, after which the table kernel is used), allowed `smem` bytes of
+// dynamic shared memory, and how many of its CTAs an SM holds.  The key is
+// compared bytewise: zero it before filling it in.
+void *jit_points_function(const PtsJitKey &k, size_t smem, int *occ);
 // Launches a compiled kernel; args[i] points at its i-th parameter.
 cudaError_t jit_launch_raw(void *fn, int grid, dim3 block, size_t smem, cudaStream_t s,
                            void **args);

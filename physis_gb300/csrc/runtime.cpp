@@ -511,7 +511,6 @@ int shape_slot(int kernel) {
 // One point-stencil map: one launch per colour it runs.
 bool launch_points_map(const Map &m, const PointStencil &ps) {
   psg::PointsArgs a{};
-  a.has_tmap = true;  // planes arrive by TMA (sizes the ring below)
   a.in = view(m.grids[0]);
   a.out = view(m.grids[1]);
   for (int d = 0; d < 3; ++d) {
@@ -535,8 +534,7 @@ bool launch_points_map(const Map &m, const PointStencil &ps) {
   a.err = rt->dev_err;
   int bw = 0, bh = 0;
   psg::points_box(a, cfg, &bw, &bh);
-  a.has_tmap = tmap_for(a.in, bw, bh, &a.tmap);
-  if (!a.has_tmap) return false;
+  if (!tmap_for(a.in, bw, bh, &a.tmap)) return false;
   const int colors[2] = {m.color == 2 ? 0 : m.color, 1};
   const int ncol = m.color == 2 ? 2 : 1;
   for (int c = 0; c < ncol; ++c) {

@@ -172,6 +172,30 @@ def test_random_point_stencils_bit_exact(rt, oracle, kernel_form, seed, shape, d
     assert np.array_equal(_bits(got), _bits(ref))
 
 
+# The sizes where the tiled sweep can go wrong: several items per CTA (2D, one
+# plane per item, and 3D), rings that wrap between items, tiles that are all
+# edge, more halo cells than a producer lane keeps (radius 4 in a corner),
+# wrapped reads across a whole short axis, and vectors cut by the domain.
+EDGES = [
+    # (seed, shape (nz, ny, nx), dtype, boundary, npts, radius, weighted, shrink)
+    (41, (1, 1400, 1531), np.float32, 1, 9, 1, True, False),
+    (42, (1, 900, 2310), np.float64, 2, 11, 4, True, True),
+    (43, (61, 130, 259), np.float32, 1, 40, 4, True, False),
+    (44, (40, 100, 513), np.int32, 2, 9, 1, False, True),
+    (45, (5, 4, 6), np.float32, 1, 20, 4, True, False),
+    (46, (3, 17, 127), np.float32, 2, 12, 3, True, False),
+    (47, (2, 16, 129), np.float64, 1, 12, 2, True, False),
+    (48, (130, 1, 5), np.int64, 1, 8, 4, False, False),
+]
+
+
+@pytest.mark.parametrize("seed,shape,dtype,boundary,npts,radius,weighted,shrink", EDGES)
+def test_point_sweep_edges_bit_exact(rt, oracle, kernel_form, seed, shape, dtype, boundary, npts,
+                                     radius, weighted, shrink):
+    test_random_point_stencils_bit_exact(rt, oracle, kernel_form, seed, shape, dtype, boundary,
+                                         npts, radius, weighted, shrink)
+
+
 @pytest.mark.parametrize("warps,rows", [(8, 2), (8, 1), (4, 2), (16, 1), (2, 2), (1, 1), (8, 4), (4, 4)])
 def test_point_launch_shapes_do_not_change_results(rt, oracle, kernel_form, warps, rows):
     rng = np.random.default_rng(42)
