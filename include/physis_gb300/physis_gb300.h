@@ -342,6 +342,14 @@ int PSWarmStartPrepareWeights(const float *w, void *w_fwd, void *w_bwd, void *st
 int PSWarmStartAdam(float *w, const float *g, float *m, float *v, long long n, float lr, float b1,
                     float b2, float eps, int step, void *stream);
 
+/* PSWarmStartAdam over a whole network's parameters, stored together as
+ * w[layers][27][16][16] then bias[layers][16] (g, m and v alike), and
+ * PSWarmStartPrepareWeights of every layer's new weights into
+ * w_fwd[layers][27][16][16] and w_bwd[layers][27][16][16], in one launch. */
+int PSWarmStartAdamLayers(float *w, const float *g, float *m, float *v, int layers, float lr,
+                          float b1, float b2, float eps, int step, void *w_fwd, void *w_bwd,
+                          void *stream);
+
 /* dy (channel 0) = 2 (pred - target) / n, other channels 0; partials[i]
  * (one per 256 values) = sum of squared errors, in FP64. */
 int PSWarmStartLoss(const float *pred, const float *target, long long n, void *dy,

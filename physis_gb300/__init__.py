@@ -59,7 +59,7 @@ PSLoadTuneCache PSClearTuning PSGetStencilPlan PSBatchCreate PSBatchRun PSBatchF
 PSSetBatchShape __PSStencilMapRedBlack __PSStencilMapRed __PSStencilMapBlack
 PSStencilMapColorV PSPointStencilNew PSStencilFunctionNew
 PSStencilFunctionCheck PSWarmStartConv PSWarmStartWeightGrad PSWarmStartPrepareWeights
-PSWarmStartAdam PSWarmStartLoss PSWarmStartPool PSWarmStartPoolTarget
+PSWarmStartAdam PSWarmStartAdamLayers PSWarmStartLoss PSWarmStartPool PSWarmStartPoolTarget
 PSWarmStartUpsample PSWarmStartUpsampleAdd PSWarmStartResidualSource
 PSWarmStartAddCorrection""".split()
 
@@ -193,6 +193,8 @@ def lib():
     L.PSWarmStartPrepareWeights.argtypes = [vp, vp, vp, vp]
     L.PSWarmStartAdam.argtypes = [vp, vp, vp, vp, ctypes.c_longlong, ctypes.c_float,
                                   ctypes.c_float, ctypes.c_float, ctypes.c_float, i, vp]
+    f = ctypes.c_float
+    L.PSWarmStartAdamLayers.argtypes = [vp, vp, vp, vp, i, f, f, f, f, i, vp, vp, vp]
     L.PSWarmStartLoss.argtypes = [vp, vp, ctypes.c_longlong, vp, vp, vp]
     fp = ctypes.POINTER(PSWarmStartFields)
     L.PSWarmStartPool.argtypes = [fp, vp, vp]
@@ -202,7 +204,7 @@ def lib():
     L.PSWarmStartResidualSource.argtypes = [fp, vp, vp, ctypes.c_float, vp, i, vp]
     L.PSWarmStartAddCorrection.argtypes = [fp, vp, ctypes.c_float, vp, vp]
     for name in ("PSWarmStartConv", "PSWarmStartWeightGrad", "PSWarmStartPrepareWeights",
-                 "PSWarmStartAdam", "PSWarmStartLoss", "PSWarmStartPool",
+                 "PSWarmStartAdam", "PSWarmStartAdamLayers", "PSWarmStartLoss", "PSWarmStartPool",
                  "PSWarmStartPoolTarget", "PSWarmStartUpsample", "PSWarmStartUpsampleAdd",
                  "PSWarmStartResidualSource", "PSWarmStartAddCorrection"):
         getattr(L, name).restype = i

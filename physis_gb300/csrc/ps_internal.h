@@ -236,6 +236,8 @@ int nn_wgrad(const void *x, const void *dy, float *part, int S, float *dw, float
 int nn_prep_weights(const float *w, void *wf, void *wb, cudaStream_t s);
 int nn_adam(float *w, const float *g, float *m, float *v, long long n, float lr, float b1,
             float b2, float eps, int step, cudaStream_t s);
+int nn_adam_layers(float *w, const float *g, float *m, float *v, int layers, float lr, float b1,
+                   float b2, float eps, int step, void *wf, void *wb, cudaStream_t s);
 int nn_mse(const float *pred, const float *tgt, long long n, void *dy, double *part,
            cudaStream_t s);
 int nn_pool_inputs(const NNFields &f, void *out, cudaStream_t s);

@@ -2393,6 +2393,15 @@ int PSWarmStartAdam(float *w, const float *g, float *m, float *v, long long n, f
                    "PSWarmStartAdam");
 }
 
+int PSWarmStartAdamLayers(float *w, const float *g, float *m, float *v, int layers, float lr,
+                          float b1, float b2, float eps, int step, void *w_fwd, void *w_bwd,
+                          void *stream) {
+  if (!w || !g || !m || !v || !w_fwd || !w_bwd) return ws_status(-1, "PSWarmStartAdamLayers");
+  return ws_status(psg::nn_adam_layers(w, g, m, v, layers, lr, b1, b2, eps, step, w_fwd, w_bwd,
+                                       ws_stream(stream)),
+                   "PSWarmStartAdamLayers");
+}
+
 int PSWarmStartLoss(const float *pred, const float *target, long long n, void *dy,
                     double *partials, void *stream) {
   if (!pred || !target || !dy || !partials) return ws_status(-1, "PSWarmStartLoss");

@@ -266,28 +266,37 @@ def coarse_shape(shape, factor):
 
 class Net:
     """6 conv layers 3x3x3 x 16 channels, ReLU between, on the coarse grid.
-    FP32 master weights and Adam moments; BF16 copies for the kernels."""
+    FP32 master weights and Adam moments; BF16 copies for the kernels.  The
+    weights of all layers, then their biases, lie in one buffer (gradients,
+    moments and BF16 copies alike), so that an optimiser step is one launch;
+    w, b, grads, ... are views of them."""
 
     def __init__(self, seed=0):
         import torch
         self.torch = torch
         dev = "cuda"
         rng = np.random.default_rng(seed)
-        self.w, self.b = [], []
+        per, nb = 27 * C * C, C
+        self._flat = [torch.zeros(LAYERS * (per + nb), device=dev) for _ in range(4)]
+
+        def views(flat):
+            w = [flat[l * per:(l + 1) * per].view(27, C, C) for l in range(LAYERS)]
+            o = LAYERS * per
+            return w, [flat[o + l * nb:o + (l + 1) * nb] for l in range(LAYERS)]
+
+        self.w, self.b = views(self._flat[0])
         for l in range(LAYERS):
             fan_in = 27 * (CIN if l == 0 else C)
             std = math.sqrt(2.0 / fan_in) if l < LAYERS - 1 else 0.1 * math.sqrt(1.0 / fan_in)
             w = rng.normal(0, std, size=(27, C, C)).astype(np.float32)
             if l == 0:
                 w[:, CIN:, :] = 0.0
-            self.w.append(torch.tensor(w, device=dev))
-            self.b.append(torch.zeros(C, device=dev))
+            self.w[l].copy_(torch.tensor(w))
         self.params = self.w + self.b
-        self.grads = [torch.zeros_like(p) for p in self.params]
-        self.m = [torch.zeros_like(p) for p in self.params]
-        self.v = [torch.zeros_like(p) for p in self.params]
-        self.wf = [torch.empty(27 * C * C, dtype=torch.bfloat16, device=dev) for _ in range(LAYERS)]
-        self.wb = [torch.empty(27 * C * C, dtype=torch.bfloat16, device=dev) for _ in range(LAYERS)]
+        self.grads, self.m, self.v = [sum(views(f), []) for f in self._flat[1:]]
+        self._half = [torch.empty((LAYERS, per), dtype=torch.bfloat16, device=dev)
+                      for _ in range(2)]
+        self.wf, self.wb = list(self._half[0]), list(self._half[1])
         self.step = 0
         self._acts = None
         self.prepare()
@@ -296,26 +305,23 @@ class Net:
         return ctypes.c_void_p(self.torch.cuda.current_stream().cuda_stream)
 
     def prepare(self):
-        L = ps.lib()
+        L, stream = ps.lib(), self.stream()
         for l in range(LAYERS):
-            _ok(L.PSWarmStartPrepareWeights(_p(self.w[l]), _p(self.wf[l]), _p(self.wb[l]),
-                                            self.stream()))
+            _ok(L.PSWarmStartPrepareWeights(_p(self.w[l]), _p(self.wf[l]), _p(self.wb[l]), stream))
 
     def forward(self, x, dims):
         """x: BF16 tensor [B*Z*Y*X*16]; returns the FP32 channel-0 output."""
         torch = self.torch
         B, Z, Y, X = dims
         n = B * Z * Y * X
-        L = ps.lib()
-        acts = [x]
+        L, stream = ps.lib(), self.stream()
+        acts = [x] + list(torch.empty((LAYERS, n * C), dtype=torch.bfloat16, device="cuda"))
         out0 = torch.empty(n, dtype=torch.float32, device="cuda")
         for l in range(LAYERS):
-            y = torch.empty(n * C, dtype=torch.bfloat16, device="cuda")
             last = l == LAYERS - 1
-            _ok(L.PSWarmStartConv(_p(acts[-1]), _p(self.wf[l]), _p(self.b[l]), None,
-                                  0 if last else 1, _p(y), _p(out0) if last else None,
-                                  B, Z, Y, X, self.stream()))
-            acts.append(y)
+            _ok(L.PSWarmStartConv(_p(acts[l]), _p(self.wf[l]), _p(self.b[l]), None,
+                                  0 if last else 1, _p(acts[l + 1]), _p(out0) if last else None,
+                                  B, Z, Y, X, stream))
         self._acts = acts
         return out0
 
@@ -324,27 +330,25 @@ class Net:
         torch = self.torch
         B, Z, Y, X = dims
         n = B * Z * Y * X
-        L = ps.lib()
+        L, stream = ps.lib(), self.stream()
         nsplit = work.numel() // (27 * C * C + C)
+        dx = list(torch.empty((2, n * C), dtype=torch.bfloat16, device="cuda"))
         g = dy
         for l in range(LAYERS - 1, -1, -1):
             _ok(L.PSWarmStartWeightGrad(_p(self._acts[l]), _p(g), _p(work), nsplit,
                                         _p(self.grads[l]), _p(self.grads[LAYERS + l]),
-                                        B, Z, Y, X, self.stream()))
+                                        B, Z, Y, X, stream))
             if l:
-                dx = torch.empty(n * C, dtype=torch.bfloat16, device="cuda")
                 _ok(L.PSWarmStartConv(_p(g), _p(self.wb[l]), None, _p(self._acts[l]), 0,
-                                      _p(dx), None, B, Z, Y, X, self.stream()))
-                g = dx
+                                      _p(dx[l % 2]), None, B, Z, Y, X, stream))
+                g = dx[l % 2]
 
     def adam(self, lr, b1=0.9, b2=0.999, eps=1e-8):
         self.step += 1
-        L = ps.lib()
-        for p, g, m, v in zip(self.params, self.grads, self.m, self.v):
-            _ok(L.PSWarmStartAdam(_p(p), _p(g), _p(m), _p(v), p.numel(), ctypes.c_float(lr),
-                                  ctypes.c_float(b1), ctypes.c_float(b2), ctypes.c_float(eps),
-                                  self.step, self.stream()))
-        self.prepare()
+        w, g, m, v = self._flat
+        _ok(ps.lib().PSWarmStartAdamLayers(_p(w), _p(g), _p(m), _p(v), LAYERS, lr, b1, b2, eps,
+                                           self.step, _p(self._half[0]), _p(self._half[1]),
+                                           self.stream()))
 
 
 def _p(t):

@@ -98,3 +98,31 @@ def test_conv_edges(rt, dims, masked):
     if not masked:
         assert np.allclose(y0.cpu().numpy().reshape(dims), ref[..., 0], rtol=3e-5,
                            atol=3e-5 * np.abs(ref).max())
+
+
+# One launch over the whole network against the per-layer calls it replaces:
+# the same arithmetic, so the same weights, moments and BF16 copies up to one
+# FP32 rounding (contraction may differ between the kernels): 2^-23 relative
+# on the moments, the update itself being at most lr.
+@pytest.mark.parametrize("layers", [1, 3, 6])
+def test_adam_layers_matches_single_calls(rt, layers):
+    L = ps.lib()
+    per, n = 27 * 256, layers * (27 * 256 + 16)
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    w, g, m = (torch.randn(n, generator=gen, device="cuda") for _ in range(3))
+    v = torch.rand(n, generator=gen, device="cuda")
+    w2, m2, v2 = w.clone(), m.clone(), v.clone()
+    half = torch.zeros((2, layers, per), dtype=torch.bfloat16, device="cuda")
+    half2 = torch.zeros_like(half)
+    assert L.PSWarmStartAdamLayers(_p(w), _p(g), _p(m), _p(v), layers, 1e-2, 0.9, 0.999, 1e-8, 3,
+                                   _p(half[0]), _p(half[1]), _stream()) == 0
+    assert L.PSWarmStartAdam(_p(w2), _p(g), _p(m2), _p(v2), n, 1e-2, 0.9, 0.999, 1e-8, 3,
+                             _stream()) == 0
+    for l in range(layers):
+        assert L.PSWarmStartPrepareWeights(_p(w[l * per:]), _p(half2[0, l]), _p(half2[1, l]),
+                                           _stream()) == 0
+    torch.cuda.synchronize()
+    assert torch.allclose(m, m2, rtol=2 ** -23, atol=0) and torch.allclose(v, v2, rtol=2 ** -23,
+                                                                           atol=0)
+    assert (w - w2).abs().max() <= 2 ** -22 * w2.abs().max()
+    assert torch.equal(half.view(torch.int16), half2.view(torch.int16))
