@@ -98,6 +98,28 @@ cudaError_t launch_temporal7(const Temporal7Args &a, const MarchConfig &cfg,
                              const CUtensorMap *tin, int *dev_err, int sm_count,
                              cudaStream_t s);
 
+// ---- Whole DIFFUSION7 runs of small grids (resident7.cu) -------------------
+constexpr int kResident7MaxK = 4;
+struct Resident7Plan {
+  int by, bz;  // rows of a brick in y and z
+  int k;       // steps between exchanges
+  double us;   // estimated time per step
+};
+struct Resident7Args {
+  GridView g1, g2;  // step 0 in g1; ends with step `steps` in g1, steps - 1 in g2
+  double coef[7];   // map argument order: ce cw cn cs ct cb cc
+  int steps;        // even
+  Resident7Plan plan;
+  void *packets;    // resident7_packet_bytes() that only these launches write
+  unsigned base;    // no packet carries more; the launch leaves at most base + steps
+  int *err;
+};
+size_t resident7_packet_bytes(int nx, int ny, int nz, int esz);
+size_t resident7_smem(const Resident7Plan &q, int nx, int ny, int nz, int esz);
+// The cheapest brick and depth by the cost model; false if no brick fits.
+bool choose_resident7(int nx, int ny, int nz, int esz, int sms, Resident7Plan *best);
+cudaError_t launch_resident7(const Resident7Args &a, cudaStream_t s);
+
 // ---- Himeno 19-point Jacobi (himeno19.cu) --------------------------------
 struct Himeno19Args {
   GridView g[14];  // p0 p1 a0 a1 a2 a3 b0 b1 b2 c0 c1 c2 bnd wrk1

@@ -17,6 +17,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <chrono>
 #include <cstdarg>
@@ -68,6 +69,14 @@ struct Grid {
   void *dev;
 };
 
+// Launch shape of the 7-point sweeps unless the user or the autotuner chooses.
+constexpr MarchConfig kDefaultShape{8, 2, 4, 0, 0};
+
+bool same_cfg(const MarchConfig &a, const MarchConfig &b) {
+  return a.warps == b.warps && a.rows == b.rows && a.ns == b.ns && a.ns2 == b.ns2 &&
+         a.ctas_per_sm == b.ctas_per_sm;
+}
+
 // How a run executes: the sweep's launch shape and, for temporal-eligible
 // pairs, the temporal depth and the passes' shape.
 struct Plan {
@@ -114,6 +123,13 @@ struct Runtime {
   MarchConfig shapes[kNumKernels];
   int tblock[kNumKernels] = {};            // temporal steps per pass (<= 1: off)
   MarchConfig tshapes[kNumKernels];        // launch shape of temporal passes
+  // resident7.cu: the exchange packets (grown to the largest grid run so far),
+  // the number none of them exceeds, and the plans chosen so far by {nx, ny,
+  // nz, element size} (by = 0: none fits)
+  void *res_packets = nullptr;
+  size_t res_bytes = 0;
+  unsigned res_base = 0;
+  std::map<std::array<int, 4>, psg::Resident7Plan> res_plans;
   std::vector<TmapEntry> tmaps;
   int fail_allocs = 0;
   bool fma = false;  // temporal passes may contract multiply-adds
@@ -669,6 +685,17 @@ bool pair_eligible(const Map &a, const Map &b) {
   return true;
 }
 
+// Runs of fewer iterations stay with ordinary launches.
+constexpr int kResidentMinIter = 4;
+
+// Time per step of plain sweeps of g, in us: float 4.9 at 64^3 (launch and
+// latency), 5.0 at 96^3 and 6.0 at 128^3; double 19.2 up to 64^3 (four planes
+// of a 64 x 16 tile on the FP64 pipe) and 34.6 at 80^3.
+double plain_sweep_us(const Grid &g) {
+  const double cells = (double)g.dim[0] * g.dim[1] * g.dim[2];
+  return g.type == PS_FLOAT ? 4.5 + cells * 8 / 12e6 : std::max(18.0, 1.2 * 13 * cells / 0.42e6);
+}
+
 bool temporal_pair(const Map &a, const Map &b) {
   const int k = temporal_depth(a);
   return k >= 2 && k <= psg::temporal7_max_k(a.grids[0]->esz) && pair_eligible(a, b);
@@ -701,6 +728,89 @@ bool run_temporal(const Map &a, int iter) {
   // cur holds step total, oth step total-1.
   g1->dev = cur.ptr;
   g2->dev = oth.ptr;
+  return true;
+}
+
+// Exchange packets of at least `bytes` (zeroed when new, and before their
+// numbers could wrap around); false if there is no memory for them.
+bool resident_packets(size_t bytes) {
+  const bool wrap = rt->res_base > 0x7fffffffu;
+  if (bytes <= rt->res_bytes && !wrap) return true;
+  if (bytes > rt->res_bytes) {
+    cudaStreamSynchronize(rt->stream);
+    cudaFree(rt->res_packets);
+    rt->res_packets = nullptr;
+    rt->res_bytes = 0;
+    if (rt->fail_allocs > 0 || cudaMalloc(&rt->res_packets, bytes) != cudaSuccess) {
+      cudaGetLastError();
+      rt->res_packets = nullptr;
+      return false;
+    }
+    rt->res_bytes = bytes;
+  }
+  rt->res_base = 0;
+  if (cudaMemsetAsync(rt->res_packets, 0, rt->res_bytes, rt->stream) == cudaSuccess) return true;
+  cudaGetLastError();
+  cudaFree(rt->res_packets);
+  rt->res_packets = nullptr;
+  rt->res_bytes = 0;
+  return false;
+}
+
+// The plan for running (a, b) x iter in one launch (resident7.cu), or nullptr
+// if another path is to run it: runs whose launch shape the user or the
+// autotuner chose, stream capture, short runs, and grids that do not fit on
+// chip or are estimated to be faster as plain sweeps.
+const psg::Resident7Plan *resident_plan(const Map &a, const Map &b, int iter) {
+  if (!pair_eligible(a, b) || a.has_plan ||
+      !same_cfg(rt->shapes[shape_slot(a.kernel)], kDefaultShape))
+    return nullptr;
+  if (iter < kResidentMinIter || iter > (1 << 28)) return nullptr;
+  const char *e = getenv("PS_RESIDENT");
+  if (e && e[0] == '0') return nullptr;
+  const Grid *g = a.grids[0];
+  const std::array<int, 4> key = {g->dim[0], g->dim[1], g->dim[2], g->esz};
+  auto hit = rt->res_plans.find(key);
+  if (hit == rt->res_plans.end()) {
+    psg::Resident7Plan q{};
+    if (!psg::choose_resident7(key[0], key[1], key[2], key[3], rt->sm_count, &q) ||
+        q.us > 0.9 * plain_sweep_us(*g))
+      q.by = 0;
+    hit = rt->res_plans.emplace(key, q).first;
+  }
+  if (hit->second.by == 0) return nullptr;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(rt->stream, &cap) != cudaSuccess ||
+      cap != cudaStreamCaptureStatusNone) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  return resident_packets(psg::resident7_packet_bytes(key[0], key[1], key[2], key[3]))
+             ? &hit->second
+             : nullptr;
+}
+
+// *ran is false, with no error, if the device cannot hold the launch's CTAs at
+// once (a process limited to some of its SMs).
+bool run_resident(const Map &a, int iter, const psg::Resident7Plan &plan, bool *ran) {
+  psg::Resident7Args r{};
+  r.g1 = view(a.grids[0]);
+  r.g2 = view(a.grids[1]);
+  for (int i = 0; i < 7; ++i) r.coef[i] = a.scalars[i];
+  r.steps = 2 * iter;
+  r.plan = plan;
+  r.packets = rt->res_packets;
+  r.base = rt->res_base;
+  r.err = rt->dev_err;
+  const cudaError_t e = psg::launch_resident7(r, rt->stream);
+  *ran = e != cudaErrorCooperativeLaunchTooLarge && e != cudaErrorNotSupported;
+  if (!*ran) {
+    cudaGetLastError();
+    return true;
+  }
+  if (!cuda_ok(e, "resident7 launch")) return false;
+  rt->res_base += (unsigned)r.steps;
+  ++rt->launches;
   return true;
 }
 
@@ -1075,11 +1185,6 @@ void graph_signature(const std::vector<Map *> &ms, std::vector<void *> *ptrs,
   }
 }
 
-bool same_cfg(const MarchConfig &a, const MarchConfig &b) {
-  return a.warps == b.warps && a.rows == b.rows && a.ns == b.ns && a.ns2 == b.ns2 &&
-         a.ctas_per_sm == b.ctas_per_sm;
-}
-
 void drop_graphs_for(const Grid *g) {
   for (size_t i = 0; i < g_graphs.size();) {
     bool uses = false;
@@ -1404,6 +1509,11 @@ bool run_maps(const std::vector<Map *> &ms, int iter) {
     // every iteration went into tuning trials
   } else if (ms.size() == 2 && temporal_pair(*ms[0], *ms[1])) {
     if (!run_temporal(*ms[0], iter)) return false;
+  } else if (const psg::Resident7Plan *q =
+                 ms.size() == 2 ? resident_plan(*ms[0], *ms[1], iter) : nullptr) {
+    bool ran = false;
+    if (!run_resident(*ms[0], iter, *q, &ran)) return false;
+    if (!ran && !run_plain(ms, iter)) return false;
   } else {
     if (!run_plain(ms, iter)) return false;
   }
@@ -1605,7 +1715,7 @@ void PSInitV(int trace) {
   for (int i = 0; i < kNumEvents; ++i) cudaEventCreate(&r->events[i]);
   // Default launch shapes (the autotuner may replace them):
   // {warps, rows per thread, ring stages, second-ring stages, CTAs per SM}.
-  for (int k = 0; k < kNumKernels; ++k) r->shapes[k] = MarchConfig{8, 2, 4, 0, 0};
+  for (int k = 0; k < kNumKernels; ++k) r->shapes[k] = kDefaultShape;
   for (int k = 0; k < kNumKernels; ++k) {
     r->tshapes[k] = MarchConfig{8, 4, 3, 0, 0};
     r->tblock[k] = 1;
@@ -1639,6 +1749,7 @@ void PSFinalize(void) {
   cudaFree(rt->partials);
   cudaFree(rt->ticket);
   cudaFree(rt->results);
+  cudaFree(rt->res_packets);
   for (int i = 0; i < kNumEvents; ++i) cudaEventDestroy(rt->events[i]);
   cudaEventDestroy(rt->fork);
   cudaEventDestroy(rt->join);

@@ -165,6 +165,58 @@ def test_diffusion_64cubed_100_steps_then_reduce(rt, oracle):
     g.free()
 
 
+# Whole runs in one launch (grids that fit on chip): ragged bricks, rows that
+# are no whole number of vectors and that start inside a warp, a last epoch of
+# one step, one brick per axis, bricks thinner than the halo, double precision.
+# The launch count shows which path ran: one kernel, or one per sweep.
+@pytest.mark.parametrize("shape,dtype,iters,one", [
+    ((32, 32, 32), np.float32, 5, True), ((25, 26, 1), np.float32, 6, True),
+    ((47, 33, 40), np.float32, 7, True), ((67, 63, 65), np.float32, 4, True),
+    ((13, 200, 50), np.float32, 8, True), ((300, 4, 7), np.float32, 9, True),
+    ((64, 10, 300), np.float32, 5, True), ((96, 95, 97), np.float32, 6, True),
+    ((31, 33, 35), np.float64, 6, True), ((60, 11, 129), np.float64, 5, True),
+    ((64, 64, 64), np.float32, 3, False), ((8, 8, 64), np.float32, 6, False),
+    ((200, 200, 200), np.float32, 4, False)])
+def test_diffusion_run_in_one_launch(rt, oracle, monkeypatch, shape, dtype, iters, one):
+    nz, ny, nx = shape
+    init = synth.uniform(shape, 21).astype(dtype)
+    r1, r2 = init.copy(), np.zeros_like(init)
+    oracle.run7(oracle.V_DIFFUSION7, r1, r2, (0, nx, 0, ny, 0, nz), DIFF_COEF, iter=iters)
+    for env, launches in (("1", 1 if one else 2 * iters), ("0", 2 * iters)):
+        monkeypatch.setenv("PS_RESIDENT", env)
+        n0 = ps.launch_count()
+        a, b = run_pingpong(ps.PS_KERNEL_DIFFUSION7, init, ps.full_domain(shape), DIFF_COEF,
+                            iters, dtype)
+        assert ps.launch_count() - n0 == launches
+        assert np.array_equal(_bits(a), _bits(r1))
+        assert np.array_equal(_bits(b), _bits(r2))
+
+
+def test_one_launch_runs_repeat_and_keep_their_storage(rt, oracle):
+    # three runs of two grids in turn: exchange packets of earlier runs and of
+    # the other grid size stay behind; each run continues from the last
+    shapes = [(40, 40, 40), (34, 50, 60)]
+    grids, refs = [], []
+    for shape in shapes:
+        init = synth.uniform(shape, 22)
+        g = [ps.Grid(shape), ps.Grid(shape)]
+        g[0].copyin(init)
+        m = [ps.stencil_map(ps.PS_KERNEL_DIFFUSION7, ps.full_domain(shape), q, DIFF_COEF)
+             for q in (g, g[::-1])]
+        grids.append((g, m, [x.dev_ptr for x in g]))
+        refs.append((init.copy(), np.zeros_like(init)))
+    for iters in (4, 9, 5):
+        for (g, m, ptrs), (r1, r2), (nz, ny, nx) in zip(grids, refs, shapes):
+            ps.stencil_run(m, iters)
+            oracle.run7(oracle.V_DIFFUSION7, r1, r2, (0, nx, 0, ny, 0, nz), DIFF_COEF, iter=iters)
+            assert np.array_equal(_bits(g[0].copyout()), _bits(r1))
+            assert np.array_equal(_bits(g[1].copyout()), _bits(r2))
+            assert [x.dev_ptr for x in g] == ptrs
+    for g, _, _ in grids:
+        g[0].free()
+        g[1].free()
+
+
 SHAPES = [(9, 17, 33), (5, 3, 130), (1, 1, 7), (40, 67, 45), (2, 130, 4),
           (16, 16, 256)]
 
