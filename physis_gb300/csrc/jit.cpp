@@ -139,7 +139,7 @@ bool load_driver(std::string *err) {
 
 // ---- the device prelude -----------------------------------------------------
 // PSGrid{1,2,3}D{Float,Double,Int,Long} are one device struct per element
-// type; `cur` is the element the map's current point emits to.  Index
+// type; `e` is the element the map's current point emits to.  Index
 // arithmetic as the reference's (physis_cuda.h:237-269): x fastest, periodic
 // reads wrap with (i + n) % n.
 const char *kPrelude = R"PSJIT(
@@ -147,7 +147,7 @@ const char *kPrelude = R"PSJIT(
 typedef int PSIndex;
 // Kernel parameter (host layout: GridArg in jit.cpp).
 template <typename T> struct __PSGridArg {
-  T *p; long long row; long long plane; int nx; int ny; int nz; int rank; long long cur;
+  T *p; long long row; long long plane; int nx; int ny; int nz; int rank;
 };
 // What the stencil function sees.  For a grid the tiled entry staged in
 // shared memory (staged == 1) the entry also records the cell being computed
@@ -158,14 +158,14 @@ template <typename T> struct __PSGridArg {
 // const make every test and index a constant; any other read is tested at
 // run time and falls back to global memory outside the window.
 template <typename T> struct __PSGridDev {
-  T *p; long long row; long long plane; int nx; int ny; int nz; int rank; long long cur;
+  T *p; long long row; long long plane; int nx; int ny; int nz; int rank; T *e;
   int staged, rx, ry, rz, sw, cx, cy, cz;
   const T *c[9];
 };
 template <typename T> __device__ __forceinline__ __PSGridDev<T> __ps_dev(const __PSGridArg<T> &a) {
   __PSGridDev<T> g;
   g.p = a.p; g.row = a.row; g.plane = a.plane; g.nx = a.nx; g.ny = a.ny; g.nz = a.nz;
-  g.rank = a.rank; g.cur = 0; g.staged = 0;
+  g.rank = a.rank; g.e = nullptr; g.staged = 0;
   return g;
 }
 #define __PS_GRID_TYPES(N, T) \
@@ -216,7 +216,7 @@ template <typename T> __device__ __forceinline__ int __ps_dim(const __PSGridDev<
 }
 // Grids of a user-defined element type: the source's own struct definition
 // and DeclareGrid line; PSGridEmitUtype(g.m, v) reaches __PS_EMITU as
-// __PS_EMITU((g).p[(g).cur].m, v) (the front end rewrites the call), i.e. a
+// __PS_EMITU((g).e[0].m, v) (the front end rewrites the call), i.e. a
 // store to member m of the point being computed.
 #define DeclareGrid1D(N, T) typedef __PSGridDev<T> PSGrid1D##N
 #define DeclareGrid2D(N, T) typedef __PSGridDev<T> PSGrid2D##N
@@ -224,11 +224,12 @@ template <typename T> __device__ __forceinline__ int __ps_dim(const __PSGridDev<
 #define __PS_EMITU(lhs, v) ((void)((lhs) = (v)))
 #define PSGridGet(g, ...) __ps_get((g), __VA_ARGS__)
 #define PSGridGetPeriodic(g, ...) __ps_getp((g), __VA_ARGS__)
-#define PSGridEmit(g, v) ((void)((g).p[(g).cur] = (v)))
+#define PSGridEmit(g, v) ((void)((g).e[0] = (v)))
 #define PSGridDim(g, d) __ps_dim((g), (d))
 
 // ---- staging for the tiled entry ----
-template <int S> __device__ __forceinline__ int __ps_slot(int z) { return ((z % S) + S) % S; }
+// Opaque TMA descriptor (the layout of CUtensorMap: 128 bytes, 64-aligned).
+struct alignas(64) __PSTmap { unsigned long long opaque[16]; };
 template <bool PER> __device__ __forceinline__ int __ps_fit(int v, int n) {
   if (PER) {
     if ((unsigned)v >= (unsigned)n) {
@@ -239,40 +240,38 @@ template <bool PER> __device__ __forceinline__ int __ps_fit(int v, int n) {
   }
   return min(max(v, 0), n - 1);
 }
-// Plane zp (unwrapped) of the W x H window at (x0 - RX, y0 - RY) into its
-// ring slot.  vec (the CTA's window lies inside the grid in x and every
-// window row starts on a 16-byte boundary): 16-byte cp.async chunks, rows
-// clamped or wrapped in y.  Otherwise one cp.async per cell, warp w copying
-// rows w, w + 8, ..., cells outside the grid wrapped (PER) or clamped.
-template <typename T, int W, int H, int S, int RX, int RY, bool PER>
-__device__ __forceinline__ void __ps_stage(T *ring, const __PSGridArg<T> &a, int x0, int y0,
-                                           bool vec, int zp) {
-  T *dst = ring + __ps_slot<S>(zp) * (W * H);
-  const T *src = a.p + (long long)__ps_fit<PER>(zp, a.nz) * a.plane;
-  if (vec) {
-    constexpr int V = 16 / (int)sizeof(T), NV = W / V;
-    for (int e = threadIdx.x; e < NV * H; e += 256) {
-      const int r = e / NV, c = e - r * NV;
-      const T *srow = src + (long long)__ps_fit<PER>(y0 - RY + r, a.ny) * a.row + (x0 - RX);
-      psg::cp_async16(dst + r * W + c * V, srow + c * V);
-    }
-    return;
-  }
-  const int lane = threadIdx.x & 31;
-  for (int r = threadIdx.x >> 5; r < H; r += 8) {
-    const T *srow = src + (long long)__ps_fit<PER>(y0 - RY + r, a.ny) * a.row;
-    T *drow = dst + r * W;
-#pragma unroll
-    for (int c = lane; c < W; c += 32)
-      psg::cp_async_small<(int)sizeof(T)>(drow + c, srow + __ps_fit<PER>(x0 - RX + c, a.nx));
-  }
+// Whether the W x H window at (xs, ys) has cells outside an nx x ny plane.
+__device__ __forceinline__ bool __ps_crosses(int xs, int ys, int w, int h, int nx, int ny) {
+  return xs < 0 || ys < 0 || xs + w > nx || ys + h > ny;
 }
-// Whether a window of width W at x0 - RX can be staged in 16-byte chunks.
-template <typename T, int W, int RX>
-__device__ __forceinline__ bool __ps_vec_ok(const __PSGridArg<T> &a, int x0) {
-  const T *row0 = a.p + (x0 - RX);
-  return x0 - RX >= 0 && x0 - RX + W <= a.nx &&
-         ((unsigned long long)row0 & 15) == 0 && ((a.row * (long long)sizeof(T)) & 15) == 0;
+// One plane of a staged window (W x H cells at (xs, ys), TMA-filled with zeros
+// outside the grid): the warp rewrites the outside cells that a halo of RX x
+// RY can reach with the wrapped (PER, fetched from the grid's plane zg) or
+// nearest (copied within the window) values.
+template <typename T, int W, int H, int RX, int RY, bool PER>
+__device__ __forceinline__ void __ps_edges(T *box, const __PSGridArg<T> &a, int xs, int ys,
+                                           int zg, int lane) {
+  const int c0 = max(0, -RX - xs), c1 = min(W, a.nx + RX - xs);
+  const int r0 = max(0, -RY - ys), r1 = min(H, a.ny + RY - ys);
+  const int rin0 = max(r0, -ys), rin1 = min(r1, a.ny - ys);
+  const int cl = max(c0, -xs), cr = min(c1, a.nx - xs);
+  const T *plane = a.p + (long long)zg * a.plane;
+  for (int r = r0; r < r1; ++r) {
+    if (r >= rin0 && r < rin1) continue;
+    const int y = __ps_fit<PER>(ys + r, a.ny);
+    for (int c = c0 + lane; c < c1; c += 32) {
+      const int x = __ps_fit<PER>(xs + c, a.nx);
+      box[r * W + c] = PER ? plane[(long long)y * a.row + x] : box[(y - ys) * W + (x - xs)];
+    }
+  }
+  const int nc = (cl - c0) + (c1 - cr);
+  if (nc <= 0) return;
+  for (int r = rin0 + lane; r < rin1; r += 32)
+    for (int k = 0; k < nc; ++k) {
+      const int c = k < cl - c0 ? c0 + k : cr + (k - (cl - c0));
+      const int x = __ps_fit<PER>(xs + c, a.nx);
+      box[r * W + c] = PER ? plane[(long long)(ys + r) * a.row + x] : box[r * W + (x - xs)];
+    }
 }
 )PSJIT";
 
@@ -281,7 +280,6 @@ struct GridArg {
   void *p;
   long long row, plane;
   int nx, ny, nz, rank;
-  long long cur;
 };
 
 std::string trim(const std::string &s) {
@@ -483,27 +481,49 @@ std::string entry_source(const JitKernel &k) {
   for (size_t i = 0; i < k.params.size(); ++i) {
     if (!k.params[i].grid) continue;
     const std::string g = "g" + std::to_string(i);
-    s += "    " + g + ".cur = " + cur_expr(k.params[i], g) + ";\n";
+    s += "    " + g + ".e = " + g + ".p + (" + cur_expr(k.params[i], g) + ");\n";
   }
   s += "    " + call_source(k) + "  }\n}\n";
   return s;
 }
 
 // ---- the tiled entry ---------------------------------------------------------
-// A CTA of 256 threads owns a 64 x 16 (x, y) tile and a chunk of z.  Grids
-// the stencil reads at neighbour offsets (and never emits to) are staged:
-// each z step copies one plane of the tile plus halo into a ring of
-// shared-memory planes with cp.async, kAhead planes ahead of the compute, and
-// the function's reads inside the window come from there.  The reads themselves
-// are unchanged, so every result is bit-identical to the plain entry's.
+// A CTA of four warps and a producer warp owns a 64 x 16 (x, y) tile and a
+// chunk of z; a thread computes eight consecutive rows of one column.  Grids
+// the stencil reads at neighbour offsets (and never emits to) are staged: a
+// ring of shared-memory planes of the tile plus halo, one TMA box per plane,
+// loaded a step ahead of the compute by the producer warp, which on edge tiles
+// also gives the cells outside the grid their values.  The function's reads
+// inside the window come from there.  The reads themselves are unchanged, so
+// every result is bit-identical to the plain entry's.
+//
+// Issue slots are what such a kernel is short of, so:
+// * the eight rows share their loads (the window positions of a thread's cells
+//   differ by constants, so equal reads are one load to the compiler) and a
+//   step's fixed work;
+// * warps whose cells all lie at least one cell inside the domain's grids and
+//   inside the domain run a copy of the function that may assume so: the
+//   comparisons of a function that treats the faces itself fold away;
+// * boxes arrive by TMA, where cp.async took a quarter of the instructions.
+// Measured, one sweep against the cp.async entry (256 threads, two by two cells
+// each, CTA barriers): clamped 7-point function at 400 x 384 x 320 float 90
+// against 154 us (48 instructions a cell against 92, 65 % of the HBM rate),
+// 27-point function at 258 x 258 x 200 double 686 against 727 us (the FP64
+// pipe's time is 556).
 constexpr int kTileX = 64, kTileY = 16;
-constexpr int kAhead = 3;                   // planes in flight ahead of the compute
-constexpr size_t kStageBudget = 96 * 1024;  // two or more CTAs per SM
+constexpr int kTileRows = 8;                              // rows per thread
+constexpr int kTileWarps = kTileX / 32 * kTileY / kTileRows;
+constexpr int kTileThreads = 32 * (kTileWarps + 1);
+constexpr size_t kStageBudget = 80 * 1024;                // two or more CTAs per SM
+constexpr size_t kStageHead = 128;                        // mbarriers in front of the rings
 
 // Ring planes of a grid staged with z halo rz: the 2 rz + 1 planes a step
-// reads, kAhead in flight, and one more so that a plane is never refilled
-// while a thread still one step behind reads it.
-int ring_planes(int rz) { return 2 * rz + 2 + kAhead; }
+// reads and the next one.
+int ring_planes(int rz) { return 2 * rz + 2; }
+// Bytes of one of them (TMA destinations are 128-byte aligned).
+size_t plane_bytes(const JitStage &st) {
+  return ((size_t)st.w * (kTileY + 2 * st.ry) * st.esz + 127) / 128 * 128;
+}
 
 // Splits the argument list of the call whose '(' is at src[open] into its
 // top-level arguments; npos-safe (returns false if unbalanced).
@@ -595,10 +615,10 @@ void choose_stages(JitKernel *k) {
     st.rz = r[2];
     st.periodic = periodic;
     st.esz = (p.type == kFloat || p.type == kInt) ? 4 : 8;
-    const int v = 16 / st.esz;  // the window's x halo: rx rounded up to 16 bytes
-    st.rxw = (st.rx + v - 1) / v * v;
-    st.bytes = (size_t)ring_planes(st.rz) * (kTileX + 2 * st.rxw) * (kTileY + 2 * st.ry) * st.esz;
-    st.bytes = (st.bytes + 15) / 16 * 16;
+    // the window starts on 16 bytes, up to v - 1 cells left of the halo
+    const int v = 16 / st.esz;
+    st.w = (kTileX + 2 * st.rx + 2 * (v - 1)) / v * v;
+    st.bytes = (size_t)ring_planes(st.rz) * plane_bytes(st);
     if (k->stage_smem + st.bytes > kStageBudget) continue;
     st.off = k->stage_smem;
     k->stage_smem += st.bytes;
@@ -607,87 +627,151 @@ void choose_stages(JitKernel *k) {
 }
 
 std::string tiled_entry_source(const JitKernel &k) {
-  std::string s =
-      "\nextern \"C\" __global__ void __launch_bounds__(256) __ps_entry_t(int dmin0, int dmax0, "
-      "int dmin1, int dmax1, int dmin2, int dmax2, int ntx, int zlen" +
-      entry_params(k) + ") {\n"
-      "  extern __shared__ __align__(16) unsigned char __ps_sm[];\n"
-      "  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;\n"
-      "  const int x0 = dmin0 + (int)(blockIdx.x % (unsigned)ntx) * " + std::to_string(kTileX) +
-      ";\n"
-      "  const int y0 = dmin1 + (int)(blockIdx.x / (unsigned)ntx) * " + std::to_string(kTileY) +
-      ";\n"
-      "  const int zs = dmin2 + (int)blockIdx.y * zlen;\n"
-      "  const int ze = min(zs + zlen, dmax2);\n"
-      "  if (zs >= ze) return;\n";
-  for (size_t i = 0; i < k.params.size(); ++i)
-    if (k.params[i].grid)
-      s += "  auto g" + std::to_string(i) + " = __ps_dev(a" + std::to_string(i) + ");\n";
-  // prologue: the planes step zs reads (one commit group), then the planes
-  // ahead of it one group each; step z adds plane z + rz + kAhead and waits
-  // until at most kAhead groups are pending, i.e. plane z + rz has landed.
-  std::string first, ahead, next;
+  const auto N = [](long long v) { return std::to_string(v); };
+  std::string s = "\nextern \"C\" __global__ void __launch_bounds__(" + N(kTileThreads) +
+                  ") __ps_entry_t(int dmin0, int dmax0, int dmin1, int dmax1, int dmin2, "
+                  "int dmax2, int ntx, int zlen, int *err";
+  for (size_t j = 0; j < k.stages.size(); ++j)
+    s += ", const __grid_constant__ __PSTmap tm" + N(j);
+  s += entry_params(k) + ") {\n"
+       "  extern __shared__ __align__(128) unsigned char __ps_raw[];\n"
+       "  unsigned char *__ps_sm = __ps_raw + ((128u - (psg::smem_u32(__ps_raw) & 127u)) & 127u);\n"
+       // barriers: group loaded (full), box landed (raw), step done (empty), two each
+       "  unsigned long long *full = reinterpret_cast<unsigned long long *>(__ps_sm), *raw = full + 2,"
+       " *empty = full + 4;\n"
+       "  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;\n"
+       "  const int x0 = dmin0 + (int)(blockIdx.x % (unsigned)ntx) * " + N(kTileX) + ";\n"
+       "  const int y0 = dmin1 + (int)(blockIdx.x / (unsigned)ntx) * " + N(kTileY) + ";\n"
+       "  const int zs = dmin2 + (int)blockIdx.y * zlen;\n"
+       "  const int n = min(zs + zlen, dmax2) - zs;\n"
+       "  if (n <= 0) return;\n"
+       "  if (threadIdx.x == 0) {\n"
+       "    for (int i = 0; i < 2; ++i) {\n"
+       "      psg::mbar_init(&full[i], 1);\n      psg::mbar_init(&raw[i], 1);\n"
+       "      psg::mbar_init(&empty[i], " + N(kTileWarps) + ");\n    }\n"
+       "    psg::fence_barrier_init();\n  }\n"
+       "  __syncthreads();\n";
+  // the staged grids' rings and windows
+  std::string edge, init, step, fixi, fixs;
+  size_t bytes0 = 0, bytes1 = 0;
   for (size_t j = 0; j < k.stages.size(); ++j) {
     const JitStage &st = k.stages[j];
-    const std::string i = std::to_string(st.param), sj = std::to_string(j);
+    const std::string i = N(st.param), sj = N(j);
     const std::string T = scalar_ctype(k.params[st.param].type);
-    const int W = kTileX + 2 * st.rxw, H = kTileY + 2 * st.ry, S = ring_planes(st.rz);
-    const std::string rz = std::to_string(st.rz), vj = "v" + sj;
-    const std::string stage = "__ps_stage<" + T + ", " + std::to_string(W) + ", " +
-                              std::to_string(H) + ", " + std::to_string(S) + ", " +
-                              std::to_string(st.rxw) + ", " + std::to_string(st.ry) + ", " +
-                              (st.periodic ? "true" : "false") + ">(s" + sj + ", a" + i +
-                              ", x0, y0, " + vj + ", ";
+    const int W = st.w, H = kTileY + 2 * st.ry, S = ring_planes(st.rz);
+    const size_t pe = plane_bytes(st) / st.esz;
+    const std::string fit = std::string("__ps_fit<") + (st.periodic ? "true" : "false") + ">";
     s += "  " + T + " *s" + sj + " = reinterpret_cast<" + T + " *>(__ps_sm + " +
-         std::to_string(st.off) + ");\n";
-    s += "  const bool " + vj + " = __ps_vec_ok<" + T + ", " + std::to_string(W) + ", " +
-         std::to_string(st.rxw) + ">(a" + i + ", x0);\n";
-    s += "  g" + i + ".staged = 1; g" + i + ".rx = " + std::to_string(st.rxw) + "; g" + i +
-         ".ry = " + std::to_string(st.ry) + "; g" + i + ".rz = " + rz + "; g" + i + ".sw = " +
-         std::to_string(W) + ";\n";
-    first += "  for (int d = -" + rz + "; d <= " + rz + "; ++d) " + stage + "zs + d);\n";
-    ahead += "    if (zs + a < ze) " + stage + "zs + " + rz + " + a);\n";
-    next += "      " + stage + "z + " + rz + " + " + std::to_string(kAhead) + ");\n";
+         N(kStageHead + st.off) + ");\n";
+    s += "  const int xs" + sj + " = (x0 - " + N(st.rx) + ") & ~" + N(16 / st.esz - 1) + ", ys" + sj +
+         " = y0 - " + N(st.ry) + ";\n";
+    edge += (j ? " || " : "") + ("__ps_crosses(xs" + sj + ", ys" + sj + ", " + N(W) + ", " + N(H) +
+            ", a" + i + ".nx, a" + i + ".ny)");
+    bytes0 += (size_t)(2 * st.rz + 1) * W * H * st.esz;
+    bytes1 += (size_t)W * H * st.esz;
+    const std::string load = "psg::tma_load_3d(s" + sj + " + ", at = ", &tm" + sj + ", xs" + sj +
+                             ", ys" + sj + ", " + fit + "(";
+    const std::string fix = "__ps_edges<" + T + ", " + N(W) + ", " + N(H) + ", " + N(st.rx) + ", " +
+                            N(st.ry) + ", " + (st.periodic ? "true" : "false") + ">(s" + sj + " + ";
+    // group 0: planes zs - rz .. zs + rz in slots 0 .. 2 rz; group i: plane
+    // zs + i + rz in slot (i + 2 rz) % S
+    init += "        for (int d = 0; d <= " + N(2 * st.rz) + "; ++d) " + load + "d * " + N(pe) + at +
+            "zs - " + N(st.rz) + " + d, a" + i + ".nz), bar);\n";
+    step += "        " + load + "(i + " + N(2 * st.rz) + ") % " + N(S) + " * " + N(pe) + at + "zs + i + " +
+            N(st.rz) + ", a" + i + ".nz), bar);\n";
+    fixi += "        for (int d = 0; d <= " + N(2 * st.rz) + "; ++d) " + fix + "d * " + N(pe) + ", a" + i +
+            ", xs" + sj + ", ys" + sj + ", " + fit + "(zs - " + N(st.rz) + " + d, a" + i + ".nz), lane);\n";
+    fixs += "        " + fix + "(i + " + N(2 * st.rz) + ") % " + N(S) + " * " + N(pe) + ", a" + i + ", xs" +
+            sj + ", ys" + sj + ", " + fit + "(zs + i + " + N(st.rz) + ", a" + i + ".nz), lane);\n";
   }
-  s += first + "  psg::cp_async_commit();\n";
-  s += "  for (int a = 1; a < " + std::to_string(kAhead) + "; ++a) {\n" + ahead +
-       "    psg::cp_async_commit();\n  }\n";
-  s += "  for (int z = zs; z < ze; ++z) {\n"
-       "    if (z + " + std::to_string(kAhead) + " < ze) {\n" + next + "    }\n"
-       "    psg::cp_async_commit();\n"
-       "    psg::cp_async_wait<" + std::to_string(kAhead) + ">();\n"
-       "    __syncthreads();\n";
-  // per step: each staged grid's plane pointers; per cell: the cell's
-  // coordinates and its position in those planes
-  std::string cell;
-  for (size_t j = 0; j < k.stages.size(); ++j) {
-    const JitStage &st = k.stages[j];
-    const std::string g = "g" + std::to_string(st.param), sj = std::to_string(j);
-    const int W = kTileX + 2 * st.rxw, S = ring_planes(st.rz);
-    const std::string rz = std::to_string(st.rz);
-    s += "    const " + scalar_ctype(k.params[st.param].type) + " *pl" + sj + "[9];\n";
-    s += "    for (int d = -" + rz + "; d <= " + rz + "; ++d) pl" + sj + "[d + 4] = s" + sj +
-         " + __ps_slot<" + std::to_string(S) + ">(z + d) * " +
-         std::to_string(W * (kTileY + 2 * st.ry)) + ";\n";
-    cell += "          " + g + ".cx = x; " + g + ".cy = y; " + g + ".cz = z;\n";
-    cell += "          for (int d = -" + rz + "; d <= " + rz + "; ++d) " + g + ".c[d + 4] = pl" +
-            sj + "[d + 4] + (y - y0 + " + std::to_string(st.ry) + ") * " + std::to_string(W) +
-            " + (x - x0 + " + std::to_string(st.rxw) + ");\n";
-  }
-  s += "#pragma unroll\n"
-       "    for (int jy = 0; jy < " + std::to_string(kTileY / 8) + "; ++jy) {\n"
-       "      const int y = y0 + warp + 8 * jy;\n"
-       "#pragma unroll\n"
-       "      for (int jx = 0; jx < " + std::to_string(kTileX / 32) + "; ++jx) {\n"
-       "        const int x = x0 + lane + 32 * jx;\n"
-       "        if (x < dmax0 && y < dmax1) {\n" + cell;
+  s += "  if (warp == " + N(kTileWarps) + ") {\n"
+       "    const bool edge = " + edge + ";\n"
+       "    for (int i = 0; i < n; ++i) {\n"
+       "      // group i replaces the plane that step i - 2 read last\n"
+       "      if (i >= 2 && !__all_sync(0xffffffffu, psg::mbar_wait(&empty[i & 1], ((i - 2) >> 1) & 1, err)))"
+       " return;\n"
+       "      unsigned long long *bar = edge ? &raw[i & 1] : &full[i & 1];\n"
+       "      if (lane == 0) {\n"
+       "        psg::mbar_arrive_expect_tx(bar, i ? " + N(bytes1) + "u : " + N(bytes0) + "u);\n"
+       "        if (i == 0) {\n" + init + "        } else {\n" + step + "        }\n      }\n"
+       "      if (!edge) continue;\n"
+       "      if (!__all_sync(0xffffffffu, psg::mbar_wait(bar, (i >> 1) & 1, err))) return;\n"
+       "      if (i == 0) {\n" + fixi + "      } else {\n" + fixs + "      }\n"
+       "      asm volatile(\"fence.proxy.async.shared::cta;\" ::: \"memory\");\n"
+       "      __syncwarp();\n"
+       "      if (lane == 0) psg::mbar_arrive(&full[i & 1]);\n    }\n"
+       "    // the last copies land before the CTA may end\n"
+       "    for (int i = max(0, n - 2); i < n; ++i)\n"
+       "      psg::mbar_wait(&full[i & 1], (i >> 1) & 1, nullptr, 1u << 16);\n"
+       "    return;\n  }\n";
+  // consumers
+  s += "  const int x = x0 + lane + 32 * (warp % " + N(kTileX / 32) + ");\n"
+       "  const int yb = y0 + " + N(kTileRows) + " * (warp / " + N(kTileX / 32) + ");\n";
+  std::string inner = "__all_sync(0xffffffffu, x >= dmin0 && x < dmax0 && yb + " +
+                      N(kTileRows) + " <= dmax1", zin, assume;
   for (size_t i = 0; i < k.params.size(); ++i) {
     if (!k.params[i].grid) continue;
-    const std::string g = "g" + std::to_string(i);
-    s += "          " + g + ".cur = " + cur_expr(k.params[i], g) + ";\n";
+    const JitParam &p = k.params[i];
+    const std::string si = N(i), g = "g" + si, a = "a" + si;
+    s += "  auto " + g + " = __ps_dev(" + a + ");\n";
+    // the element of the thread's first row, advanced by a plane per step
+    s += "  auto *e" + si + " = " + a + ".p + (" +
+         (p.rank == 1 ? std::string("x")
+          : p.rank == 2 ? "(long long)yb * " + a + ".row + x"
+                        : "(long long)zs * " + a + ".plane + (long long)yb * " + a + ".row + x") + ");\n";
+    if (p.rank != 3) continue;
+    inner += " && x >= 1 && x < " + a + ".nx - 1 && yb >= 1 && yb + " + N(kTileRows) + " <= " + a +
+             ".ny - 1";
+    zin += " && z < " + a + ".nz - 1";
+    for (const char *d : {"x", "y", "z"}) {
+      const std::string dim = g + ".n" + d;
+      assume += std::string("__builtin_assume(") + d + " < " + dim + " - 1); __builtin_assume(" + d +
+                " + 1 < " + dim + "); ";
+    }
   }
-  s += "          " + call_source(k) + "        }\n      }\n    }\n  }\n"
-       "  psg::cp_async_wait<0>();\n}\n";
+  s += "  const bool inner = " + inner + ");\n";
+  for (size_t j = 0; j < k.stages.size(); ++j) {
+    const JitStage &st = k.stages[j];
+    const std::string g = "g" + N(st.param);
+    s += "  " + g + ".staged = 1; " + g + ".rx = " + N(st.rx) + "; " + g + ".ry = " + N(st.ry) + "; " + g +
+         ".rz = " + N(st.rz) + "; " + g + ".sw = " + N(st.w) + ";\n";
+    s += "  const int w" + N(j) + " = (yb - ys" + N(j) + ") * " + N(st.w) + " + (x - xs" +
+         N(j) + ");\n";
+  }
+  s += "  bool ok = true;\n"
+       "  for (int i = 0; i < n; ++i) {\n"
+       "    const int z = zs + i;\n"
+       "    if (ok) ok = __all_sync(0xffffffffu, psg::mbar_wait(&full[i & 1], (i >> 1) & 1, err));\n"
+       "    if (ok) {\n";
+  std::string cell, advance;
+  for (size_t j = 0; j < k.stages.size(); ++j) {
+    const JitStage &st = k.stages[j];
+    const std::string g = "g" + N(st.param), sj = N(j);
+    const int S = ring_planes(st.rz);
+    s += "      const " + scalar_ctype(k.params[st.param].type) + " *pl" + sj + "[" + N(2 * st.rz + 1) + "];\n"
+         "#pragma unroll\n"
+         "      for (int d = 0; d <= " + N(2 * st.rz) + "; ++d) pl" + sj + "[d] = s" + sj +
+         " + (i + d) % " + N(S) + " * " + N(plane_bytes(st) / st.esz) + " + w" + sj + ";\n";
+    cell += "          " + g + ".cx = x; " + g + ".cy = y; " + g + ".cz = z;\n"
+            "          for (int d = 0; d <= " + N(2 * st.rz) + "; ++d) " + g + ".c[d + " + N(4 - st.rz) +
+            "] = pl" + sj + "[d] + r * " + N(st.w) + ";\n";
+  }
+  for (size_t i = 0; i < k.params.size(); ++i) {
+    if (!k.params[i].grid) continue;
+    const JitParam &p = k.params[i];
+    const std::string si = N(i);
+    cell += "          g" + si + ".e = e" + si + (p.rank == 1 ? "" : " + r * a" + si + ".row") + ";\n";
+    if (p.rank == 3) advance += "    e" + si + " += a" + si + ".plane;\n";
+  }
+  const std::string rows = "#pragma unroll\n        for (int r = 0; r < " + N(kTileRows) + "; ++r) {\n"
+                           "          const int y = yb + r;\n";
+  s += "      if (inner && z > 0" + zin + ") {\n" + rows +
+       "          __builtin_assume(x > 0); __builtin_assume(y > 0); __builtin_assume(z > 0); " + assume +
+       "\n" + cell + "          " + call_source(k) + "        }\n      } else {\n" + rows +
+       "          if (x < dmin0 || x >= dmax0 || y >= dmax1) continue;\n" + cell + "          " +
+       call_source(k) + "        }\n      }\n    }\n"
+       "    __syncwarp();\n"
+       "    if (lane == 0) psg::mbar_arrive(&empty[i & 1]);\n" + advance + "  }\n}\n";
   return s;
 }
 
@@ -695,11 +779,11 @@ std::string tiled_entry_source(const JitKernel &k) {
 
 namespace {
 
-// PSGridEmitUtype(g.member, v) -> __PS_EMITU((g).p[(g).cur].member, v): the
+// PSGridEmitUtype(g.member, v) -> __PS_EMITU((g).e[0].member, v): the
 // member expression is applied to the point being computed.
 std::string rewrite_emit_utype(const std::string &src) {
   static const std::regex re("\\bPSGridEmitUtype\\s*\\(\\s*([A-Za-z_]\\w*)");
-  return std::regex_replace(src, re, "__PS_EMITU(($1).p[($1).cur]");
+  return std::regex_replace(src, re, "__PS_EMITU(($1).e[0]");
 }
 
 // One device global per user-type grid parameter holding its element size,
@@ -776,6 +860,9 @@ bool jit_build(const char *source, const char *name, JitKernel *k, std::vector<c
   return false;
 }
 
+// Dynamic shared memory of the tiled entry (with slack to align its base).
+static size_t stage_dynamic(const JitKernel &k) { return 128 + kStageHead + k.stage_smem; }
+
 bool jit_compile(const char *source, const char *name, JitKernel *k, std::string *err) {
   std::vector<char> image;
   if (!jit_build(source, name, k, &image, err) || !load_driver(err)) return false;
@@ -793,14 +880,15 @@ bool jit_compile(const char *source, const char *name, JitKernel *k, std::string
   if (!k->stages.empty()) {
     if (g_drv.get(&fn_t, mod, "__ps_entry_t") != CUDA_SUCCESS ||
         g_drv.set_attr(fn_t, CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES,
-                       (int)k->stage_smem) != CUDA_SUCCESS) {
+                       (int)stage_dynamic(*k)) != CUDA_SUCCESS) {
       fn_t = nullptr;
       k->stages.clear();
       k->stage_smem = 0;
     }
   }
   k->tiled_occ = 0;
-  if (fn_t && (g_drv.occupancy(&k->tiled_occ, fn_t, 256, k->stage_smem) != CUDA_SUCCESS ||
+  if (fn_t && (g_drv.occupancy(&k->tiled_occ, fn_t, kTileThreads, stage_dynamic(*k)) !=
+                   CUDA_SUCCESS ||
                k->tiled_occ < 1)) {
     k->tiled_occ = 0;
     fn_t = nullptr;
@@ -850,7 +938,7 @@ bool tiled_enabled() {
 // of a grid that the same launch writes would be stale); red/black maps and
 // everything else run the plain entry.
 cudaError_t jit_launch(const JitKernel &k, const Box &dom, int color, const GridView *grids,
-                       const double *scalars, int sm_count, cudaStream_t s) {
+                       const double *scalars, int sm_count, int *dev_err, cudaStream_t s) {
   const int nxd = dom.max[0] - dom.min[0], nyd = dom.max[1] - dom.min[1],
             nzd = dom.max[2] - dom.min[2];
   if (nxd <= 0 || nyd <= 0 || nzd <= 0) return cudaSuccess;
@@ -870,32 +958,23 @@ cudaError_t jit_launch(const JitKernel &k, const Box &dom, int color, const Grid
   if (tiled) {
     const long long ntx = (nxd + kTileX - 1) / kTileX, nty = (nyd + kTileY - 1) / kTileY;
     const long long tiles = ntx * nty;
-    // z chunks: the count whose waves of resident CTAs finish with the least
-    // idle time, counting each chunk's warm-up planes (2 rz + kAhead) as work
+    // z chunks: one wave of resident CTAs while chunks are short, else chunks
+    // of five planes (times the stencil's z radius): many small CTAs even out
+    // edge tiles and tails, and neighbouring chunks' halo planes come from L2
+    // (400 x 384 x 320, 7 points: 90 us a sweep with 5 planes, 98 with 36, 116
+    // with 32 -- a little over one wave -- and 146 with 64; a double 27-point sweep
+    // 686, 725, 776 and 1031 us for 5, 12, 32 and 64).
     const long long want = std::max(1LL, (long long)k.tiled_occ * sm_count);
-    int ovh = kAhead;
-    for (const JitStage &st : k.stages) ovh = std::max(ovh, 2 * st.rz + kAhead);
-    const long long c0 = std::max(1LL, (want + tiles - 1) / tiles);
-    const long long cmax = std::max(1LL, std::min(16 * c0, (long long)(nzd + 7) / 8));
-    long long chunks = 1;
-    int zlen = nzd;
-    double best = -1.0;
-    for (long long c = std::min(c0, cmax); c <= cmax; ++c) {
-      const int zl = (int)((nzd + c - 1) / c);
-      const long long cc = (nzd + zl - 1) / zl;
-      const long long waves = (tiles * cc + want - 1) / want;
-      const double eff = (double)tiles * nzd / ((double)want * waves * (zl + ovh));
-      if (eff > best + 1e-9) {
-        best = eff;
-        chunks = cc;
-        zlen = zl;
-      }
-    }
+    int rz = 1;
+    for (const JitStage &st : k.stages) rz = std::max(rz, st.rz);
+    const int zlen = (int)std::max({1LL, std::min((long long)nzd * tiles / want, 5LL * rz),
+                                    (nzd + 65534LL) / 65535});
+    const long long chunks = (nzd + zlen - 1) / zlen;
     if (tiles > 0x7fffffffLL || chunks > 65535) return cudaErrorInvalidConfiguration;
     gx = (unsigned)tiles;
     gy = (unsigned)chunks;
     gz = 1;
-    bx = 256;
+    bx = kTileThreads;
     by = 1;
     const int h[8] = {dom.min[0], dom.max[0], dom.min[1], dom.max[1],
                       dom.min[2], dom.max[2], (int)ntx, zlen};
@@ -920,7 +999,7 @@ cudaError_t jit_launch(const JitKernel &k, const Box &dom, int color, const Grid
   }
 
   // argument storage: 8 ints, then each parameter at its alignment
-  std::vector<unsigned char> buf(64 + 64 * k.params.size());
+  std::vector<unsigned char> buf(64 + 64 * k.params.size() + 16);
   std::vector<void *> args;
   size_t off = 0;
   auto put = [&](const void *v, size_t n, size_t align) {
@@ -930,6 +1009,18 @@ cudaError_t jit_launch(const JitKernel &k, const Box &dom, int color, const Grid
     off += n;
   };
   for (int v : head) put(&v, 4, 4);
+  std::vector<CUtensorMap> maps(tiled ? k.stages.size() : 0);
+  if (tiled) {
+    put(&dev_err, 8, 8);
+    for (size_t j = 0; j < maps.size(); ++j) {
+      const JitStage &st = k.stages[j];
+      int g = 0;
+      for (int i = 0; i < st.param; ++i) g += k.params[i].grid ? 1 : 0;
+      if (!make_tmap_3d(&maps[j], grids[g], st.w, kTileY + 2 * st.ry))
+        return cudaErrorInvalidValue;
+      args.push_back(&maps[j]);
+    }
+  }
   int gi = 0, si = 0;
   for (const JitParam &p : k.params) {
     if (p.grid) {
@@ -942,7 +1033,6 @@ cudaError_t jit_launch(const JitKernel &k, const Box &dom, int color, const Grid
       a.ny = g.ny;
       a.nz = g.nz;
       a.rank = p.rank;
-      a.cur = 0;
       put(&a, sizeof(a), 8);
     } else {
       const double v = scalars[si++];
@@ -955,7 +1045,7 @@ cudaError_t jit_launch(const JitKernel &k, const Box &dom, int color, const Grid
     }
   }
   const CUresult r = g_drv.launch(static_cast<CUfunction>(tiled ? k.func_tiled : k.func), gx,
-                                  gy, gz, bx, by, 1, tiled ? (unsigned)k.stage_smem : 0,
+                                  gy, gz, bx, by, 1, tiled ? (unsigned)stage_dynamic(k) : 0,
                                   static_cast<CUstream>(s), args.data(), nullptr);
   return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorLaunchFailure;
 }

@@ -174,13 +174,13 @@ struct JitParam {
   std::string utype;      // kUser grids: the element type (DeclareGrid's "struct Point")
   int esz = 0;            // kUser grids: its size in bytes (read from the module; 0 unknown)
 };
-// A grid the tiled entry stages in shared memory: planes of (64 + 2 rxw) x
-// (16 + 2 ry) cells around the CTA's tile (rxw: rx rounded up to 16 bytes),
-// a ring of 2 rz + 5 of them.
+// A grid the tiled entry stages in shared memory: planes of w x (16 + 2 ry)
+// cells around the CTA's 64 x 16 tile, starting on 16 bytes in x, a ring of
+// 2 rz + 2 of them.
 struct JitStage {
   int param;            // index into params
   int rx, ry, rz;       // halo widths the stencil's reads need
-  int rxw;              // x halo of the staged window
+  int w;                // width of the staged window
   bool periodic;        // halo cells wrap (else clamp to the grid)
   int esz;              // element size
   size_t off, bytes;    // byte range in dynamic shared memory
@@ -207,7 +207,7 @@ void jit_unload(JitKernel *k);
 // Runs the compiled stencil over dom (color -1 every point, 0 red, 1 black):
 // grids[] and scalars[] in parameter order.
 cudaError_t jit_launch(const JitKernel &k, const Box &dom, int color, const GridView *grids,
-                       const double *scalars, int sm_count, cudaStream_t s);
+                       const double *scalars, int sm_count, int *dev_err, cudaStream_t s);
 
 // Point stencils compiled per stencil (jit.cpp compiles points_body.cuh with
 // the table below as constants).  The key is everything the generated code

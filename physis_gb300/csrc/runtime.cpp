@@ -601,7 +601,7 @@ bool launch_function_map(const Map &m, const psg::JitKernel &f) {
   const int ncol = m.color == 2 ? 2 : 1;
   for (int c = 0; c < ncol; ++c) {
     cudaError_t e = psg::jit_launch(f, box, colors[c], views, m.scalars.data(), rt->sm_count,
-                                    rt->stream);
+                                    rt->dev_err, rt->stream);
     if (!cuda_ok(e, "stencil function launch")) return false;
     ++rt->launches;
   }

@@ -475,3 +475,89 @@ def test_benchmark_functions_match_oracle_and_builtin(rt, oracle):
     assert np.array_equal(_bits(b.copyout()), _bits(c.copyout()))
     for g in (a, b, c):
         g.free()
+
+
+def _sum_source(name, pts, ctype, gtype, periodic):
+    get = "PSGridGetPeriodic" if periodic else "PSGridGet"
+
+    def at(v, d):
+        return v if d == 0 else f"{v} {'+' if d > 0 else '-'} {abs(d)}"
+    terms = " + ".join(f"{get}(a, {at('x', p[0])}, {at('y', p[1])}, {at('z', p[2])})" for p in pts)
+    return (f"void {name}(const int x, const int y, const int z, PSGrid3D{gtype} a, "
+            f"PSGrid3D{gtype} b) {{\n  {ctype} v = {terms};\n  PSGridEmit(b, v);\n}}\n")
+
+
+# The sizes where the tiled entry can go wrong: domains that start off a
+# 16-byte boundary, one-cell remainders of the tile in x and y, chunks of one
+# plane, halos up to 4 in one axis and none in another, windows that cross the
+# grid on every side, wrapped halos, and each element type.  Sums in the given
+# order, so the oracle's bits.
+@pytest.mark.parametrize("shape,dtype,periodic,radius,lo", [
+    ((9, 17, 65), np.float32, False, (1, 1, 1), (1, 1, 1)),
+    ((7, 34, 131), np.float32, False, (4, 1, 2), (5, 3, 2)),
+    ((12, 16, 64), np.float32, True, (1, 1, 1), (0, 0, 0)),
+    ((5, 19, 70), np.float64, True, (3, 4, 2), (0, 0, 0)),
+    ((3, 50, 129), np.float64, False, (1, 0, 1), (3, 7, 1)),
+    ((2, 5, 9), np.int32, True, (2, 2, 1), (0, 0, 0)),
+    ((40, 33, 67), np.int64, False, (2, 3, 0), (2, 4, 1)),
+    ((60, 15, 200), np.float32, True, (0, 2, 4), (0, 0, 0))])
+def test_function_tiles_and_edges_bit_exact(rt, oracle, shape, dtype, periodic, radius, lo):
+    nz, ny, nx = shape
+    names = {np.float32: ("float", "Float"), np.float64: ("double", "Double"),
+             np.int32: ("int", "Int"), np.int64: ("long long", "Long")}
+    rng = np.random.default_rng(51)
+    pts = [(0, 0, 0)] + [tuple(int(rng.integers(-r, r + 1)) for r in radius) for _ in range(9)]
+    pts += [tuple(radius), tuple(-r for r in radius)]
+    src = (rng.integers(-1000, 1000, size=shape) if np.issubdtype(dtype, np.integer)
+           else rng.uniform(-1, 1, size=shape)).astype(dtype)
+    out0 = src[::-1].copy()
+    dom = ((0, nx, 0, ny, 0, nz) if periodic else
+           tuple(v for n, r, a in zip((nx, ny, nz), radius, lo) for v in (max(a, r), n - r)))
+    ref = out0.copy()
+    oracle.points(src, ref, dom, pts, boundary=1 if periodic else 0)
+    name = "s_" + "_".join(str(v) for v in shape)
+    k = ps.stencil_function(_sum_source(name, pts, *names[dtype], periodic), name)
+    a, b = _grid(src), _grid(out0)
+    _run(k, ps.domain(*dom), [a, b])
+    assert np.array_equal(_bits(b.copyout()), _bits(ref))
+    a.free()
+    b.free()
+
+
+TWO_STAGED = r"""
+void two(const int x, const int y, const int z, PSGrid3DFloat a, PSGrid3DDouble k,
+         PSGrid3DFloat out, PSGrid2DFloat m) {
+  int nx = PSGridDim(a, 0), ny = PSGridDim(a, 1), nz = PSGridDim(a, 2);
+  float c = PSGridGet(a, x, y, z);
+  float w = x > 0 ? PSGridGet(a, x - 1, y, z) : c;
+  float e = x + 1 < nx ? PSGridGet(a, x + 1, y, z) : c;
+  float n = y >= 1 ? PSGridGet(a, x, y - 1, z) : c;
+  float s = y <= ny - 2 ? PSGridGet(a, x, y + 1, z) : c;
+  float b = z == 0 ? c : PSGridGet(a, x, y, z - 1);
+  float t = z == nz - 1 ? c : PSGridGet(a, x, y, z + 1);
+  double q = PSGridGetPeriodic(k, x, y - 2, z) + PSGridGetPeriodic(k, x + 2, y, z)
+      + PSGridGetPeriodic(k, x, y, z + 2);
+  if (x != 5) PSGridEmit(out, (float)(q * (double)(w + e + n + s + b + t)) + PSGridGet(m, x, y));
+}
+"""
+
+
+def test_function_with_two_staged_grids_and_its_own_faces(rt, monkeypatch):
+    # two staged grids of different types, radii and boundary rules, faces the
+    # function treats itself in several spellings, a conditional emit and a 2D
+    # grid: the tiled entry's bits against the plain entry's
+    shape = (11, 37, 150)
+    rng = np.random.default_rng(52)
+    arrays = [rng.uniform(-1, 1, size=shape).astype(t) for t in (np.float32, np.float64, np.float32)]
+    m = rng.uniform(-1, 1, size=shape[1:]).astype(np.float32)
+    k = ps.stencil_function(TWO_STAGED, "two")
+    got = {}
+    for tiled in ("1", "0"):
+        monkeypatch.setenv("PS_FUNCTION_TILED", tiled)
+        gs = [_grid(v) for v in arrays] + [_grid(m)]
+        _run(k, ps.domain(0, 150, 1, 37, 0, 11), gs)
+        got[tiled] = gs[2].copyout()
+        for g in gs:
+            g.free()
+    assert np.array_equal(_bits(got["1"]), _bits(got["0"]))
+    assert not np.array_equal(got["1"], arrays[2])

@@ -30,7 +30,9 @@ def _p(t):
 
 
 def _stream():
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    # PyTorch's default stream is handle 0, which the library takes for its own
+    # stream; 1 is CUDA's name for the default stream (cudaStreamLegacy)
+    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream or 1)
 
 
 # FP32 sums of n products of O(1) BF16 values, added in runs of 16 (a tensor
