@@ -12,7 +12,7 @@
 // accumulates 27 taps x 2 n-tiles) when PS_WARMSTART_TC=0 asks for it.  The
 // backward-data pass is the same kernel with the weights flipped in space and
 // transposed in channels; the weight gradient is a K = voxels GEMM per tap
-// (wgrad_pad_kernel; wgrad_kernel where a slab does not fit), split over CTAs
+// (wgrad_run_kernel; wgrad_kernel for unaligned tensors), split over CTAs
 // and reduced in a fixed order (deterministic).
 // Pooling (fine grids -> coarse network input), the MSE gradient, Adam and
 // cubic upsampling (coarse prediction -> fine warm start) complete the
@@ -525,48 +525,50 @@ conv_pad_kernel(const __grid_constant__ CUtensorMap tmx, const __nv_bfloat16 *__
   }
 }
 
-// ---- weight gradient over padded slabs -------------------------------------------
+// ---- weight gradient -----------------------------------------------------------
 //
 // dW[t][in][out] = sum over voxels v of X[v + d_t][in] * dY[v][out]: a GEMM
 // per tap with M = N = 16 and K = voxels.  M = 16 is below tcgen05's smallest
-// tile, so the products run on mma.sync.m16n8k16.  X and dY are staged as
-// padded slabs (two stages, so the next slab loads while this one is used);
-// padding contributes zeros.  Warp w owns the three x taps of its (z, y)
-// offset for every voxel of the CTA, so nothing is summed across warps: per 16
-// voxels it reads dY's fragment and three of X (ldmatrix.trans turns
-// [voxel][channel] rows into K = voxel fragments; eight 16-byte rows of a half
-// plane are 128 contiguous bytes, no bank conflicts) and issues six products.
-// The CTAs of a split form a cluster that adds its sums through distributed
-// shared memory in rank order, so the caller's work buffer holds nsplit
-// partials whatever the number of CTAs and results repeat bit for bit.
-// Bound: 54 products per 16 padded voxels on the mma.sync pipe (about 10
-// cycles each per sub-partition: 62 us of the case below); shared memory hands
-// out 36 ldmatrix tiles of 512 B for them (144 cycles, 54 us).  Measured on
-// 1024 x 17 x 9 x 9 voxels, nsplit 64: 137 us against 1760 us of wgrad_kernel
-// (2-byte gathers from L2 for each tap); on 32 instances 12.3 against 60 us.
-// What is left is balance: nine warps on four sub-partitions, 2.5 CTAs per SM.
-constexpr int kPwWarps = 9;   // one per (z, y) tap offset
-constexpr int kPwThreads = 32 * kPwWarps;
-constexpr int kPwMaxCluster = 8;
-constexpr size_t kPwSmem = 74 * 1024;   // three CTAs per SM
-constexpr size_t kPwMaxSmem = 200 * 1024;
-constexpr int kPwSums = kTaps * kC * kC + kPwWarps * kC;
+// tile, so the products run on mma.sync.m16n8k16.
+//
+// CTAs (g, s) make the nine taps of z offset g - 1 for split s.  Split s takes
+// every S-th run of 128 voxels; its warp w the w-th 16 of each run, in ascending
+// order, so each FP32 accumulator sees the products in the order that
+// wgrad_kernel gives them, and the results are the same bits (a training run is
+// sensitive to the last one: it decides BF16 roundings of the weights).  X rows
+// of a run and of its y and x neighbours are one contiguous stretch of memory
+// (three, one per y offset, where rows of the grid are longer than a run); they
+// and the run's dY rows arrive by cp.async, three runs ahead.  They sit in two
+// planes of 8-channel halves, so the eight 16-byte rows of an ldmatrix phase
+// are 128 contiguous bytes (no bank conflicts); ldmatrix.trans turns
+// [voxel][channel] rows into K = voxel fragments.  A lane follows the
+// coordinates of the voxel whose row it hands to ldmatrix, and hands it a row
+// of zeros where the tap leaves the grid.
+// Bound: 54 products per 16 voxels, about 10 cycles each on a sub-partition's
+// mma.sync pipe (40 us of the case below were the CTAs even over the SMs).
+// Measured, 1024 x 17 x 9 x 9 voxels, 64 splits: 135 us (167 with eight-warp
+// CTAs; wgrad_kernel, two-byte gathers from L2 for every tap, 1760); 32
+// instances 13 us (60).
+// A split's eight warps are two CTAs of four (a cluster, whose sums are added
+// through distributed shared memory): 384 of them even out better over the SMs
+// than 192 of eight.
+constexpr int kWgHalves = 2;
+constexpr int kWgWarps = kConvWarps / kWgHalves;
+constexpr int kWgThreads = 32 * kWgWarps;
+constexpr int kWgRun = 16 * kWgWarps;     // voxels of a CTA's half run
+constexpr int kWgStages = 4;
 
-// Half planes of X (zs + 2 planes) and dY (zs planes); a last chunk of 16
-// voxels may read past the planes (zeroed once, never written again).
-__host__ __device__ constexpr int pw_half_x(int zs, int P, int px, int pre) {
-  return pre + (((zs + 2) * P + 16 + px + 1) * 16 + 127) / 128 * 128;
+// Staging of a run's X rows: `segs` stretches of `len` rows, a tap's y offset
+// being `pitch` staged rows.
+struct WgRows {
+  int segs, len, pitch;
+};
+__host__ __device__ inline WgRows wg_rows(int X) {
+  const int run = kWgRun + 2;
+  return X <= run ? WgRows{1, run + 2 * X, X} : WgRows{3, run, run};
 }
-__host__ __device__ constexpr int pw_half_y(int zs, int P) {
-  return ((zs * P + 16) * 16 + 127) / 128 * 128;
-}
-__host__ __device__ constexpr int pw_stage(int zs, int P, int px, int pre) {
-  return 2 * (pw_half_x(zs, P, px, pre) + pw_half_y(zs, P));
-}
-size_t pw_smem(const PadGeom &g) {
-  const size_t n = 128 + 128 + 2 * (size_t)pw_stage(g.zs, g.P, g.px, g.pre);
-  const size_t sums = 128 + 128 + (size_t)kPwSums * 4;  // reuses the stages
-  return n < sums ? sums : n;
+__host__ __device__ inline int wg_stage_bytes(const WgRows &r) {
+  return (r.segs * r.len + kWgRun) * 32;
 }
 
 __device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], uint32_t addr) {
@@ -576,129 +578,204 @@ __device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], uint32_t add
                : "memory");
 }
 
-__global__ void __launch_bounds__(kPwThreads, 3)
-wgrad_pad_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant__ CUtensorMap tmy,
-                 float *__restrict__ part, float *__restrict__ bpart, Dims d, PadGeom g, int items,
-                 int *err) {
-  namespace cg = cooperative_groups;
-  extern __shared__ __align__(128) unsigned char pw_raw[];
+__device__ __forceinline__ void cp_async16_to(uint32_t dst, const void *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst),
+               "l"(__cvta_generic_to_global(src))
+               : "memory");
+}
+
+__global__ void __cluster_dims__(kWgHalves, 1, 1) __launch_bounds__(kWgThreads, 4)
+wgrad_run_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restrict__ dy,
+                 float *__restrict__ part, float *__restrict__ bpart, Dims d, WgRows rows) {
+  extern __shared__ __align__(128) unsigned char wg_smem[];
+  __shared__ float bred[kWgWarps][kC];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  // the same offset in every CTA of the cluster
-  unsigned char *smem = pw_raw + ((128u - (smem_u32(pw_raw) & 127u)) & 127u);
-  unsigned long long *bars = reinterpret_cast<unsigned long long *>(smem);
-  unsigned char *stage0 = smem + 128;
-  const int hx = pw_half_x(g.zs, g.P, g.px, g.pre), hy = pw_half_y(g.zs, g.P);
-  const int sbytes = 2 * (hx + hy);
-  const int rank = blockIdx.x, s = blockIdx.y, C = gridDim.x;
-  const int cta = s * C + rank, nctas = C * gridDim.y;
+  const int g = blockIdx.x / kWgHalves, half = blockIdx.x % kWgHalves;
+  const int s = blockIdx.y, S = gridDim.y;
+  const int dz = g - 1;
+  const long long YX = (long long)d.Y * d.X;
+  constexpr int kFull = kWgHalves * kWgRun;
+  const long long runs = (d.nvox + kFull - 1) / kFull;
+  const int n = s < runs ? (int)((runs - s + S - 1) / S) : 0;  // this split's runs
+  const int XR = rows.segs * rows.len;                          // staged X rows
+  const uint32_t sbytes = wg_stage_bytes(rows);
+  const uint32_t zero_row = smem_u32(wg_smem), sm0 = zero_row + 16;
+  if (tid < 4) reinterpret_cast<uint32_t *>(wg_smem)[tid] = 0u;
 
-  for (int i = tid; i < 2 * sbytes / 16; i += kPwThreads)
-    reinterpret_cast<uint4 *>(stage0)[i] = make_uint4(0u, 0u, 0u, 0u);
-  if (tid == 0) {
-    mbar_init(&bars[0], 1);
-    mbar_init(&bars[1], 1);
-    fence_barrier_init();
-  }
-  // the zeros before the TMA boxes that overwrite most of them
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-  __syncthreads();
-
-  auto issue = [&](int item, int st) {
-    const int b = item / g.nslab, z0 = (item - b * g.nslab) * g.zs;
-    const uint32_t base = smem_u32(stage0) + st * sbytes, bar = smem_u32(&bars[st]);
-    mbar_arrive_expect_tx(&bars[st], 2u * (unsigned)((2 * g.zs + 2) * g.P * 16));
-    for (int h = 0; h < 2; ++h) {
-      tma_load_5d(base + h * hx + g.pre, &tmx, 8 * h, 0, 0, z0 - 1, b, bar);
-      tma_load_5d(base + 2 * hx + h * hy, &tmy, 8 * h, 0, 0, z0, b, bar);
+  // Staging: 16-byte unit i of a stretch is half i & 1 of row i >> 1.  Rows
+  // outside the tensor are left alone (no lane reads them).
+  const uint32_t xdst = ((tid & 1) * XR + (tid >> 1)) * 16;
+  const uint32_t ydst = XR * 32 + ((tid & 1) * kWgRun + (tid >> 1)) * 16;
+  const long long hop = (long long)S * kFull;  // voxels from one run to the next
+  const long long v_first = (long long)s * kFull + half * kWgRun;
+  long long v_next = v_first;  // first voxel of the next run to stage
+  const char *ysrc = reinterpret_cast<const char *>(dy) + v_next * 32 + tid * 16;
+  long long x_next = v_next + dz * YX - d.X - 1;  // its first X row
+  const char *xsrc = reinterpret_cast<const char *>(x) + x_next * 32 + tid * 16;
+  auto load = [&](int stage) {
+    uint32_t dst = sm0 + stage * sbytes;
+    const bool whole = x_next >= 0 && v_next + kWgRun <= d.nvox &&
+                       x_next + (long long)(rows.segs - 1) * d.X + rows.len <= d.nvox;
+    if (whole || v_next + (tid >> 1) < d.nvox) cp_async16_to(dst + ydst, ysrc);
+    dst += xdst;
+    const char *src = xsrc;
+    if (whole) {
+      // 132 units or more: one per thread, one more for some, rarely others
+      const int units = 2 * rows.len;
+      for (int sg = 0; sg < rows.segs; ++sg) {
+        cp_async16_to(dst, src);
+        if (tid + kWgThreads < units) cp_async16_to(dst + kWgThreads * 8, src + kWgThreads * 16);
+#pragma unroll 1
+        for (int i = tid + 2 * kWgThreads; i < units; i += kWgThreads)
+          cp_async16_to(dst + (i - tid) * 8, src + (i - tid) * 16);
+        dst += rows.len * 16;
+        src += (long long)d.X * 32;
+      }
+    } else {
+      long long row = x_next;
+#pragma unroll 1
+      for (int sg = 0; sg < rows.segs; ++sg) {
+#pragma unroll 1
+        for (int i = tid; i < 2 * rows.len; i += kWgThreads) {
+          const long long k = row + (i >> 1);
+          if (k >= 0 && k < d.nvox) cp_async16_to(dst + (i - tid) * 8, src + (i - tid) * 16);
+        }
+        dst += rows.len * 16;
+        src += (long long)d.X * 32;
+        row += d.X;
+      }
     }
+    v_next += hop;
+    x_next += hop;
+    ysrc += hop * 32;
+    xsrc += hop * 32;
   };
-  if (tid == 0) {
-    if (cta < items) issue(cta, 0);
-    if (cta + nctas < items) issue(cta + nctas, 1);
-  }
 
-  float acc[3][2][4] = {};
-  float bacc[2][4] = {};  // ones x dY: this warp's share of the bias gradient
-  const uint32_t ones[4] = {0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u};
-  // this lane's row of an ldmatrix.x4: voxel lv of the chunk, channel half lh
+  // This lane's row of an ldmatrix.x4: voxel lv of its warp's 16, channel half
+  // lh.  Coordinates of that voxel, advanced by S runs at a time.
   const int lv = (lane & 7) + ((lane >> 4) << 3), lh = (lane >> 3) & 1;
-  const uint32_t xl = lh * hx + g.pre +
-                      (lv + (warp / 3) * g.P + (warp % 3 - 1) * g.px - 1) * 16;
-  const uint32_t yl = 2 * hx + lh * hy + lv * 16;
-  const int chunks = (g.zs * g.P + 15) / 16;
+  long long v = v_first + warp * 16 + lv;
+  int cx, cy, cz;
+  {
+    const long long q = v / d.X;
+    cx = (int)(v - q * d.X);
+    cy = (int)(q % d.Y);
+    cz = (int)((q / d.Y) % d.Z);
+  }
+  const int sx = (int)(hop % d.X), sy = (int)((hop / d.X) % d.Y), sz = (int)((hop / YX) % d.Z);
+  const uint32_t xrow = (lh * XR + warp * 16 + lv) * 16;
+  const uint32_t yrow = XR * 32 + (lh * kWgRun + warp * 16 + lv) * 16;
+  const uint32_t ypitch = rows.pitch * 16;
 
-  int st = 0;
-  uint32_t phase = 0;
-  bool ok = true;
-  for (int item = cta; item < items; item += nctas) {
-    if (!mbar_wait(&bars[st], phase, err)) ok = false;
-    uint32_t xa = smem_u32(stage0) + st * sbytes + xl;
-    uint32_t ya = smem_u32(stage0) + st * sbytes + yl;
-    int bias = warp + 1;
-#pragma unroll 4
-    for (int c = 0; c < chunks; ++c) {
-      uint32_t b[4], a[3][4];
-      ldmatrix_x4_trans(b, ya);
+  float acc[9][2][4] = {};
+  float bsum0 = 0.f, bsum1 = 0.f;
 #pragma unroll
-      for (int k = 0; k < 3; ++k) ldmatrix_x4_trans(a[k], xa + k * 16);
+  for (int t = 0; t < kWgStages - 1; ++t) {
+    if (t < n) load(t);
+    cp_async_commit();
+  }
+  int stage = 0, fill = kWgStages - 1;
+  for (int t = 0; t < n; ++t) {
+    cp_async_wait<kWgStages - 2>();
+    __syncthreads();  // the run has landed; the stage read a run ago is free
+    if (t + kWgStages - 1 < n) load(fill);
+    cp_async_commit();
+    if (++fill == kWgStages) fill = 0;
+    const uint32_t st = sm0 + stage * sbytes;
+    if (++stage == kWgStages) stage = 0;
+
+    const bool in = v < d.nvox;
+    const bool z = in && (unsigned)(cz + dz) < (unsigned)d.Z;
+    const bool yok[3] = {z && cy > 0, z, z && cy < d.Y - 1};
+    const bool xok[3] = {cx > 0, true, cx < d.X - 1};
+    uint32_t b[4];
+    ldmatrix_x4_trans(b, in ? st + yrow : zero_row);
+    uint32_t xa = st + xrow;
+#pragma unroll
+    for (int ky = 0; ky < 3; ++ky) {
+      uint32_t a[3][4];
+#pragma unroll
+      for (int k = 0; k < 3; ++k)
+        ldmatrix_x4_trans(a[k], yok[ky] && xok[k] ? xa + 16 * k : zero_row);
 #pragma unroll
       for (int k = 0; k < 3; ++k) {
-        mma_16816(acc[k][0], a[k], b[0], b[2]);
-        mma_16816(acc[k][1], a[k], b[1], b[3]);
+        mma_16816(acc[ky * 3 + k][0], a[k], b[0], b[2]);
+        mma_16816(acc[ky * 3 + k][1], a[k], b[1], b[3]);
       }
-      if (--bias == 0) {  // every ninth chunk: the warps share dY's sums evenly
-        bias = kPwWarps;
-        mma_16816(bacc[0], ones, b[0], b[2]);
-        mma_16816(bacc[1], ones, b[1], b[3]);
-      }
-      xa += 256;
-      ya += 256;
+      xa += ypitch;
     }
-    ok = __syncthreads_and(ok);  // every warp is done with the stage
-    if (!ok) break;
-    if (tid == 0 && item + 2 * nctas < items) issue(item + 2 * nctas, st);
-    if ((st ^= 1) == 0) phase ^= 1u;
+    if (g == 1) {
+      const uint32_t bb[4] = {b[0], b[2], b[1], b[3]};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float lo = __uint_as_float(bb[i] << 16), hi = __uint_as_float(bb[i] & 0xffff0000u);
+        if (i < 2) bsum0 += lo + hi;
+        else bsum1 += lo + hi;
+      }
+    }
+    v += hop;
+    cx += sx;
+    cy += sy;
+    cz += sz;
+    if (cx >= d.X) {
+      cx -= d.X;
+      ++cy;
+    }
+    if (cy >= d.Y) {
+      cy -= d.Y;
+      ++cz;
+    }
+    if (cz >= d.Z) cz -= d.Z;
   }
-  if (!ok && tid == 0) {
-    // give copies still in flight a bounded chance to land
-    for (int i = 0; i < 2; ++i)
-      for (uint32_t q = 0; q < 2; ++q) mbar_wait(&bars[i], q, nullptr, 1024);
-  }
-  __syncthreads();
+  cp_async_wait<0>();  // only empty groups can remain
 
-  float *sums = reinterpret_cast<float *>(stage0);
-  const int gq = lane >> 2, q = lane & 3;
-#pragma unroll
-  for (int k = 0; k < 3; ++k)
-#pragma unroll
-    for (int n = 0; n < 2; ++n)
-#pragma unroll
-      for (int i = 0; i < 2; ++i)
-        *reinterpret_cast<float2 *>(sums + (warp * 3 + k) * kC * kC + (gq + i * 8) * kC + n * 8 +
-                                    2 * q) = make_float2(acc[k][n][2 * i], acc[k][n][2 * i + 1]);
-  if (gq == 0) {
-#pragma unroll
-    for (int n = 0; n < 2; ++n)
-      *reinterpret_cast<float2 *>(sums + kTaps * kC * kC + warp * kC + n * 8 + 2 * q) =
-          make_float2(bacc[n][0], bacc[n][1]);
-  }
+  // warps' sums, added in warp order over the cluster, three taps at a time
+  namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
-  cl.sync();
-  const int n = kTaps * kC * kC;
-  for (int i = tid + rank * kPwThreads; i < n + kC; i += C * kPwThreads) {
-    float v = 0.f;
-    if (i < n) {
-      for (int r = 0; r < C; ++r) v += cl.map_shared_rank(sums, r)[i];
-      part[(long long)s * n + i] = v;
-    } else {
-      for (int r = 0; r < C; ++r) {
-        const float *p = cl.map_shared_rank(sums, r);
-        for (int k = 0; k < kPwWarps; ++k) v += p[i + k * kC];
-      }
-      bpart[s * kC + (i - n)] = v;
-    }
+  float *red = reinterpret_cast<float *>(wg_smem);
+  constexpr int kSums = 3 * kC * kC;
+  const int gq = lane >> 2, q = lane & 3;
+  bsum0 += __shfl_xor_sync(0xffffffffu, bsum0, 1);
+  bsum0 += __shfl_xor_sync(0xffffffffu, bsum0, 2);
+  bsum1 += __shfl_xor_sync(0xffffffffu, bsum1, 1);
+  bsum1 += __shfl_xor_sync(0xffffffffu, bsum1, 2);
+  if (q == 0) {
+    bred[warp][gq] = bsum0;
+    bred[warp][gq + 8] = bsum1;
   }
-  cl.sync();  // no CTA leaves while its sums are still being read
+#pragma unroll
+  for (int ky = 0; ky < 3; ++ky) {
+    if (ky == 0) __syncthreads();  // the stages are free
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+#pragma unroll
+      for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+          *reinterpret_cast<float2 *>(red + warp * kSums + k * kC * kC + (gq + i * 8) * kC +
+                                      m * 8 + 2 * q) =
+              make_float2(acc[ky * 3 + k][m][2 * i], acc[ky * 3 + k][m][2 * i + 1]);
+    cl.sync();
+    for (int i = tid + half * kWgThreads; i < kSums; i += kWgHalves * kWgThreads) {
+      float f = 0.f;
+#pragma unroll
+      for (int r = 0; r < kWgHalves; ++r) {
+        const float *from = cl.map_shared_rank(red, r);
+#pragma unroll
+        for (int w = 0; w < kWgWarps; ++w) f += from[w * kSums + i];
+      }
+      part[((long long)s * kTaps + g * 9 + ky * 3) * kC * kC + i] = f;
+    }
+    if (ky == 0 && g == 1 && half == 0 && tid < kC) {
+      float f = 0.f;
+      for (int r = 0; r < kWgHalves; ++r) {
+        const float *from = cl.map_shared_rank(&bred[0][0], r);
+        for (int w = 0; w < kWgWarps; ++w) f += from[w * kC + tid];
+      }
+      bpart[s * kC + tid] = f;
+    }
+    cl.sync();  // read before it is overwritten, or the CTA leaves
+  }
 }
 
 // Partial weight gradients: block (t, s) sums over the s-th share of the
@@ -775,30 +852,44 @@ wgrad_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restric
   }
 }
 
-// Sums the splits' partials in a fixed order: eight lanes per gradient, each
-// over every eighth split, then a shuffle tree (a thread per gradient walking
-// 64 partials one after the other took 5.1 us, latency-bound).
+// Sums the splits' partials in split order: 64 gradients per CTA, four threads
+// fetching each one's partials of 64 splits, one adding them (one thread
+// walking through memory took 5.1 us for 64 splits).
 __global__ void __launch_bounds__(256)
 wgrad_reduce_kernel(const float *__restrict__ part, const float *__restrict__ bpart, int S,
                     float *__restrict__ dw, float *__restrict__ db) {
-  // a warp holds four gradients' worth of lanes: neighbouring lanes read
-  // neighbouring gradients of the same split
-  const int lane = threadIdx.x & 31;
-  const int i = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 4 + (lane & 3);
-  const int k = lane >> 2;
+  __shared__ float buf[64][65];
+  const int c = threadIdx.x & 63, k = threadIdx.x >> 6;
+  const int i = blockIdx.x * 64 + c;
   const int n = kTaps * kC * kC;
+  const bool on = i < n || (i < n + kC && db);
+  const float *src = i < n ? part + i : bpart + (i - n);
+  const int step = i < n ? n : kC;
   float v = 0.f;
-  if (i < n) {
-    for (int s = k; s < S; s += 8) v += part[(long long)s * n + i];
-  } else if (i < n + kC && db) {
-    for (int s = k; s < S; s += 8) v += bpart[s * kC + (i - n)];
-  }
+  for (int s0 = 0; s0 < S; s0 += 64) {
+    float u[16];
 #pragma unroll
-  for (int o = 4; o < 32; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  if (k == 0) {
-    if (i < n) dw[i] = v;
-    else if (i < n + kC && db) db[i - n] = v;
+    for (int j = 0; j < 16; ++j) {
+      const int s = s0 + k * 16 + j;
+      u[j] = on && s < S ? src[(long long)s * step] : 0.f;
+    }
+#pragma unroll
+    for (int j = 0; j < 16; ++j) buf[k * 16 + j][c] = u[j];
+    __syncthreads();
+    if (on && k == 0) {
+      const int m = min(64, S - s0);
+      if (m == 64) {
+#pragma unroll
+        for (int j = 0; j < 64; ++j) v += buf[j][c];
+      } else {
+        for (int j = 0; j < m; ++j) v += buf[j][c];
+      }
+    }
+    __syncthreads();
   }
+  if (!on || k) return;
+  if (i < n) dw[i] = v;
+  else db[i - n] = v;
 }
 
 // FP32 master [27][in][out] -> BF16 forward [27][out][in] and backward-data
@@ -1250,70 +1341,28 @@ int nn_conv(const void *x, const void *w, const float *bias, const void *mask, i
   return (int)cudaGetLastError();
 }
 
-// wgrad_pad_kernel over slabs, or false if the planes are too large to stage
-// or the tensors not aligned for TMA.
-static bool launch_wgrad_pad(const void *x, const void *dy, float *part, float *bpart, int S,
-                             const Dims &d, cudaStream_t s, cudaError_t *e) {
-  if (d.X > 255 || d.Y > 255 || !aligned16(x) || !aligned16(dy)) return false;
-  const int sms = sm_count();
-  PadGeom g = pad_geom(d, 1, 1);
-  int zmax = 0;  // most planes per slab with three CTAs per SM, else with one
-  for (size_t limit : {kPwSmem, kPwMaxSmem}) {
-    for (int z = 1; z <= d.Z && z <= 254; ++z) {
-      g.zs = z;
-      if (pw_smem(g) > limit) break;
-      zmax = z;
-    }
-    if (zmax) break;
-  }
-  if (!zmax) return false;
-  g = pad_geom(d, zmax, 3LL * sms);
-  const long long items = (long long)d.B * g.nslab;
-  if (items > 0x3fffffff) return false;
-  CUtensorMap tmx, tmy;
-  if (!tmap_slab(&tmx, x, d, g.px, d.Y + 1, g.zs + 2) ||
-      !tmap_slab(&tmy, dy, d, g.px, d.Y + 1, g.zs))
-    return false;
-  // CTAs per split: up to 2.6 per SM in all.  Three fit, but a cluster's CTAs
-  // stay within one GPC, and 64 clusters of 7 (2.95 per SM) did not all find
-  // room at once: the last few ran alone (147 us, against 137 us with 6).
-  long long c = 26LL * sms / (10LL * S);
-  if (c > (items + S - 1) / S) c = (items + S - 1) / S;
-  if (c > kPwMaxCluster) c = kPwMaxCluster;
-  if (c < 1) c = 1;
-  const size_t smem = pw_smem(g);
-  *e = cudaFuncSetAttribute(wgrad_pad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                            (int)smem);
-  if (*e != cudaSuccess) return true;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)c, (unsigned)S);
-  cfg.blockDim = dim3(kPwThreads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = (unsigned)c;
-  at[0].val.clusterDim.y = 1;
-  at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  *e = cudaLaunchKernelEx(&cfg, wgrad_pad_kernel, tmx, tmy, part, bpart, d, g, (int)items, g_err);
-  return true;
-}
-
 int nn_wgrad(const void *x, const void *dy, float *part, int S, float *dw, float *db, int B,
              int Z, int Y, int X, cudaStream_t s) {
   Dims d{B, Z, Y, X, (long long)B * Z * Y * X};
   if (S < 1) return -1;
   float *bpart = part + (long long)S * kTaps * kC * kC;
-  cudaError_t e = cudaSuccess;
-  if (!launch_wgrad_pad(x, dy, part, bpart, S, d, s, &e))
-    wgrad_kernel<<<dim3(kTaps, S), 32 * kConvWarps, 0, s>>>(
-        static_cast<const __nv_bfloat16 *>(x), static_cast<const __nv_bfloat16 *>(dy), part, bpart,
-        d);
-  if (e != cudaSuccess) return (int)e;
+  const __nv_bfloat16 *xb = static_cast<const __nv_bfloat16 *>(x);
+  const __nv_bfloat16 *yb = static_cast<const __nv_bfloat16 *>(dy);
+  // wgrad_kernel's two-byte loads take any pointer, cp.async 16-byte ones
+  if (aligned16(x) && aligned16(dy)) {
+    const WgRows rows = wg_rows(X);
+    const int stages = 16 + kWgStages * wg_stage_bytes(rows);
+    const int sums = kWgWarps * 3 * kC * kC * 4;
+    const int smem = stages > sums ? stages : sums;
+    const cudaError_t e = cudaFuncSetAttribute(
+        wgrad_run_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return (int)e;
+    wgrad_run_kernel<<<dim3(3 * kWgHalves, S), kWgThreads, smem, s>>>(xb, yb, part, bpart, d, rows);
+  } else {
+    wgrad_kernel<<<dim3(kTaps, S), 32 * kConvWarps, 0, s>>>(xb, yb, part, bpart, d);
+  }
   const int n = kTaps * kC * kC + kC;
-  wgrad_reduce_kernel<<<(n + 31) / 32, 256, 0, s>>>(part, bpart, S, dw, db);
+  wgrad_reduce_kernel<<<(n + 63) / 64, 256, 0, s>>>(part, bpart, S, dw, db);
   return (int)cudaGetLastError();
 }
 

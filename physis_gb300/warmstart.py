@@ -302,7 +302,7 @@ class Net:
         self.prepare()
 
     def stream(self):
-        return ctypes.c_void_p(self.torch.cuda.current_stream().cuda_stream)
+        return _stream()
 
     def prepare(self):
         L, stream = ps.lib(), self.stream()
@@ -351,6 +351,14 @@ class Net:
                                            self.stream()))
 
 
+def _stream():
+    """PyTorch's current stream for the C API.  Its default stream has handle
+    0, which the library takes for its own stream (nothing orders the two); 1
+    is CUDA's name for the default stream (cudaStreamLegacy)."""
+    import torch
+    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream or 1)
+
+
 def _p(t):
     return None if t is None else ctypes.c_void_p(t.data_ptr())
 
@@ -366,8 +374,7 @@ def loss_grad(pred, target, work64):
     import torch
     n = pred.numel()
     dy = torch.empty(n * C, dtype=torch.bfloat16, device="cuda")
-    _ok(ps.lib().PSWarmStartLoss(_p(pred), _p(target), n, _p(dy), _p(work64),
-                                 ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    _ok(ps.lib().PSWarmStartLoss(_p(pred), _p(target), n, _p(dy), _p(work64), _stream()))
     nb = (n + 255) // 256
     return float(work64[:nb].cpu().numpy().sum()) / n, dy
 
@@ -539,6 +546,7 @@ def predict_into(net, stack, data_scales, factor, mirrors=1, restarts=0, nu=0,
     itself, the last approach runs like a zero start's, which ends at a
     fixed point."""
     import torch
+    ps.synchronize()  # sweeps still running on the library's stream
     wscale, pscale = data_scales
     zc, yc, xc = coarse_shape(stack.shape, factor)
     n = stack.count

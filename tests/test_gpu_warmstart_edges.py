@@ -128,3 +128,25 @@ def test_adam_layers_matches_single_calls(rt, layers):
                                                                            atol=0)
     assert (w - w2).abs().max() <= 2 ** -22 * w2.abs().max()
     assert torch.equal(half.view(torch.int16), half2.view(torch.int16))
+
+
+@pytest.mark.parametrize("batch", [16, 47])
+def test_loss_is_that_of_its_own_prediction(rt, batch):
+    # the host reads the loss right after the kernels were issued, on PyTorch's
+    # default stream: it must be this step's, step after step
+    from physis_gb300 import warmstart as ws
+    dims = (batch, 16, 16, 16)
+    gen = torch.Generator(device="cuda").manual_seed(6)
+    n = int(np.prod(dims))
+    x = torch.randn(n * 16, generator=gen, device="cuda").to(torch.bfloat16)
+    t = torch.randn(n, generator=gen, device="cuda")
+    net = ws.Net(7)
+    work = torch.empty(64 * (27 * 256 + 16), device="cuda")
+    work64 = torch.empty((n + 255) // 256, dtype=torch.float64, device="cuda")
+    for _ in range(4):
+        pred = net.forward(x, dims)
+        loss, dy = ws.loss_grad(pred, t, work64)
+        net.backward(dy, dims, work)
+        net.adam(2e-3)
+        true = float(((pred - t).double() ** 2).mean())  # FP32 difference, as the kernel's
+        assert abs(loss - true) <= 1e-9 * true
