@@ -112,10 +112,14 @@ struct Runtime {
   cudaEvent_t fork = nullptr, join = nullptr;
   int sm_count = 0;
   bool trace = false;
-  int *dev_err = nullptr;
+  // The device error word and the results live in pinned host memory that the
+  // kernels write through these device addresses: after a synchronisation the
+  // host reads them where they are, without a copy and a second wait.
+  int *dev_err = nullptr, *host_err = nullptr;
   uint64_t *partials = nullptr;
   unsigned *ticket = nullptr;
-  uint64_t *results = nullptr;  // slot 0: reductions, slot 1: residuals
+  uint64_t *results = nullptr;  // slot 0: reductions, slot 1: residuals (device address)
+  volatile uint64_t *host_results = nullptr;
   cudaEvent_t events[kNumEvents] = {};
   long long launches = 0;
   std::deque<Map> maps;  // deque: references stay valid as maps are added
@@ -241,30 +245,19 @@ GridView view(const Grid *g) {
   return v;
 }
 
-// Checks the device error word; a device-side wait that gave up leaves a
-// non-zero value.  Also re-arms the reduction ticket, which an interrupted
-// reduction may have left non-zero.
-bool check_device_errors() {
-  int h = 0;
-  if (!cuda_ok(cudaMemcpyAsync(&h, rt->dev_err, sizeof(int), cudaMemcpyDeviceToHost,
-                               rt->stream), "read device error word"))
-    return false;
-  if (!cuda_ok(cudaStreamSynchronize(rt->stream), "cudaStreamSynchronize")) return false;
-  if (h != 0) {
-    cudaMemsetAsync(rt->dev_err, 0, sizeof(int), rt->stream);
-    cudaMemsetAsync(rt->ticket, 0, sizeof(unsigned), rt->stream);
-    cudaStreamSynchronize(rt->stream);
-    return fail(PS_ERR_DEVICE_TIMEOUT,
-                "a device-side wait gave up (error bits 0x%x); results of the "
-                "affected launch are invalid", h);
-  }
-  return true;
-}
-
+// Waits for the runtime's stream and checks the device error word; a
+// device-side wait that gave up leaves a non-zero value.  Also re-arms the
+// reduction ticket, which an interrupted reduction may have left non-zero.
 bool sync_rt() {
-  cudaError_t e = cudaStreamSynchronize(rt->stream);
-  if (!cuda_ok(e, "cudaStreamSynchronize")) return false;
-  return check_device_errors();
+  if (!cuda_ok(cudaStreamSynchronize(rt->stream), "cudaStreamSynchronize")) return false;
+  const int h = *const_cast<volatile int *>(rt->host_err);
+  if (h == 0) return true;
+  *const_cast<volatile int *>(rt->host_err) = 0;
+  cudaMemsetAsync(rt->ticket, 0, sizeof(unsigned), rt->stream);
+  cudaStreamSynchronize(rt->stream);
+  return fail(PS_ERR_DEVICE_TIMEOUT,
+              "a device-side wait gave up (error bits 0x%x); results of the "
+              "affected launch are invalid", h);
 }
 
 bool same_view(const GridView &a, const GridView &b) {
@@ -1527,10 +1520,9 @@ bool run_maps(const std::vector<Map *> &ms, int iter) {
 }
 
 bool read_result(int slot, uint64_t *bits) {
-  if (!cuda_ok(cudaMemcpyAsync(bits, rt->results + slot, 8, cudaMemcpyDeviceToHost,
-                               rt->stream), "read reduction result"))
-    return false;
-  return sync_rt();
+  if (!sync_rt()) return false;
+  *bits = rt->host_results[slot];
+  return true;
 }
 
 bool reduce_grid(Grid *g, int op, uint64_t *bits) {
@@ -1702,16 +1694,20 @@ void PSInitV(int trace) {
       !cuda_ok(cudaStreamCreateWithFlags(&r->side, cudaStreamNonBlocking), "cudaStreamCreate") ||
       !cuda_ok(cudaEventCreateWithFlags(&r->fork, cudaEventDisableTiming), "cudaEventCreate") ||
       !cuda_ok(cudaEventCreateWithFlags(&r->join, cudaEventDisableTiming), "cudaEventCreate") ||
-      !cuda_ok(cudaMalloc(&r->dev_err, sizeof(int)), "cudaMalloc") ||
+      !cuda_ok(cudaHostAlloc(reinterpret_cast<void **>(&r->host_err), 128, cudaHostAllocMapped),
+               "cudaHostAlloc") ||
+      !cuda_ok(cudaHostGetDevicePointer(reinterpret_cast<void **>(&r->dev_err), r->host_err, 0),
+               "cudaHostGetDevicePointer") ||
       !cuda_ok(cudaMalloc(&r->partials, sizeof(uint64_t) * kMaxPartials), "cudaMalloc") ||
-      !cuda_ok(cudaMalloc(&r->ticket, sizeof(unsigned)), "cudaMalloc") ||
-      !cuda_ok(cudaMalloc(&r->results, sizeof(uint64_t) * 8), "cudaMalloc")) {
+      !cuda_ok(cudaMalloc(&r->ticket, sizeof(unsigned)), "cudaMalloc")) {
     delete r;
     return;
   }
-  cudaMemset(r->dev_err, 0, sizeof(int));
+  // the error word, then eight results on the next 64 bytes
+  memset(r->host_err, 0, 128);
+  r->host_results = reinterpret_cast<uint64_t *>(r->host_err) + 8;
+  r->results = reinterpret_cast<uint64_t *>(r->dev_err) + 8;
   cudaMemset(r->ticket, 0, sizeof(unsigned));
-  cudaMemset(r->results, 0, sizeof(uint64_t) * 8);
   for (int i = 0; i < kNumEvents; ++i) cudaEventCreate(&r->events[i]);
   // Default launch shapes (the autotuner may replace them):
   // {warps, rows per thread, ring stages, second-ring stages, CTAs per SM}.
@@ -1745,10 +1741,10 @@ void PSFinalize(void) {
   for (Batch &b : g_batches) batch_release(b);
   g_batches.clear();
   for (psg::JitKernel &k : rt->funcs) psg::jit_unload(&k);
-  cudaFree(rt->dev_err);
+  psg::nn_set_error_word(nullptr);
+  cudaFreeHost(rt->host_err);
   cudaFree(rt->partials);
   cudaFree(rt->ticket);
-  cudaFree(rt->results);
   cudaFree(rt->res_packets);
   for (int i = 0; i < kNumEvents; ++i) cudaEventDestroy(rt->events[i]);
   cudaEventDestroy(rt->fork);
