@@ -4,11 +4,11 @@
 
 namespace psg {
 
-int choose_zchunk(int tiles, int nz, int resident) {
-  return choose_zchunk_overhead(tiles, nz, resident, 1);
+int choose_zchunk(int tiles, int nz, int resident, int fill) {
+  return choose_zchunk_overhead(tiles, nz, resident, 1, fill);
 }
 
-int choose_zchunk_overhead(int tiles, int nz, int resident, int overhead) {
+int choose_zchunk_overhead(int tiles, int nz, int resident, int overhead, int fill) {
   if (nz <= 1 || tiles <= 0 || resident <= 0) return nz > 0 ? nz : 1;
   int best_len = nz;
   double best = -1.0;
@@ -28,7 +28,7 @@ int choose_zchunk_overhead(int tiles, int nz, int resident, int overhead) {
       best = eff;
       best_len = len;
     }
-    if (len <= 4) break;
+    if (len <= 4 && items >= fill) break;
   }
   return best_len;
 }

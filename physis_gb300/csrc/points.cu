@@ -134,7 +134,10 @@ template <typename T>
 int schedule(PtsParams<T> *p, int occ, int sm_count) {
   const int resident = sm_count * occ;
   const int nzd = p->dmax2 - p->dmin2;
-  p->zlen = choose_zchunk_overhead(p->tiles, nzd, resident, p->rzl + p->rzh + 1);
+  // chunks as short as fills every resident CTA: loading runs ahead into a CTA's
+  // next item, so a short chunk's halo planes cost little (33 x 65 x 79, 27
+  // points: 5.4 us a sweep against 7.7 with four planes)
+  p->zlen = choose_zchunk_overhead(p->tiles, nzd, resident, p->rzl + p->rzh + 1, resident);
   const int chunks = (nzd + p->zlen - 1) / p->zlen;
   p->items = (long long)p->tiles * chunks;
   return (int)(p->items < resident ? p->items : resident);

@@ -194,12 +194,12 @@ __device__ __forceinline__ void pts_term(T (&acc)[RY][kPtsVX], const T *src, int
 struct PtsPos {
   int tx, ty, chunk;
 };
-__device__ __forceinline__ PtsPos pts_split(long long item, int tiles_x, int tiles) {
+__device__ __forceinline__ PtsPos pts_split(unsigned item, unsigned tiles_x, unsigned tiles) {
+  const unsigned chunk = item / tiles, tile = item - chunk * tiles, ty = tile / tiles_x;
   PtsPos q;
-  q.chunk = (int)(item / tiles);
-  const int tile = (int)(item - (long long)q.chunk * tiles);
-  q.ty = tile / tiles_x;
-  q.tx = tile - q.ty * tiles_x;
+  q.chunk = (int)chunk;
+  q.ty = (int)ty;
+  q.tx = (int)(tile - ty * tiles_x);
   return q;
 }
 __device__ __forceinline__ void pts_advance(PtsPos &q, const PtsPos &step, int tiles_x,

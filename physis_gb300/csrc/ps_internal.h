@@ -62,10 +62,14 @@ struct MarchConfig {
 // spent on useful planes, counting whole rounds of `resident` items and one
 // extra plane of pipeline start-up per item.  Shared by the marching kernels
 // (march.cpp).
-int choose_zchunk(int tiles, int nz, int resident);
+// Chunks are at least four planes long once there are `fill` items: a short
+// chunk's halo planes cost more than they spread, except on a GPU that would
+// stay partly idle (64^3 on 128 x 16 tiles is 64 items of four planes: 4.9 us a
+// sweep, 3.8 with shorter ones; double precision 19.3 and 11.0).
+int choose_zchunk(int tiles, int nz, int resident, int fill = 0);
 // The same with `overhead` start-up planes per item (a k-step temporal pass
 // reads 2k extra input planes per item).
-int choose_zchunk_overhead(int tiles, int nz, int resident, int overhead);
+int choose_zchunk_overhead(int tiles, int nz, int resident, int overhead, int fill = 0);
 
 // Builds a 3D tiled tensor map over g with box {box_w, box_h, 1} elements.
 // Implemented in runtime.cpp (driver entry point looked up at run time).

@@ -103,7 +103,7 @@ cudaError_t launch_ry(S7Params<T> p, int tiles, int nzd, const MarchConfig &cfg,
   const int per_sm = (cfg.ctas_per_sm > 0 && cfg.ctas_per_sm < oc) ? cfg.ctas_per_sm : oc;
   const int resident = sm_count * per_sm;
   p.tiles = tiles;
-  p.zlen = choose_zchunk(tiles, nzd, resident);
+  p.zlen = choose_zchunk(tiles, nzd, resident, sm_count);
   p.items = (int64_t)tiles * ((nzd + p.zlen - 1) / p.zlen);
   int64_t grid = resident;
   if (grid > p.items) grid = p.items;
