@@ -1068,7 +1068,8 @@ std::string points_source(const PtsJitKey &k) {
   snprintf(buf, sizeof(buf), "  static constexpr int kN = %d;\n", k.n);
   s += buf;
   s += "  static constexpr int kW = " + std::to_string(k.w) + ", kPlanes = " +
-       std::to_string(k.planes) + ", kCentre = " + std::to_string(k.centre) + ";\n";
+       std::to_string(k.planes) + ", kCentre = " + std::to_string(k.centre) +
+       ", kLX = " + std::to_string(k.lx) + ";\n";
   s += "  static constexpr int kDx[kN] = {";
   for (int i = 0; i < k.n; ++i) s += (i ? ", " : "") + std::to_string(k.dx[i]);
   s += "};\n  static constexpr int kDy[kN] = {";
@@ -1082,6 +1083,8 @@ std::string points_source(const PtsJitKey &k) {
   }
   s += "};\n";
   snprintf(buf, sizeof(buf), "%d", k.w);
+  s += "  template <typename T> static __device__ __forceinline__ int lx("
+       "const psg::PtsParams<T> &) { return kLX; }\n";
   s += "  template <typename T> static __device__ __forceinline__ int w(const psg::PtsParams<T> &)"
        " { return " + std::string(buf) + "; }\n";
   s += "  template <typename T> static __device__ __forceinline__ int nstage("

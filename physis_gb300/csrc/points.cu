@@ -11,10 +11,10 @@
 // neighbour sums of the reference's system tests (27-point, 9-point 2D,
 // 3-point 1D, asymmetric, hole, periodic variants, red/black).
 //
-// Design.  A tile is 128 cells wide in x and warps*RY rows high; a lane owns
-// RY rows of 16 bytes of consecutive cells (two such groups for 8-byte types)
-// in the compiled form, RY rows of four lane-strided cells in the table form;
-// work items are (z-chunk, tile) pairs in chunk-major order taken round-robin
+// Design.  A tile is 128 cells wide in x and warps*RY rows high, or 64 or 32
+// cells wide and two or four times as high (points_lanes); a lane owns RY rows
+// of 16 bytes of consecutive cells (two such groups for 8-byte types) in the
+// compiled form, RY rows of four lane-strided cells in the table form; work items are (z-chunk, tile) pairs in chunk-major order taken round-robin
 // by a persistent grid, as in the 7-point kernels.
 // * Each z-plane of the tile plus its x/y halo arrives in a ring of
 //   shared-memory planes by one TMA 3D box load (mbarrier per stage, bounded
@@ -23,8 +23,8 @@
 //   that the offsets reach are then rewritten through the boundary map
 //   (periodic cells from the opposite face, clamped ones from the face); the
 //   compute loop is the same for every rule.
-// * The ring holds rzl + rzh + 1 planes for the stencil's z extent plus
-//   planes in flight ahead of the newest one a step reads; loading runs on
+// * The ring holds rzl + rzh + 1 planes for the stencil's z extent plus one or
+//   two planes in flight ahead of the newest one a step reads; loading runs on
 //   into a CTA's next item.  A producer warp issues the boxes and rewrites the
 //   halo cells (their values fetched a plane ahead); consumer warps release
 //   stages one by one, so no step ends in a CTA barrier.
@@ -33,8 +33,8 @@
 // instructions a cell), HBM where it is narrow.  Measured, float, per sweep,
 // against lane-strided cells, halos rewritten by all threads between two CTA
 // barriers and no loading across items: 27 points periodic at 320 x 300 x 257
-// 63 against 198 us, 9 points periodic at 4099 x 3001 21 against 41 us, one
-// colour of the 7-point clamped stencil at 319 x 257 x 255 42 against 94 us.
+// 58 against 198 us, 9 points periodic at 4099 x 3001 21 against 41 us, one
+// colour of the 7-point clamped stencil at 319 x 257 x 255 36 against 94 us.
 // * The sweep body (points_body.cuh) is compiled two ways: here with the
 //   point table (shared-memory offset, plane lag, weight) copied to shared
 //   memory once per CTA and walked in order, and by jit.cpp with NVRTC per
@@ -64,10 +64,18 @@ pts_kernel(const __grid_constant__ PtsParams<T> p, const __grid_constant__ PtsTm
   pts_body<T, RY, UNIT, PtsTableSpec>(p, &tm, smem);
 }
 
-// Planes in flight ahead of the newest plane a step reads: one, as a deeper
-// ring costs CTAs (at 512^3 two or three ran the 7-point stencil 4-15 % and the
-// 27-point one 1-2 % slower, measured when CTA barriers ended each step).
-constexpr int kPtsAhead = 1;
+// Planes in flight ahead of the newest plane a step reads: two where four CTAs
+// still fit an SM, else one (27 points periodic, float, 320 x 300 x 257: 57.9 us
+// a sweep, against 59.8 with five CTAs and one plane and 59.9 with three CTAs
+// and three; red/black 319 x 257 x 255 35.8, 37.2 and 37.9 us a colour).
+size_t ring_bytes(const PointsArgs &a, const int lo[3], const int hi[3], int w, int h,
+                  int *nstage) {
+  const size_t stage = ((size_t)w * h * a.in.esz + 127) / 128 * 128;
+  const int planes = hi[2] - lo[2] + 1;
+  const size_t fixed = 128 + (size_t)kPtsRingOffset;
+  *nstage = planes + (planes + 2 <= kPtsMaxStages && fixed + (planes + 2) * stage <= 56 * 1024 ? 2 : 1);
+  return fixed + (size_t)*nstage * stage;
+}
 
 // Offsets' extent per axis: lo <= 0 <= hi.
 void extents(const PointsArgs &a, int lo[3], int hi[3]) {
@@ -81,7 +89,7 @@ void extents(const PointsArgs &a, int lo[3], int hi[3]) {
 
 // Fills everything but zlen / items (those need the occupancy).
 template <typename T>
-void fill_params(const PointsArgs &a, int warps, int ry, PtsParams<T> *pp) {
+void fill_params(const PointsArgs &a, int warps, int ry, int lx, PtsParams<T> *pp) {
   constexpr int VEC = 16 / (int)sizeof(T);
   PtsParams<T> &p = *pp;
   memset(&p, 0, sizeof(p));
@@ -111,10 +119,11 @@ void fill_params(const PointsArgs &a, int warps, int ry, PtsParams<T> *pp) {
   p.rzh = hi[2];
   p.lp = (-lo[0] + VEC - 1) / VEC * VEC;
   const int rp = (hi[0] + VEC - 1) / VEC * VEC;
-  p.w = p.lp + kPtsTX + rp;
-  const int TY = warps * ry;
+  const int TX = kPtsVX * lx, TY = warps * ry * (32 / lx);
+  p.lx = lx;
+  p.w = p.lp + TX + rp;
   p.rows_h = TY + p.ryl + hi[1];
-  p.nstage = p.rzl + p.rzh + 1 + kPtsAhead;
+  ring_bytes(a, lo, hi, p.w, p.rows_h, &p.nstage);
   p.plane_elems = p.rows_h * p.w;
   p.pstride = (int)(((size_t)p.plane_elems * sizeof(T) + 127) / 128 * 128 / sizeof(T));
   p.err = a.err;
@@ -124,7 +133,7 @@ void fill_params(const PointsArgs &a, int warps, int ry, PtsParams<T> *pp) {
     p.wt[i] = (T)a.w[i];
   }
   p.xbase = a.dom.min[0] / VEC * VEC;
-  p.tiles_x = (a.dom.max[0] - p.xbase + kPtsTX - 1) / kPtsTX;
+  p.tiles_x = (a.dom.max[0] - p.xbase + TX - 1) / TX;
   const int tiles_y = (a.dom.max[1] - a.dom.min[1] + TY - 1) / TY;
   p.tiles = p.tiles_x * tiles_y;
 }
@@ -154,9 +163,9 @@ bool jit_enabled() {
 }
 
 template <typename T, int RY, bool UNIT>
-cudaError_t launch_t(const PointsArgs &a, int warps, int sm_count, cudaStream_t s) {
+cudaError_t launch_t(const PointsArgs &a, int warps, int lx, int sm_count, cudaStream_t s) {
   PtsParams<T> p;
-  fill_params<T>(a, warps, RY, &p);
+  fill_params<T>(a, warps, RY, lx, &p);
   const size_t smem = smem_for(p);
   PtsTmap tm;
   memset(&tm, 0, sizeof(tm));
@@ -177,6 +186,7 @@ cudaError_t launch_t(const PointsArgs &a, int warps, int sm_count, cudaStream_t 
     key.min_ctas = 65536 / (regs * 32 * (warps + 1));
     if (key.min_ctas < 1) key.min_ctas = 1;
     key.unit = UNIT;
+    key.lx = lx;
     key.w = p.w;
     key.nstage = p.nstage;
     key.pstride = p.pstride;
@@ -212,36 +222,72 @@ cudaError_t launch_t(const PointsArgs &a, int warps, int sm_count, cudaStream_t 
 template <typename T>
 cudaError_t launch_type(const PointsArgs &a, const MarchConfig &cfg, int sm_count,
                         cudaStream_t s) {
-  const int warps = cfg.warps;
+  const int warps = cfg.warps, lx = points_lanes(a, cfg);
   if (cfg.rows >= 4)
-    return a.unit ? launch_t<T, 4, true>(a, warps, sm_count, s)
-                  : launch_t<T, 4, false>(a, warps, sm_count, s);
+    return a.unit ? launch_t<T, 4, true>(a, warps, lx, sm_count, s)
+                  : launch_t<T, 4, false>(a, warps, lx, sm_count, s);
   if (cfg.rows >= 2)
-    return a.unit ? launch_t<T, 2, true>(a, warps, sm_count, s)
-                  : launch_t<T, 2, false>(a, warps, sm_count, s);
-  return a.unit ? launch_t<T, 1, true>(a, warps, sm_count, s)
-                : launch_t<T, 1, false>(a, warps, sm_count, s);
+    return a.unit ? launch_t<T, 2, true>(a, warps, lx, sm_count, s)
+                  : launch_t<T, 2, false>(a, warps, lx, sm_count, s);
+  return a.unit ? launch_t<T, 1, true>(a, warps, lx, sm_count, s)
+                : launch_t<T, 1, false>(a, warps, lx, sm_count, s);
 }
 
 }  // namespace
 
 int points_rows(const MarchConfig &cfg) { return cfg.rows >= 4 ? 4 : (cfg.rows >= 2 ? 2 : 1); }
 
-void points_box(const PointsArgs &a, const MarchConfig &cfg, int *w, int *h) {
+namespace {
+
+// TMA box of one ring plane and shared memory with tiles of lx lanes in x.
+void box_for(const PointsArgs &a, const MarchConfig &cfg, int lx, int *w, int *h) {
   const int vec = 16 / a.in.esz;
   int lo[3], hi[3];
   extents(a, lo, hi);
-  *w = (-lo[0] + vec - 1) / vec * vec + kPtsTX + (hi[0] + vec - 1) / vec * vec;
-  *h = cfg.warps * points_rows(cfg) - lo[1] + hi[1];
+  *w = (-lo[0] + vec - 1) / vec * vec + kPtsVX * lx + (hi[0] + vec - 1) / vec * vec;
+  *h = cfg.warps * points_rows(cfg) * (32 / lx) - lo[1] + hi[1];
+}
+
+size_t smem_bytes_for(const PointsArgs &a, const MarchConfig &cfg, int lx) {
+  int lo[3], hi[3], w, h, nstage;
+  extents(a, lo, hi);
+  box_for(a, cfg, lx, &w, &h);
+  return ring_bytes(a, lo, hi, w, h, &nstage);
+}
+
+}  // namespace
+
+// Lanes side by side in x.  All three shapes hold the same cells, so the one
+// that covers the domain with the fewest cells loaded (tiles x box) is taken,
+// the wider one unless a narrower one saves 3 %.  Against 128-cell tiles, per
+// sweep: 64-cell tiles, 27 points periodic 320 x 300 x 257 59.8 against 63 us,
+// 27 points 60^3 4.3 against 4.9, 7 points 50 x 300 x 300 12.4 against 17.2;
+// 32-cell tiles, double, 7 points 40 x 66 x 100 18 against 32 us.
+int points_lanes(const PointsArgs &a, const MarchConfig &cfg) {
+  const int vec = 16 / a.in.esz;
+  const int nx = a.dom.max[0] - a.dom.min[0] / vec * vec, ny = a.dom.max[1] - a.dom.min[1];
+  int best = 32;
+  double cost = 0;
+  for (int lx = 32; lx >= 8; lx /= 2) {
+    const int tx = kPtsVX * lx, ty = cfg.warps * points_rows(cfg) * (32 / lx);
+    int w, h;
+    box_for(a, cfg, lx, &w, &h);
+    if (lx < 32 && (h > 256 || smem_bytes_for(a, cfg, lx) > 220 * 1024)) continue;
+    const double c = (double)((nx + tx - 1) / tx) * ((ny + ty - 1) / ty) * w * h;
+    if (lx == 32 || c < 0.97 * cost) {
+      best = lx;
+      cost = c;
+    }
+  }
+  return best;
+}
+
+void points_box(const PointsArgs &a, const MarchConfig &cfg, int *w, int *h) {
+  box_for(a, cfg, points_lanes(a, cfg), w, h);
 }
 
 size_t points_smem_bytes(const PointsArgs &a, const MarchConfig &cfg) {
-  int lo[3], hi[3], w, h;
-  extents(a, lo, hi);
-  points_box(a, cfg, &w, &h);
-  const int nstage = -lo[2] + hi[2] + 1 + kPtsAhead;
-  const size_t stage = ((size_t)w * h * a.in.esz + 127) / 128 * 128;
-  return 128 + (size_t)kPtsRingOffset + (size_t)nstage * stage;
+  return smem_bytes_for(a, cfg, points_lanes(a, cfg));
 }
 
 cudaError_t launch_points(const PointsArgs &a, const MarchConfig &cfg, int sm_count,

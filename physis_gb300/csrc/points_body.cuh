@@ -13,8 +13,7 @@
 
 namespace psg {
 
-constexpr int kPtsTX = 128;       // tile width in cells
-constexpr int kPtsVX = 4;         // cells per lane and row
+constexpr int kPtsVX = 4;         // cells per lane and row; a tile is kPtsVX * lx cells wide
 constexpr int kPtsMaxPoints = 64;
 // Shared memory: point table (run-time spec only: offsets, lags, weights),
 // then the ring's mbarriers (full, empty, raw), then the ring (128-byte
@@ -42,6 +41,7 @@ struct PtsParams {
   int rxl, rxh, ryl, ryh, rzl, rzh;  // extent of the offsets per axis
   int lp, w, rows_h, nstage, plane_elems;
   int pstride;       // ring stage stride in elements (128-byte multiple)
+  int lx;            // lanes side by side in x: 32, 16 or 8 (the others take rows further down)
   int xbase, tiles_x, tiles, zlen;
   long long items;
   int *err;          // device error word (bounded waits that give up)
@@ -121,6 +121,8 @@ __device__ __forceinline__ int pts_halo_cell(const PtsParams<T> &p, const PtsHal
 struct PtsTableSpec {
   static constexpr bool kStatic = false;
   template <typename T>
+  static __device__ __forceinline__ int lx(const PtsParams<T> &p) { return p.lx; }
+  template <typename T>
   static __device__ __forceinline__ int w(const PtsParams<T> &p) { return p.w; }
   template <typename T>
   static __device__ __forceinline__ int nstage(const PtsParams<T> &p) { return p.nstage; }
@@ -142,9 +144,10 @@ __device__ __forceinline__ PtsVec<T> pts_ld16(const T *src) {
 }
 
 // Compiled spec.  acc[r][c] (+)= w * the point's value for the cells of row r:
-// lane l owns the VEC = 16 / sizeof(T) consecutive cells from
-// 32 VEC j + VEC l of each of the 4 / VEC column groups j.  Every read is an
-// aligned 16-byte shared load (conflict-free); a point's row and x offset only
+// lane l of the LX side by side owns the VEC = 16 / sizeof(T) consecutive cells
+// from LX VEC j + VEC l of each of the 4 / VEC column groups j.  Every read is an
+// aligned 16-byte shared load (conflict-free, as a load goes by quarter warps
+// and eight lanes are always consecutive); a point's row and x offset only
 // select cells of such vectors, and the compiler issues each vector once per
 // step however many points and rows use it (a 27-point stencil needs 3 planes
 // x 6 rows x 3 vectors for 16 cells, 3.4 loads a cell).
@@ -160,7 +163,7 @@ __device__ __forceinline__ void pts_point(T (&acc)[RY][kPtsVX], const T *const *
     for (int c = 0; c < kPtsVX; ++c) {
       const int j = c / VEC, i = c % VEC + DX;
       const int vi = (i + 8 * VEC) / VEC - 8, e = i - vi * VEC;
-      const T v = pts_ld16<T>(pl[LAG] + cell0 + (r + DY) * S::kW + j * 32 * VEC + vi * VEC)
+      const T v = pts_ld16<T>(pl[LAG] + cell0 + (r + DY) * S::kW + j * S::kLX * VEC + vi * VEC)
                       .v[e];
       const T t = UNIT ? v : R::mul(wk, v);
       acc[r][c] = K == 0 ? t : R::add(acc[r][c], t);
@@ -174,16 +177,16 @@ __device__ __forceinline__ void pts_points(T (&acc)[RY][kPtsVX], const T *const 
   }
 }
 
-// Table spec: acc[r][j] (+)= w * src[r*W + 32*j]; `first` starts the sum.
+// Table spec: acc[r][j] (+)= w * src[r*W + LX*j]; `first` starts the sum.
 template <typename T, int RY, bool UNIT>
-__device__ __forceinline__ void pts_term(T (&acc)[RY][kPtsVX], const T *src, int W, T wk,
+__device__ __forceinline__ void pts_term(T (&acc)[RY][kPtsVX], const T *src, int W, int LX, T wk,
                                          bool first) {
   typedef RN<T> R;
 #pragma unroll
   for (int r = 0; r < RY; ++r)
 #pragma unroll
     for (int j = 0; j < kPtsVX; ++j) {
-      const T v = src[r * W + 32 * j];
+      const T v = src[r * W + LX * j];
       const T t = UNIT ? v : R::mul(wk, v);
       acc[r][j] = first ? t : R::add(acc[r][j], t);
     }
@@ -242,7 +245,8 @@ __device__ __forceinline__ void pts_body(const PtsParams<T> &p, const void *tmap
   unsigned long long *full = reinterpret_cast<unsigned long long *>(smem + kPtsTableBytes);
   unsigned long long *empty = full + kPtsMaxStages, *raw = empty + kPtsMaxStages;
   T *ring = reinterpret_cast<T *>(smem + kPtsRingOffset);
-  const int W = S::w(p), NST = S::nstage(p), PS = S::pstride(p);
+  const int W = S::w(p), NST = S::nstage(p), PS = S::pstride(p), LX = S::lx(p);
+  const int TX = kPtsVX * LX;
 
   const int lane = threadIdx.x, warp = threadIdx.y;
   const int consumers = blockDim.y - 1;  // warps
@@ -264,7 +268,7 @@ __device__ __forceinline__ void pts_body(const PtsParams<T> &p, const void *tmap
   }
   __syncthreads();
 
-  const int TY = consumers * RY;
+  const int TY = consumers * RY * (32 / LX);
   const int zext = p.rzl + p.rzh;
   const int tiles_y = p.tiles / p.tiles_x;
   PtsPos pos = pts_split(blockIdx.x, p.tiles_x, p.tiles);
@@ -279,12 +283,12 @@ __device__ __forceinline__ void pts_body(const PtsParams<T> &p, const void *tmap
     for (long long item = blockIdx.x; item < p.items; item += gridDim.x) {
       const int zs = p.dmin2 + pos.chunk * p.zlen;
       const int n = min(p.zlen, p.dmax2 - zs) + zext;
-      const int x0 = p.xbase + pos.tx * kPtsTX, y0 = p.dmin1 + pos.ty * TY;
+      const int x0 = p.xbase + pos.tx * TX, y0 = p.dmin1 + pos.ty * TY;
       pts_advance(pos, step, p.tiles_x, tiles_y);
       PtsHalo h;
       h.total = 0;
       if (p.boundary != kPtsNone &&
-          !(x0 - p.rxl >= 0 && x0 + kPtsTX + p.rxh <= p.nx && y0 - p.ryl >= 0 &&
+          !(x0 - p.rxl >= 0 && x0 + TX + p.rxh <= p.nx && y0 - p.ryl >= 0 &&
             y0 - p.ryl + p.rows_h <= p.ny))
         h = pts_halo(p, x0, y0, W);
       const bool fix = h.total > 0;
@@ -373,7 +377,8 @@ __device__ __forceinline__ void pts_body(const PtsParams<T> &p, const void *tmap
 
   // first cell of the lane's first row relative to a plane: its vector
   // (compiled spec) or its first lane-strided cell (table spec)
-  const int cell0 = S::kStatic ? (warp * RY + p.ryl) * W + p.lp + lane * VEC : warp * RY * W + lane;
+  const int xl = lane % LX, row0 = (warp * (32 / LX) + lane / LX) * RY;
+  const int cell0 = S::kStatic ? (row0 + p.ryl) * W + p.lp + xl * VEC : row0 * W + xl;
   bool ok = true;
   // Slot of plane z - rzl of the current step, the next slot to wait for, and
   // the parity of each slot's next completion (bit s).
@@ -382,23 +387,23 @@ __device__ __forceinline__ void pts_body(const PtsParams<T> &p, const void *tmap
   for (long long item = blockIdx.x; item < p.items; item += gridDim.x) {
     const int zs = p.dmin2 + pos.chunk * p.zlen;
     const int ze = min(zs + p.zlen, p.dmax2);
-    const int x0 = p.xbase + pos.tx * kPtsTX;
+    const int x0 = p.xbase + pos.tx * TX;
     const int y0 = p.dmin1 + pos.ty * TY;
     pts_advance(pos, step, p.tiles_x, tiles_y);
     // cells of the lane in the domain: bit c of colmask, bit r of rowmask
     unsigned colmask = 0, rowmask = 0;
 #pragma unroll
     for (int c = 0; c < kPtsVX; ++c) {
-      const int x = S::kStatic ? x0 + (c / VEC) * 32 * VEC + lane * VEC + c % VEC
-                               : x0 + lane + 32 * c;
+      const int x = S::kStatic ? x0 + (c / VEC) * LX * VEC + xl * VEC + c % VEC
+                               : x0 + xl + LX * c;
       if (x >= p.dmin0 && x < p.dmax0) colmask |= 1u << c;
     }
 #pragma unroll
     for (int r = 0; r < RY; ++r)
-      if (y0 + warp * RY + r < p.dmax1) rowmask |= 1u << r;
+      if (y0 + row0 + r < p.dmax1) rowmask |= 1u << r;
     const bool whole = colmask == (1u << kPtsVX) - 1u && rowmask == (1u << RY) - 1u;
-    T *dst = p.out + (long long)zs * p.plane + (long long)(y0 + warp * RY) * p.row + x0 +
-             lane * (S::kStatic ? VEC : 1);
+    T *dst = p.out + (long long)zs * p.plane + (long long)(y0 + row0) * p.row + x0 +
+             xl * (S::kStatic ? VEC : 1);
 
     int waited = 0;  // planes of this item that have landed
     for (int z = zs; z < ze; ++z, dst += p.plane) {
@@ -428,11 +433,11 @@ __device__ __forceinline__ void pts_body(const PtsParams<T> &p, const void *tmap
             for (int r = 0; r < RY; ++r)
 #pragma unroll
               for (int c = 0; c < kPtsVX; ++c) {
-                const int x = x0 + (c / VEC) * 32 * VEC + lane * VEC + c % VEC;
+                const int x = x0 + (c / VEC) * LX * VEC + xl * VEC + c % VEC;
                 const T own =
-                    pts_ld16<T>(pl[S::kCentre] + cell0 + r * S::kW + (c / VEC) * 32 * VEC)
+                    pts_ld16<T>(pl[S::kCentre] + cell0 + r * S::kW + (c / VEC) * LX * VEC)
                         .v[c % VEC];
-                if ((x + y0 + warp * RY + r + z + p.color) & 1) acc[r][c] = own;
+                if ((x + y0 + row0 + r + z + p.color) & 1) acc[r][c] = own;
               }
           }
 #pragma unroll
@@ -441,7 +446,7 @@ __device__ __forceinline__ void pts_body(const PtsParams<T> &p, const void *tmap
 #pragma unroll
             for (int j = 0; j < kPtsVX / VEC; ++j) {
               const unsigned m = (colmask >> (j * VEC)) & ((1u << VEC) - 1u);
-              T *d = dst + r * p.row + j * 32 * VEC;
+              T *d = dst + r * p.row + j * LX * VEC;
               if (whole || m == (1u << VEC) - 1u) {
                 union { uint4 u; T t[VEC]; } c;
 #pragma unroll
@@ -458,17 +463,18 @@ __device__ __forceinline__ void pts_body(const PtsParams<T> &p, const void *tmap
           for (int k = 0; k < p.n; ++k) {
             int s = cs + s_lag[k];
             if (s >= NST) s -= NST;
-            pts_term<T, RY, UNIT>(acc, ring + s * PS + cell0 + s_off[k], W, s_w[k], k == 0);
+            pts_term<T, RY, UNIT>(acc, ring + s * PS + cell0 + s_off[k], W, LX, s_w[k],
+                                  k == 0);
           }
 #pragma unroll
           for (int r = 0; r < RY; ++r) {
-            const int y = y0 + warp * RY + r;
+            const int y = y0 + row0 + r;
             const bool row_on = ((rowmask >> r) & 1u) &&
-                                (p.color < 0 || ((x0 + lane + y + z + p.color) & 1) == 0);
+                                (p.color < 0 || ((x0 + xl + y + z + p.color) & 1) == 0);
             if (row_on) {
 #pragma unroll
               for (int j = 0; j < kPtsVX; ++j)
-                if ((colmask >> j) & 1u) dst[r * p.row + 32 * j] = acc[r][j];
+                if ((colmask >> j) & 1u) dst[r * p.row + LX * j] = acc[r][j];
             }
           }
         }

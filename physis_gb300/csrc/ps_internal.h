@@ -159,9 +159,12 @@ struct PointsArgs {
   int *err;          // device error word
   CUtensorMap tmap;  // maps `in` with the box points_box() gives
 };
-// cfg.warps x points_rows(cfg) (1, 2 or 4) rows per tile; the other fields
+// cfg.warps warps of points_rows(cfg) (1, 2 or 4) rows a lane; the other fields
 // are unused.
 int points_rows(const MarchConfig &cfg);
+// Lanes side by side in x (32, 16 or 8): tiles of 4 * lanes cells by
+// cfg.warps * points_rows(cfg) * 32 / lanes rows.
+int points_lanes(const PointsArgs &a, const MarchConfig &cfg);
 // The TMA box of one ring plane: w cells by h rows.
 void points_box(const PointsArgs &a, const MarchConfig &cfg, int *w, int *h);
 size_t points_smem_bytes(const PointsArgs &a, const MarchConfig &cfg);
@@ -221,6 +224,7 @@ struct PtsJitKey {
   int ry, warps, n;          // warps: consumers (the CTA has one more)
   int min_ctas;              // per SM, for the register limit
   bool unit;
+  int lx;                    // lanes side by side in x
   int w, nstage, pstride;
   int planes, centre;        // z extent of the points, lag of the cell's own plane
   int dx[kMaxPoints], dy[kMaxPoints], lag[kMaxPoints];

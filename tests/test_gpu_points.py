@@ -196,6 +196,25 @@ def test_point_sweep_edges_bit_exact(rt, oracle, kernel_form, seed, shape, dtype
                                          npts, radius, weighted, shrink)
 
 
+NARROW = [
+    # grids that 64- and 32-cell tiles cover with fewer cells, their edges one
+    # cell off, and boxes too high for the narrowest
+    (51, (9, 70, 65), np.float32, 1, 27, 1, True, False),
+    (52, (7, 129, 33), np.float64, 2, 14, 2, True, True),
+    (53, (11, 63, 31), np.int32, 1, 9, 1, False, False),
+    (54, (3, 130, 192), np.int64, 2, 20, 4, True, False),
+    (55, (1, 513, 161), np.float32, 1, 9, 1, True, True),
+    (56, (17, 64, 7), np.float64, 1, 12, 3, True, False),
+]
+
+
+@pytest.mark.parametrize("seed,shape,dtype,boundary,npts,radius,weighted,shrink", NARROW)
+def test_narrow_point_tiles_bit_exact(rt, oracle, kernel_form, seed, shape, dtype, boundary, npts,
+                                      radius, weighted, shrink):
+    test_random_point_stencils_bit_exact(rt, oracle, kernel_form, seed, shape, dtype, boundary,
+                                         npts, radius, weighted, shrink)
+
+
 @pytest.mark.parametrize("warps,rows", [(8, 2), (8, 1), (4, 2), (16, 1), (2, 2), (1, 1), (8, 4), (4, 4)])
 def test_point_launch_shapes_do_not_change_results(rt, oracle, kernel_form, warps, rows):
     rng = np.random.default_rng(42)
@@ -258,6 +277,14 @@ def test_red_black_bit_exact(rt, oracle, kernel_form, seed, shape, dtype, bounda
     got = dg.copyout()
     dg.free()
     assert np.array_equal(_bits(got), _bits(ref))
+
+
+@pytest.mark.parametrize("seed,shape,dtype,boundary", [
+    (61, (9, 67, 63), np.float32, 2), (62, (6, 70, 34), np.float64, 1),
+    (63, (4, 34, 162), np.int32, 1)])
+def test_red_black_narrow_tiles(rt, oracle, kernel_form, seed, shape, dtype, boundary):
+    test_red_black_bit_exact(rt, oracle, kernel_form, seed, shape, dtype, boundary, sc.P7_RB,
+                             True, 0, 2)
 
 
 def test_red_black_builtins(rt, oracle):
