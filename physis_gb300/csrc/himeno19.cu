@@ -73,6 +73,8 @@ himeno19_kernel(const __grid_constant__ HimenoMaps maps, const HParams p) {
     fence_barrier_init();
   }
   __syncthreads();
+  if (p.early) launch_dependents();
+  wait_for_predecessors();
 
   HRing pprod, pcons, cprod, ccons;
   bool ok = true;
@@ -192,8 +194,8 @@ cudaError_t launch_himeno19(const Himeno19Args &a, const MarchConfig &cfg,
   int64_t grid = resident;
   if (grid > p.items) grid = p.items;
   if (a.gosa && grid > sink.max_partials) grid = sink.max_partials;
-  kern<<<(unsigned)grid, dim3(32, cfg.warps, 1), smem, s>>>(maps, p);
-  return cudaGetLastError();
+  p.early = grid == resident;
+  return launch_kernel(kern, (unsigned)grid, dim3(32, cfg.warps, 1), smem, s, a.overlap, maps, p);
 }
 
 }  // namespace psg

@@ -96,8 +96,7 @@ struct Driver {
   bool tried = false, ok = false;
   CUresult (*load)(CUmodule *, const void *) = nullptr;
   CUresult (*get)(CUfunction *, CUmodule, const char *) = nullptr;
-  CUresult (*launch)(CUfunction, unsigned, unsigned, unsigned, unsigned, unsigned, unsigned,
-                     unsigned, CUstream, void **, void **) = nullptr;
+  CUresult (*launch)(const CUlaunchConfig *, CUfunction, void **, void **) = nullptr;
   CUresult (*unload)(CUmodule) = nullptr;
   CUresult (*set_attr)(CUfunction, CUfunction_attribute, int) = nullptr;
   CUresult (*occupancy)(int *, CUfunction, int, size_t) = nullptr;
@@ -122,7 +121,7 @@ bool load_driver(std::string *err) {
   };
   g_drv.load = reinterpret_cast<decltype(g_drv.load)>(sym("cuModuleLoadData"));
   g_drv.get = reinterpret_cast<decltype(g_drv.get)>(sym("cuModuleGetFunction"));
-  g_drv.launch = reinterpret_cast<decltype(g_drv.launch)>(sym("cuLaunchKernel"));
+  g_drv.launch = reinterpret_cast<decltype(g_drv.launch)>(sym("cuLaunchKernelEx"));
   g_drv.unload = reinterpret_cast<decltype(g_drv.unload)>(sym("cuModuleUnload"));
   g_drv.set_attr = reinterpret_cast<decltype(g_drv.set_attr)>(sym("cuFuncSetAttribute"));
   g_drv.occupancy = reinterpret_cast<decltype(g_drv.occupancy)>(
@@ -464,12 +463,13 @@ std::string call_source(const JitKernel &k) {
 std::string entry_source(const JitKernel &k) {
   std::string s =
       "\nextern \"C\" __global__ void __launch_bounds__(256) __ps_entry(int dmin0, int dmax0, "
-      "int dmin1, int dmax1, int dmin2, int dmax2, int color, int zlen" +
+      "int dmin1, int dmax1, int dmin2, int dmax2, int color, int zlen, int early" +
       entry_params(k) + ") {\n";
   for (size_t i = 0; i < k.params.size(); ++i)
     if (k.params[i].grid)
       s += "  auto g" + std::to_string(i) + " = __ps_dev(a" + std::to_string(i) + ");\n";
-  s += "  const int tx = blockIdx.x * blockDim.x + threadIdx.x;\n"
+  s += "  if (early) psg::launch_dependents();\n  psg::wait_for_predecessors();\n"
+       "  const int tx = blockIdx.x * blockDim.x + threadIdx.x;\n"
        "  const int y = dmin1 + blockIdx.y * blockDim.y + threadIdx.y;\n"
        "  if (y >= dmax1) return;\n"
        "  const int zs = dmin2 + blockIdx.z * zlen;\n"
@@ -630,7 +630,7 @@ std::string tiled_entry_source(const JitKernel &k) {
   const auto N = [](long long v) { return std::to_string(v); };
   std::string s = "\nextern \"C\" __global__ void __launch_bounds__(" + N(kTileThreads) +
                   ") __ps_entry_t(int dmin0, int dmax0, int dmin1, int dmax1, int dmin2, "
-                  "int dmax2, int ntx, int zlen, int *err";
+                  "int dmax2, int ntx, int zlen, int early, int *err";
   for (size_t j = 0; j < k.stages.size(); ++j)
     s += ", const __grid_constant__ __PSTmap tm" + N(j);
   s += entry_params(k) + ") {\n"
@@ -650,7 +650,8 @@ std::string tiled_entry_source(const JitKernel &k) {
        "      psg::mbar_init(&full[i], 1);\n      psg::mbar_init(&raw[i], 1);\n"
        "      psg::mbar_init(&empty[i], " + N(kTileWarps) + ");\n    }\n"
        "    psg::fence_barrier_init();\n  }\n"
-       "  __syncthreads();\n";
+       "  __syncthreads();\n"
+       "  if (early) psg::launch_dependents();\n  psg::wait_for_predecessors();\n";
   // the staged grids' rings and windows
   std::string edge, init, step, fixi, fixs;
   size_t bytes0 = 0, bytes1 = 0;
@@ -937,8 +938,30 @@ bool tiled_enabled() {
 // no staged grid shares its memory with another grid argument (a staged copy
 // of a grid that the same launch writes would be stale); red/black maps and
 // everything else run the plain entry.
+// A launch of a compiled kernel; with `overlap` it may start before the stream's
+// previous kernel ends.
+static CUresult launch_function(void *fn, dim3 grid, dim3 block, size_t smem, bool overlap,
+                                cudaStream_t s, void **args) {
+  CUlaunchAttribute at = {};
+  at.id = CU_LAUNCH_ATTRIBUTE_PROGRAMMATIC_STREAM_SERIALIZATION;
+  at.value.programmaticStreamSerializationAllowed = 1;
+  CUlaunchConfig c = {};
+  c.gridDimX = grid.x;
+  c.gridDimY = grid.y;
+  c.gridDimZ = grid.z;
+  c.blockDimX = block.x;
+  c.blockDimY = block.y;
+  c.blockDimZ = block.z;
+  c.sharedMemBytes = (unsigned)smem;
+  c.hStream = static_cast<CUstream>(s);
+  c.attrs = &at;
+  c.numAttrs = overlap ? 1 : 0;
+  return g_drv.launch(&c, static_cast<CUfunction>(fn), args, nullptr);
+}
+
 cudaError_t jit_launch(const JitKernel &k, const Box &dom, int color, const GridView *grids,
-                       const double *scalars, int sm_count, int *dev_err, cudaStream_t s) {
+                       const double *scalars, int sm_count, int *dev_err, bool overlap,
+                       cudaStream_t s) {
   const int nxd = dom.max[0] - dom.min[0], nyd = dom.max[1] - dom.min[1],
             nzd = dom.max[2] - dom.min[2];
   if (nxd <= 0 || nyd <= 0 || nzd <= 0) return cudaSuccess;
@@ -954,7 +977,7 @@ cudaError_t jit_launch(const JitKernel &k, const Box &dom, int color, const Grid
       if (j != sgi && grids[j].ptr == grids[sgi].ptr) tiled = false;
   }
   unsigned gx, gy, gz, bx, by;
-  int head[8];
+  int head[9];
   if (tiled) {
     const long long ntx = (nxd + kTileX - 1) / kTileX, nty = (nyd + kTileY - 1) / kTileY;
     const long long tiles = ntx * nty;
@@ -976,8 +999,8 @@ cudaError_t jit_launch(const JitKernel &k, const Box &dom, int color, const Grid
     gz = 1;
     bx = kTileThreads;
     by = 1;
-    const int h[8] = {dom.min[0], dom.max[0], dom.min[1], dom.max[1],
-                      dom.min[2], dom.max[2], (int)ntx, zlen};
+    const int h[9] = {dom.min[0], dom.max[0], dom.min[1], dom.max[1], dom.min[2], dom.max[2],
+                      (int)ntx,   zlen,       tiles * chunks >= want};
     memcpy(head, h, sizeof(h));
   } else {
     bx = 64;
@@ -993,12 +1016,12 @@ cudaError_t jit_launch(const JitKernel &k, const Box &dom, int color, const Grid
     nz = (nzd + zlen - 1) / zlen;
     if (gy > 65535 || nz > 65535) return cudaErrorInvalidConfiguration;
     gz = (unsigned)nz;
-    const int h[8] = {dom.min[0], dom.max[0], dom.min[1], dom.max[1],
-                      dom.min[2], dom.max[2], color, zlen};
+    const int h[9] = {dom.min[0], dom.max[0], dom.min[1], dom.max[1],           dom.min[2],
+                      dom.max[2], color,      zlen,       gx * gy * nz >= want};
     memcpy(head, h, sizeof(h));
   }
 
-  // argument storage: 8 ints, then each parameter at its alignment
+  // argument storage: 9 ints, then each parameter at its alignment
   std::vector<unsigned char> buf(64 + 64 * k.params.size() + 16);
   std::vector<void *> args;
   size_t off = 0;
@@ -1044,9 +1067,8 @@ cudaError_t jit_launch(const JitKernel &k, const Box &dom, int color, const Grid
       }
     }
   }
-  const CUresult r = g_drv.launch(static_cast<CUfunction>(tiled ? k.func_tiled : k.func), gx,
-                                  gy, gz, bx, by, 1, tiled ? (unsigned)stage_dynamic(k) : 0,
-                                  static_cast<CUstream>(s), args.data(), nullptr);
+  const CUresult r = launch_function(tiled ? k.func_tiled : k.func, dim3(gx, gy, gz), dim3(bx, by),
+                                     tiled ? stage_dynamic(k) : 0, overlap, s, args.data());
   return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorLaunchFailure;
 }
 
@@ -1161,11 +1183,9 @@ void *jit_points_function(const PtsJitKey &k, size_t smem, int *occ) {
   return fn;
 }
 
-cudaError_t jit_launch_raw(void *fn, int grid, dim3 block, size_t smem, cudaStream_t s,
-                           void **args) {
-  const CUresult r = g_drv.launch(static_cast<CUfunction>(fn), (unsigned)grid, 1, 1, block.x,
-                                  block.y, block.z, (unsigned)smem, static_cast<CUstream>(s),
-                                  args, nullptr);
+cudaError_t jit_launch_raw(void *fn, int grid, dim3 block, size_t smem, bool overlap,
+                           cudaStream_t s, void **args) {
+  const CUresult r = launch_function(fn, dim3(grid), block, smem, overlap, s, args);
   return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorLaunchFailure;
 }
 

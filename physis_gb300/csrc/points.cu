@@ -52,6 +52,7 @@
 #include <cstring>
 
 #include "points_body.cuh"
+#include "ps_device.cuh"
 #include "ps_internal.h"
 
 namespace psg {
@@ -149,6 +150,7 @@ int schedule(PtsParams<T> *p, int occ, int sm_count) {
   p->zlen = choose_zchunk_overhead(p->tiles, nzd, resident, p->rzl + p->rzh + 1, resident);
   const int chunks = (nzd + p->zlen - 1) / p->zlen;
   p->items = (long long)p->tiles * chunks;
+  p->early = p->items >= resident;
   return (int)(p->items < resident ? p->items : resident);
 }
 
@@ -203,7 +205,7 @@ cudaError_t launch_t(const PointsArgs &a, int warps, int lx, int sm_count, cudaS
     if (fn && occ >= 1) {
       const int grid = schedule(&p, occ, sm_count);
       void *args[2] = {&p, &tm};
-      return jit_launch_raw(fn, grid, dim3(32, warps + 1, 1), smem, s, args);
+      return jit_launch_raw(fn, grid, dim3(32, warps + 1, 1), smem, a.overlap, s, args);
     }
   }
   auto kern = pts_kernel<T, RY, UNIT>;
@@ -215,8 +217,7 @@ cudaError_t launch_t(const PointsArgs &a, int warps, int lx, int sm_count, cudaS
   if (e != cudaSuccess) return e;
   if (occ < 1) return cudaErrorInvalidConfiguration;
   const int grid = schedule(&p, occ, sm_count);
-  kern<<<grid, dim3(32, warps + 1, 1), smem, s>>>(p, tm);
-  return cudaGetLastError();
+  return launch_kernel(kern, (unsigned)grid, dim3(32, warps + 1, 1), smem, s, a.overlap, p, tm);
 }
 
 template <typename T>

@@ -44,6 +44,7 @@ struct PtsParams {
   int lx;            // lanes side by side in x: 32, 16 or 8 (the others take rows further down)
   int xbase, tiles_x, tiles, zlen;
   long long items;
+  int early;         // the next launch's CTAs may take places while this one runs
   int *err;          // device error word (bounded waits that give up)
   int off[kPtsMaxPoints];  // shared offset of point i relative to the cell
   int lag[kPtsMaxPoints];  // rzl + dz_i: the point's plane relative to z - rzl
@@ -267,6 +268,8 @@ __device__ __forceinline__ void pts_body(const PtsParams<T> &p, const void *tmap
     }
   }
   __syncthreads();
+  if (p.early) launch_dependents();
+  wait_for_predecessors();
 
   const int TY = consumers * RY * (32 / LX);
   const int zext = p.rzl + p.rzh;

@@ -54,6 +54,21 @@ struct RN<long long> {
   static __device__ __forceinline__ long long mul(long long a, long long b) { return (long long)((U)a * (U)b); }
 };
 
+// Launches that may overlap: `launch_dependents` lets the next launch's CTAs
+// take free places on the SMs before this one ends, `wait` returns once the
+// launches before this one have ended and their writes are visible.  Neither
+// does anything in a launch without the attribute.
+// A launch that leaves places free keeps its dependents waiting until its CTAs
+// end: they would crowd into the free places, several to an SM while others have
+// none (a double 64^3 sweep 13.9 us against 10.2, a double 27-point function at
+// 60^3 37 against 20.4).  One that fills the GPU lets them in at its start.
+__device__ __forceinline__ void launch_dependents() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void wait_for_predecessors() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // Error bits written into the runtime's device error word.
 enum : int {
   kDevErrWaitTimeout = 1,  // an mbarrier wait ran past its iteration limit

@@ -17,6 +17,24 @@ __device__ __forceinline__ void prefetch_tmap(const CUtensorMap *map) {
                : "memory");
 }
 
+// A launch that, with `overlap`, may start while the stream's previous kernel
+// still runs (the kernel then waits with wait_for_predecessors()).
+template <typename... P, typename... A>
+cudaError_t launch_kernel(void (*kern)(P...), unsigned grid, dim3 block, size_t smem,
+                          cudaStream_t s, bool overlap, A &&...args) {
+  cudaLaunchConfig_t c = {};
+  c.gridDim = dim3(grid);
+  c.blockDim = block;
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = &at;
+  c.numAttrs = overlap ? 1 : 0;
+  return cudaLaunchKernelEx(&c, kern, static_cast<P>(args)...);
+}
+
 // 16-byte vector of T held as VEC scalars.
 template <typename T>
 struct V16 {

@@ -81,6 +81,7 @@ struct Stencil7Args {
   GridView in, out;
   Box dom;
   double coef[7];  // map argument order: ce cw cn cs ct cb cc
+  bool overlap;    // the launch may start before the stream's previous kernel ends
 };
 // Number of bytes of dynamic shared memory the launch will use.
 size_t stencil7_smem_bytes(int esz, const MarchConfig &cfg);
@@ -95,6 +96,7 @@ struct Temporal7Args {
   double coef[7];  // map argument order: ce cw cn cs ct cb cc
   int k;
   bool fma;        // contract each multiply-add (else bit-exact to k plain steps)
+  bool overlap;
 };
 int temporal7_max_k(int esz);
 size_t temporal7_smem_bytes(int esz, const MarchConfig &cfg, int k);
@@ -130,6 +132,7 @@ struct Himeno19Args {
   Box dom;
   float omega;
   bool gosa;       // fused residual sum of ss*ss
+  bool overlap;
 };
 struct ResidualSink {
   double *partials;     // one FP64 partial per CTA
@@ -156,6 +159,7 @@ struct PointsArgs {
   int d[kMaxPoints][3];
   double w[kMaxPoints];
   bool unit;         // every weight is 1: terms are the point values
+  bool overlap;
   int *err;          // device error word
   CUtensorMap tmap;  // maps `in` with the box points_box() gives
 };
@@ -214,7 +218,8 @@ void jit_unload(JitKernel *k);
 // Runs the compiled stencil over dom (color -1 every point, 0 red, 1 black):
 // grids[] and scalars[] in parameter order.
 cudaError_t jit_launch(const JitKernel &k, const Box &dom, int color, const GridView *grids,
-                       const double *scalars, int sm_count, int *dev_err, cudaStream_t s);
+                       const double *scalars, int sm_count, int *dev_err, bool overlap,
+                       cudaStream_t s);
 
 // Point stencils compiled per stencil (jit.cpp compiles points_body.cuh with
 // the table below as constants).  The key is everything the generated code
@@ -236,8 +241,8 @@ struct PtsJitKey {
 // compared bytewise: zero it before filling it in.
 void *jit_points_function(const PtsJitKey &k, size_t smem, int *occ);
 // Launches a compiled kernel; args[i] points at its i-th parameter.
-cudaError_t jit_launch_raw(void *fn, int grid, dim3 block, size_t smem, cudaStream_t s,
-                           void **args);
+cudaError_t jit_launch_raw(void *fn, int grid, dim3 block, size_t smem, bool overlap,
+                           cudaStream_t s, void **args);
 
 // ---- Learned warm start (nn.cu) -------------------------------------------
 // Fine stacked grids of a batch of Himeno instances (float, row pitch

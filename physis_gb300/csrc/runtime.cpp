@@ -136,6 +136,9 @@ struct Runtime {
   std::map<std::array<int, 4>, psg::Resident7Plan> res_plans;
   std::vector<TmapEntry> tmaps;
   int fail_allocs = 0;
+  // sweeps of the current run may start before the one ahead of them ends (not
+  // while the user captures the stream: a captured launch's edge would be one)
+  bool overlap = false;
   bool fma = false;  // temporal passes may contract multiply-adds
   bool autotune = false;
   std::string tune_path;  // JSON-lines cache file ("" = in memory only)
@@ -541,6 +544,7 @@ bool launch_points_map(const Map &m, const PointStencil &ps) {
     else cfg.warps /= 2;
   }
   a.err = rt->dev_err;
+  a.overlap = rt->overlap;
   int bw = 0, bh = 0;
   psg::points_box(a, cfg, &bw, &bh);
   if (!tmap_for(a.in, bw, bh, &a.tmap)) return false;
@@ -558,6 +562,7 @@ bool launch_points_map(const Map &m, const PointStencil &ps) {
 // One plain sweep of a 7-point-family map with explicit input/output views.
 bool launch_s7(const Map &m, const GridView &in, const GridView &out) {
   psg::Stencil7Args a{};
+  a.overlap = rt->overlap;
   a.kernel = m.kernel;
   a.in = in;
   a.out = out;
@@ -594,7 +599,7 @@ bool launch_function_map(const Map &m, const psg::JitKernel &f) {
   const int ncol = m.color == 2 ? 2 : 1;
   for (int c = 0; c < ncol; ++c) {
     cudaError_t e = psg::jit_launch(f, box, colors[c], views, m.scalars.data(), rt->sm_count,
-                                    rt->dev_err, rt->stream);
+                                    rt->dev_err, rt->overlap, rt->stream);
     if (!cuda_ok(e, "stencil function launch")) return false;
     ++rt->launches;
   }
@@ -615,6 +620,7 @@ bool launch_map(const Map &m, bool want_gosa) {
   cudaError_t e;
   if (m.kernel == PS_KERNEL_HIMENO19 || m.kernel == PS_KERNEL_HIMENO19_GOSA) {
     psg::Himeno19Args a{};
+    a.overlap = rt->overlap;
     for (int i = 0; i < 14; ++i) a.g[i] = view(m.grids[i]);
     a.dom = box;
     a.omega = (float)m.scalars[0];
@@ -645,6 +651,7 @@ bool launch_t7(const Map &m, const GridView &in, const GridView &out, int k) {
   a.out = out;
   a.k = k;
   a.fma = rt->fma;
+  a.overlap = rt->overlap;
   for (int i = 0; i < 7; ++i) a.coef[i] = m.scalars[i];
   const MarchConfig cfg = m.has_plan ? m.plan.tshape : rt->tshapes[shape_slot(m.kernel)];
   const int vec = 16 / in.esz;
@@ -681,12 +688,15 @@ bool pair_eligible(const Map &a, const Map &b) {
 // Runs of fewer iterations stay with ordinary launches.
 constexpr int kResidentMinIter = 4;
 
-// Time per step of plain sweeps of g, in us: float 4.9 at 64^3 (launch and
-// latency), 5.0 at 96^3 and 6.0 at 128^3; double 19.2 up to 64^3 (four planes
-// of a 64 x 16 tile on the FP64 pipe) and 34.6 at 80^3.
+// Time per step of plain sweeps of g, in us: float 2.5 at 32^3 (launch and
+// latency), 3.4 at 64^3, 4.9 at 96^3 and 5.8 from 110^3 to 120^3; double 3.9 for each plane of
+// a 64 x 16 tile that an SM computes (its FP64 pipe): 6.2 up to 48^3, 10.2 at
+// 64^3.
 double plain_sweep_us(const Grid &g) {
   const double cells = (double)g.dim[0] * g.dim[1] * g.dim[2];
-  return g.type == PS_FLOAT ? 4.5 + cells * 8 / 12e6 : std::max(18.0, 1.2 * 13 * cells / 0.42e6);
+  if (g.type == PS_FLOAT) return 2.5 + std::min(cells / 0.42e6, 3.3);
+  const long long planes = (long long)((g.dim[0] + 63) / 64) * ((g.dim[1] + 15) / 16) * g.dim[2];
+  return 2.3 + 3.9 * (double)((planes + rt->sm_count - 1) / rt->sm_count);
 }
 
 bool temporal_pair(const Map &a, const Map &b) {
@@ -750,6 +760,16 @@ bool resident_packets(size_t bytes) {
   return false;
 }
 
+// True if the runtime's stream is being captured.
+bool capturing() {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(rt->stream, &cap) == cudaSuccess &&
+      cap == cudaStreamCaptureStatusNone)
+    return false;
+  cudaGetLastError();
+  return true;
+}
+
 // The plan for running (a, b) x iter in one launch (resident7.cu), or nullptr
 // if another path is to run it: runs whose launch shape the user or the
 // autotuner chose, stream capture, short runs, and grids that do not fit on
@@ -772,12 +792,7 @@ const psg::Resident7Plan *resident_plan(const Map &a, const Map &b, int iter) {
     hit = rt->res_plans.emplace(key, q).first;
   }
   if (hit->second.by == 0) return nullptr;
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(rt->stream, &cap) != cudaSuccess ||
-      cap != cudaStreamCaptureStatusNone) {
-    cudaGetLastError();
-    return nullptr;
-  }
+  if (capturing()) return nullptr;
   return resident_packets(psg::resident7_packet_bytes(key[0], key[1], key[2], key[3]))
              ? &hit->second
              : nullptr;
@@ -1491,7 +1506,22 @@ bool batch_stale(const Batch &b) {
   return false;
 }
 
+// Lets a run's sweeps overlap for as long as the guard lives: a sweep's CTAs take
+// the places that the one before it gives up, set up their barriers and wait
+// there for it to end.  Per sweep, in turn and overlapped, us: 7 points float
+// 64^3 4.2 and 3.2 (one launch a sweep), 512^3 166.6 and 165.0; 9 points
+// 4099 x 3001 19.8 and 17.8; a colour of 319 x 257 x 255 34.9 and 31.9; a 7-point
+// function 400 x 384 x 320 90 and 87.  PS_OVERLAP=0 turns it off.
+struct OverlapGuard {
+  OverlapGuard() {
+    const char *e = getenv("PS_OVERLAP");
+    rt->overlap = !(e && e[0] == '0') && !capturing();
+  }
+  ~OverlapGuard() { rt->overlap = false; }
+};
+
 bool run_maps(const std::vector<Map *> &ms, int iter) {
+  OverlapGuard guard;
   std::chrono::steady_clock::time_point t0;
   if (rt->trace) {
     fprintf(stderr, "Physis: Stencil started\n");

@@ -21,6 +21,7 @@ struct S7Params {
   int zlen;       // planes per z-chunk
   int64_t items;  // tiles * chunks
   int ns;
+  int early;      // the next launch's CTAs may take places while this one runs
   T cc, cw, ce, cs, cn, cb, ct;  // expression order of DIFFUSION7
   int *err;
 };

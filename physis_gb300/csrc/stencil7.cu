@@ -60,6 +60,8 @@ s7_march_kernel(const __grid_constant__ CUtensorMap tin, const S7Params<T> p) {
     fence_barrier_init();
   }
   __syncthreads();
+  if (p.early) launch_dependents();
+  wait_for_predecessors();
 
   // Producer (thread 0) and consumer (all threads) positions in the ring.
   RingPos prod, cons;
@@ -80,7 +82,7 @@ s7_march_kernel(const __grid_constant__ CUtensorMap tin, const S7Params<T> p) {
 
 template <typename T, int K, int RY>
 cudaError_t launch_ry(S7Params<T> p, int tiles, int nzd, const MarchConfig &cfg,
-                      const CUtensorMap *tin, int sm_count, cudaStream_t st) {
+                      const CUtensorMap *tin, int sm_count, bool overlap, cudaStream_t st) {
   const size_t smem = stencil7_smem_bytes((int)sizeof(T), cfg);
   static size_t attr_set = 0;     // dynamic shared memory opted in so far
   static int occ_cached[17][17];  // [warps][ns] -> CTAs per SM (0 = unknown)
@@ -108,8 +110,8 @@ cudaError_t launch_ry(S7Params<T> p, int tiles, int nzd, const MarchConfig &cfg,
   int64_t grid = resident;
   if (grid > p.items) grid = p.items;
   if (grid < 1) grid = 1;
-  kern<<<(unsigned)grid, dim3(32, cfg.warps, 1), smem, st>>>(*tin, p);
-  return cudaGetLastError();
+  p.early = grid == resident;
+  return launch_kernel(kern, (unsigned)grid, dim3(32, cfg.warps, 1), smem, st, overlap, *tin, p);
 }
 
 template <typename T, int K>
@@ -152,10 +154,10 @@ cudaError_t launch_t(const Stencil7Args &a, const MarchConfig &cfg,
   p.tiles_x = (ex + TX - 1) / TX;
   const int tiles = p.tiles_x * ((ey + ty - 1) / ty);
   switch (cfg.rows) {
-    case 1: return launch_ry<T, K, 1>(p, tiles, ez, cfg, tin, sm_count, st);
-    case 2: return launch_ry<T, K, 2>(p, tiles, ez, cfg, tin, sm_count, st);
-    case 4: return launch_ry<T, K, 4>(p, tiles, ez, cfg, tin, sm_count, st);
-    case 8: return launch_ry<T, K, 8>(p, tiles, ez, cfg, tin, sm_count, st);
+    case 1: return launch_ry<T, K, 1>(p, tiles, ez, cfg, tin, sm_count, a.overlap, st);
+    case 2: return launch_ry<T, K, 2>(p, tiles, ez, cfg, tin, sm_count, a.overlap, st);
+    case 4: return launch_ry<T, K, 4>(p, tiles, ez, cfg, tin, sm_count, a.overlap, st);
+    case 8: return launch_ry<T, K, 8>(p, tiles, ez, cfg, tin, sm_count, a.overlap, st);
   }
   return cudaErrorInvalidConfiguration;
 }

@@ -45,6 +45,7 @@ struct TParams {
   int tiles_x, tiles, zlen;
   int64_t items;
   int ns;
+  int early;           // the next launch's CTAs may take places while this one runs
   T cc, cw, ce, cs, cn, cb, ct;
   int *err;
 };
@@ -217,6 +218,8 @@ t7_kernel(const __grid_constant__ CUtensorMap tin, const TParams<T> p) {
   // keep the (discarded) border cells finite.
   for (int i = tid; i < (K - 1) * 2 * plane_elems; i += nthreads) bufs[i] = T(0);
   __syncthreads();
+  if (p.early) launch_dependents();
+  wait_for_predecessors();
 
   int pstage = 0, cstage = 0;
   uint32_t pphase = 0, cphase = 0;
@@ -322,7 +325,7 @@ t7_kernel(const __grid_constant__ CUtensorMap tin, const TParams<T> p) {
 
 template <typename T, int RY, int K, bool FMA>
 cudaError_t launch_k(TParams<T> p, const MarchConfig &cfg, const CUtensorMap *tin,
-                     int sm_count, cudaStream_t st) {
+                     int sm_count, bool overlap, cudaStream_t st) {
   constexpr int VEC = 16 / (int)sizeof(T);
   constexpr int TXO = 30 * VEC;
   const int tye = cfg.warps * cfg.rows;
@@ -349,30 +352,30 @@ cudaError_t launch_k(TParams<T> p, const MarchConfig &cfg, const CUtensorMap *ti
   p.items = (int64_t)p.tiles * ((p.nz + p.zlen - 1) / p.zlen);
   int64_t grid = resident;
   if (grid > p.items) grid = p.items;
-  kern<<<(unsigned)grid, dim3(32, cfg.warps, 1), smem, st>>>(*tin, p);
-  return cudaGetLastError();
+  p.early = grid == resident;
+  return launch_kernel(kern, (unsigned)grid, dim3(32, cfg.warps, 1), smem, st, overlap, *tin, p);
 }
 
 template <typename T, int RY, bool FMA>
 cudaError_t launch_rows(const TParams<T> &p, const MarchConfig &cfg, const CUtensorMap *tin,
-                        int sm_count, cudaStream_t st) {
+                        int sm_count, bool overlap, cudaStream_t st) {
   constexpr int VEC = 16 / (int)sizeof(T);
-  if (p.k <= 2) return launch_k<T, RY, 2, FMA>(p, cfg, tin, sm_count, st);
-  if (p.k <= 3) return launch_k<T, RY, 3, FMA>(p, cfg, tin, sm_count, st);
+  if (p.k <= 2) return launch_k<T, RY, 2, FMA>(p, cfg, tin, sm_count, overlap, st);
+  if (p.k <= 3) return launch_k<T, RY, 3, FMA>(p, cfg, tin, sm_count, overlap, st);
   if constexpr (VEC >= 4) {
-    if (p.k <= 4) return launch_k<T, RY, 4, FMA>(p, cfg, tin, sm_count, st);
-    if (p.k <= 5) return launch_k<T, RY, 5, FMA>(p, cfg, tin, sm_count, st);
+    if (p.k <= 4) return launch_k<T, RY, 4, FMA>(p, cfg, tin, sm_count, overlap, st);
+    if (p.k <= 5) return launch_k<T, RY, 5, FMA>(p, cfg, tin, sm_count, overlap, st);
   }
   return cudaErrorInvalidValue;
 }
 
 template <typename T, bool FMA>
 cudaError_t launch_shape(const TParams<T> &p, const MarchConfig &cfg, const CUtensorMap *tin,
-                         int sm_count, cudaStream_t st) {
+                         int sm_count, bool overlap, cudaStream_t st) {
   switch (cfg.rows) {
-    case 1: return launch_rows<T, 1, FMA>(p, cfg, tin, sm_count, st);
-    case 2: return launch_rows<T, 2, FMA>(p, cfg, tin, sm_count, st);
-    case 4: return launch_rows<T, 4, FMA>(p, cfg, tin, sm_count, st);
+    case 1: return launch_rows<T, 1, FMA>(p, cfg, tin, sm_count, overlap, st);
+    case 2: return launch_rows<T, 2, FMA>(p, cfg, tin, sm_count, overlap, st);
+    case 4: return launch_rows<T, 4, FMA>(p, cfg, tin, sm_count, overlap, st);
   }
   return cudaErrorInvalidConfiguration;
 }
@@ -399,8 +402,8 @@ cudaError_t launch_t(const Temporal7Args &a, const MarchConfig &cfg, const CUten
   p.err = dev_err;
   if (cfg.warps < 1 || cfg.warps > 8 || cfg.ns < 2 || cfg.ns > 16)
     return cudaErrorInvalidConfiguration;
-  return a.fma ? launch_shape<T, true>(p, cfg, tin, sm_count, st)
-               : launch_shape<T, false>(p, cfg, tin, sm_count, st);
+  return a.fma ? launch_shape<T, true>(p, cfg, tin, sm_count, a.overlap, st)
+               : launch_shape<T, false>(p, cfg, tin, sm_count, a.overlap, st);
 }
 
 }  // namespace

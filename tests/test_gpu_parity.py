@@ -192,6 +192,48 @@ def test_diffusion_run_in_one_launch(rt, oracle, monkeypatch, shape, dtype, iter
         assert np.array_equal(_bits(b), _bits(r2))
 
 
+AVERAGE = """
+void average(const int x, const int y, const int z, PSGrid3D%s in, PSGrid3D%s out) {
+  PSGridEmit(out, (PSGridGet(in, x, y, z) + PSGridGetPeriodic(in, x + 1, y, z) +
+                   PSGridGetPeriodic(in, x, y - 1, z) + PSGridGetPeriodic(in, x, y, z + 1)) / 4);
+}
+"""
+
+
+# A run's launches may start while the one ahead of them still runs: every kind
+# of sweep after every other, each reading what the one before wrote and
+# overwriting what it read, on a grid smaller than the GPU and one that fills it,
+# launched directly and from a graph.  In turn (PS_OVERLAP=0) gives the same bits.
+@pytest.mark.parametrize("shape,dtype,iters", [
+    ((7, 20, 70), np.float32, 3), ((12, 33, 41), np.float64, 19),
+    ((96, 130, 260), np.float32, 18), ((60, 70, 200), np.float64, 3)])
+def test_overlapping_sweeps_keep_their_order(rt, monkeypatch, shape, dtype, iters):
+    c = "Float" if dtype == np.float32 else "Double"
+    init = synth.uniform(shape, 23).astype(dtype)
+    f = ps.stencil_function(AVERAGE % (c, c), "average")
+    pts = [(0, 0, 0), (-1, 0, 0), (1, 1, 0), (0, 0, -1), (0, -1, 1)]
+    k = ps.point_stencil(pts, weights=[0.3, 0.2, 0.2, 0.15, 0.15], boundary=2)
+    dom = ps.full_domain(shape)
+    got = {}
+    for env in ("1", "0"):
+        monkeypatch.setenv("PS_OVERLAP", env)
+        a, b = ps.Grid(shape, dtype), ps.Grid(shape, dtype)
+        a.copyin(init)
+        b.copyin(init)
+        ps.stencil_run([
+            ps.stencil_map(ps.PS_KERNEL_DIFFUSION7, dom, [a, b], DIFF_COEF),
+            ps.stencil_map(k, dom, [b, a]),
+            ps.stencil_map(f, dom, [a, b]),
+            ps.stencil_map_color(ps.PS_KERNEL_DIFFUSION7, 2, dom, [b], DIFF_COEF),
+            ps.stencil_map(ps.PS_KERNEL_DIFFUSION7, dom, [b, a], DIFF_COEF),
+            ps.stencil_map(f, dom, [a, b]), ps.stencil_map(k, dom, [b, a])], iters)
+        got[env] = a.copyout().copy(), b.copyout().copy()
+        a.free()
+        b.free()
+    for x, y in zip(got["1"], got["0"]):
+        assert np.array_equal(_bits(x), _bits(y))
+
+
 def test_one_launch_runs_repeat_and_keep_their_storage(rt, oracle):
     # three runs of two grids in turn: exchange packets of earlier runs and of
     # the other grid size stay behind; each run continues from the last
