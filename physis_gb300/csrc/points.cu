@@ -50,6 +50,7 @@
 //   sequential REF one.
 #include <cstdlib>
 #include <cstring>
+#include <type_traits>
 
 #include "points_body.cuh"
 #include "ps_device.cuh"
@@ -148,10 +149,19 @@ int schedule(PtsParams<T> *p, int occ, int sm_count) {
   // next item, so a short chunk's halo planes cost little (33 x 65 x 79, 27
   // points: 5.4 us a sweep against 7.7 with four planes)
   p->zlen = choose_zchunk_overhead(p->tiles, nzd, resident, p->rzl + p->rzh + 1, resident);
+  // Wide enough double stencils are bound by the FP64 pipes, whose shares even out
+  // best with one CTA per plane of a tile, handed to whichever SM is free (7
+  // points 300 x 200 x 250: 364 us a sweep against 416); with fewer than 16 rounds
+  // the round-robin is as good.
+  const int planes = p->rzl + p->rzh + 1;
+  const bool spread = std::is_same<T, double>::value && p->n >= 2 * planes &&
+                      (long long)p->tiles * nzd >= 16LL * resident &&
+                      (long long)p->tiles * nzd <= 0x7fffffff;
+  if (spread) p->zlen = 1;
   const int chunks = (nzd + p->zlen - 1) / p->zlen;
   p->items = (long long)p->tiles * chunks;
   p->early = p->items >= resident;
-  return (int)(p->items < resident ? p->items : resident);
+  return (int)(p->items < resident || spread ? p->items : resident);
 }
 
 template <typename T>

@@ -405,6 +405,7 @@ __device__ __forceinline__ void pts_body(const PtsParams<T> &p, const void *tmap
     for (int r = 0; r < RY; ++r)
       if (y0 + row0 + r < p.dmax1) rowmask |= 1u << r;
     const bool whole = colmask == (1u << kPtsVX) - 1u && rowmask == (1u << RY) - 1u;
+    const bool any = __any_sync(0xffffffffu, colmask && rowmask);  // else nothing to do
     T *dst = p.out + (long long)zs * p.plane + (long long)(y0 + row0) * p.row + x0 +
              xl * (S::kStatic ? VEC : 1);
 
@@ -418,7 +419,7 @@ __device__ __forceinline__ void pts_body(const PtsParams<T> &p, const void *tmap
         if (++wslot == NST) wslot = 0;
       }
 
-      if (ok) {
+      if (ok && any) {
         T acc[RY][kPtsVX];
         if constexpr (S::kStatic) {
           const T *pl[S::kPlanes];

@@ -125,6 +125,8 @@ __device__ __forceinline__ bool s7_item(const CUtensorMap *tin, const S7Params<T
     }
 #pragma unroll
     for (int r = 0; r < RY; ++r) {
+      // double precision is short of FP64 issue: nothing for rows outside
+      if (sizeof(T) == 8 && y + r >= p.dmax1) break;
       T o[VEC];
       if (K == kKernelCopy) {
 #pragma unroll

@@ -105,12 +105,18 @@ cudaError_t launch_ry(S7Params<T> p, int tiles, int nzd, const MarchConfig &cfg,
   const int per_sm = (cfg.ctas_per_sm > 0 && cfg.ctas_per_sm < oc) ? cfg.ctas_per_sm : oc;
   const int resident = sm_count * per_sm;
   p.tiles = tiles;
-  p.zlen = choose_zchunk(tiles, nzd, resident, sm_count);
+  // Double precision has one bound, the FP64 pipe of an SM, so it is the SMs'
+  // shares that must be even: one CTA per plane of a tile, which the hardware hands to
+  // whichever SM is free, instead of a round-robin of longer chunks (155 x 105 x 127
+  // 68.7 us a sweep against 85, 300 x 200 x 250 404 against 428, 72^3 21.9 against
+  // 34; two planes cost 0-13 % more, four 1-28 %).
+  const bool spread = std::is_same<T, double>::value && K != kKernelCopy && cfg.ctas_per_sm == 0;
+  p.zlen = spread ? 1 : choose_zchunk(tiles, nzd, resident, sm_count);
   p.items = (int64_t)tiles * ((nzd + p.zlen - 1) / p.zlen);
   int64_t grid = resident;
-  if (grid > p.items) grid = p.items;
+  if (grid > p.items || spread) grid = p.items;
   if (grid < 1) grid = 1;
-  p.early = grid == resident;
+  p.early = grid >= resident;
   return launch_kernel(kern, (unsigned)grid, dim3(32, cfg.warps, 1), smem, st, overlap, *tin, p);
 }
 

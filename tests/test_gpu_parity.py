@@ -192,6 +192,34 @@ def test_diffusion_run_in_one_launch(rt, oracle, monkeypatch, shape, dtype, iter
         assert np.array_equal(_bits(b), _bits(r2))
 
 
+# Double sweeps go plane by plane to whichever SM is free and skip rows outside
+# the domain: domains that end inside a tile and a warp's rows, one plane, enough
+# planes for several rounds, and point stencils on either side of their rule.
+@pytest.mark.parametrize("shape,dom", [
+    ((5, 17, 66), None), ((1, 40, 70), None), ((90, 33, 130), (1, 129, 1, 32, 1, 89)),
+    ((40, 50, 65), (3, 60, 5, 38, 2, 39)), ((130, 150, 200), None)])
+def test_double_sweeps_plane_by_plane(rt, oracle, shape, dom):
+    nz, ny, nx = shape
+    dom = dom or (0, nx, 0, ny, 0, nz)
+    init = synth.uniform(shape, 24).astype(np.float64)
+    r1, r2 = init.copy(), init.copy()
+    oracle.run7(oracle.V_DIFFUSION7, r1, r2, dom, DIFF_COEF, iter=2)
+    a, b = run_pingpong(ps.PS_KERNEL_DIFFUSION7, init, ps.domain(*dom), DIFF_COEF, 2, np.float64)
+    assert np.array_equal(_bits(a), _bits(r1))
+    assert np.array_equal(_bits(b), _bits(r2))
+    pts = [(0, 0, 0), (-1, 0, 0), (1, 0, 0), (0, 1, 0), (0, -1, 0), (0, 0, -1), (0, 0, 1)]
+    w = [0.4, 0.1, 0.1, 0.1, 0.1, 0.1, 0.1]
+    out = np.zeros_like(init)
+    oracle.points(init, out, dom, pts, weights=w, boundary=2)
+    g = [ps.Grid(shape, np.float64) for _ in range(2)]
+    g[0].copyin(init)
+    ps.stencil_run([ps.stencil_map(ps.point_stencil(pts, weights=w, boundary=2), ps.domain(*dom), g)])
+    got = g[1].copyout()
+    for x in g:
+        x.free()
+    assert np.array_equal(_bits(got), _bits(out))
+
+
 AVERAGE = """
 void average(const int x, const int y, const int z, PSGrid3D%s in, PSGrid3D%s out) {
   PSGridEmit(out, (PSGridGet(in, x, y, z) + PSGridGetPeriodic(in, x + 1, y, z) +
