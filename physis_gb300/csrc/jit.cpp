@@ -984,13 +984,19 @@ cudaError_t jit_launch(const JitKernel &k, const Box &dom, int color, const Grid
     // z chunks: one wave of resident CTAs while chunks are short, else chunks
     // of five planes (times the stencil's z radius): many small CTAs even out
     // edge tiles and tails, and neighbouring chunks' halo planes come from L2
-    // (400 x 384 x 320, 7 points: 90 us a sweep with 5 planes, 98 with 36, 116
-    // with 32 -- a little over one wave -- and 146 with 64; a double 27-point sweep
-    // 686, 725, 776 and 1031 us for 5, 12, 32 and 64).
+    // (400 x 384 x 320, 7 points: 88 us a sweep with 5 planes, 98 with 2, 129 with
+    // 1, 91 with 12).  Double functions are bound by the SMs' FP64 pipes, which
+    // chunks of one plane (or the radius) share out best: 27 points 281 x 194 x 51
+    // 152 us with 1 plane, 157 with 2, 195 with 3, 164 with 5; 258 x 258 x 200 674,
+    // 676, 677 and 684; 7 points 200 x 150 x 180 163, 167, 174 and 180.
     const long long want = std::max(1LL, (long long)k.tiled_occ * sm_count);
     int rz = 1;
-    for (const JitStage &st : k.stages) rz = std::max(rz, st.rz);
-    const int zlen = (int)std::max({1LL, std::min((long long)nzd * tiles / want, 5LL * rz),
+    bool fp64 = false;
+    for (const JitStage &st : k.stages) {
+      rz = std::max(rz, st.rz);
+      fp64 |= k.params[st.param].type == kDouble;
+    }
+    const int zlen = (int)std::max({1LL, std::min((long long)nzd * tiles / want, (fp64 ? 1LL : 5LL) * rz),
                                     (nzd + 65534LL) / 65535});
     const long long chunks = (nzd + zlen - 1) / zlen;
     if (tiles > 0x7fffffffLL || chunks > 65535) return cudaErrorInvalidConfiguration;

@@ -524,6 +524,12 @@ def test_function_tiles_and_edges_bit_exact(rt, oracle, shape, dtype, periodic, 
     b.free()
 
 
+# Double functions take chunks of one plane, or of the radius, in many rounds.
+@pytest.mark.parametrize("shape,radius", [((60, 150, 200), (1, 1, 1)), ((41, 90, 330), (2, 1, 3))])
+def test_double_function_chunks_bit_exact(rt, oracle, shape, radius):
+    test_function_tiles_and_edges_bit_exact(rt, oracle, shape, np.float64, True, radius, (0, 0, 0))
+
+
 TWO_STAGED = r"""
 void two(const int x, const int y, const int z, PSGrid3DFloat a, PSGrid3DDouble k,
          PSGrid3DFloat out, PSGrid2DFloat m) {
