@@ -7,14 +7,13 @@
 // of all problems form one list, problem after problem and chunk-major within
 // a problem; a persistent grid of SMs x occupancy CTAs takes items
 // round-robin, so small problems fill the GPU together and large ones keep
-// the chunk-major locality of the single-run kernels.  A CTA finds an item's
-// problem by binary search over the problems' first item indices and runs
-// the shared per-item body (s7_body.cuh / himeno_body.cuh) with that
+// the chunk-major locality of the single-run kernels.  A CTA's items ascend, so
+// it finds an item's problem by stepping on from the last one's, and runs the
+// shared per-item body (s7_body.cuh / himeno_body.cuh) with that
 // problem's parameters and tensor maps, both read from global memory.
 // Problem kinds: the 7-point family (DIFFUSION7, SUM7, COPY; 1, 2 or 4 rows
-// per thread) and the plain Himeno sweep, float grids.  The kernel is built
-// per family (FAM = kBatch7, kBatchHimeno) so that each launch carries only
-// its family's registers and shared memory; a batch holding both families
+// per thread) and the plain Himeno sweep, float grids.  Each family has its own
+// kernel so that each launch carries only its family's registers and shared memory; a batch holding both families
 // launches one of each per step.
 #include "batch.h"
 #include "himeno_body.cuh"
@@ -44,69 +43,91 @@ __device__ __forceinline__ bool s7_rows(const BatchProblem &bp, int parity,
                               prod, cons);
 }
 
-template <int FAM>
+// Problem of an item at or after those of problem `q`: items of a CTA ascend.
+__device__ __forceinline__ int batch_problem(const BatchProblem *__restrict__ probs, int nprob,
+                                             int64_t item, int q) {
+  while (q + 1 < nprob && probs[q + 1].item_begin <= item) ++q;
+  return q;
+}
+
 __global__ void __launch_bounds__(256, 1)
-batch_kernel(const BatchProblem *__restrict__ probs, int nprob, const CUtensorMap *tmaps,
-             int64_t total_items, int parity, int ns7, int nsp, int nsc) {
+batch7_kernel(const BatchProblem *__restrict__ probs, int nprob, const CUtensorMap *tmaps,
+              int64_t total_items, int parity, int ns7) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   unsigned char *smem = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);
-  uint64_t *full7 = reinterpret_cast<uint64_t *>(smem);
-  uint64_t *pfull = full7 + ns7;
-  uint64_t *cfull = pfull + nsp;
-  unsigned char *data = smem + s7_bar_bytes(ns7 + nsp + nsc);
-  // The 7-point ring and the Himeno rings share the data region: an item
-  // consumes every plane it issues before the next item starts.
-  float *ring7 = reinterpret_cast<float *>(data);
-  const int TYh = blockDim.y;
-  const int p_elems = (int)(h_align128((uint32_t)(kHimW * (TYh + 2) * 4)) / 4);
-  float *pring = reinterpret_cast<float *>(data);
-  float *cring = pring + nsp * p_elems;
-
+  uint64_t *full = reinterpret_cast<uint64_t *>(smem);
+  float *ring = reinterpret_cast<float *>(smem + s7_bar_bytes(ns7));
   const int tid = threadIdx.y * 32 + threadIdx.x;
   if (tid == 0) {
-    for (int s = 0; s < ns7 + nsp + nsc; ++s) mbar_init(&full7[s], 1);
+    for (int s = 0; s < ns7; ++s) mbar_init(&full[s], 1);
     fence_barrier_init();
   }
   __syncthreads();
 
-  RingPos prod7, cons7;
-  HRing pprod, pcons, cprod, ccons;
-  float acc = 0.0f;
+  RingPos prod, cons;
   bool ok = true;
+  int q = 0;
   for (int64_t item = blockIdx.x; item < total_items && ok; item += gridDim.x) {
-    int lo = 0, hi = nprob - 1;  // last problem whose first item <= item
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (probs[mid].item_begin <= item) lo = mid;
-      else hi = mid - 1;
-    }
-    const BatchProblem &bp = probs[lo];
+    q = batch_problem(probs, nprob, item, q);
+    const BatchProblem &bp = probs[q];
     const int64_t local = item - bp.item_begin;
     const int chunk = (int)(local / bp.tiles);
     const int tile = (int)(local - (int64_t)chunk * bp.tiles);
     const int zs = bp.dmin2 + chunk * bp.zlen;
     const int ze = min(zs + bp.zlen, bp.dmax2);
-    if constexpr (FAM == kBatch7) {
-      switch (bp.kind) {
-        case kKernelDiffusion7:
-          ok = s7_rows<kKernelDiffusion7>(bp, parity, tmaps, full7, ring7, tile, zs, ze, prod7,
-                                          cons7);
-          break;
-        case kKernelSum7:
-          ok = s7_rows<kKernelSum7>(bp, parity, tmaps, full7, ring7, tile, zs, ze, prod7, cons7);
-          break;
-        default:
-          ok = s7_rows<kKernelCopy>(bp, parity, tmaps, full7, ring7, tile, zs, ze, prod7, cons7);
-          break;
-      }
-    } else {
-      ok = himeno_item<false>(tmaps + bp.tmap[parity], tmaps + bp.cmap, bp.him[parity], pfull,
-                              cfull, pring, cring, tile, zs, ze, pprod, pcons, cprod, ccons, acc);
+    switch (bp.kind) {
+      case kKernelDiffusion7:
+        ok = s7_rows<kKernelDiffusion7>(bp, parity, tmaps, full, ring, tile, zs, ze, prod, cons);
+        break;
+      case kKernelSum7:
+        ok = s7_rows<kKernelSum7>(bp, parity, tmaps, full, ring, tile, zs, ze, prod, cons);
+        break;
+      default:
+        ok = s7_rows<kKernelCopy>(bp, parity, tmaps, full, ring, tile, zs, ze, prod, cons);
+        break;
     }
   }
   if (!ok && tid == 0) {
-    for (int s = 0; s < ns7 + nsp + nsc; ++s) mbar_wait(&full7[s], 0, nullptr, 1024);
+    for (int s = 0; s < ns7; ++s) mbar_wait(&full[s], 0, nullptr, 1024);
   }
+}
+
+__global__ void __maxnreg__(128)
+batch_himeno_kernel(const BatchProblem *__restrict__ probs, int nprob, const CUtensorMap *tmaps,
+                    int64_t total_items, int parity, int nsp, int nsc) {
+  const int warps = blockDim.y - 1;  // consumers; the last warp is the producer
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  unsigned char *smem = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);
+  const HimSmem h = him_smem(smem, nsp, nsc, warps);
+  const int lane = threadIdx.x, row = threadIdx.y, tid = row * 32 + lane;
+  if (tid == 0) him_init(h, nsp, nsc, warps);
+  __syncthreads();
+
+  HRing pprod, cprod, pcons, prel, ccons;
+  float acc = 0.0f;
+  bool ok = true;
+  int q = 0;
+  if (row < warps || lane == 0) {
+    for (int64_t item = blockIdx.x; item < total_items && ok; item += gridDim.x) {
+      q = batch_problem(probs, nprob, item, q);
+      const BatchProblem &bp = probs[q];
+      const HParams &p = bp.him[parity];
+      const int local = (int)(item - bp.item_begin);
+      const int chunk = local / bp.tiles, tile = local - chunk * bp.tiles;
+      const int zs = bp.dmin2 + chunk * bp.zlen;
+      const int ze = min(zs + bp.zlen, bp.dmax2);
+      if (row == warps)
+        ok = himeno_produce(tmaps + bp.tmap[parity], tmaps + bp.cmap, p, h, warps, bp.lx, tile, zs,
+                            ze, pprod, cprod);
+      else if (bp.lx == 32)
+        ok = himeno_consume<false, 32>(p, h, warps, tile, zs, ze, pcons, prel, ccons, acc);
+      else if (bp.lx == 16)
+        ok = himeno_consume<false, 16>(p, h, warps, tile, zs, ze, pcons, prel, ccons, acc);
+      else
+        ok = himeno_consume<false, 8>(p, h, warps, tile, zs, ze, pcons, prel, ccons, acc);
+    }
+  }
+  if (!__syncthreads_and(ok) && tid == 0) him_drain(h, nsp, nsc);
 }
 
 }  // namespace
@@ -115,14 +136,17 @@ size_t batch_smem_bytes(const BatchShape &sh, int fam) {
   const size_t r7 = (size_t)sh.ns7 * s7_stage_bytes((uint32_t)(34 * 4 * (sh.warps * sh.max_rows + 2) * 4));
   const size_t rh = (size_t)sh.nsp * h_align128((uint32_t)(kHimW * (sh.warps + 2) * 4)) +
                     (size_t)sh.nsc * kHimCoef * kHimTX * sh.warps * 4;
-  return 128 + (size_t)s7_bar_bytes(sh.ns7 + sh.nsp + sh.nsc) + (fam == kBatch7 ? r7 : rh);
+  return 128 + (fam == kBatch7 ? (size_t)s7_bar_bytes(sh.ns7) + r7
+                               : (size_t)h_bar_bytes(2 * (sh.nsp + sh.nsc)) + rh);
 }
 
 namespace {
 const void *batch_fn(int fam) {
-  return fam == kBatch7 ? reinterpret_cast<const void *>(batch_kernel<kBatch7>)
-                        : reinterpret_cast<const void *>(batch_kernel<kBatchHimeno>);
+  return fam == kBatch7 ? reinterpret_cast<const void *>(batch7_kernel)
+                        : reinterpret_cast<const void *>(batch_himeno_kernel);
 }
+// Himeno CTAs have a producer warp besides.
+int batch_warps(const BatchShape &sh, int fam) { return sh.warps + (fam == kBatchHimeno ? 1 : 0); }
 }  // namespace
 
 int batch_occupancy(const BatchShape &sh, int fam) {
@@ -130,7 +154,8 @@ int batch_occupancy(const BatchShape &sh, int fam) {
   const size_t smem = batch_smem_bytes(sh, fam);
   if (cudaFuncSetAttribute(batch_fn(fam), cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)smem) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&oc, batch_fn(fam), 32 * sh.warps, smem) !=
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&oc, batch_fn(fam),
+                                                    32 * batch_warps(sh, fam), smem) !=
           cudaSuccess) {
     cudaGetLastError();
     return 0;
@@ -142,12 +167,13 @@ cudaError_t launch_batch(const BatchProblem *probs_dev, int nprob, const CUtenso
                          int64_t total_items, int parity, const BatchShape &sh, int grid, int fam,
                          cudaStream_t s) {
   const size_t smem = batch_smem_bytes(sh, fam);
+  const dim3 block(32, batch_warps(sh, fam), 1);
   if (fam == kBatch7)
-    batch_kernel<kBatch7><<<grid, dim3(32, sh.warps, 1), smem, s>>>(
-        probs_dev, nprob, tmaps_dev, total_items, parity, sh.ns7, sh.nsp, sh.nsc);
+    batch7_kernel<<<grid, block, smem, s>>>(probs_dev, nprob, tmaps_dev, total_items, parity,
+                                            sh.ns7);
   else
-    batch_kernel<kBatchHimeno><<<grid, dim3(32, sh.warps, 1), smem, s>>>(
-        probs_dev, nprob, tmaps_dev, total_items, parity, sh.ns7, sh.nsp, sh.nsc);
+    batch_himeno_kernel<<<grid, block, smem, s>>>(probs_dev, nprob, tmaps_dev, total_items, parity,
+                                                  sh.nsp, sh.nsc);
   return cudaGetLastError();
 }
 

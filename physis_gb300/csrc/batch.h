@@ -10,6 +10,7 @@ namespace psg {
 struct BatchProblem {
   int kind;            // kKernelDiffusion7 / kKernelSum7 / kKernelCopy / kKernelHimeno19
   int rows;            // 7-point: rows per thread (1, 2 or 4)
+  int lx;              // Himeno: lanes side by side in x
   int64_t item_begin;  // index of this problem's first item in the batch
   int64_t items;
   int tiles, zlen, dmin2, dmax2;

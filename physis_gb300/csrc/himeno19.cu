@@ -10,14 +10,16 @@
 // Design (persistent, like the 7-point kernel: (z-chunk, tile) work items in
 // chunk-major order taken round-robin by SMs x occupancy CTAs, so resident
 // CTAs march the same z-chunk of neighbouring tiles; a tile is 128 x warps
-// cells in x,y):
+// cells in x,y, or 64 or 32 cells wide and higher, see himeno19_lanes):
 // * p planes with a one-cell y halo and a 4-cell (16-byte) x halo arrive by
 //   TMA into a ring of `ns` stages; the sweep at plane z reads planes z-1, z
 //   and z+1 from the ring (the 19-point stencil needs xy neighbours on all
 //   three planes, so a register queue alone does not suffice);
 // * the 12 centre-only coefficient arrays (a0..a3, b0..b2, c0..c2, bnd,
-//   wrk1) arrive as 12 TMA boxes of 128 x warps per plane into a second ring
+//   wrk1) arrive as 12 TMA boxes of the tile per plane into a second ring
 //   of `ns2` stages, all signalled by one mbarrier per stage;
+// * a producer warp fills both rings, on into the CTA's next item; consumer
+//   warps release stages one by one, so nothing drains between items;
 // * one thread per 4 consecutive x cells: 16-byte shared loads, x neighbours
 //   by warp shuffles, one 16-byte store;
 // * the arithmetic keeps the reference's expression order, round-to-nearest
@@ -25,14 +27,19 @@
 // * residual: FP32 per thread, FP32 warp-shuffle + block tree, one FP64
 //   partial per CTA, and the last CTA to finish (atomic ticket) adds the
 //   partials in FP64 in a fixed order (deterministic run to run).
+// Bound: HBM, 14 arrays of 4 bytes a cell; 257 x 257 x 513 takes 290 us with the
+// residual, 270 at the copy rate.  Against 128-cell tiles filled by a consumer
+// between CTA barriers, a sweep with its residual read back: 200^3 100 against
+// 114 us, 142 x 245 x 97 57 and 74, 65^3 28 and 37.  All coefficients loaded before any is
+// used takes 155 registers for 96, one CTA of three per SM and 4 % more time.
 #include "himeno_body.cuh"
 
 namespace psg {
 namespace {
 
 struct HimenoMaps {
-  CUtensorMap p;               // p0 with halo box {kHimW, TY+2, 1}
-  CUtensorMap coef[kHimCoef];  // box {kHimTX, TY, 1}
+  CUtensorMap p;               // p0 with the tile's halo box
+  CUtensorMap coef[kHimCoef];  // the tile's box
 };
 
 __device__ __forceinline__ float warp_sum(float v) {
@@ -46,21 +53,13 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
-template <bool GOSA>
-__global__ void __launch_bounds__(256, 1)
+template <bool GOSA, int LX>
+__global__ void __maxnreg__(128)
 himeno19_kernel(const __grid_constant__ HimenoMaps maps, const HParams p) {
-  typedef RN<float> R;
-  const int TY = blockDim.y;
-  const int nsp = p.nsp, nsc = p.nsc;
-  const uint32_t p_bytes = (uint32_t)(kHimW * (TY + 2) * 4);
-  const int p_elems = (int)(h_align128(p_bytes) / 4);  // stage stride
-
+  const int warps = blockDim.y - 1;  // consumers; the last warp is the producer
   extern __shared__ __align__(128) unsigned char smem_raw[];
   unsigned char *smem = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);
-  uint64_t *pfull = reinterpret_cast<uint64_t *>(smem);
-  uint64_t *cfull = pfull + nsp;
-  float *pring = reinterpret_cast<float *>(smem + h_bar_bytes(nsp + nsc));
-  float *cring = pring + nsp * p_elems;
+  const HimSmem h = him_smem(smem, p.nsp, p.nsc, warps);
   __shared__ float red[32];
   __shared__ int last_cta;
 
@@ -68,42 +67,39 @@ himeno19_kernel(const __grid_constant__ HimenoMaps maps, const HParams p) {
   const int tid = row * 32 + lane;
   if (tid == 0) {
     prefetch_tmap(&maps.p);
-    for (int s = 0; s < nsp; ++s) mbar_init(&pfull[s], 1);
-    for (int s = 0; s < nsc; ++s) mbar_init(&cfull[s], 1);
-    fence_barrier_init();
+    him_init(h, p.nsp, p.nsc, warps);
   }
   __syncthreads();
   if (p.early) launch_dependents();
   wait_for_predecessors();
 
-  HRing pprod, pcons, cprod, ccons;
+  HRing pprod, cprod, pcons, prel, ccons;
   bool ok = true;
   float acc = 0.0f;
-  for (int64_t item = blockIdx.x; item < p.items && ok; item += gridDim.x) {
-    const int chunk = (int)(item / p.tiles);
-    const int tile = (int)(item - (int64_t)chunk * p.tiles);
-    const int zs = p.dmin2 + chunk * p.zlen;
-    const int ze = min(zs + p.zlen, p.dmax2);
-    ok = himeno_item<GOSA>(&maps.p, maps.coef, p, pfull, cfull, pring, cring, tile, zs, ze,
-                           pprod, pcons, cprod, ccons, acc);
-  }
-  if (!ok) {
-    if (tid == 0) {
-      // Give copies still in flight a bounded chance to land before exit.
-      for (int s = 0; s < nsp; ++s) mbar_wait(&pfull[s], 0, nullptr, 1024);
-      for (int s = 0; s < nsc; ++s) mbar_wait(&cfull[s], 0, nullptr, 1024);
+  if (row < warps || lane == 0) {
+    for (int64_t item = blockIdx.x; item < p.items && ok; item += gridDim.x) {
+      const int chunk = (int)(item / p.tiles);
+      const int tile = (int)(item - (int64_t)chunk * p.tiles);
+      const int zs = p.dmin2 + chunk * p.zlen;
+      const int ze = min(zs + p.zlen, p.dmax2);
+      ok = row < warps ? himeno_consume<GOSA, LX>(p, h, warps, tile, zs, ze, pcons, prel, ccons, acc)
+                       : himeno_produce(&maps.p, maps.coef, p, h, warps, LX, tile, zs, ze, pprod,
+                                        cprod);
     }
+  }
+  if (!__syncthreads_and(ok)) {
+    if (tid == 0) him_drain(h, p.nsp, p.nsc);
     return;
   }
   if (!GOSA) return;
 
   // Residual: FP32 block tree, FP64 partial per CTA, FP64 final combine.
   acc = warp_sum(acc);
-  if (lane == 0) red[row] = acc;
+  if (lane == 0 && row < warps) red[row] = acc;
   __syncthreads();
   if (tid == 0) {
     float bs = 0.0f;
-    for (int w = 0; w < TY; ++w) bs = __fadd_rn(bs, red[w]);
+    for (int w = 0; w < warps; ++w) bs = __fadd_rn(bs, red[w]);
     p.partials[blockIdx.x] = (double)bs;
     __threadfence();
     const unsigned prev = atomicAdd(p.ticket, 1u);
@@ -126,10 +122,42 @@ himeno19_kernel(const __grid_constant__ HimenoMaps maps, const HParams p) {
 
 size_t himeno19_smem_bytes(const MarchConfig &cfg) {
   // 128 bytes of slack for aligning the dynamic shared-memory base
-  return 128 + (size_t)h_bar_bytes(cfg.ns + cfg.ns2) +
+  return 128 + (size_t)h_bar_bytes(2 * (cfg.ns + cfg.ns2)) +
          (size_t)cfg.ns * h_align128((uint32_t)(kHimW * (cfg.warps + 2) * 4)) +
          (size_t)cfg.ns2 * kHimCoef * kHimTX * cfg.warps * 4;
 }
+
+// Lanes side by side in x: all tiles hold the same cells, so the widest is
+// taken unless a narrower one covers the domain with 3 % fewer (a batch of 24
+// problems 39 to 160 wide: 271 us a step, 299 with 128-cell tiles and no producer).
+int himeno19_lanes(const Box &dom, int warps) {
+  const int nx = dom.max[0] - dom.min[0] / 4 * 4, ny = dom.max[1] - dom.min[1];
+  int best = 32;
+  double cost = 0;
+  for (int lx = 32; lx >= 8; lx /= 2) {
+    const int tx = 4 * lx, ty = him_rows(warps, lx);
+    const double c = (double)((nx + tx - 1) / tx) * ((ny + ty - 1) / ty);
+    if (lx == 32 || c < 0.97 * cost) {
+      best = lx;
+      cost = c;
+    }
+  }
+  return best;
+}
+
+void himeno19_boxes(int lx, int warps, int p_box[2], int c_box[2]) {
+  c_box[0] = 4 * lx;
+  c_box[1] = him_rows(warps, lx);
+  p_box[0] = c_box[0] + 8;
+  p_box[1] = c_box[1] + 2;
+}
+
+namespace {
+template <int LX>
+auto him_kernel(bool gosa) {
+  return gosa ? himeno19_kernel<true, LX> : himeno19_kernel<false, LX>;
+}
+}  // namespace
 
 cudaError_t launch_himeno19(const Himeno19Args &a, const MarchConfig &cfg,
                             const CUtensorMap *tmaps, const ResidualSink &sink,
@@ -163,15 +191,20 @@ cudaError_t launch_himeno19(const Himeno19Args &a, const MarchConfig &cfg,
   if (cfg.warps < 1 || cfg.warps > 8 || cfg.ns < 3 || cfg.ns > 16 || cfg.ns2 < 1 ||
       cfg.ns2 > 8)
     return cudaErrorInvalidConfiguration;
-  p.tiles_x = (ex + kHimTX - 1) / kHimTX;
-  p.tiles = p.tiles_x * ((ey + cfg.warps - 1) / cfg.warps);
+  const int lx = himeno19_lanes(a.dom, cfg.warps);
+  const int tx = 4 * lx, ty = him_rows(cfg.warps, lx);
+  p.tiles_x = (ex + tx - 1) / tx;
+  p.tiles = p.tiles_x * ((ey + ty - 1) / ty);
   const size_t smem = himeno19_smem_bytes(cfg);
   // Opt in to the dynamic shared memory this launch needs (the kernel also
   // has a little static shared memory, so the opt-in is the exact size).
-  static size_t attr_set[2] = {0, 0};
-  static int occ[2][9][17][9];  // [gosa][warps][ns][ns2] -> CTAs per SM
-  auto kern = a.gosa ? himeno19_kernel<true> : himeno19_kernel<false>;
-  size_t &have = attr_set[a.gosa ? 1 : 0];
+  static size_t attr_set[2][3] = {};
+  static int occ[2][3][9][17][9];  // [gosa][lanes][warps][ns][ns2] -> CTAs per SM
+  const int gi = a.gosa ? 1 : 0, li = lx == 32 ? 0 : lx == 16 ? 1 : 2;
+  auto kern = lx == 32 ? him_kernel<32>(a.gosa) : lx == 16 ? him_kernel<16>(a.gosa)
+                                                           : him_kernel<8>(a.gosa);
+  const int threads = 32 * (cfg.warps + 1);
+  size_t &have = attr_set[gi][li];
   if (smem > have) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem);
@@ -180,10 +213,9 @@ cudaError_t launch_himeno19(const Himeno19Args &a, const MarchConfig &cfg,
   }
   // The round-robin schedule assumes every CTA is resident: never launch
   // more per SM than fit.
-  int &oc = occ[a.gosa ? 1 : 0][cfg.warps][cfg.ns][cfg.ns2];
+  int &oc = occ[gi][li][cfg.warps][cfg.ns][cfg.ns2];
   if (oc == 0) {
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&oc, kern, 32 * cfg.warps,
-                                                                  smem);
+    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&oc, kern, threads, smem);
     if (e != cudaSuccess) return e;
     if (oc < 1) oc = 1;
   }
@@ -195,7 +227,7 @@ cudaError_t launch_himeno19(const Himeno19Args &a, const MarchConfig &cfg,
   if (grid > p.items) grid = p.items;
   if (a.gosa && grid > sink.max_partials) grid = sink.max_partials;
   p.early = grid == resident;
-  return launch_kernel(kern, (unsigned)grid, dim3(32, cfg.warps, 1), smem, s, a.overlap, maps, p);
+  return launch_kernel(kern, (unsigned)grid, dim3(32, cfg.warps + 1, 1), smem, s, a.overlap, maps, p);
 }
 
 }  // namespace psg

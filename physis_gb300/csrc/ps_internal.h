@@ -141,6 +141,10 @@ struct ResidualSink {
   double *result;       // where the FP64 total goes
 };
 size_t himeno19_smem_bytes(const MarchConfig &cfg);
+// Lanes side by side in x (32, 16 or 8) of the tiles that cover dom best with
+// `warps` warps, and the {w, h} boxes of p and of the coefficients.
+int himeno19_lanes(const Box &dom, int warps);
+void himeno19_boxes(int lx, int warps, int p_box[2], int c_box[2]);
 cudaError_t launch_himeno19(const Himeno19Args &a, const MarchConfig &cfg,
                             const CUtensorMap *tmaps /* 13: p0-halo, 12 coef */,
                             const ResidualSink &sink, int *dev_err, int sm_count,

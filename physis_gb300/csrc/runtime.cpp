@@ -627,9 +627,11 @@ bool launch_map(const Map &m, bool want_gosa) {
     a.gosa = want_gosa;
     const MarchConfig cfg = m.has_plan ? m.plan.shape : rt->shapes[shape_slot(m.kernel)];
     CUtensorMap maps[13];
-    if (!tmap_for(view(m.grids[0]), 136, cfg.warps + 2, &maps[0])) return false;
+    int pb[2], cb[2];
+    psg::himeno19_boxes(psg::himeno19_lanes(box, cfg.warps), cfg.warps, pb, cb);
+    if (!tmap_for(view(m.grids[0]), pb[0], pb[1], &maps[0])) return false;
     for (int i = 0; i < 12; ++i)
-      if (!tmap_for(view(m.grids[2 + i]), 128, cfg.warps, &maps[1 + i])) return false;
+      if (!tmap_for(view(m.grids[2 + i]), cb[0], cb[1], &maps[1 + i])) return false;
     psg::ResidualSink sink;
     sink.partials = reinterpret_cast<double *>(rt->partials);
     sink.max_partials = kMaxPartials;
@@ -1383,9 +1385,20 @@ bool batch_build(Batch &b) {
     const Grid *g = m0->grids[0];
     bp.kind = m0->kernel;
     bp.rows = rows[r];
-    const int tyy = bp.kind == PS_KERNEL_HIMENO19 ? b.shape.warps : b.shape.warps * bp.rows;
-    const int xbase = (m0->dom.min[0] / 4) * 4;
-    const int tiles_x = (m0->dom.max[0] - xbase + 127) / 128;
+    const bool him = bp.kind == PS_KERNEL_HIMENO19;
+    // tile: 128 cells x warps * rows, or Himeno's choice
+    int tile[2] = {128, b.shape.warps * bp.rows}, pbox[2] = {136, tile[1] + 2};
+    if (him) {
+      psg::Box box;
+      for (int d = 0; d < 3; ++d) {
+        box.min[d] = m0->dom.min[d];
+        box.max[d] = m0->dom.max[d];
+      }
+      bp.lx = psg::himeno19_lanes(box, b.shape.warps);
+      psg::himeno19_boxes(bp.lx, b.shape.warps, pbox, tile);
+    }
+    const int xbase = (m0->dom.min[0] / 4) * 4, tyy = tile[1];
+    const int tiles_x = (m0->dom.max[0] - xbase + tile[0] - 1) / tile[0];
     bp.tiles = tiles_x * ((m0->dom.max[1] - m0->dom.min[1] + tyy - 1) / tyy);
     const int nzd = m0->dom.max[2] - m0->dom.min[2];
     bp.zlen = psg::choose_zchunk(bp.tiles, nzd, resident[fam]);
@@ -1398,11 +1411,10 @@ bool batch_build(Batch &b) {
       const Map *m = b.maps[(size_t)r * M + (par % M)];
       const GridView in = view(m->grids[0]), out = view(m->grids[1]);
       CUtensorMap t;
-      const int box_h = (bp.kind == PS_KERNEL_HIMENO19 ? b.shape.warps : tyy) + 2;
-      if (!tmap_for(in, 136, box_h, &t)) return false;
+      if (!tmap_for(in, pbox[0], pbox[1], &t)) return false;
       bp.tmap[par] = (int)tmaps.size();
       tmaps.push_back(t);
-      if (bp.kind == PS_KERNEL_HIMENO19) {
+      if (him) {
         psg::HParams &h = bp.him[par];
         h.out = static_cast<float *>(out.ptr);
         h.row = out.pitch / 4;
@@ -1425,7 +1437,7 @@ bool batch_build(Batch &b) {
         if (par == 0) {
           bp.cmap = (int)tmaps.size();
           for (int i = 0; i < 12; ++i) {
-            if (!tmap_for(view(m->grids[2 + i]), 128, b.shape.warps, &t)) return false;
+            if (!tmap_for(view(m->grids[2 + i]), tile[0], tile[1], &t)) return false;
             tmaps.push_back(t);
           }
         }

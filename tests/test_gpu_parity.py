@@ -379,6 +379,38 @@ def test_himeno_random_coefficients_bit_exact(rt, oracle, shape, launch):
             ps.set_launch_shape(k, *HIMENO_SHAPES[0])
 
 
+# Tiles of 64 and 32 cells, their remainders, and more planes than one item's.
+@pytest.mark.parametrize("shape", [(7, 70, 40), (12, 37, 200), (5, 18, 66), (60, 66, 146)])
+@pytest.mark.parametrize("launch", [(4, 1, 4, 2, 0), (8, 1, 3, 1, 0)])
+def test_himeno_narrow_tiles_bit_exact(rt, oracle, shape, launch):
+    test_himeno_random_coefficients_bit_exact(rt, oracle, shape, launch)
+
+
+def test_himeno_batch_of_every_tile_width(rt, oracle):
+    keep, runs, refs = [], [], []
+    for shape in [(30, 40, 128), (7, 70, 40), (40, 18, 66), (5, 66, 146), (33, 9, 200)]:
+        arrays = _himeno_random(shape, 70 + shape[0])
+        gs = himeno_grids(shape, arrays)
+        keep += gs
+        nz, ny, nx = shape
+        domt = (1, nx - 1, 1, ny - 1, 1, nz - 1)
+        runs.append([ps.stencil_map(ps.PS_KERNEL_HIMENO19, ps.domain(*domt), p + gs[2:], [0.8])
+                     for p in (gs[:2], gs[1::-1])])
+        g = [a.copy() for a in arrays]
+        for _ in range(36):
+            oracle.himeno19(g, domt, np.float32(0.8))
+            g[0], g[1] = g[1], g[0]
+        refs.append((gs, g))
+    b = ps.batch_create(runs)
+    ps.batch_run(b, 18)
+    for gs, g in refs:
+        assert np.array_equal(_bits(gs[0].copyout()), _bits(g[0]))
+        assert np.array_equal(_bits(gs[1].copyout()), _bits(g[1]))
+    ps.batch_free(b)
+    for g in keep:
+        g.free()
+
+
 def _himeno_random_case(oracle, shape):
     arrays = _himeno_random(shape, 11)
     gs = himeno_grids(shape, arrays)
