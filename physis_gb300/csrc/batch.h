@@ -10,7 +10,7 @@ namespace psg {
 struct BatchProblem {
   int kind;            // kKernelDiffusion7 / kKernelSum7 / kKernelCopy / kKernelHimeno19
   int rows;            // 7-point: rows per thread (1, 2 or 4)
-  int lx;              // Himeno: lanes side by side in x
+  int lx;              // lanes side by side in x
   int64_t item_begin;  // index of this problem's first item in the batch
   int64_t items;
   int tiles, zlen, dmin2, dmax2;
@@ -23,6 +23,7 @@ struct BatchProblem {
 struct BatchShape {
   int warps;     // CTA = 32 x warps threads
   int max_rows;  // largest 7-point rows per thread in the batch
+  int stage7;    // bytes of a 7-point ring stage (0: the widest tile's)
   int ns7;       // 7-point ring stages
   int nsp, nsc;  // Himeno p ring and coefficient ring stages
 };

@@ -3,7 +3,7 @@
 //
 // The reference launches one kernel per map per step
 // (translator/cuda_runtime_builder.cc:1512-1583).  A small grid's step is then
-// all launch and latency: 3.4 us at 64^3 replayed from a CUDA graph, for 0.2 us
+// all launch and latency: 2.6 us at 64^3 replayed from a CUDA graph, for 0.2 us
 // of L2 traffic.
 //
 // Design.  The grid is cut into bricks, full rows in x and by x bz rows in y
@@ -347,8 +347,8 @@ size_t resident7_smem(const Resident7Plan &q, int nx, int ny, int nz, int esz) {
 // Cost per epoch, fitted on GB300 to 32^3 .. 128^3: 1.1 us for the exchange,
 // 0.33 us of latency per step, and per 16-byte vector 0.83 ns computed (7.7 ns
 // in double precision, whose pipe is the bound) and 0.6 ns of halo.  Measured
-// per step against sweeps replayed from a graph: 32^3 0.9 against 2.5 us, 64^3 1.5
-// against 3.4 (k = 2, bricks of 5 x 6 rows), 96^3 3.0 against 4.9, 120^3 5.0
+// per step against sweeps replayed from a graph: 32^3 0.9 against 2.6 us, 64^3 1.5
+// against 2.6 (k = 2, bricks of 5 x 6 rows), 96^3 3.0 against 4.9, 120^3 5.0
 // against 5.8, 128^3 5.4 and 5.4; double 32^3 3.1 against 6.1, 64^3 9.4 against
 // 10.2.
 bool choose_resident7(int nx, int ny, int nz, int esz, int sms, Resident7Plan *best) {

@@ -574,10 +574,12 @@ bool launch_s7(const Map &m, const GridView &in, const GridView &out) {
       a.dom.min[2] >= a.dom.max[2])
     return true;
   for (int i = 0; i < 7; ++i) a.coef[i] = i < (int)m.scalars.size() ? m.scalars[i] : 0.0;
-  const int vec = 16 / in.esz;
   const MarchConfig cfg = m.has_plan ? m.plan.shape : rt->shapes[shape_slot(m.kernel)];
   CUtensorMap t;
-  if (!tmap_for(in, 34 * vec, cfg.warps * cfg.rows + 2, &t)) return false;
+  int bw = 0, bh = 0;
+  psg::stencil7_box(in.esz, cfg, psg::stencil7_lanes(a.dom, in.esz, in.type == PS_DOUBLE, cfg), &bw,
+                    &bh);
+  if (!tmap_for(in, bw, bh, &t)) return false;
   cudaError_t e = psg::launch_stencil7(a, cfg, &t, rt->dev_err, rt->sm_count, rt->stream);
   if (!cuda_ok(e, "stencil7 launch")) return false;
   ++rt->launches;
@@ -690,10 +692,10 @@ bool pair_eligible(const Map &a, const Map &b) {
 // Runs of fewer iterations stay with ordinary launches.
 constexpr int kResidentMinIter = 4;
 
-// Time per step of plain sweeps of g, in us: float 2.5 at 32^3 (launch and
-// latency), 3.4 at 64^3, 4.9 at 96^3 and 5.8 from 110^3 to 120^3; double 3.9 for each plane of
-// a 64 x 16 tile that an SM computes (its FP64 pipe): 6.2 up to 48^3, 10.2 at
-// 64^3.
+// Time per step of plain sweeps of g, in us, a little low: float 2.6 up to 64^3
+// (launch and latency), 4.9 at 96^3 and 5.8 from 110^3 to 120^3; double 3.9 for each
+// plane of a 64 x 16 tile that an SM computes (its FP64 pipe): 6.1 at 32^3, 10.2 at
+// 64^3, 22 at 80^3.
 double plain_sweep_us(const Grid &g) {
   const double cells = (double)g.dim[0] * g.dim[1] * g.dim[2];
   if (g.type == PS_FLOAT) return 2.5 + std::min(cells / 0.42e6, 3.3);
@@ -1315,8 +1317,8 @@ struct Batch {
   long long graph_launches = 0;       // kernels one replay of graph runs
 };
 std::vector<Batch> g_batches;
-// {warps, max rows (computed per batch), 7-point stages, Himeno p / coef stages}
-psg::BatchShape g_batch_shape{4, 4, 4, 4, 2};
+// {warps, max rows and stage bytes (computed per batch), 7-point stages, Himeno p / coef stages}
+psg::BatchShape g_batch_shape{4, 4, 0, 4, 4, 2};
 int g_batch_rows = 4;  // rows per thread of untuned 7-point runs in a batch
 
 void batch_release(Batch &b) {
@@ -1333,6 +1335,23 @@ bool batch_kind_ok(int k) {
          k == PS_KERNEL_HIMENO19;
 }
 
+// Tile and p / input box of a problem: 4 lx cells by the rows its warps take.
+void batch_tile(const psg::BatchShape &sh, const Map &m, int rows, int lx, int tile[2],
+                int pbox[2]) {
+  if (m.kernel == PS_KERNEL_HIMENO19) {
+    psg::himeno19_boxes(lx, sh.warps, pbox, tile);
+    return;
+  }
+  psg::stencil7_box(4, MarchConfig{sh.warps, rows, sh.ns7, 0, 0}, lx, &pbox[0], &pbox[1]);
+  tile[0] = pbox[0] - 8;
+  tile[1] = pbox[1] - 2;
+}
+
+int batch_tiles(const Map &m, const int tile[2]) {
+  const int nx = m.dom.max[0] - (m.dom.min[0] / 4) * 4, ny = m.dom.max[1] - m.dom.min[1];
+  return (nx + tile[0] - 1) / tile[0] * ((ny + tile[1] - 1) / tile[1]);
+}
+
 // (Re)builds the device tables of a batch from its maps' current grids.
 bool batch_build(Batch &b) {
   batch_release(b);
@@ -1341,7 +1360,8 @@ bool batch_build(Batch &b) {
   const int M = b.maps_per_run;
   b.shape = g_batch_shape;
   b.shape.max_rows = 1;
-  std::vector<int> rows(b.nruns, g_batch_rows);
+  b.shape.stage7 = 0;
+  std::vector<int> rows(b.nruns, g_batch_rows), lanes(b.nruns, 32);
   for (int r = 0; r < b.nruns; ++r) {
     const Map *m = b.maps[(size_t)r * M];
     if (m->kernel != PS_KERNEL_HIMENO19 && m->has_plan &&
@@ -1349,6 +1369,20 @@ bool batch_build(Batch &b) {
       rows[r] = m->plan.shape.rows;
     if (m->kernel != PS_KERNEL_HIMENO19 && rows[r] > b.shape.max_rows)
       b.shape.max_rows = rows[r];
+    psg::Box box;
+    for (int d = 0; d < 3; ++d) {
+      box.min[d] = m->dom.min[d];
+      box.max[d] = m->dom.max[d];
+    }
+    if (m->kernel == PS_KERNEL_HIMENO19) {
+      lanes[r] = psg::himeno19_lanes(box, b.shape.warps);
+    } else {
+      const MarchConfig cfg{b.shape.warps, rows[r], b.shape.ns7, 0, 0};
+      lanes[r] = psg::stencil7_lanes(box, 4, false, cfg);
+      int w = 0, h = 0;
+      psg::stencil7_box(4, cfg, lanes[r], &w, &h);
+      b.shape.stage7 = std::max(b.shape.stage7, (int)psg::s7_stage_bytes((uint32_t)(w * h * 4)));
+    }
   }
   // problems ordered by kernel family (each family is one launch), runs in
   // their given order inside a family
@@ -1374,6 +1408,22 @@ bool batch_build(Batch &b) {
     if (occ < 1) return fail(PS_ERR_CUDA, "batch kernel does not fit on an SM");
     resident[f] = rt->sm_count * occ;
   }
+  // Chunks short enough for every resident CTA, up to four planes, and then to
+  // about four rounds of them, up to eight (the 24-problem batch 258 us a step,
+  // 264 with each problem cut as it would be alone, up to 21 planes).
+  int chunk[2] = {1, 1};
+  for (int f = 0; f < 2; ++f) {
+    double planes = 0;
+    for (int r = 0; r < b.nruns; ++r) {
+      if (family(r) != f) continue;
+      const Map *m = b.maps[(size_t)r * M];
+      int tile[2], pbox[2];
+      batch_tile(b.shape, *m, rows[r], lanes[r], tile, pbox);
+      planes += (double)batch_tiles(*m, tile) * (m->dom.max[2] - m->dom.min[2]);
+    }
+    const double per = planes / std::max(resident[f], 1);
+    chunk[f] = per <= 4 ? std::max(1, (int)ceil(per)) : std::max(4, std::min(8, (int)(per / 4)));
+  }
   std::vector<psg::BatchProblem> probs(b.nruns);
   std::vector<CUtensorMap> tmaps;
   for (int i = 0; i < b.nruns; ++i) {
@@ -1386,22 +1436,15 @@ bool batch_build(Batch &b) {
     bp.kind = m0->kernel;
     bp.rows = rows[r];
     const bool him = bp.kind == PS_KERNEL_HIMENO19;
-    // tile: 128 cells x warps * rows, or Himeno's choice
-    int tile[2] = {128, b.shape.warps * bp.rows}, pbox[2] = {136, tile[1] + 2};
-    if (him) {
-      psg::Box box;
-      for (int d = 0; d < 3; ++d) {
-        box.min[d] = m0->dom.min[d];
-        box.max[d] = m0->dom.max[d];
-      }
-      bp.lx = psg::himeno19_lanes(box, b.shape.warps);
-      psg::himeno19_boxes(bp.lx, b.shape.warps, pbox, tile);
-    }
-    const int xbase = (m0->dom.min[0] / 4) * 4, tyy = tile[1];
+    bp.lx = lanes[r];
+    int tile[2], pbox[2];
+    batch_tile(b.shape, *m0, bp.rows, bp.lx, tile, pbox);
+    const int xbase = (m0->dom.min[0] / 4) * 4;
     const int tiles_x = (m0->dom.max[0] - xbase + tile[0] - 1) / tile[0];
-    bp.tiles = tiles_x * ((m0->dom.max[1] - m0->dom.min[1] + tyy - 1) / tyy);
+    bp.tiles = batch_tiles(*m0, tile);
     const int nzd = m0->dom.max[2] - m0->dom.min[2];
-    bp.zlen = psg::choose_zchunk(bp.tiles, nzd, resident[fam]);
+    const int chunks = std::max(1, (nzd + chunk[fam] - 1) / chunk[fam]);
+    bp.zlen = std::max(1, (nzd + chunks - 1) / chunks);
     bp.items = (int64_t)bp.tiles * ((nzd + bp.zlen - 1) / bp.zlen);
     bp.item_begin = b.total_items[fam];
     b.total_items[fam] += bp.items;
@@ -1455,6 +1498,7 @@ bool batch_build(Batch &b) {
         q.dmax0 = m->dom.max[0];
         q.dmax1 = m->dom.max[1];
         q.dmax2 = m->dom.max[2];
+        q.lx = bp.lx;
         q.xbase = xbase;
         q.tiles_x = tiles_x;
         q.tiles = bp.tiles;
@@ -2708,7 +2752,7 @@ void PSBatchRun(int batch, int iter) {
 
 void PSSetBatchShape(int warps, int rows, int ns7, int nsp, int nsc) {
   if (!need_rt("PSSetBatchShape")) return;
-  psg::BatchShape sh{warps, 4, ns7, nsp, nsc};
+  psg::BatchShape sh{warps, 4, 0, ns7, nsp, nsc};
   if (warps < 1 || warps > 8 || !(rows == 1 || rows == 2 || rows == 4) || ns7 < 2 ||
       ns7 > 8 || nsp < 3 || nsp > 8 || nsc < 1 || nsc > 4 ||
       psg::batch_smem_bytes(sh, psg::kBatch7) > 227 * 1024 ||

@@ -15,6 +15,7 @@ struct S7Params {
   int64_t plane;  // out elements per z-plane
   int nx, ny, nz;
   int dmin0, dmin1, dmin2, dmax0, dmax1, dmax2;
+  int lx;         // lanes side by side in x: 32, 16 or 8 (the others take rows further down)
   int xbase;      // x of the first tile (multiple of VEC)
   int tiles_x;    // tiles per y-band
   int tiles;      // tiles_x * tiles per x-column
@@ -41,38 +42,65 @@ struct RingPos {
   }
 };
 
+// How a CTA's threads agree and refill the ring.  S7Block: no producer; thread 0
+// issues an item's planes, each when a CTA barrier shows that every thread is
+// done with its stage.  Other kinds (batch.cu) have done(ok), called by each
+// thread when it is done with a plane, and last() when it is done with the
+// item's last one besides, and fill the ring themselves.
+struct S7Block {
+  static constexpr bool kIssues = true;
+  const CUtensorMap *tin;
+  RingPos prod;
+};
+
 // Marches tile `tile` of p over planes [zs, ze).  `full` are the ring's ns
-// mbarriers, `ring` its stages (stride plane_elems elements), TY the tile
-// height (blockDim.y * RY).  prod/cons persist across items.  Returns false
-// if a bounded wait gave up (the whole CTA agrees).
-template <typename T, int K, int RY>
-__device__ __forceinline__ bool s7_item(const CUtensorMap *tin, const S7Params<T> &p,
-                                        uint64_t *full, T *ring, int plane_elems,
-                                        uint32_t plane_bytes, int TY, int tile, int zs,
-                                        int ze, RingPos &prod, RingPos &cons) {
+// mbarriers, `ring` its stages (stride plane_elems elements).  Tiles are LX
+// vectors of 16 bytes wide (LX = 32, or p.lx if NARROW) and warps * RY * 32 / LX
+// rows high.  cons and sync persist across items.  Returns false if a bounded
+// wait gave up.
+template <typename T, int K, int RY, bool NARROW, class Sync>
+__device__ __forceinline__ bool s7_item(const S7Params<T> &p, uint64_t *full, T *ring,
+                                        int plane_elems, int warps, int tile, int zs, int ze,
+                                        RingPos &cons, Sync &sync) {
   constexpr int VEC = 16 / (int)sizeof(T);
-  constexpr int TX = 32 * VEC;
-  constexpr int W = TX + 2 * VEC;  // shared row width in elements
   constexpr bool kClamp = (K == kKernelDiffusion7);
   typedef RN<T> R;
+  const int LX = NARROW ? p.lx : 32;
+  const int TX = LX * VEC, W = TX + 2 * VEC;  // W: shared row width in elements
+  const int TY = warps * RY * (32 / LX);
   const int ns = p.ns;
   const int lane = threadIdx.x, warp = threadIdx.y;
   const int tid = warp * 32 + lane;
-  const int rows0 = warp * RY;                          // first own row in the tile
-  const int cen0 = (rows0 + 1) * W + VEC + lane * VEC;  // own first row, centre
+  const int xl = NARROW ? lane & (LX - 1) : lane;
+  const int rows0 = NARROW ? (warp * (32 / LX) + lane / LX) * RY : warp * RY;  // first own row in the tile
+  const int cen0 = (rows0 + 1) * W + VEC + xl * VEC;  // own first row, centre
   bool ok = true;
 
   const int x0 = p.xbase + (tile % p.tiles_x) * TX;
   const int y0 = p.dmin1 + (tile / p.tiles_x) * TY;
+
   const int nplanes = ze - zs + 2;  // planes zs-1 .. ze
 
   // Issues plane q (global plane zs-1+q) into the producer's next stage.
   auto issue = [&](int q) {
-    mbar_arrive_expect_tx(&full[prod.stage], plane_bytes);
-    tma_load_3d(ring + prod.stage * plane_elems, tin, x0 - VEC, y0 - 1, zs - 1 + q,
-                &full[prod.stage]);
-    prod.advance(ns);
+    if constexpr (Sync::kIssues) {
+      mbar_arrive_expect_tx(&full[sync.prod.stage], (uint32_t)(W * (TY + 2) * sizeof(T)));
+      tma_load_3d(ring + sync.prod.stage * plane_elems, sync.tin, x0 - VEC, y0 - 1, zs - 1 + q,
+                  &full[sync.prod.stage]);
+      sync.prod.advance(ns);
+    }
   };
+  // Agreement after a plane.
+  auto done = [&]() {
+    if constexpr (Sync::kIssues) ok = __syncthreads_and(ok);
+    else ok = sync.done(ok);
+  };
+  if constexpr (Sync::kIssues) {
+    if (tid == 0) {
+      const int n0 = min(ns, nplanes);
+      for (int q = 0; q < n0; ++q) issue(q);
+    }
+  }
   // Waits for the next plane in issue order; returns its stage.
   auto wait_next = [&]() -> const T * {
     if (!mbar_wait(&full[cons.stage], cons.phase, p.err)) ok = false;
@@ -81,10 +109,6 @@ __device__ __forceinline__ bool s7_item(const CUtensorMap *tin, const S7Params<T
     return pl;
   };
 
-  if (tid == 0) {
-    const int n0 = min(ns, nplanes);
-    for (int q = 0; q < n0; ++q) issue(q);
-  }
   T b[RY][VEC], c[RY][VEC], t[RY][VEC];
   const T *pm = wait_next();   // plane zs-1
   const T *cur = wait_next();  // plane zs
@@ -97,18 +121,18 @@ __device__ __forceinline__ bool s7_item(const CUtensorMap *tin, const S7Params<T
       for (int i = 0; i < VEC; ++i) b[r][i] = c[r][i];
     }
   }
-  ok = __syncthreads_and(ok);
+  done();
   if (!ok) return false;
-  if (tid == 0 && ns < nplanes) issue(ns);
+  if (Sync::kIssues && tid == 0 && ns < nplanes) issue(ns);
 
-  const int x = x0 + lane * VEC;
+  const int x = x0 + xl * VEC;
   const int y = y0 + rows0;  // first own row
+  const int ywarp = y0 + warp * RY * (32 / LX);  // the warp's first row
   const bool vec_in = (x >= p.dmin0) && (x + VEC <= p.dmax0);
   const bool west_face = kClamp && (x == 0);            // element 0 clamps west
   const int east_elem = kClamp ? (p.nx - 1 - x) : -1;  // element clamping east
 
   for (int z = zs; z < ze; ++z) {
-    const int q = z - zs + 1;  // plane index of z
     const T *nxt = wait_next();
     T n[VEC], s[VEC];
 #pragma unroll
@@ -126,7 +150,7 @@ __device__ __forceinline__ bool s7_item(const CUtensorMap *tin, const S7Params<T
 #pragma unroll
     for (int r = 0; r < RY; ++r) {
       // double precision is short of FP64 issue: nothing for rows outside
-      if (sizeof(T) == 8 && y + r >= p.dmax1) break;
+      if (sizeof(T) == 8 && ywarp + r >= p.dmax1) break;
       T o[VEC];
       if (K == kKernelCopy) {
 #pragma unroll
@@ -150,8 +174,8 @@ __device__ __forceinline__ bool s7_item(const CUtensorMap *tin, const S7Params<T
         }
         T left = shfl_up1(c[r][VEC - 1]);
         T right = shfl_down1(c[r][0]);
-        if (lane == 0) left = cur[cen0 + r * W - 1];
-        if (lane == 31) right = cur[cen0 + r * W + VEC];
+        if (xl == 0) left = cur[cen0 + r * W - 1];
+        if (xl == LX - 1) right = cur[cen0 + r * W + VEC];
 #pragma unroll
         for (int i = 0; i < VEC; ++i) {
           T w = (i == 0) ? left : c[r][i - 1];
@@ -199,11 +223,13 @@ __device__ __forceinline__ bool s7_item(const CUtensorMap *tin, const S7Params<T
         c[r][i] = t[r][i];
       }
     cur = nxt;
-    ok = __syncthreads_and(ok);
+    done();
     if (!ok) return false;
     // Plane q is consumed by every thread: refill its stage with q + ns.
-    if (tid == 0 && q + ns < nplanes) issue(q + ns);
+    const int q = z - zs + 1;
+    if (Sync::kIssues && tid == 0 && q + ns < nplanes) issue(q + ns);
   }
+  if constexpr (!Sync::kIssues) sync.last();  // plane ze, in registers since the last step
   return true;
 }
 

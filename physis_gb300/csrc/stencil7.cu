@@ -19,6 +19,9 @@
 //   (TMA wants 16-byte aligned x) arrives by one TMA 3D box load into a
 //   ring of `ns` shared-memory stages; one mbarrier per stage signals
 //   arrival.  Stage and phase advance incrementally (no divisions).
+// * A tile is 32 vectors wide, or 16 or 8 and higher, whichever covers the domain
+//   best (stencil7_lanes): float 300^3 39.6 us a sweep against 46.7, 143 x 379 x 429
+//   38.4 against 60.8, 64^3 2.6 against 3.2; 512^3, on the widest, 165.
 // * Each thread owns one 16-byte vector column of RY rows: the z neighbours
 //   come from a register queue (b, c, t), the y neighbours of inner rows from
 //   the thread's own registers (only the rows above and below the column are
@@ -37,15 +40,28 @@
 namespace psg {
 namespace {
 
-template <typename T, int K, int RY>
+void box_for(int esz, const MarchConfig &cfg, int lx, int *w, int *h) {
+  *w = (lx + 2) * (16 / esz);
+  *h = cfg.warps * cfg.rows * (32 / lx) + 2;
+}
+
+size_t smem_bytes_for(int esz, const MarchConfig &cfg, int lx) {
+  int w, h;
+  box_for(esz, cfg, lx, &w, &h);
+  // 128 bytes of slack for aligning the dynamic shared-memory base
+  return 128 + (size_t)s7_bar_bytes(cfg.ns) + (size_t)cfg.ns * s7_stage_bytes((uint32_t)(w * h * esz));
+}
+
+
+template <typename T, int K, int RY, bool NARROW>
 __global__ void __launch_bounds__(512, 1)
 s7_march_kernel(const __grid_constant__ CUtensorMap tin, const S7Params<T> p) {
   constexpr int VEC = 16 / (int)sizeof(T);
-  constexpr int W = 34 * VEC;  // shared row width in elements
-  const int TY = blockDim.y * RY;
+  const int LX = NARROW ? p.lx : 32;
+  const int TX = LX * VEC, TY = blockDim.y * RY * (32 / LX);
+  const uint32_t plane_bytes = (uint32_t)((TX + 2 * VEC) * (TY + 2) * sizeof(T));
   // Each ring stage starts on a 128-byte boundary (required of the shared
   // destination of cp.async.bulk.tensor).
-  const uint32_t plane_bytes = (uint32_t)(W * (TY + 2) * sizeof(T));
   const int plane_elems = (int)(s7_stage_bytes(plane_bytes) / sizeof(T));
 
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -63,16 +79,15 @@ s7_march_kernel(const __grid_constant__ CUtensorMap tin, const S7Params<T> p) {
   if (p.early) launch_dependents();
   wait_for_predecessors();
 
-  // Producer (thread 0) and consumer (all threads) positions in the ring.
-  RingPos prod, cons;
+  S7Block sync{&tin};
+  RingPos cons;
   bool ok = true;
   for (int64_t item = blockIdx.x; item < p.items && ok; item += gridDim.x) {
     const int chunk = (int)(item / p.tiles);
     const int tile = (int)(item - (int64_t)chunk * p.tiles);
     const int zs = p.dmin2 + chunk * p.zlen;
     const int ze = min(zs + p.zlen, p.dmax2);
-    ok = s7_item<T, K, RY>(&tin, p, full, ring, plane_elems, plane_bytes, TY, tile, zs, ze,
-                           prod, cons);
+    ok = s7_item<T, K, RY, NARROW>(p, full, ring, plane_elems, blockDim.y, tile, zs, ze, cons, sync);
   }
   if (!ok && tid == 0) {
     // Give copies still in flight a bounded chance to land before exit.
@@ -80,13 +95,13 @@ s7_march_kernel(const __grid_constant__ CUtensorMap tin, const S7Params<T> p) {
   }
 }
 
-template <typename T, int K, int RY>
+template <typename T, int K, int RY, bool NARROW>
 cudaError_t launch_ry(S7Params<T> p, int tiles, int nzd, const MarchConfig &cfg,
                       const CUtensorMap *tin, int sm_count, bool overlap, cudaStream_t st) {
-  const size_t smem = stencil7_smem_bytes((int)sizeof(T), cfg);
+  const size_t smem = smem_bytes_for((int)sizeof(T), cfg, p.lx);
   static size_t attr_set = 0;     // dynamic shared memory opted in so far
-  static int occ_cached[17][17];  // [warps][ns] -> CTAs per SM (0 = unknown)
-  auto kern = s7_march_kernel<T, K, RY>;
+  static int occ_cached[2][17][17];  // [lanes 8][warps][ns] -> CTAs per SM (0 = unknown)
+  auto kern = s7_march_kernel<T, K, RY, NARROW>;
   if (smem > attr_set) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem);
@@ -96,7 +111,7 @@ cudaError_t launch_ry(S7Params<T> p, int tiles, int nzd, const MarchConfig &cfg,
   const int threads = 32 * cfg.warps;
   // The round-robin schedule assumes every CTA is resident: never launch
   // more per SM than fit.
-  int &oc = occ_cached[cfg.warps][cfg.ns];
+  int &oc = occ_cached[p.lx == 8][cfg.warps][cfg.ns];
   if (oc == 0) {
     cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&oc, kern, threads, smem);
     if (e != cudaSuccess) return e;
@@ -107,9 +122,9 @@ cudaError_t launch_ry(S7Params<T> p, int tiles, int nzd, const MarchConfig &cfg,
   p.tiles = tiles;
   // Double precision has one bound, the FP64 pipe of an SM, so it is the SMs'
   // shares that must be even: one CTA per plane of a tile, which the hardware hands to
-  // whichever SM is free, instead of a round-robin of longer chunks (155 x 105 x 127
-  // 68.7 us a sweep against 85, 300 x 200 x 250 404 against 428, 72^3 21.9 against
-  // 34; two planes cost 0-13 % more, four 1-28 %).
+  // whichever SM is free, instead of a round-robin of longer chunks (on 64-cell tiles
+  // 155 x 105 x 127 68.7 us a sweep against 85, 300 x 200 x 250 404 against 428, 72^3
+  // 21.9 against 34; two planes cost 0-13 % more, four 1-28 %).
   const bool spread = std::is_same<T, double>::value && K != kKernelCopy && cfg.ctas_per_sm == 0;
   p.zlen = spread ? 1 : choose_zchunk(tiles, nzd, resident, sm_count);
   p.items = (int64_t)tiles * ((nzd + p.zlen - 1) / p.zlen);
@@ -120,12 +135,18 @@ cudaError_t launch_ry(S7Params<T> p, int tiles, int nzd, const MarchConfig &cfg,
   return launch_kernel(kern, (unsigned)grid, dim3(32, cfg.warps, 1), smem, st, overlap, *tin, p);
 }
 
+template <typename T, int K, int RY>
+cudaError_t launch_lx(const S7Params<T> &p, int tiles, int nzd, const MarchConfig &cfg,
+                      const CUtensorMap *tin, int sm_count, bool overlap, cudaStream_t st) {
+  return p.lx == 32 ? launch_ry<T, K, RY, false>(p, tiles, nzd, cfg, tin, sm_count, overlap, st)
+                    : launch_ry<T, K, RY, true>(p, tiles, nzd, cfg, tin, sm_count, overlap, st);
+}
+
 template <typename T, int K>
 cudaError_t launch_t(const Stencil7Args &a, const MarchConfig &cfg,
                      const CUtensorMap *tin, int *dev_err, int sm_count,
                      cudaStream_t st) {
   constexpr int VEC = 16 / (int)sizeof(T);
-  constexpr int TX = 32 * VEC;
   S7Params<T> p;
   p.out = static_cast<T *>(a.out.ptr);
   p.row = a.out.pitch / (int64_t)sizeof(T);
@@ -156,14 +177,15 @@ cudaError_t launch_t(const Stencil7Args &a, const MarchConfig &cfg,
   if (ex <= 0 || ey <= 0 || ez <= 0) return cudaSuccess;
   if (cfg.warps < 1 || cfg.warps > 16 || cfg.ns < 2 || cfg.ns > 16)
     return cudaErrorInvalidConfiguration;
-  const int ty = cfg.warps * cfg.rows;
-  p.tiles_x = (ex + TX - 1) / TX;
+  p.lx = stencil7_lanes(a.dom, (int)sizeof(T), std::is_same<T, double>::value, cfg);
+  const int tx = p.lx * VEC, ty = cfg.warps * cfg.rows * (32 / p.lx);
+  p.tiles_x = (ex + tx - 1) / tx;
   const int tiles = p.tiles_x * ((ey + ty - 1) / ty);
   switch (cfg.rows) {
-    case 1: return launch_ry<T, K, 1>(p, tiles, ez, cfg, tin, sm_count, a.overlap, st);
-    case 2: return launch_ry<T, K, 2>(p, tiles, ez, cfg, tin, sm_count, a.overlap, st);
-    case 4: return launch_ry<T, K, 4>(p, tiles, ez, cfg, tin, sm_count, a.overlap, st);
-    case 8: return launch_ry<T, K, 8>(p, tiles, ez, cfg, tin, sm_count, a.overlap, st);
+    case 1: return launch_lx<T, K, 1>(p, tiles, ez, cfg, tin, sm_count, a.overlap, st);
+    case 2: return launch_lx<T, K, 2>(p, tiles, ez, cfg, tin, sm_count, a.overlap, st);
+    case 4: return launch_lx<T, K, 4>(p, tiles, ez, cfg, tin, sm_count, a.overlap, st);
+    case 8: return launch_lx<T, K, 8>(p, tiles, ez, cfg, tin, sm_count, a.overlap, st);
   }
   return cudaErrorInvalidConfiguration;
 }
@@ -187,13 +209,37 @@ cudaError_t launch_type(const Stencil7Args &a, const MarchConfig &cfg,
 
 }  // namespace
 
-size_t stencil7_smem_bytes(int esz, const MarchConfig &cfg) {
+size_t stencil7_smem_bytes(int esz, const MarchConfig &cfg) { return smem_bytes_for(esz, cfg, 32); }
+
+// Lanes side by side in x.  All shapes hold the same cells: the one that covers
+// the domain with the fewest cells loaded (tiles x box) is taken, for double the
+// fewest computed (rows outside are skipped, a warp's rows at a time), the wider
+// unless a narrower one saves 3 %, or for double 8 %: its narrow form takes more
+// registers (300 x 200 x 250 428 us with 5 % fewer cells, 403 on the widest tile;
+// 155 x 105 x 127 62.6 with 11 % fewer, 68.7 on the widest).
+int stencil7_lanes(const Box &dom, int esz, bool fp64, const MarchConfig &cfg) {
   const int vec = 16 / esz;
-  const int w = 32 * vec + 2 * vec;
-  const int ty = cfg.warps * cfg.rows;
-  // 128 bytes of slack for aligning the dynamic shared-memory base
-  return 128 + (size_t)s7_bar_bytes(cfg.ns) +
-         (size_t)cfg.ns * s7_stage_bytes((uint32_t)(w * (ty + 2) * esz));
+  const int nx = dom.max[0] - dom.min[0] / vec * vec, ny = dom.max[1] - dom.min[1];
+  int best = 32;
+  double cost = 0;
+  for (int lx = 32; lx >= 8; lx /= 2) {
+    int w, h;
+    box_for(esz, cfg, lx, &w, &h);
+    if (lx < 32 && (h > 256 || smem_bytes_for(esz, cfg, lx) > 200 * 1024)) continue;
+    const int tx = lx * vec, ty = h - 2, rows = lx == 32 ? 1 : 32 / lx * cfg.rows;
+    const double tiles_x = (nx + tx - 1) / tx;
+    const double c = fp64 ? tiles_x * tx * ((ny + rows - 1) / rows * rows)
+                          : tiles_x * ((ny + ty - 1) / ty) * w * h;
+    if (lx == 32 || c < (fp64 ? 0.92 : 0.97) * cost) {
+      best = lx;
+      cost = c;
+    }
+  }
+  return best;
+}
+
+void stencil7_box(int esz, const MarchConfig &cfg, int lx, int *w, int *h) {
+  box_for(esz, cfg, lx, w, h);
 }
 
 cudaError_t launch_stencil7(const Stencil7Args &a, const MarchConfig &cfg,

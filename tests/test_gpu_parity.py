@@ -386,6 +386,54 @@ def test_himeno_narrow_tiles_bit_exact(rt, oracle, shape, launch):
     test_himeno_random_coefficients_bit_exact(rt, oracle, shape, launch)
 
 
+# 7-point sweeps on 64- and 32-cell tiles: remainders in both axes, domains that
+# end inside a lane's vector, every type; and a batch of every tile width, one
+# problem thinner than a chunk.
+@pytest.mark.parametrize("shape", [(5, 70, 65), (40, 129, 33), (3, 66, 161), (4, 130, 30)])
+@pytest.mark.parametrize("dtype", [np.float32, np.float64, np.int32, np.int64])
+def test_narrow_sweeps_bit_exact(rt, oracle, shape, dtype):
+    nz, ny, nx = shape
+    rng = np.random.default_rng(31)
+    integer = np.issubdtype(dtype, np.integer)
+    init = (rng.integers(-1000, 1000, shape) if integer else rng.random(shape)).astype(dtype)
+    cases = [(ps.PS_KERNEL_SUM7, oracle.V_SUM7, (), (1, nx - 1, 1, ny - 1, 1, nz - 1))]
+    if not integer:
+        cases.append((ps.PS_KERNEL_DIFFUSION7, oracle.V_DIFFUSION7, DIFF_COEF,
+                      (0, nx, 0, ny, 0, nz)))
+        cases.append((ps.PS_KERNEL_DIFFUSION7, oracle.V_DIFFUSION7, DIFF_COEF,
+                      (3, nx - 2, 1, ny - 5, 0, nz)))
+    for kernel, variant, coef, dom in cases:
+        r1, r2 = init.copy(), init.copy()
+        oracle.run7(variant, r1, r2, dom, coef, iter=2)
+        a, b = run_pingpong(kernel, init, ps.domain(*dom), coef, 2, dtype)
+        assert np.array_equal(_bits(a), _bits(r1))
+        assert np.array_equal(_bits(b), _bits(r2))
+
+
+def test_batch_of_every_tile_width(rt, oracle):
+    runs, refs = [], []
+    for i, shape in enumerate([(30, 40, 128), (2, 70, 40), (40, 18, 66), (5, 66, 146), (33, 9, 200)]):
+        init = synth.uniform(shape, 80 + i)
+        nz, ny, nx = shape
+        g = [ps.Grid(shape), ps.Grid(shape)]
+        for x in g:
+            x.copyin(init)
+        runs.append([ps.stencil_map(ps.PS_KERNEL_DIFFUSION7, ps.full_domain(shape), p, DIFF_COEF)
+                     for p in (g, g[::-1])])
+        r1, r2 = init.copy(), init.copy()
+        oracle.run7(oracle.V_DIFFUSION7, r1, r2, (0, nx, 0, ny, 0, nz), DIFF_COEF, iter=18)
+        refs.append((g, r1, r2))
+    b = ps.batch_create(runs)
+    ps.batch_run(b, 18)
+    for g, r1, r2 in refs:
+        assert np.array_equal(_bits(g[0].copyout()), _bits(r1))
+        assert np.array_equal(_bits(g[1].copyout()), _bits(r2))
+    ps.batch_free(b)
+    for g, _, _ in refs:
+        for x in g:
+            x.free()
+
+
 def test_himeno_batch_of_every_tile_width(rt, oracle):
     keep, runs, refs = [], [], []
     for shape in [(30, 40, 128), (7, 70, 40), (40, 18, 66), (5, 66, 146), (33, 9, 200)]:
