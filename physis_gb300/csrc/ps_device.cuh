@@ -20,10 +20,10 @@ __device__ __forceinline__ void prefetch_tmap(const CUtensorMap *map) {
 // A launch that, with `overlap`, may start while the stream's previous kernel
 // still runs (the kernel then waits with wait_for_predecessors()).
 template <typename... P, typename... A>
-cudaError_t launch_kernel(void (*kern)(P...), unsigned grid, dim3 block, size_t smem,
+cudaError_t launch_kernel(void (*kern)(P...), dim3 grid, dim3 block, size_t smem,
                           cudaStream_t s, bool overlap, A &&...args) {
   cudaLaunchConfig_t c = {};
-  c.gridDim = dim3(grid);
+  c.gridDim = grid;
   c.blockDim = block;
   c.dynamicSmemBytes = smem;
   c.stream = s;

@@ -150,3 +150,35 @@ def test_loss_is_that_of_its_own_prediction(rt, batch):
         net.adam(2e-3)
         true = float(((pred - t).double() ** 2).mean())  # FP32 difference, as the kernel's
         assert abs(loss - true) <= 1e-9 * true
+
+
+@pytest.mark.parametrize("side", [False, True])
+def test_overlapping_launches_keep_their_order(rt, monkeypatch, side):
+    # every launch of a step may start as the one before it ends; in turn
+    # (PS_OVERLAP=0) gives the same bits, on PyTorch's stream and on another
+    from physis_gb300 import warmstart as ws
+    dims = (9, 17, 9, 9)
+    n = int(np.prod(dims))
+    gen = torch.Generator(device="cuda").manual_seed(8)
+    x = torch.randn(n * 16, generator=gen, device="cuda").to(torch.bfloat16)
+    t = torch.randn(n, generator=gen, device="cuda")
+    torch.cuda.synchronize()
+    got = []
+    for env in ("0", "1", "1"):
+        monkeypatch.setenv("PS_OVERLAP", env)
+        with torch.cuda.stream(torch.cuda.Stream() if side else torch.cuda.default_stream()):
+            net = ws.Net(7)
+            work = torch.empty(64 * (27 * 256 + 16), device="cuda")
+            work64 = torch.empty((n + 255) // 256, dtype=torch.float64, device="cuda")
+            losses = []
+            for _ in range(6):
+                loss, dy = ws.loss_grad(net.forward(x, dims), t, work64)
+                net.backward(dy, dims, work)
+                net.adam(2e-3)
+                losses.append(float(loss))
+            out = net.forward(x, dims).clone()
+            torch.cuda.current_stream().synchronize()
+        got.append((losses, out))
+    for losses, out in got[1:]:
+        assert losses == got[0][0]
+        assert torch.equal(out, got[0][1])
