@@ -1152,7 +1152,7 @@ def run_gpu_points(args, dist):
                                         if args.workload.startswith("points")
                                         else ("64x4 threads, one per (x, y), z-chunked"
                                               if os.environ.get("PS_FUNCTION_TILED") == "0"
-                                              else "64x16 tiles of 256 threads, z-chunked, "
+                                              else "64x16 tiles of 4 warps and a producer warp, z-chunked, "
                                                    "staged grids in shared memory")),
                        "l2": "inputs larger than L2" if N >= 256 else "fits L2"},
             "gpu_launches": int(launches),

@@ -119,12 +119,14 @@ int PSGetSMCount(void);
 
 /* ---- 4. Launch shapes and the autotuner -------------------------------- */
 
-/* Launch shape of a persistent z-marching sweep.  A CTA owns tiles 32
- * lanes x 16 bytes wide in x and warps*rows cells high in y and marches them
- * along z; each thread holds a column of `rows` rows in registers.  ns is
+/* Launch shape of a z-marching sweep.  A CTA owns tiles 32 lanes x 16 bytes
+ * wide in x and warps*rows cells high in y, or 16 or 8 lanes wide and two or
+ * four times as high where that covers the domain with fewer cells, and marches
+ * them along z; each thread holds a column of `rows` rows in registers.  ns is
  * the number of shared-memory ring stages (planes in flight + 2), ns2 the
  * stages of Himeno's coefficient ring, ctas_per_sm the persistent grid size
- * per SM (0 = as many as fit).  A field <= 0 keeps the current value
+ * per SM (0 = as many as fit; double 7-point sweeps then launch one CTA per
+ * plane of a tile).  A field <= 0 keeps the current value
  * (ctas_per_sm <= 0 selects "as many as fit").  Himeno kernels take
  * rows == 1 and at most 8 warps. */
 typedef struct {

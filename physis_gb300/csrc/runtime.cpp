@@ -1541,7 +1541,7 @@ bool batch_launch(Batch &b, int parity) {
   if (both && (!cuda_ok(cudaEventRecord(rt->fork, rt->stream), "cudaEventRecord") ||
                !cuda_ok(cudaStreamWaitEvent(rt->side, rt->fork, 0), "cudaStreamWaitEvent")))
     return false;
-  for (int f = 0; f < 2; ++f) {
+  for (int f : {psg::kBatchHimeno, psg::kBatch7}) {
     if (!b.nprob[f]) continue;
     cudaStream_t s = (both && f == psg::kBatchHimeno) ? rt->side : rt->stream;
     cudaError_t e = psg::launch_batch(b.probs_dev + b.prob_off[f], b.nprob[f], b.tmaps_dev,
