@@ -33,8 +33,8 @@
 // instructions a cell), HBM where it is narrow.  Measured, float, per sweep,
 // against lane-strided cells, halos rewritten by all threads between two CTA
 // barriers and no loading across items: 27 points periodic at 320 x 300 x 257
-// 58 against 198 us, 9 points periodic at 4099 x 3001 21 against 41 us, one
-// colour of the 7-point clamped stencil at 319 x 257 x 255 36 against 94 us.
+// 55 against 198 us, 9 points periodic at 4099 x 3001 18 against 41 us, one
+// colour of the 7-point clamped stencil at 319 x 257 x 255 32 against 94 us.
 // * The sweep body (points_body.cuh) is compiled two ways: here with the
 //   point table (shared-memory offset, plane lag, weight) copied to shared
 //   memory once per CTA and walked in order, and by jit.cpp with NVRTC per

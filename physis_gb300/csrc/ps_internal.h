@@ -44,9 +44,9 @@ struct Box {
   int max[3];
 };
 
-// Launch shape of a persistent 2.5D z-marching stencil kernel.  A tile is
-// 32 lanes x 16 bytes wide in x and warps*rows rows high; each thread owns a
-// column of `rows` rows.  `ns` is the number of shared-memory ring stages
+// Launch shape of a 2.5D z-marching stencil kernel.  A tile is 32 lanes x 16
+// bytes wide in x and warps*rows rows high, or 16 or 8 lanes wide and two or four
+// times as high; each thread owns a column of `rows` rows.  `ns` is the number of shared-memory ring stages
 // for the marched field, `ns2` that of a second ring (Himeno's coefficient
 // planes).  The grid is SMs x ctas_per_sm CTAs (0 = as many as fit).
 struct MarchConfig {
