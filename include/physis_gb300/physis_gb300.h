@@ -122,7 +122,9 @@ int PSGetSMCount(void);
 /* Launch shape of a z-marching sweep.  A CTA owns tiles 32 lanes x 16 bytes
  * wide in x and warps*rows cells high in y, or 16 or 8 lanes wide and two or
  * four times as high where that covers the domain with fewer cells, and marches
- * them along z; each thread holds a column of `rows` rows in registers.  ns is
+ * them along z; each thread holds a column of `rows` rows in registers.  (Point
+ * sweeps of the default shape, 4 warps of 4 rows, take 3 warps where that saves
+ * cells.)  ns is
  * the number of shared-memory ring stages (planes in flight + 2), ns2 the
  * stages of Himeno's coefficient ring, ctas_per_sm the persistent grid size
  * per SM (0 = as many as fit; double 7-point sweeps then launch one CTA per

@@ -506,9 +506,9 @@ std::string entry_source(const JitKernel &k) {
 //   comparisons of a function that treats the faces itself fold away;
 // * boxes arrive by TMA, where cp.async took a quarter of the instructions.
 // Measured, one sweep against the cp.async entry (256 threads, two by two cells
-// each, CTA barriers): clamped 7-point function at 400 x 384 x 320 float 90
-// against 154 us (48 instructions a cell against 92, 65 % of the HBM rate),
-// 27-point function at 258 x 258 x 200 double 686 against 727 us (the FP64
+// each, CTA barriers): clamped 7-point function at 400 x 384 x 320 float 87
+// against 154 us (52 instructions a cell against 92, 66 % of the HBM rate),
+// 27-point function at 258 x 258 x 200 double 673 against 727 us (the FP64
 // pipe's time is 556).
 constexpr int kTileX = 64, kTileY = 16;
 constexpr int kTileRows = 8;                              // rows per thread

@@ -34,7 +34,7 @@
 // against lane-strided cells, halos rewritten by all threads between two CTA
 // barriers and no loading across items: 27 points periodic at 320 x 300 x 257
 // 55 against 198 us, 9 points periodic at 4099 x 3001 18 against 41 us, one
-// colour of the 7-point clamped stencil at 319 x 257 x 255 32 against 94 us.
+// colour of the 7-point clamped stencil at 319 x 257 x 255 28 against 94 us.
 // * The sweep body (points_body.cuh) is compiled two ways: here with the
 //   point table (shared-memory offset, plane lag, weight) copied to shared
 //   memory once per CTA and walked in order, and by jit.cpp with NVRTC per
@@ -274,7 +274,7 @@ size_t smem_bytes_for(const PointsArgs &a, const MarchConfig &cfg, int lx) {
 // sweep: 64-cell tiles, 27 points periodic 320 x 300 x 257 59.8 against 63 us,
 // 27 points 60^3 4.3 against 4.9, 7 points 50 x 300 x 300 12.4 against 17.2;
 // 32-cell tiles, double, 7 points 40 x 66 x 100 18 against 32 us.
-int points_lanes(const PointsArgs &a, const MarchConfig &cfg) {
+static int best_lanes(const PointsArgs &a, const MarchConfig &cfg, double *cells) {
   const int vec = 16 / a.in.esz;
   const int nx = a.dom.max[0] - a.dom.min[0] / vec * vec, ny = a.dom.max[1] - a.dom.min[1];
   int best = 32;
@@ -290,7 +290,25 @@ int points_lanes(const PointsArgs &a, const MarchConfig &cfg) {
       cost = c;
     }
   }
+  *cells = cost;
   return best;
+}
+
+int points_lanes(const PointsArgs &a, const MarchConfig &cfg) {
+  double cells;
+  return best_lanes(a, cfg, &cells);
+}
+
+// Consumer warps of the default shape: three where the lower tiles load 3 % fewer
+// cells than four warps' (red/black 319 x 257 x 255 28.8 us a colour against 33.0,
+// tiles of 24 rows for 257; where neither saves, four are up to 2 % faster or slower).
+int points_warps(const PointsArgs &a, const MarchConfig &cfg) {
+  MarchConfig three = cfg;
+  three.warps = 3;
+  double c3, c4;
+  best_lanes(a, three, &c3);
+  best_lanes(a, cfg, &c4);
+  return c3 < 0.97 * c4 ? 3 : cfg.warps;
 }
 
 void points_box(const PointsArgs &a, const MarchConfig &cfg, int *w, int *h) {

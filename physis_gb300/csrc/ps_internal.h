@@ -177,6 +177,8 @@ int points_rows(const MarchConfig &cfg);
 // Lanes side by side in x (32, 16 or 8): tiles of 4 * lanes cells by
 // cfg.warps * points_rows(cfg) * 32 / lanes rows.
 int points_lanes(const PointsArgs &a, const MarchConfig &cfg);
+// Warps for maps without a shape of their own (cfg is the default one).
+int points_warps(const PointsArgs &a, const MarchConfig &cfg);
 // The TMA box of one ring plane: w cells by h rows.
 void points_box(const PointsArgs &a, const MarchConfig &cfg, int *w, int *h);
 size_t points_smem_bytes(const PointsArgs &a, const MarchConfig &cfg);

@@ -71,6 +71,7 @@ struct Grid {
 
 // Launch shape of the 7-point sweeps unless the user or the autotuner chooses.
 constexpr MarchConfig kDefaultShape{8, 2, 4, 0, 0};
+constexpr MarchConfig kPointsShape{4, 4, 4, 0, 0};
 
 bool same_cfg(const MarchConfig &a, const MarchConfig &b) {
   return a.warps == b.warps && a.rows == b.rows && a.ns == b.ns && a.ns2 == b.ns2 &&
@@ -538,6 +539,7 @@ bool launch_points_map(const Map &m, const PointStencil &ps) {
   memcpy(a.w, ps.w, sizeof(a.w));
   a.unit = ps.unit;
   MarchConfig cfg = m.has_plan ? m.plan.shape : rt->shapes[kSlotPoints];
+  if (!m.has_plan && same_cfg(cfg, kPointsShape)) cfg.warps = psg::points_warps(a, cfg);
   // the widest stencils need a shorter tile to fit their plane ring
   while (psg::points_smem_bytes(a, cfg) > 220 * 1024 && (cfg.rows > 1 || cfg.warps > 1)) {
     if (cfg.rows > 1) cfg.rows /= 2;
@@ -1804,7 +1806,7 @@ void PSInitV(int trace) {
   }
   // point stencils: 4 warps x 4 rows (a 128 x 16 tile; at 512^3 it equals 8 x 4 for the
   // 7-point stencil and is 6 % faster for the 27-point one: smaller rings, more CTAs)
-  r->shapes[kSlotPoints] = MarchConfig{4, 4, 4, 0, 0};
+  r->shapes[kSlotPoints] = kPointsShape;
   r->shapes[PS_KERNEL_HIMENO19] = MarchConfig{4, 1, 5, 2, 0};
   r->shapes[PS_KERNEL_HIMENO19_GOSA] = MarchConfig{4, 1, 5, 2, 0};
   cudaDeviceSynchronize();

@@ -215,6 +215,16 @@ def test_narrow_point_tiles_bit_exact(rt, oracle, kernel_form, seed, shape, dtyp
                                          npts, radius, weighted, shrink)
 
 
+# Heights that tiles of three warps (12, 24 or 48 rows) cover with fewer cells
+# than tiles of four, and one row more.
+@pytest.mark.parametrize("shape", [(6, 24, 128), (5, 25, 130), (4, 257, 319), (1, 600, 65),
+                                   (9, 12, 300)])
+@pytest.mark.parametrize("dtype,boundary", [(np.float32, 1), (np.float64, 2), (np.int32, 1)])
+def test_three_warp_tiles_bit_exact(rt, oracle, kernel_form, shape, dtype, boundary):
+    test_random_point_stencils_bit_exact(rt, oracle, kernel_form, 57, shape, dtype, boundary, 12,
+                                         1, True, False)
+
+
 @pytest.mark.parametrize("warps,rows", [(8, 2), (8, 1), (4, 2), (16, 1), (2, 2), (1, 1), (8, 4), (4, 4)])
 def test_point_launch_shapes_do_not_change_results(rt, oracle, kernel_form, warps, rows):
     rng = np.random.default_rng(42)
