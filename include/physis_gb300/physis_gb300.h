@@ -321,9 +321,12 @@ PSStencil PSStencilMapColorV(int kernel, int color, const PSDomain3D *dom, int n
  * (no counterpart in the reference).  Network tensors are channels-last
  * [batch][z][y][x][16] BF16 in device memory; weights are FP32 masters
  * [27 taps][16 in][16 out] (tap = (dz+1)*9 + (dy+1)*3 + (dx+1)) with BF16
- * copies for the kernels.  Every call takes device pointers and a stream
- * (NULL: the runtime's stream), allocates nothing, and returns PS_OK or an
- * error code (also recorded). */
+ * copies for the kernels.  Every call takes device pointers and a stream,
+ * allocates nothing, and returns PS_OK or an error code (also recorded).
+ * NULL is CUDA's default stream (as for PSReduceNoAlloc), kept in one order
+ * with the runtime's stream: the call sees what the runtime was asked to do
+ * before it, and the runtime's later calls see what it writes.  With another
+ * stream the caller orders the two. */
 
 /* y = epilogue(conv3x3x3(x, w_fwd) + bias) with zero padding; epilogue:
  * ReLU if relu != 0; times (mask > 0) if mask != NULL (the backward-data

@@ -111,6 +111,12 @@ struct Runtime {
   // joined back into `stream` by the two events
   cudaStream_t side = nullptr;
   cudaEvent_t fork = nullptr, join = nullptr;
+  // The PSWarmStart* calls' default stream is CUDA's; `order` carries the waits
+  // between it and `stream`.  default_work: it has work that `stream` is not
+  // ordered after; own_work: the reverse; stream_out: PSGetStream has given
+  // `stream` away, so work on it is not all seen here.
+  cudaEvent_t order = nullptr;
+  bool default_work = false, own_work = true, stream_out = false;
   int sm_count = 0;
   bool trace = false;
   // The device error word and the results live in pinned host memory that the
@@ -207,12 +213,35 @@ bool cuda_ok(cudaError_t e, const char *what) {
   return fail(PS_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
 }
 
-bool need_rt(const char *fn) {
-  if (rt) return true;
-  return fail(PS_ERR_NOT_INITIALIZED, "%s called before PSInit", fn);
+// True if the runtime's stream is being captured.
+bool capturing() {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(rt->stream, &cap) == cudaSuccess &&
+      cap == cudaStreamCaptureStatusNone)
+    return false;
+  cudaGetLastError();
+  return true;
 }
 
-Grid *as_grid(void *g, const char *fn) {
+// The runtime's stream waits for what PSWarmStart* calls left on the default one.
+void after_default_stream() {
+  if (!rt->default_work || capturing()) return;
+  if (cudaEventRecord(rt->order, cudaStreamLegacy) == cudaSuccess &&
+      cudaStreamWaitEvent(rt->stream, rt->order, 0) == cudaSuccess)
+    rt->default_work = false;
+  else
+    cudaGetLastError();
+}
+
+// Every call that may use the runtime's stream begins here.
+bool need_rt(const char *fn) {
+  if (!rt) return fail(PS_ERR_NOT_INITIALIZED, "%s called before PSInit", fn);
+  after_default_stream();
+  rt->own_work = true;
+  return true;
+}
+
+Grid *find_grid(void *g, const char *fn) {
   Grid *p = static_cast<Grid *>(g);
   if (!rt) {
     fail(PS_ERR_NOT_INITIALIZED, "%s called before PSInit", fn);
@@ -222,6 +251,13 @@ Grid *as_grid(void *g, const char *fn) {
     fail(PS_ERR_BAD_HANDLE, "%s: %p is not a live grid", fn, g);
     return nullptr;
   }
+  return p;
+}
+
+// The same for calls that go on to use the runtime's stream.
+Grid *as_grid(void *g, const char *fn) {
+  Grid *p = find_grid(g, fn);
+  if (p) need_rt(fn);
   return p;
 }
 
@@ -764,16 +800,6 @@ bool resident_packets(size_t bytes) {
   rt->res_packets = nullptr;
   rt->res_bytes = 0;
   return false;
-}
-
-// True if the runtime's stream is being captured.
-bool capturing() {
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(rt->stream, &cap) == cudaSuccess &&
-      cap == cudaStreamCaptureStatusNone)
-    return false;
-  cudaGetLastError();
-  return true;
 }
 
 // The plan for running (a, b) x iter in one launch (resident7.cu), or nullptr
@@ -1782,6 +1808,7 @@ void PSInitV(int trace) {
       !cuda_ok(cudaStreamCreateWithFlags(&r->side, cudaStreamNonBlocking), "cudaStreamCreate") ||
       !cuda_ok(cudaEventCreateWithFlags(&r->fork, cudaEventDisableTiming), "cudaEventCreate") ||
       !cuda_ok(cudaEventCreateWithFlags(&r->join, cudaEventDisableTiming), "cudaEventCreate") ||
+      !cuda_ok(cudaEventCreateWithFlags(&r->order, cudaEventDisableTiming), "cudaEventCreate") ||
       !cuda_ok(cudaHostAlloc(reinterpret_cast<void **>(&r->host_err), 128, cudaHostAllocMapped),
                "cudaHostAlloc") ||
       !cuda_ok(cudaHostGetDevicePointer(reinterpret_cast<void **>(&r->dev_err), r->host_err, 0),
@@ -1817,6 +1844,7 @@ void PSInitV(int trace) {
 
 void PSFinalize(void) {
   if (!rt) return;
+  after_default_stream();
   cudaStreamSynchronize(rt->stream);
   for (Grid *g : rt->grids) {
     cudaFree(g->dev);
@@ -1837,6 +1865,7 @@ void PSFinalize(void) {
   for (int i = 0; i < kNumEvents; ++i) cudaEventDestroy(rt->events[i]);
   cudaEventDestroy(rt->fork);
   cudaEventDestroy(rt->join);
+  cudaEventDestroy(rt->order);
   cudaStreamDestroy(rt->side);
   cudaStreamDestroy(rt->stream);
   delete rt;
@@ -2009,7 +2038,7 @@ void __PSGridSetScalar(void *g, int nidx, PSIndex i, PSIndex j, PSIndex k, int i
 }
 
 PSIndex PSGridDim(void *g, int d) {
-  Grid *p = as_grid(g, "PSGridDim");
+  Grid *p = find_grid(g, "PSGridDim");
   if (!p) return 0;
   if (d < 0 || d >= 3) {
     fail(PS_ERR_INVALID_ARGUMENT, "PSGridDim: dimension %d", d);
@@ -2019,19 +2048,19 @@ PSIndex PSGridDim(void *g, int d) {
 }
 
 void *PSGridDevicePtr(void *g) {
-  Grid *p = as_grid(g, "PSGridDevicePtr");
+  Grid *p = find_grid(g, "PSGridDevicePtr");
   return p ? p->dev : nullptr;
 }
 size_t PSGridPitch(void *g) {
-  Grid *p = as_grid(g, "PSGridPitch");
+  Grid *p = find_grid(g, "PSGridPitch");
   return p ? p->pitch : 0;
 }
 int PSGridElemSize(void *g) {
-  Grid *p = as_grid(g, "PSGridElemSize");
+  Grid *p = find_grid(g, "PSGridElemSize");
   return p ? p->esz : 0;
 }
 int PSGridType(void *g) {
-  Grid *p = as_grid(g, "PSGridType");
+  Grid *p = find_grid(g, "PSGridType");
   return p ? p->type : -1;
 }
 
@@ -2378,7 +2407,12 @@ void PSSynchronize(void) {
   sync_rt();
 }
 
-void *PSGetStream(void) { return rt ? (void *)rt->stream : nullptr; }
+void *PSGetStream(void) {
+  if (!rt) return nullptr;
+  after_default_stream();
+  rt->stream_out = true;
+  return rt->stream;
+}
 
 void PSEventRecord(int slot) {
   if (!need_rt("PSEventRecord")) return;
@@ -2505,13 +2539,33 @@ void PSGetLaunchShape(int kernel, PSLaunchShape *shape) {
   shape->ctas_per_sm = c.ctas_per_sm;
 }
 
+// The stream of a PSWarmStart* call: the caller's, or for NULL the default one,
+// which stands in one order with the runtime's (PyTorch, whose default stream it
+// is, can read what the call writes; the runtime's calls before and after it are
+// ordered with it as well).  While the runtime's stream or a stream that the
+// default one synchronises with is captured, NULL is the runtime's stream.
 static cudaStream_t ws_stream(void *stream) {
-  if (stream) return static_cast<cudaStream_t>(stream);
-  return rt ? rt->stream : nullptr;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if ((s && s != cudaStreamLegacy) || !rt) return s;
+  cudaStreamCaptureStatus cap;
+  if (capturing() || cudaStreamIsCapturing(cudaStreamLegacy, &cap) != cudaSuccess) {
+    cudaGetLastError();
+    return s ? s : rt->stream;
+  }
+  if (rt->own_work || rt->stream_out) {
+    if (cudaEventRecord(rt->order, rt->stream) == cudaSuccess &&
+        cudaStreamWaitEvent(cudaStreamLegacy, rt->order, 0) == cudaSuccess)
+      rt->own_work = false;
+    else
+      cudaGetLastError();
+  }
+  rt->default_work = true;
+  return cudaStreamLegacy;
 }
 
 // rc: 0, -1 (invalid arguments) or a cudaError_t from the launch.
 static int ws_status(int rc, const char *what) {
+  if (rt && rt->stream_out) after_default_stream();
   if (rc == 0) return PS_OK;
   if (rc > 0) {
     fail(PS_ERR_CUDA, "%s: %s", what, cudaGetErrorString(static_cast<cudaError_t>(rc)));

@@ -352,11 +352,10 @@ class Net:
 
 
 def _stream():
-    """PyTorch's current stream for the C API.  Its default stream has handle
-    0, which the library takes for its own stream (nothing orders the two); 1
-    is CUDA's name for the default stream (cudaStreamLegacy)."""
+    """PyTorch's current stream for the C API (the default one's handle is 0,
+    which stands for the default stream there too)."""
     import torch
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream or 1)
+    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
 def _p(t):
