@@ -269,7 +269,8 @@ class Net:
     FP32 master weights and Adam moments; BF16 copies for the kernels.  The
     weights of all layers, then their biases, lie in one buffer (gradients,
     moments and BF16 copies alike), so that an optimiser step is one launch;
-    w, b, grads, ... are views of them."""
+    w, b, grads, ... are views of them.  Where a program puts tensors of its own
+    into those lists, the step goes through the lists, tensor by tensor."""
 
     def __init__(self, seed=0):
         import torch
@@ -297,9 +298,14 @@ class Net:
         self._half = [torch.empty((LAYERS, per), dtype=torch.bfloat16, device=dev)
                       for _ in range(2)]
         self.wf, self.wb = list(self._half[0]), list(self._half[1])
+        self._own = self._pointers()
         self.step = 0
         self._acts = None
         self.prepare()
+
+    def _pointers(self):
+        return [t.data_ptr() for t in self.params + self.grads + self.m + self.v + self.w
+                + self.wf + self.wb]
 
     def stream(self):
         return _stream()
@@ -345,6 +351,12 @@ class Net:
 
     def adam(self, lr, b1=0.9, b2=0.999, eps=1e-8):
         self.step += 1
+        if self._pointers() != self._own:
+            for p, g, m, v in zip(self.params, self.grads, self.m, self.v):
+                _ok(ps.lib().PSWarmStartAdam(_p(p), _p(g), _p(m), _p(v), p.numel(), lr, b1, b2,
+                                             eps, self.step, self.stream()))
+            self.prepare()
+            return
         w, g, m, v = self._flat
         _ok(ps.lib().PSWarmStartAdamLayers(_p(w), _p(g), _p(m), _p(v), LAYERS, lr, b1, b2, eps,
                                            self.step, _p(self._half[0]), _p(self._half[1]),
