@@ -397,21 +397,26 @@ conv_pad_kernel(const __grid_constant__ CUtensorMap tmx, const __nv_bfloat16 *w,
   const int ntiles = (rows + kTcM - 1) / kTcM;
 
   if (warp == 4) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                     smem_u32(tslot)),
-                 "r"(kPcCols)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     if (lane == 0) {
       for (int i = 0; i <= kPcMaxTiles; ++i) mbar_init(&bars[i], 1);
       fence_barrier_init();
-      wait_for_predecessors();
+    }
+    wait_for_predecessors();
+    if (lane == 0) {
       // planes z0 - 1 .. z0 + zs of both halves
       mbar_arrive_expect_tx(&bars[0], 2u * (unsigned)((g.zs + 2) * g.P * 16));
       for (int h = 0; h < 2; ++h)
         tma_load_5d(smem_u32(sx + h * half + g.pre), &tmx, 8 * h, 0, 0, z0 - 1, b,
                     smem_u32(&bars[0]));
     }
+    __syncwarp();
+    // after the wait: columns held while waiting could be ones that the kernel
+    // waited for, the caller's own, has yet to allocate
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     smem_u32(tslot)),
+                 "r"(kPcCols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   } else {
     wait_for_predecessors();
     // weights: out channel n's 16 in-channels as two 16-byte halves
@@ -1291,8 +1296,9 @@ static bool tmap_slab(CUtensorMap *m, const void *x, const Dims &d, int bx, int 
 // kernel waits for their writes), except while the stream is captured: the
 // captured edge would be one.  A training step of 27 launches takes 256 us with
 // it, 282 without; a layer's forward, data and weight gradients of 1024 instances
-// 283 and 291.  No kernel here lets its dependents in before its CTAs leave:
-// theirs would hold the tensor memory that its own have yet to allocate.  What
+// 283 and 291.  No kernel here lets its dependents in before its CTAs leave, and
+// none allocates tensor memory before its wait: the kernel ahead, which may be the
+// caller's and let dependents in early, could still want those columns.  What
 // these kernels read is not __restrict__, as read-only loads could be moved ahead of the wait.
 static bool may_overlap(cudaStream_t s) {
   const char *e = getenv("PS_OVERLAP");
