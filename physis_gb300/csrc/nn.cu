@@ -372,6 +372,11 @@ __host__ __device__ constexpr int pc_tiles(int zs, int P) { return (zs * P + kTc
 __host__ __device__ constexpr int pc_half(int zs, int P, int px, int pre) {
   return pre + ((pc_tiles(zs, P) * kTcM + 2 * P + px + 1) * 16 + 127) / 128 * 128;
 }
+// The largest pc_smem: 1024 rows of tiles, planes of up to 1024 voxels in rows of
+// up to 256.  The kernel is always allowed this much, not each launch's own size,
+// which another thread's launch could lower in between.
+constexpr size_t kPcMaxSmem =
+    128 + kPcHead + kPcB + 2 * (size_t)(257 * 16 + 112 + (1024 + 2 * 1024 + 257) * 16 + 112);
 size_t pc_smem(const PadGeom &g) {
   const size_t n = 128 + kPcHead + kPcB + 2 * (size_t)pc_half(g.zs, g.P, g.px, g.pre);
   return n < kPcMinSmem ? kPcMinSmem : n;
@@ -1329,7 +1334,7 @@ static bool launch_conv_pad(const void *x, const void *w, const float *bias, con
   if (!tmap_slab(&tm, x, d, g.px, d.Y + 1, g.zs + 2)) return false;
   const size_t smem = pc_smem(g);
   *e = cudaFuncSetAttribute(conv_pad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                            (int)smem);
+                            (int)kPcMaxSmem);
   if (*e != cudaSuccess) return true;
   *e = launch_kernel(conv_pad_kernel, dim3((unsigned)items), dim3(kPcThreads), smem, s, may_overlap(s),
                      tm, static_cast<const __nv_bfloat16 *>(w), bias,
@@ -1380,11 +1385,9 @@ int nn_wgrad(const void *x, const void *dy, float *part, int S, float *dw, float
     const int stages = 16 + kWgStages * wg_stage_bytes(rows);
     const int sums = kWgWarps * 3 * kC * kC * 4;
     const int smem = stages > sums ? stages : sums;
-    cudaError_t e = cudaFuncSetAttribute(wgrad_run_kernel,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e == cudaSuccess)
-      e = launch_kernel(wgrad_run_kernel, dim3(3 * kWgHalves, S), dim3(kWgThreads), smem, s,
-                        overlap, xb, yb, part, bpart, d, rows);
+    // at most 33552 bytes: under what a launch may use without asking
+    const cudaError_t e = launch_kernel(wgrad_run_kernel, dim3(3 * kWgHalves, S), dim3(kWgThreads),
+                                        smem, s, overlap, xb, yb, part, bpart, d, rows);
     if (e != cudaSuccess) return (int)e;
   } else {
     wgrad_kernel<<<dim3(kTaps, S), 32 * kConvWarps, 0, s>>>(xb, yb, part, bpart, d);

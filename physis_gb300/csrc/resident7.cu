@@ -41,6 +41,7 @@ namespace {
 
 constexpr int kResThreads = 512;
 constexpr int kResBatch = 3;             // vectors of halo a thread polls together
+constexpr size_t kResSmem = 220 * 1024;   // most dynamic shared memory of a CTA
 constexpr unsigned kResPolls = 1u << 20;  // packet reads (about 0.7 us each) before a wait gives up
 
 template <typename T>
@@ -322,7 +323,7 @@ cudaError_t launch_t(const Resident7Args &a, cudaStream_t s) {
   auto kern = one ? resident7_kernel<T, 1> : resident7_kernel<T, 2>;
   const size_t smem = resident7_smem(a.plan, p.nx, p.ny, p.nz, (int)sizeof(T));
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)smem);
+                                       (int)kResSmem);
   if (e != cudaSuccess) return e;
   void *args[] = {&p};
   return cudaLaunchCooperativeKernel(
@@ -365,7 +366,7 @@ bool choose_resident7(int nx, int ny, int nz, int esz, int sms, Resident7Plan *b
       q.k = k;
       q.by = by;
       q.bz = (nz + nbz_max - 1) / nbz_max;
-      if (resident7_smem(q, nx, ny, nz, esz) > 220 * 1024) continue;
+      if (resident7_smem(q, nx, ny, nz, esz) > kResSmem) continue;
       double vecs = 0;  // 16-byte vectors computed per epoch
       for (int j = 1; j <= k; ++j)
         vecs += (double)nvec * (by + 2 * (k - j)) * (q.bz + 2 * (k - j));
