@@ -8,7 +8,7 @@
 // a problem; a persistent grid of SMs x occupancy CTAs takes items
 // round-robin, so small problems fill the GPU together and large ones keep
 // the chunk-major locality of the single-run kernels.  A CTA's items ascend, so
-// it finds an item's problem by stepping on from the last one's, and runs the
+// it looks for an item's problem from the last one's on, and runs the
 // shared per-item body (s7_body.cuh / himeno_body.cuh) with that
 // problem's parameters and tensor maps, both read from global memory.
 // Problem kinds: the 7-point family (DIFFUSION7, SUM7, COPY; 1, 2 or 4 rows
@@ -64,10 +64,17 @@ __device__ __forceinline__ bool s7_rows(const BatchProblem &bp, int parity, uint
 }
 
 // Problem of an item at or after those of problem `q`: items of a CTA ascend.
+// Often still q; else found by bisection, as each look at a problem waits for L2.
 __device__ __forceinline__ int batch_problem(const BatchProblem *__restrict__ probs, int nprob,
                                              int64_t item, int q) {
-  while (q + 1 < nprob && probs[q + 1].item_begin <= item) ++q;
-  return q;
+  if (q + 1 >= nprob || probs[q + 1].item_begin > item) return q;
+  int lo = q + 1, hi = nprob - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (probs[mid].item_begin <= item) lo = mid;
+    else hi = mid - 1;
+  }
+  return lo;
 }
 
 __global__ void __maxnreg__(112)
