@@ -1437,8 +1437,11 @@ bool batch_build(Batch &b) {
     resident[f] = rt->sm_count * occ;
   }
   // Chunks short enough for every resident CTA, up to four planes, and then to
-  // about four rounds of them, up to eight (the 24-problem batch 258 us a step,
-  // 264 with each problem cut as it would be alone, up to 21 planes).
+  // about four rounds of them, up to eight planes for Himeno (the 24-problem batch
+  // 258 us a step, 264 with each problem cut as it would be alone, up to 21 planes)
+  // and 16 for 7 points, whose own halo planes cost more (two 400^3 grids 222 us a
+  // step against 230 with eight, one 512^3 196 against 205, 6 of 320 x 320 x 256 and
+  // 6 of 100 x 200 x 300 321 against 327).
   int chunk[2] = {1, 1};
   for (int f = 0; f < 2; ++f) {
     double planes = 0;
@@ -1450,7 +1453,7 @@ bool batch_build(Batch &b) {
       planes += (double)batch_tiles(*m, tile) * (m->dom.max[2] - m->dom.min[2]);
     }
     const double per = planes / std::max(resident[f], 1);
-    chunk[f] = per <= 4 ? std::max(1, (int)ceil(per)) : std::max(4, std::min(8, (int)(per / 4)));
+    chunk[f] = per <= 4 ? std::max(1, (int)ceil(per)) : std::max(4, std::min(f == psg::kBatch7 ? 16 : 8, (int)(per / 4)));
   }
   std::vector<psg::BatchProblem> probs(b.nruns);
   std::vector<CUtensorMap> tmaps;
