@@ -85,9 +85,13 @@ struct Stencil7Args {
 };
 // Number of bytes of dynamic shared memory the launch will use.
 size_t stencil7_smem_bytes(int esz, const MarchConfig &cfg);
+// What bounds a sweep: the cells loaded and the work on them, the FP64 pipes, or
+// memory alone.
+enum class S7Bound { kLoads, kFp64, kMemory };
+S7Bound stencil7_bound(int type, int kernel, const Box &dom);
 // Lanes side by side in x (32, 16 or 8) of the tiles that cover dom best, and
 // the {w, h} box of such a tile and its halo.
-int stencil7_lanes(const Box &dom, int esz, bool fp64, const MarchConfig &cfg);
+int stencil7_lanes(const Box &dom, int esz, S7Bound bound, const MarchConfig &cfg);
 void stencil7_box(int esz, const MarchConfig &cfg, int lx, int *w, int *h);
 cudaError_t launch_stencil7(const Stencil7Args &a, const MarchConfig &cfg,
                             const CUtensorMap *tin, int *dev_err, int sm_count,

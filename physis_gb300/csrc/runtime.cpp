@@ -615,8 +615,8 @@ bool launch_s7(const Map &m, const GridView &in, const GridView &out) {
   const MarchConfig cfg = m.has_plan ? m.plan.shape : rt->shapes[shape_slot(m.kernel)];
   CUtensorMap t;
   int bw = 0, bh = 0;
-  psg::stencil7_box(in.esz, cfg, psg::stencil7_lanes(a.dom, in.esz, in.type == PS_DOUBLE, cfg), &bw,
-                    &bh);
+  const psg::S7Bound bound = psg::stencil7_bound(in.type, m.kernel, a.dom);
+  psg::stencil7_box(in.esz, cfg, psg::stencil7_lanes(a.dom, in.esz, bound, cfg), &bw, &bh);
   if (!tmap_for(in, bw, bh, &t)) return false;
   cudaError_t e = psg::launch_stencil7(a, cfg, &t, rt->dev_err, rt->sm_count, rt->stream);
   if (!cuda_ok(e, "stencil7 launch")) return false;
@@ -1406,7 +1406,7 @@ bool batch_build(Batch &b) {
       lanes[r] = psg::himeno19_lanes(box, b.shape.warps);
     } else {
       const MarchConfig cfg{b.shape.warps, rows[r], b.shape.ns7, 0, 0};
-      lanes[r] = psg::stencil7_lanes(box, 4, false, cfg);
+      lanes[r] = psg::stencil7_lanes(box, 4, psg::S7Bound::kLoads, cfg);
       int w = 0, h = 0;
       psg::stencil7_box(4, cfg, lanes[r], &w, &h);
       b.shape.stage7 = std::max(b.shape.stage7, (int)psg::s7_stage_bytes((uint32_t)(w * h * 4)));

@@ -96,7 +96,7 @@ s7_march_kernel(const __grid_constant__ CUtensorMap tin, const S7Params<T> p) {
 }
 
 template <typename T, int K, int RY, bool NARROW>
-cudaError_t launch_ry(S7Params<T> p, int tiles, int nzd, const MarchConfig &cfg,
+cudaError_t launch_ry(S7Params<T> p, int tiles, int nzd, const MarchConfig &cfg, S7Bound bound,
                       const CUtensorMap *tin, int sm_count, bool overlap, cudaStream_t st) {
   const size_t smem = smem_bytes_for((int)sizeof(T), cfg, p.lx);
   static size_t attr_set = 0;     // dynamic shared memory opted in so far
@@ -117,7 +117,11 @@ cudaError_t launch_ry(S7Params<T> p, int tiles, int nzd, const MarchConfig &cfg,
     if (e != cudaSuccess) return e;
     if (oc < 1) oc = 1;
   }
-  const int per_sm = (cfg.ctas_per_sm > 0 && cfg.ctas_per_sm < oc) ? cfg.ctas_per_sm : oc;
+  int per_sm = (cfg.ctas_per_sm > 0 && cfg.ctas_per_sm < oc) ? cfg.ctas_per_sm : oc;
+  // SUM7 of 4-byte types fits four times, which costs locality on grids beyond L2
+  // (four sweeps of 600^3 1198 us with three CTAs, 1272 with four; 375 x 131 x 214,
+  // within L2, 56 and 51)
+  if (bound == S7Bound::kMemory && cfg.ctas_per_sm == 0 && per_sm > 3) per_sm = 3;
   const int resident = sm_count * per_sm;
   p.tiles = tiles;
   // Double precision has one bound, the FP64 pipe of an SM, so it is the SMs'
@@ -131,15 +135,16 @@ cudaError_t launch_ry(S7Params<T> p, int tiles, int nzd, const MarchConfig &cfg,
   int64_t grid = resident;
   if (grid > p.items || spread) grid = p.items;
   if (grid < 1) grid = 1;
-  p.early = grid >= resident;
+  p.early = grid >= (int64_t)sm_count * oc;  // no place left free
   return launch_kernel(kern, (unsigned)grid, dim3(32, cfg.warps, 1), smem, st, overlap, *tin, p);
 }
 
 template <typename T, int K, int RY>
-cudaError_t launch_lx(const S7Params<T> &p, int tiles, int nzd, const MarchConfig &cfg,
+cudaError_t launch_lx(const S7Params<T> &p, int tiles, int nzd, const MarchConfig &cfg, S7Bound bound,
                       const CUtensorMap *tin, int sm_count, bool overlap, cudaStream_t st) {
-  return p.lx == 32 ? launch_ry<T, K, RY, false>(p, tiles, nzd, cfg, tin, sm_count, overlap, st)
-                    : launch_ry<T, K, RY, true>(p, tiles, nzd, cfg, tin, sm_count, overlap, st);
+  return p.lx == 32
+             ? launch_ry<T, K, RY, false>(p, tiles, nzd, cfg, bound, tin, sm_count, overlap, st)
+             : launch_ry<T, K, RY, true>(p, tiles, nzd, cfg, bound, tin, sm_count, overlap, st);
 }
 
 template <typename T, int K>
@@ -177,15 +182,16 @@ cudaError_t launch_t(const Stencil7Args &a, const MarchConfig &cfg,
   if (ex <= 0 || ey <= 0 || ez <= 0) return cudaSuccess;
   if (cfg.warps < 1 || cfg.warps > 16 || cfg.ns < 2 || cfg.ns > 16)
     return cudaErrorInvalidConfiguration;
-  p.lx = stencil7_lanes(a.dom, (int)sizeof(T), std::is_same<T, double>::value, cfg);
+  const S7Bound bound = stencil7_bound(a.in.type, K, a.dom);
+  p.lx = stencil7_lanes(a.dom, (int)sizeof(T), bound, cfg);
   const int tx = p.lx * VEC, ty = cfg.warps * cfg.rows * (32 / p.lx);
   p.tiles_x = (ex + tx - 1) / tx;
   const int tiles = p.tiles_x * ((ey + ty - 1) / ty);
   switch (cfg.rows) {
-    case 1: return launch_lx<T, K, 1>(p, tiles, ez, cfg, tin, sm_count, a.overlap, st);
-    case 2: return launch_lx<T, K, 2>(p, tiles, ez, cfg, tin, sm_count, a.overlap, st);
-    case 4: return launch_lx<T, K, 4>(p, tiles, ez, cfg, tin, sm_count, a.overlap, st);
-    case 8: return launch_lx<T, K, 8>(p, tiles, ez, cfg, tin, sm_count, a.overlap, st);
+    case 1: return launch_lx<T, K, 1>(p, tiles, ez, cfg, bound, tin, sm_count, a.overlap, st);
+    case 2: return launch_lx<T, K, 2>(p, tiles, ez, cfg, bound, tin, sm_count, a.overlap, st);
+    case 4: return launch_lx<T, K, 4>(p, tiles, ez, cfg, bound, tin, sm_count, a.overlap, st);
+    case 8: return launch_lx<T, K, 8>(p, tiles, ez, cfg, bound, tin, sm_count, a.overlap, st);
   }
   return cudaErrorInvalidConfiguration;
 }
@@ -211,13 +217,29 @@ cudaError_t launch_type(const Stencil7Args &a, const MarchConfig &cfg,
 
 size_t stencil7_smem_bytes(int esz, const MarchConfig &cfg) { return smem_bytes_for(esz, cfg, 32); }
 
+// Copies have no arithmetic: 20000 x 8 x 8 in double takes 81.6 us a pair of sweeps on
+// the tiles that compute fewest cells, 61 on those that load fewest.  Seven
+// additions of 4 bytes leave memory the bound once the two grids exceed L2.
+S7Bound stencil7_bound(int type, int kernel, const Box &dom) {
+  if (kernel == kKernelCopy) return S7Bound::kLoads;
+  if (type == kDouble) return S7Bound::kFp64;
+  double bytes = 2.0 * 4;
+  for (int d = 0; d < 3; ++d) bytes *= dom.max[d] - dom.min[d];
+  const bool far = kernel == kKernelSum7 && type != kLong && bytes > 128 << 20;
+  return far ? S7Bound::kMemory : S7Bound::kLoads;
+}
+
 // Lanes side by side in x.  All shapes hold the same cells: the one that covers
 // the domain with the fewest cells loaded (tiles x box) is taken, for double the
 // fewest computed (rows outside are skipped, a warp's rows at a time), the wider
 // unless a narrower one saves 3 %, or for double 8 %: its narrow form takes more
 // registers (300 x 200 x 250 428 us with 5 % fewer cells, 403 on the widest tile;
-// 155 x 105 x 127 62.6 with 11 % fewer, 68.7 on the widest).
-int stencil7_lanes(const Box &dom, int esz, bool fp64, const MarchConfig &cfg) {
+// 155 x 105 x 127 62.6 with 11 % fewer, 68.7 on the widest).  Sweeps bound by memory
+// want long rows: 40 % (SUM7 700 x 640 x 400 893 us a run of four on the widest tile,
+// 1027 with 8 % fewer cells; 143 x 705 x 448 321 and 354 with 32 % fewer).
+int stencil7_lanes(const Box &dom, int esz, S7Bound bound, const MarchConfig &cfg) {
+  const bool fp64 = bound == S7Bound::kFp64;
+  const double saves = fp64 ? 0.92 : bound == S7Bound::kMemory ? 0.6 : 0.97;
   const int vec = 16 / esz;
   const int nx = dom.max[0] - dom.min[0] / vec * vec, ny = dom.max[1] - dom.min[1];
   int best = 32;
@@ -230,7 +252,7 @@ int stencil7_lanes(const Box &dom, int esz, bool fp64, const MarchConfig &cfg) {
     const double tiles_x = (nx + tx - 1) / tx;
     const double c = fp64 ? tiles_x * tx * ((ny + rows - 1) / rows * rows)
                           : tiles_x * ((ny + ty - 1) / ty) * w * h;
-    if (lx == 32 || c < (fp64 ? 0.92 : 0.97) * cost) {
+    if (lx == 32 || c < saves * cost) {
       best = lx;
       cost = c;
     }

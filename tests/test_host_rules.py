@@ -32,10 +32,13 @@ static PointsArgs points(const int *d, int type, int n, const int *offsets) {
 API int zchunk(int tiles, int nz, int resident, int overhead, int fill) {
   return choose_zchunk_overhead(tiles, nz, resident, overhead, fill);
 }
-API int s7(const int *d, int esz, int fp64, const int *c, int *w, int *h) {
-  const int lx = stencil7_lanes(box(d), esz, fp64 != 0, cfg(c));
+API int s7(const int *d, int esz, int bound, const int *c, int *w, int *h) {
+  const int lx = stencil7_lanes(box(d), esz, (S7Bound)bound, cfg(c));
   stencil7_box(esz, cfg(c), lx, w, h);
   return lx;
+}
+API int s7_bound(int type, int kernel, const int *d) {
+  return (int)stencil7_bound(type, kernel, box(d));
 }
 API long long s7_smem(int esz, const int *c) { return (long long)stencil7_smem_bytes(esz, cfg(c)); }
 API int himeno(const int *d, int warps, int *p, int *c) {
@@ -119,12 +122,12 @@ def _covered(d, xbase, tx, ty, zlen, grid):
 SHAPES7 = [(8, 2, 4), (4, 4, 4), (1, 1, 2), (16, 1, 4), (2, 8, 3), (16, 8, 2), (8, 4, 8)]
 
 
-@pytest.mark.parametrize("esz,fp64", [(4, 0), (8, 0), (8, 1)])
-def test_seven_point_tiles(rules, esz, fp64):
-    rnd, vec = random.Random(esz + fp64), 16 // esz
+@pytest.mark.parametrize("esz,bound", [(4, 0), (8, 0), (8, 1), (4, 2)])  # S7Bound
+def test_seven_point_tiles(rules, esz, bound):
+    rnd, vec = random.Random(esz + bound), 16 // esz
     for d, shape in itertools.product(_domains(rnd, 25), SHAPES7):
         w, h = ctypes.c_int(), ctypes.c_int()
-        lx = rules.s7(_ints(*d), esz, fp64, _ints(*shape), ctypes.byref(w), ctypes.byref(h))
+        lx = rules.s7(_ints(*d), esz, bound, _ints(*shape), ctypes.byref(w), ctypes.byref(h))
         assert lx in (8, 16, 32)
         tx, ty = lx * vec, shape[0] * shape[1] * (32 // lx)
         assert (w.value, h.value) == (tx + 2 * vec, ty + 2)
@@ -137,6 +140,32 @@ def test_seven_point_tiles(rules, esz, fp64):
             zlen = rules.zchunk(tiles, d[5] - d[4], resident, 1, fill)
             _covered(d, xbase, tx, ty, zlen, resident)
         _covered(d, xbase, tx, ty, 1, 10 ** 9)  # one CTA per plane of a tile
+
+
+def test_seven_point_bounds(rules):
+    # types kInt, kLong, kFloat, kDouble = 0..3; kernels DIFFUSION7, SUM7, COPY
+    import physis_gb300 as ps
+    small, large = _ints(0, 64, 0, 64, 0, 64), _ints(1, 599, 1, 599, 1, 599)
+    for d in (small, large):
+        assert rules.s7_bound(3, ps.PS_KERNEL_DIFFUSION7, d) == 1
+        assert rules.s7_bound(3, ps.PS_KERNEL_SUM7, d) == 1
+        assert all(rules.s7_bound(t, ps.PS_KERNEL_COPY, d) == 0 for t in range(4))
+        assert rules.s7_bound(2, ps.PS_KERNEL_DIFFUSION7, d) == 0
+        assert rules.s7_bound(1, ps.PS_KERNEL_SUM7, d) == 0
+    assert rules.s7_bound(2, ps.PS_KERNEL_SUM7, small) == 0
+    assert rules.s7_bound(2, ps.PS_KERNEL_SUM7, large) == 2
+
+    def lanes(d, esz, bound):
+        w, h = ctypes.c_int(), ctypes.c_int()
+        return rules.s7(_ints(*d), esz, bound, _ints(8, 2, 4), ctypes.byref(w), ctypes.byref(h))
+
+    # a double copy of a narrow grid loads fewest cells on the widest tiles
+    assert lanes((0, 8, 0, 8, 0, 20000), 8, 0) == 32
+    assert lanes((0, 8, 0, 8, 0, 20000), 8, 1) == 8
+    # beyond L2 SUM7 gives up long rows for a large saving only
+    assert lanes((1, 699, 1, 639, 1, 399), 4, 2) == 32
+    assert lanes((1, 699, 1, 639, 1, 399), 4, 0) == 16
+    assert lanes((0, 64, 0, 4000, 0, 900), 4, 2) == 16
 
 
 @pytest.mark.parametrize("warps", [1, 3, 4, 8])
