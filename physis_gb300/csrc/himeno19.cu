@@ -70,7 +70,9 @@ himeno19_kernel(const __grid_constant__ HimenoMaps maps, const HParams p) {
     him_init(h, p.nsp, p.nsc, warps);
   }
   __syncthreads();
-  if (p.early) launch_dependents();
+  // dependents are not let in early: CTAs that take places as they fall free lose
+  // the neighbours they share p's halos with (257 x 257 x 513, sweep after sweep:
+  // 298 us against 292)
   wait_for_predecessors();
 
   HRing pprod, cprod, pcons, prel, ccons;
@@ -226,9 +228,6 @@ cudaError_t launch_himeno19(const Himeno19Args &a, const MarchConfig &cfg,
   int64_t grid = resident;
   if (grid > p.items) grid = p.items;
   if (a.gosa && grid > sink.max_partials) grid = sink.max_partials;
-  // never early: CTAs that take places as they fall free lose the neighbours they
-  // share p's halos with (257 x 257 x 513, sweep after sweep: 298 us against 292)
-  p.early = 0;
   return launch_kernel(kern, (unsigned)grid, dim3(32, cfg.warps + 1, 1), smem, s, a.overlap, maps, p);
 }
 

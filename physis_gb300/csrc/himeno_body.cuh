@@ -24,7 +24,6 @@ struct HParams {
   int xbase, tiles_x, tiles, zlen;
   int64_t items;
   int nsp, nsc;
-  int early;  // the next launch's CTAs may take places while this one runs
   float omega;
   double *partials;
   unsigned *ticket;

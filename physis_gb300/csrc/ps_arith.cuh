@@ -157,17 +157,6 @@ __device__ __forceinline__ void tma_load_3d(void *dst, const void *map,
 }
 
 // cp.async (global -> shared, asynchronous, completion per commit group).
-__device__ __forceinline__ void cp_async16(void *dst, const void *src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)),
-               "l"(__cvta_generic_to_global(src))
-               : "memory");
-}
-template <int B>
-__device__ __forceinline__ void cp_async_small(void *dst, const void *src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(smem_u32(dst)),
-               "l"(__cvta_generic_to_global(src)), "n"(B)
-               : "memory");
-}
 __device__ __forceinline__ void cp_async_commit() {
   asm volatile("cp.async.commit_group;" ::: "memory");
 }
