@@ -1331,12 +1331,12 @@ static bool launch_conv_pad(const void *x, const void *w, const float *bias, con
   const long long items = (long long)d.B * g.nslab;
   if (items > 0x7fffffff) return false;
   // A few slabs of wide planes: one CTA makes a slab's tiles one after the other,
-  // 3.6 us and 1 us a tile, where conv_tc_kernel's CTAs share all tiles out, 8.1 us
+  // 3.6 us and 1 us a tile, where conv_tc_kernel's CTAs share all tiles out, 8.5 us
   // and 1.4 us for each tile an SM gets (2 x 10 x 4 x 200 voxels, 20 slabs of 8 tiles:
   // 11.7 against 9.3 us; 4 x 20 x 4 x 200: 11.8 against 14.4).
   const int sms = sm_count();
   if (items <= sms && 3.6 + pc_tiles(g.zs, g.P) >
-                          8.1 + 1.4 * (double)((d.nvox + kTcM - 1) / kTcM) / sms)
+                          8.5 + 1.4 * (double)((d.nvox + kTcM - 1) / kTcM) / sms)
     return false;
   CUtensorMap tm;
   if (!tmap_slab(&tm, x, d, g.px, d.Y + 1, g.zs + 2)) return false;
