@@ -117,7 +117,7 @@ constexpr int kResident7MaxK = 4;
 struct Resident7Plan {
   int by, bz;  // rows of a brick in y and z
   int k;       // steps between exchanges
-  double us;   // estimated time per step
+  double us;   // cost it was chosen by
 };
 struct Resident7Args {
   GridView g1, g2;  // step 0 in g1; ends with step `steps` in g1, steps - 1 in g2
@@ -132,6 +132,8 @@ size_t resident7_packet_bytes(int nx, int ny, int nz, int esz);
 size_t resident7_smem(const Resident7Plan &q, int nx, int ny, int nz, int esz);
 // The cheapest brick and depth by the cost model; false if no brick fits.
 bool choose_resident7(int nx, int ny, int nz, int esz, int sms, Resident7Plan *best);
+// A closer estimate of a plan's time per step than the one it was chosen by.
+double resident7_us(const Resident7Plan &q, int nx, int ny, int nz, int esz);
 cudaError_t launch_resident7(const Resident7Args &a, cudaStream_t s);
 
 // ---- Himeno 19-point Jacobi (himeno19.cu) --------------------------------

@@ -730,10 +730,11 @@ bool pair_eligible(const Map &a, const Map &b) {
 // Runs of fewer iterations stay with ordinary launches.
 constexpr int kResidentMinIter = 4;
 
-// Time per step of plain sweeps of g, in us, a little low: float 2.6 up to 64^3
-// (launch and latency), 4.9 at 96^3 and 5.8 from 110^3 to 120^3; double 3.9 for each
-// plane of a 64 x 16 tile that an SM computes (its FP64 pipe): 6.1 at 32^3, 10.2 at
-// 64^3, 22 at 80^3.
+// Time per step of plain sweeps of g in runs of a hundred, in us, cubes in mind: float
+// 2.5 up to 64^3 (launch and latency; single launches 3.2), 4.9 at 96^3 and 5.7 from
+// 110^3 to 120^3; double 3.9 for each plane of a 64 x 16 tile that an SM computes (its
+// FP64 pipe): 6.1 at 32^3, 10.2 at 64^3, 22 at 80^3.  This gives 3.1, 4.6 and 5.8, 6.2,
+// 10.1 and 25.7; thin boxes take up to twice or half of it.
 double plain_sweep_us(const Grid &g) {
   const double cells = (double)g.dim[0] * g.dim[1] * g.dim[2];
   if (g.type == PS_FLOAT) return 2.5 + std::min(cells / 0.42e6, 3.3);
@@ -818,8 +819,13 @@ const psg::Resident7Plan *resident_plan(const Map &a, const Map &b, int iter) {
   auto hit = rt->res_plans.find(key);
   if (hit == rt->res_plans.end()) {
     psg::Resident7Plan q{};
+    // Chosen by the cost, refused by the closer estimate: of 138 sizes that the cost
+    // alone takes it drops two, 124^3 float (6.35 us a step in one launch, 5.72 as
+    // sweeps) and 278 x 110 x 9 double (22.4 and 15.2).
+    const double plain = plain_sweep_us(*g);
     if (!psg::choose_resident7(key[0], key[1], key[2], key[3], rt->sm_count, &q) ||
-        q.us > 0.9 * plain_sweep_us(*g))
+        q.us > 0.9 * plain || psg::resident7_us(q, key[0], key[1], key[2], key[3]) >
+                                  (g->type == PS_FLOAT ? 1.0 : 1.1) * plain)
       q.by = 0;
     hit = rt->res_plans.emplace(key, q).first;
   }
