@@ -48,8 +48,11 @@
 //   points all have odd parity, so a pass never reads a cell it writes
 //   (other than each cell's own centre) and the parallel result equals the
 //   sequential REF one.
+#include <algorithm>
+#include <array>
 #include <cstdlib>
 #include <cstring>
+#include <map>
 #include <type_traits>
 
 #include "points_body.cuh"
@@ -195,8 +198,16 @@ cudaError_t launch_t(const PointsArgs &a, int warps, int lx, int sm_count, cudaS
     // Registers: four rows of four cells compile to 72 of 80 without spilling
     // (4-byte types, 7 to 27 points); 8-byte types need about 120.
     const int regs = a.in.esz == 4 ? 80 : 120;
-    key.min_ctas = 65536 / (regs * 32 * (warps + 1));
-    if (key.min_ctas < 1) key.min_ctas = 1;
+    // Lists that come back late to what they have loaded hold more vectors than that
+    // leaves room for: more than 28 of them (22 of 8-byte types) get the registers
+    // of two CTAs to an SM (64 points within 2 of the cell, float, 256 x 250 x 120:
+    // 56 us a sweep, 222 spilling at 72 registers; 25 points in a plane, double,
+    // 2049 x 1500: 292 and 321).  Nor are registers saved for CTAs whose ring does
+    // not fit.
+    const int live = a.live[RY == 4 ? 2 : RY == 2 ? 1 : 0];
+    int ctas = 65536 / (regs * 32 * (warps + 1));
+    if (live > (a.in.esz == 4 ? 28 : 21)) ctas = std::min(ctas, 2);
+    key.min_ctas = std::max(1, std::min(ctas, (int)(227 * 1024 / (smem + 1024))));
     key.unit = UNIT;
     key.lx = lx;
     key.w = p.w;
@@ -309,6 +320,27 @@ int points_warps(const PointsArgs &a, const MarchConfig &cfg) {
   best_lanes(a, three, &c3);
   best_lanes(a, cfg, &c4);
   return c3 < 0.97 * c4 ? 3 : cfg.warps;
+}
+
+int points_live(int n, const int (*d)[3], int esz, int rows) {
+  const int vec = 16 / esz;
+  // vectors of point k: plane, row and (column group, vector) of each of its cells
+  std::map<std::array<int, 3>, std::pair<int, int>> use;
+  for (int k = 0; k < n; ++k)
+    for (int r = 0; r < rows; ++r)
+      for (int c = 0; c < kPtsVX; ++c) {
+        const int i = c % vec + d[k][0], v = (i + 8 * vec) / vec - 8;
+        auto at = use.emplace(std::array<int, 3>{d[k][2], d[k][1] + r, c / vec * 64 + v},
+                              std::make_pair(k, k));
+        at.first->second.second = k;
+      }
+  int most = 0;
+  for (int k = 0; k < n; ++k) {
+    int live = 0;
+    for (const auto &u : use) live += u.second.first <= k && k <= u.second.second;
+    most = std::max(most, live);
+  }
+  return most;
 }
 
 void points_box(const PointsArgs &a, const MarchConfig &cfg, int *w, int *h) {

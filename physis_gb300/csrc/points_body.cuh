@@ -120,7 +120,7 @@ __device__ __forceinline__ int pts_halo_cell(const PtsParams<T> &p, const PtsHal
 // The run-time spec: the point table travels in the kernel parameters and is
 // copied to shared memory; the tile geometry comes from the parameters.
 struct PtsTableSpec {
-  static constexpr bool kStatic = false;
+  static constexpr bool kStatic = false, kWideHalo = true;
   template <typename T>
   static __device__ __forceinline__ int lx(const PtsParams<T> &p) { return p.lx; }
   template <typename T>
@@ -357,10 +357,21 @@ __device__ __forceinline__ void pts_body(const PtsParams<T> &p, const void *tmap
           if (dst[i] >= 0) box[dst[i]] = v[i];
         const T *plane =
             p.in + (long long)pts_map_axis(zs - p.rzl + done, p.nz, p.boundary) * p.plane;
-        for (int e = lane + 32 * kBatch; e < h.total; e += 32) {
-          long long from;
-          const int to = pts_halo_cell(p, h, e, W, &from);
-          box[to] = plane[from];
+        // the rest of a wide halo, kMore loads of a lane in flight at a time
+        constexpr int kMore = S::kWideHalo ? 4 : 1;
+        for (int e0 = lane + 32 * kBatch; e0 < h.total; e0 += 32 * kMore) {
+          int to[kMore];
+          T u[kMore];
+#pragma unroll
+          for (int i = 0; i < kMore; ++i) {
+            const int e = e0 + 32 * i;
+            long long from = 0;
+            to[i] = e < h.total ? pts_halo_cell(p, h, e, W, &from) : -1;
+            u[i] = plane[from];
+          }
+#pragma unroll
+          for (int i = 0; i < kMore; ++i)
+            if (to[i] >= 0) box[to[i]] = u[i];
         }
         // these writes precede the consumers' reads (the arrival below) and
         // the box that reuses the stage (the proxy fence)

@@ -173,10 +173,14 @@ struct PointsArgs {
   int d[kMaxPoints][3];
   double w[kMaxPoints];
   bool unit;         // every weight is 1: terms are the point values
+  int live[3];       // points_live() with 1, 2 and 4 rows a lane
   bool overlap;
   int *err;          // device error word
   CUtensorMap tmap;  // maps `in` with the box points_box() gives
 };
+// The most 16-byte vectors that a lane of `rows` rows holds at a time when it loads
+// each once: those between their first use and their last, in point order.
+int points_live(int n, const int (*d)[3], int esz, int rows);
 // cfg.warps warps of points_rows(cfg) (1, 2 or 4) rows a lane; the other fields
 // are unused.
 int points_rows(const MarchConfig &cfg);

@@ -92,6 +92,7 @@ struct PointStencil {
   int d[psg::kMaxPoints][3];
   double w[psg::kMaxPoints];
   bool unit = true;
+  int live[2][3] = {};  // psg::points_live() of 4- and 8-byte types, 1, 2 and 4 rows
 };
 
 struct Map {
@@ -387,6 +388,9 @@ int register_points(const PointStencil &ps) {
     return -1;
   }
   rt->points.push_back(ps);
+  PointStencil &q = rt->points.back();
+  for (int t = 0; t < 2; ++t)
+    for (int r = 0; r < 3; ++r) q.live[t][r] = psg::points_live(q.n, q.d, t ? 8 : 4, 1 << r);
   return kPointsBase + (int)rt->points.size() - 1;
 }
 
@@ -574,8 +578,17 @@ bool launch_points_map(const Map &m, const PointStencil &ps) {
   memcpy(a.d, ps.d, sizeof(a.d));
   memcpy(a.w, ps.w, sizeof(a.w));
   a.unit = ps.unit;
+  memcpy(a.live, ps.live[a.in.esz == 4 ? 0 : 1], sizeof(a.live));
   MarchConfig cfg = m.has_plan ? m.plan.shape : rt->shapes[kSlotPoints];
-  if (!m.has_plan && same_cfg(cfg, kPointsShape)) cfg.warps = psg::points_warps(a, cfg);
+  if (!m.has_plan && same_cfg(cfg, kPointsShape)) {
+    // fewer rows where the ring of four would leave one CTA to an SM (offsets of 4,
+    // or of 2 in 8-byte types): 25 points in a star of radius 4, 256 x 250 x 120,
+    // float 22 us a sweep against 32, clamped 60 against 107; radius 2, double 359
+    // against 434; and two rows where four would not hold what the list comes back to
+    if (a.live[2] > 60 && a.in.esz == 4) cfg.rows = 2;
+    while (psg::points_smem_bytes(a, cfg) > 110 * 1024 && cfg.rows > 1) cfg.rows /= 2;
+    cfg.warps = psg::points_warps(a, cfg);
+  }
   // the widest stencils need a shorter tile to fit their plane ring
   while (psg::points_smem_bytes(a, cfg) > 220 * 1024 && (cfg.rows > 1 || cfg.warps > 1)) {
     if (cfg.rows > 1) cfg.rows /= 2;
