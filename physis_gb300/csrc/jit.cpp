@@ -934,10 +934,6 @@ bool tiled_enabled() {
 
 }  // namespace
 
-// The tiled entry runs every-point maps of stencils with staged grids when
-// no staged grid shares its memory with another grid argument (a staged copy
-// of a grid that the same launch writes would be stale); red/black maps and
-// everything else run the plain entry.
 // A launch of a compiled kernel; with `overlap` it may start before the stream's
 // previous kernel ends.
 static CUresult launch_function(void *fn, dim3 grid, dim3 block, size_t smem, bool overlap,
@@ -959,6 +955,10 @@ static CUresult launch_function(void *fn, dim3 grid, dim3 block, size_t smem, bo
   return g_drv.launch(&c, static_cast<CUfunction>(fn), args, nullptr);
 }
 
+// The tiled entry runs every-point maps of stencils with staged grids when
+// no staged grid shares its memory with another grid argument (a staged copy
+// of a grid that the same launch writes would be stale) and TMA can describe
+// each of them; red/black maps and everything else run the plain entry.
 cudaError_t jit_launch(const JitKernel &k, const Box &dom, int color, const GridView *grids,
                        const double *scalars, int sm_count, int *dev_err, bool overlap,
                        cudaStream_t s) {
@@ -966,7 +966,9 @@ cudaError_t jit_launch(const JitKernel &k, const Box &dom, int color, const Grid
             nzd = dom.max[2] - dom.min[2];
   if (nxd <= 0 || nyd <= 0 || nzd <= 0) return cudaSuccess;
   bool tiled = k.func_tiled && color < 0 && tiled_enabled() && k.tiled_occ > 0;
-  for (const JitStage &st : k.stages) {
+  std::vector<CUtensorMap> maps(tiled ? k.stages.size() : 0);
+  for (size_t t = 0; t < maps.size() && tiled; ++t) {
+    const JitStage &st = k.stages[t];
     int gi = 0, sgi = -1;
     for (size_t i = 0; i < k.params.size(); ++i)
       if (k.params[i].grid) {
@@ -975,6 +977,7 @@ cudaError_t jit_launch(const JitKernel &k, const Box &dom, int color, const Grid
       }
     for (int j = 0; j < gi && tiled; ++j)
       if (j != sgi && grids[j].ptr == grids[sgi].ptr) tiled = false;
+    if (tiled) tiled = make_tmap_3d(&maps[t], grids[sgi], st.w, kTileY + 2 * st.ry);
   }
   unsigned gx, gy, gz, bx, by;
   int head[9];
@@ -1038,17 +1041,9 @@ cudaError_t jit_launch(const JitKernel &k, const Box &dom, int color, const Grid
     off += n;
   };
   for (int v : head) put(&v, 4, 4);
-  std::vector<CUtensorMap> maps(tiled ? k.stages.size() : 0);
   if (tiled) {
     put(&dev_err, 8, 8);
-    for (size_t j = 0; j < maps.size(); ++j) {
-      const JitStage &st = k.stages[j];
-      int g = 0;
-      for (int i = 0; i < st.param; ++i) g += k.params[i].grid ? 1 : 0;
-      if (!make_tmap_3d(&maps[j], grids[g], st.w, kTileY + 2 * st.ry))
-        return cudaErrorInvalidValue;
-      args.push_back(&maps[j]);
-    }
+    for (CUtensorMap &m : maps) args.push_back(&m);
   }
   int gi = 0, si = 0;
   for (const JitParam &p : k.params) {

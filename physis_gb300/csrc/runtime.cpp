@@ -318,7 +318,8 @@ bool tmap_for(const GridView &v, int w, int h, CUtensorMap *out) {
   e.v = v;
   e.w = w;
   e.h = h;
-  if (!psg::make_tmap_3d(&e.map, v, w, h)) return false;
+  if (!psg::make_tmap_3d(&e.map, v, w, h))
+    return fail(PS_ERR_CUDA, "cuTensorMapEncodeTiled failed for box %dx%d", w, h);
   rt->tmaps.push_back(e);
   *out = e.map;
   return true;
@@ -1727,7 +1728,7 @@ bool reduce_kernel_form(void *v, int op, int kernel, const __PSDomain &dom, int 
 namespace psg {
 
 bool make_tmap_3d(CUtensorMap *map, const GridView &g, int box_w, int box_h) {
-  if (!g_encode) return fail(PS_ERR_CUDA, "cuTensorMapEncodeTiled unavailable");
+  if (!g_encode) return false;
   CUtensorMapDataType dt;
   switch (g.type) {
     case kFloat: dt = CU_TENSOR_MAP_DATA_TYPE_FLOAT32; break;
@@ -1739,14 +1740,9 @@ bool make_tmap_3d(CUtensorMap *map, const GridView &g, int box_w, int box_h) {
   cuuint64_t strides[2] = {(cuuint64_t)g.pitch, (cuuint64_t)g.pitch * (cuuint64_t)g.ny};
   cuuint32_t box[3] = {(cuuint32_t)box_w, (cuuint32_t)box_h, 1};
   cuuint32_t estr[3] = {1, 1, 1};
-  CUresult r = g_encode(map, dt, 3, g.ptr, dims, strides, box, estr,
-                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS)
-    return fail(PS_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d) for box %dx%d", (int)r,
-                box_w, box_h);
-  return true;
+  return g_encode(map, dt, 3, g.ptr, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 }  // namespace psg
