@@ -297,7 +297,7 @@ int PSStencilFunctionNew(const char *source, const char *name);
  * loading it (no device or PSInit needed).  Returns PS_OK, else
  * PS_ERR_INVALID_ARGUMENT (the reason and compiler log, truncated, in
  * log[0..logsize)) or PS_ERR_UNSUPPORTED without NVRTC.  On success log
- * names the grids the tiled entry stages in shared memory, one
+ * names the grids the tiled entry stages in shared memory with a halo, one
  * "staged <grid> <rx> <ry> <rz> <clamp|periodic>;" each ("" if none). */
 int PSStencilFunctionCheck(const char *source, const char *name, char *log, size_t logsize);
 

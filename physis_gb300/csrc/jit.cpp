@@ -489,7 +489,8 @@ std::string entry_source(const JitKernel &k) {
 
 // ---- the tiled entry ---------------------------------------------------------
 // A CTA of four warps and a producer warp owns a 64 x 16 (x, y) tile and a
-// chunk of z; a thread computes eight consecutive rows of one column.  Grids
+// chunk of z; a thread computes eight consecutive rows of one column (or eight warps
+// and four rows, see choose_form).  Grids
 // the stencil reads at neighbour offsets (and never emits to) are staged: a
 // ring of shared-memory planes of the tile plus halo, one TMA box per plane,
 // loaded a step ahead of the compute by the producer warp, which on edge tiles
@@ -498,7 +499,7 @@ std::string entry_source(const JitKernel &k) {
 // every result is bit-identical to the plain entry's.
 //
 // Issue slots are what such a kernel is short of, so:
-// * the eight rows share their loads (the window positions of a thread's cells
+// * a thread's rows share their loads (the window positions of a thread's cells
 //   differ by constants, so equal reads are one load to the compiler) and a
 //   step's fixed work;
 // * warps whose cells all lie at least one cell inside the domain's grids and
@@ -511,9 +512,8 @@ std::string entry_source(const JitKernel &k) {
 // 27-point function at 258 x 258 x 200 double 673 against 727 us (the FP64
 // pipe's time is 556).
 constexpr int kTileX = 64, kTileY = 16;
-constexpr int kTileRows = 8;                              // rows per thread
-constexpr int kTileWarps = kTileX / 32 * kTileY / kTileRows;
-constexpr int kTileThreads = 32 * (kTileWarps + 1);
+int tile_warps(int rows) { return kTileX / 32 * kTileY / rows; }  // rows: per thread, 8 or 4
+int tile_threads(int rows) { return 32 * (tile_warps(rows) + 1); }
 constexpr size_t kStageBudget = 80 * 1024;                // two or more CTAs per SM
 constexpr size_t kStageHead = 128;                        // mbarriers in front of the rings
 
@@ -556,6 +556,146 @@ bool call_args(const std::string &src, size_t open, std::vector<std::string> *ar
   return false;
 }
 
+// How the source text reads a grid parameter of the stencil.
+struct GridUse {
+  int reads = 0;                 // PSGridGet / PSGridGetPeriodic of it
+  bool emitted = false;          // a PSGridEmit anywhere in the source names it
+  bool off_centre = false, periodic = false;
+  int r[3] = {0, 0, 0};          // halo widths
+};
+
+std::vector<GridUse> grid_uses(const JitKernel &k) {
+  std::vector<GridUse> uses(k.params.size());
+  const std::string &src = k.source;
+  const std::regex emit_re("\\bPSGridEmit(?:Utype)?\\s*\\(\\s*(\\w+)");
+  for (auto it = std::sregex_iterator(src.begin(), src.end(), emit_re);
+       it != std::sregex_iterator(); ++it)
+    for (size_t pi = 0; pi < uses.size(); ++pi)
+      if (k.params[pi].grid && k.params[pi].name == (*it)[1].str()) uses[pi].emitted = true;
+  const std::regex get_re("\\bPSGridGet(Periodic)?\\s*\\(");
+  for (auto it = std::sregex_iterator(src.begin(), src.end(), get_re);
+       it != std::sregex_iterator(); ++it) {
+    const size_t open = it->position(0) + it->length(0) - 1;
+    std::vector<std::string> args;
+    size_t close = 0;
+    if (!call_args(src, open, &args, &close) || args.size() != 4) continue;
+    for (size_t pi = 0; pi < uses.size(); ++pi) {
+      if (!k.params[pi].grid || k.params[pi].rank != 3 || trim(args[0]) != k.params[pi].name)
+        continue;
+      GridUse &u = uses[pi];
+      ++u.reads;
+      if ((*it)[1].matched) u.periodic = true;
+      for (int d = 0; d < 3; ++d) {
+        std::smatch m;
+        const std::string a = trim(args[d + 1]);
+        static const std::regex lit_re("^(\\w+)\\s*(?:([+-])\\s*([0-9]+))?$");
+        if (std::regex_match(a, m, lit_re) && m[1].str() == k.idx[d]) {
+          const int c = m[3].matched ? std::atoi(m[3].str().c_str()) : 0;
+          if (c) u.off_centre = true;
+          u.r[d] = std::max(u.r[d], std::min(c, 4));
+        } else {
+          u.off_centre = true;
+          u.r[d] = std::max(u.r[d], 1);
+        }
+      }
+    }
+  }
+  return uses;
+}
+
+// Stages parameter pi if it can be and the budget lasts.
+bool add_stage(JitKernel *k, size_t pi, const GridUse &u) {
+  const JitParam &p = k->params[pi];
+  if (!p.grid || p.rank != 3 || p.type == kUser || u.emitted) return false;
+  JitStage st;
+  st.param = (int)pi;
+  st.rx = u.r[0];
+  st.ry = u.r[1];
+  st.rz = u.r[2];
+  st.periodic = u.periodic;
+  st.esz = (p.type == kFloat || p.type == kInt) ? 4 : 8;
+  // the window starts on 16 bytes, up to v - 1 cells left of the halo
+  const int v = 16 / st.esz;
+  st.w = (kTileX + 2 * st.rx + 2 * (v - 1)) / v * v;
+  st.bytes = (size_t)ring_planes(st.rz) * plane_bytes(st);
+  if (k->stage_smem + st.bytes > kStageBudget) return false;
+  st.off = k->stage_smem;
+  k->stage_smem += st.bytes;
+  k->stages.push_back(st);
+  return true;
+}
+
+void no_stages(JitKernel *k) {
+  k->stages.clear();
+  k->stage_smem = 0;
+}
+
+// The form of the tiled entry, or none.  Its threads make up for few warps with
+// rows whose loads do not wait for one another; a read from global memory does wait
+// (for the row before it to be stored: the compiler cannot tell that the two do not
+// overlap), so a stencil that leaves grids unstaged takes another form.  Times of
+// four sweeps, in us, 256 x 256 x 128 and 400 x 384 x 320:
+// * 4-byte grids read at the cell only are staged as well, where that leaves none
+//   (two coefficient grids 136 and 562; unstaged in eight rows 355 and 1905, in
+//   four 193 and 1081, plain entry 201 and 1301);
+// * where one with a halo is left: four rows, eight warps (four inputs 328 and
+//   1575; eight rows 419 and 2181, plain 510 and 3175);
+// * else (an emitted grid that is read; many grids, whose rows would each hold a
+//   register per grid) the plain entry (Himeno's 14 grids 472 and 3038; eight rows
+//   2728 and 15732);
+// * 8-byte grids, whose bound is the FP64 pipe: four rows on eight warps for a few
+//   unstaged reads (three coefficients 670 and 3929; eight rows 742 and 4384, plain
+//   689 and 4347), the plain entry for more or for two staged grids, whose rings
+//   leave few CTAs to an SM (1171 and 7240; 1231 and 7372).
+// Under 4 M cells (2^22) there are too few planes for a CTA to be worth the ring's
+// start: plain (two coefficients 300 x 20 x 400 50, staged 79), also for one grid
+// read three or more planes away (a star of radius 4, 61 and 160; 187 and 704
+// above, 299 and 2041 plain).
+void choose_form(JitKernel *k, const std::vector<GridUse> &uses) {
+  int grids = 0, left = 0, rz = 0;
+  bool wide = false, left_off = false;
+  for (size_t pi = 0; pi < uses.size(); ++pi) {
+    if (!uses[pi].reads) continue;
+    const JitParam &p = k->params[pi];
+    ++grids;
+    wide |= p.type == kDouble || p.type == kLong;
+    bool staged = false;
+    for (const JitStage &st : k->stages) staged |= st.param == (int)pi;
+    if (staged) {
+      rz = std::max(rz, uses[pi].r[2]);
+    } else {
+      left += uses[pi].reads;
+      left_off |= uses[pi].off_centre;
+    }
+  }
+  if (!left) {
+    if (wide && k->stages.size() > 1) return no_stages(k);
+    if (rz >= 3) {
+      k->min_ctas = 3;
+      k->plain_below = 1 << 22;
+    }
+    return;
+  }
+  if (grids > 8 || (wide && left > 6)) return no_stages(k);
+  k->plain_below = 1 << 22;
+  if (wide) {
+    k->rows = 4;
+    k->min_ctas = 4;
+    return;
+  }
+  if (left_off) {
+    k->rows = 4;
+    k->min_ctas = 3;
+    return;
+  }
+  for (size_t pi = 0; pi < uses.size(); ++pi) {
+    bool staged = false;
+    for (const JitStage &st : k->stages) staged |= st.param == (int)pi;
+    if (uses[pi].reads && !staged && !add_stage(k, pi, uses[pi])) return no_stages(k);
+  }
+  if (k->stages.size() > 2) k->min_ctas = 3;
+}
+
 // Chooses the staged grids of a 3D stencil from its source text.  A grid is
 // staged when some PSGridGet / PSGridGetPeriodic of it reads off the centre
 // and no PSGridEmit anywhere in the source names it.  A coordinate written
@@ -565,71 +705,18 @@ bool call_args(const std::string &src, size_t open, std::vector<std::string> *ar
 // any read outside the staged window to global memory, so the choice affects
 // speed only, never results.
 void choose_stages(JitKernel *k) {
-  k->stages.clear();
-  k->stage_smem = 0;
+  no_stages(k);
   if (k->nd != 3) return;
-  const std::string &src = k->source;
-  std::vector<std::string> emitted;
-  {
-    const std::regex emit_re("\\bPSGridEmit(?:Utype)?\\s*\\(\\s*(\\w+)");
-    for (auto it = std::sregex_iterator(src.begin(), src.end(), emit_re);
-         it != std::sregex_iterator(); ++it)
-      emitted.push_back((*it)[1].str());
-  }
-  const std::regex get_re("\\bPSGridGet(Periodic)?\\s*\\(");
-  for (size_t pi = 0; pi < k->params.size(); ++pi) {
-    const JitParam &p = k->params[pi];
-    if (!p.grid || p.rank != 3 || p.type == kUser) continue;
-    bool is_emitted = false;
-    for (const std::string &e : emitted) is_emitted |= (e == p.name);
-    if (is_emitted) continue;
-    int r[3] = {0, 0, 0};
-    bool off_centre = false, periodic = false;
-    for (auto it = std::sregex_iterator(src.begin(), src.end(), get_re);
-         it != std::sregex_iterator(); ++it) {
-      const size_t open = it->position(0) + it->length(0) - 1;
-      std::vector<std::string> args;
-      size_t close = 0;
-      if (!call_args(src, open, &args, &close) || args.size() != 4 || trim(args[0]) != p.name)
-        continue;
-      if ((*it)[1].matched) periodic = true;
-      for (int d = 0; d < 3; ++d) {
-        std::smatch m;
-        const std::string a = trim(args[d + 1]);
-        static const std::regex lit_re("^(\\w+)\\s*(?:([+-])\\s*([0-9]+))?$");
-        if (std::regex_match(a, m, lit_re) && m[1].str() == k->idx[d]) {
-          const int c = m[3].matched ? std::atoi(m[3].str().c_str()) : 0;
-          if (c) off_centre = true;
-          r[d] = std::max(r[d], std::min(c, 4));
-        } else {
-          off_centre = true;
-          r[d] = std::max(r[d], 1);
-        }
-      }
-    }
-    if (!off_centre) continue;
-    JitStage st;
-    st.param = (int)pi;
-    st.rx = r[0];
-    st.ry = r[1];
-    st.rz = r[2];
-    st.periodic = periodic;
-    st.esz = (p.type == kFloat || p.type == kInt) ? 4 : 8;
-    // the window starts on 16 bytes, up to v - 1 cells left of the halo
-    const int v = 16 / st.esz;
-    st.w = (kTileX + 2 * st.rx + 2 * (v - 1)) / v * v;
-    st.bytes = (size_t)ring_planes(st.rz) * plane_bytes(st);
-    if (k->stage_smem + st.bytes > kStageBudget) continue;
-    st.off = k->stage_smem;
-    k->stage_smem += st.bytes;
-    k->stages.push_back(st);
-  }
+  const std::vector<GridUse> uses = grid_uses(*k);
+  for (size_t pi = 0; pi < uses.size(); ++pi)
+    if (uses[pi].off_centre) add_stage(k, pi, uses[pi]);
+  if (!k->stages.empty()) choose_form(k, uses);
 }
 
 std::string tiled_entry_source(const JitKernel &k) {
   const auto N = [](long long v) { return std::to_string(v); };
-  std::string s = "\nextern \"C\" __global__ void __launch_bounds__(" + N(kTileThreads) +
-                  ") __ps_entry_t(int dmin0, int dmax0, int dmin1, int dmax1, int dmin2, "
+  std::string s = "\nextern \"C\" __global__ void __launch_bounds__(" + N(tile_threads(k.rows)) +
+                  (k.min_ctas ? ", " + N(k.min_ctas) : std::string()) + ") __ps_entry_t(int dmin0, int dmax0, int dmin1, int dmax1, int dmin2, "
                   "int dmax2, int ntx, int zlen, int early, int *err";
   for (size_t j = 0; j < k.stages.size(); ++j)
     s += ", const __grid_constant__ __PSTmap tm" + N(j);
@@ -648,7 +735,7 @@ std::string tiled_entry_source(const JitKernel &k) {
        "  if (threadIdx.x == 0) {\n"
        "    for (int i = 0; i < 2; ++i) {\n"
        "      psg::mbar_init(&full[i], 1);\n      psg::mbar_init(&raw[i], 1);\n"
-       "      psg::mbar_init(&empty[i], " + N(kTileWarps) + ");\n    }\n"
+       "      psg::mbar_init(&empty[i], " + N(tile_warps(k.rows)) + ");\n    }\n"
        "    psg::fence_barrier_init();\n  }\n"
        "  __syncthreads();\n"
        "  if (early) psg::launch_dependents();\n  psg::wait_for_predecessors();\n";
@@ -685,7 +772,7 @@ std::string tiled_entry_source(const JitKernel &k) {
     fixs += "        " + fix + "(i + " + N(2 * st.rz) + ") % " + N(S) + " * " + N(pe) + ", a" + i + ", xs" +
             sj + ", ys" + sj + ", " + fit + "(zs + i + " + N(st.rz) + ", a" + i + ".nz), lane);\n";
   }
-  s += "  if (warp == " + N(kTileWarps) + ") {\n"
+  s += "  if (warp == " + N(tile_warps(k.rows)) + ") {\n"
        "    const bool edge = " + edge + ";\n"
        "    for (int i = 0; i < n; ++i) {\n"
        "      // group i replaces the plane that step i - 2 read last\n"
@@ -707,9 +794,9 @@ std::string tiled_entry_source(const JitKernel &k) {
        "    return;\n  }\n";
   // consumers
   s += "  const int x = x0 + lane + 32 * (warp % " + N(kTileX / 32) + ");\n"
-       "  const int yb = y0 + " + N(kTileRows) + " * (warp / " + N(kTileX / 32) + ");\n";
+       "  const int yb = y0 + " + N(k.rows) + " * (warp / " + N(kTileX / 32) + ");\n";
   std::string inner = "__all_sync(0xffffffffu, x >= dmin0 && x < dmax0 && yb + " +
-                      N(kTileRows) + " <= dmax1", zin, assume;
+                      N(k.rows) + " <= dmax1", zin, assume;
   for (size_t i = 0; i < k.params.size(); ++i) {
     if (!k.params[i].grid) continue;
     const JitParam &p = k.params[i];
@@ -721,7 +808,7 @@ std::string tiled_entry_source(const JitKernel &k) {
           : p.rank == 2 ? "(long long)yb * " + a + ".row + x"
                         : "(long long)zs * " + a + ".plane + (long long)yb * " + a + ".row + x") + ");\n";
     if (p.rank != 3) continue;
-    inner += " && x >= 1 && x < " + a + ".nx - 1 && yb >= 1 && yb + " + N(kTileRows) + " <= " + a +
+    inner += " && x >= 1 && x < " + a + ".nx - 1 && yb >= 1 && yb + " + N(k.rows) + " <= " + a +
              ".ny - 1";
     zin += " && z < " + a + ".nz - 1";
     for (const char *d : {"x", "y", "z"}) {
@@ -764,7 +851,7 @@ std::string tiled_entry_source(const JitKernel &k) {
     cell += "          g" + si + ".e = e" + si + (p.rank == 1 ? "" : " + r * a" + si + ".row") + ";\n";
     if (p.rank == 3) advance += "    e" + si + " += a" + si + ".plane;\n";
   }
-  const std::string rows = "#pragma unroll\n        for (int r = 0; r < " + N(kTileRows) + "; ++r) {\n"
+  const std::string rows = "#pragma unroll\n        for (int r = 0; r < " + N(k.rows) + "; ++r) {\n"
                            "          const int y = yb + r;\n";
   s += "      if (inner && z > 0" + zin + ") {\n" + rows +
        "          __builtin_assume(x > 0); __builtin_assume(y > 0); __builtin_assume(z > 0); " + assume +
@@ -888,7 +975,7 @@ bool jit_compile(const char *source, const char *name, JitKernel *k, std::string
     }
   }
   k->tiled_occ = 0;
-  if (fn_t && (g_drv.occupancy(&k->tiled_occ, fn_t, kTileThreads, stage_dynamic(*k)) !=
+  if (fn_t && (g_drv.occupancy(&k->tiled_occ, fn_t, tile_threads(k->rows), stage_dynamic(*k)) !=
                    CUDA_SUCCESS ||
                k->tiled_occ < 1)) {
     k->tiled_occ = 0;
@@ -926,10 +1013,12 @@ void jit_unload(JitKernel *k) {
 
 namespace {
 
-// PS_FUNCTION_TILED=0 runs every map on the plain entry (read per launch).
-bool tiled_enabled() {
+// PS_FUNCTION_TILED=0 runs every map on the plain entry, =1 every map on the tiled
+// one that it can run, however small (read per launch).
+bool tiled_wanted(const JitKernel &k, long long cells) {
   const char *e = getenv("PS_FUNCTION_TILED");
-  return !(e && e[0] == '0');
+  if (e && e[0] == '0') return false;
+  return (e && e[0] == '1') || cells >= k.plain_below;
 }
 
 }  // namespace
@@ -965,7 +1054,8 @@ cudaError_t jit_launch(const JitKernel &k, const Box &dom, int color, const Grid
   const int nxd = dom.max[0] - dom.min[0], nyd = dom.max[1] - dom.min[1],
             nzd = dom.max[2] - dom.min[2];
   if (nxd <= 0 || nyd <= 0 || nzd <= 0) return cudaSuccess;
-  bool tiled = k.func_tiled && color < 0 && tiled_enabled() && k.tiled_occ > 0;
+  bool tiled = k.func_tiled && color < 0 && k.tiled_occ > 0 &&
+               tiled_wanted(k, (long long)nxd * nyd * nzd);
   std::vector<CUtensorMap> maps(tiled ? k.stages.size() : 0);
   for (size_t t = 0; t < maps.size() && tiled; ++t) {
     const JitStage &st = k.stages[t];
@@ -1006,7 +1096,7 @@ cudaError_t jit_launch(const JitKernel &k, const Box &dom, int color, const Grid
     gx = (unsigned)tiles;
     gy = (unsigned)chunks;
     gz = 1;
-    bx = kTileThreads;
+    bx = (unsigned)tile_threads(k.rows);
     by = 1;
     const int h[9] = {dom.min[0], dom.max[0], dom.min[1], dom.max[1], dom.min[2], dom.max[2],
                       (int)ntx,   zlen,       tiles * chunks >= want};

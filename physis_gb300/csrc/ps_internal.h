@@ -224,6 +224,9 @@ struct JitKernel {
   int ngrids = 0, nscalars = 0;
   std::vector<JitStage> stages;   // grids the tiled entry stages (3D only)
   size_t stage_smem = 0;
+  // the tiled entry's form: rows per thread, CTAs per SM its registers must allow
+  // (0: no bound), and the cells of a domain under which the plain entry runs
+  int rows = 8, min_ctas = 0, plain_below = 0;
   void *module = nullptr, *func = nullptr;
   void *func_tiled = nullptr;     // __ps_entry_t, when stages is not empty
   int tiled_occ = 0;              // its resident CTAs per SM

@@ -2214,9 +2214,10 @@ int PSStencilFunctionCheck(const char *source, const char *name, char *log, size
   if (psg::jit_build(source, name, &k, &image, &why)) {
     std::string rep;
     for (const psg::JitStage &st : k.stages)
-      rep += "staged " + k.params[st.param].name + " " + std::to_string(st.rx) + " " +
-             std::to_string(st.ry) + " " + std::to_string(st.rz) +
-             (st.periodic ? " periodic;" : " clamp;");
+      if (st.rx || st.ry || st.rz)
+        rep += "staged " + k.params[st.param].name + " " + std::to_string(st.rx) + " " +
+               std::to_string(st.ry) + " " + std::to_string(st.rz) +
+               (st.periodic ? " periodic;" : " clamp;");
     if (log && logsize) snprintf(log, logsize, "%s", rep.c_str());
     return PS_OK;
   }

@@ -35,6 +35,8 @@ the library's kernels.
 import ctypes
 import math
 import time
+from itertools import chain
+from operator import is_, methodcaller
 
 import numpy as np
 
@@ -304,8 +306,9 @@ class Net:
         self.prepare()
 
     def _pointers(self):
-        return [t.data_ptr() for t in self.params + self.grads + self.m + self.v + self.w
-                + self.wf + self.wb]
+        # w's tensors are the first of params unless a program replaced some
+        return list(map(_ptr, chain(self.params, self.grads, self.m, self.v, self.wf, self.wb,
+                                    () if all(map(is_, self.w, self.params)) else self.w)))
 
     def stream(self):
         return _stream()
@@ -370,8 +373,11 @@ def _stream():
     return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
+_ptr = methodcaller("data_ptr")
+
+
 def _p(t):
-    return None if t is None else ctypes.c_void_p(t.data_ptr())
+    return None if t is None else t.data_ptr()
 
 
 def _ok(code):
