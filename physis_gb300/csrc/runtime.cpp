@@ -2567,7 +2567,9 @@ static cudaStream_t ws_stream(void *stream) {
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if ((s && s != cudaStreamLegacy) || !rt) return s;
   cudaStreamCaptureStatus cap;
-  if (capturing() || cudaStreamIsCapturing(cudaStreamLegacy, &cap) != cudaSuccess) {
+  // (only who was given the runtime's stream can capture it)
+  if ((rt->stream_out && capturing()) ||
+      cudaStreamIsCapturing(cudaStreamLegacy, &cap) != cudaSuccess) {
     cudaGetLastError();
     return s ? s : rt->stream;
   }

@@ -324,14 +324,15 @@ class Net:
         B, Z, Y, X = dims
         n = B * Z * Y * X
         L, stream = ps.lib(), self.stream()
-        acts = [x] + list(torch.empty((LAYERS, n * C), dtype=torch.bfloat16, device="cuda"))
+        acts = torch.empty((LAYERS, n * C), dtype=torch.bfloat16, device="cuda")
         out0 = torch.empty(n, dtype=torch.float32, device="cuda")
+        src, dst, layer = _p(x), _p(acts), n * C * 2  # bytes
         for l in range(LAYERS):
             last = l == LAYERS - 1
-            _ok(L.PSWarmStartConv(_p(acts[l]), _p(self.wf[l]), _p(self.b[l]), None,
-                                  0 if last else 1, _p(acts[l + 1]), _p(out0) if last else None,
-                                  B, Z, Y, X, stream))
-        self._acts = acts
+            _ok(L.PSWarmStartConv(src, _p(self.wf[l]), _p(self.b[l]), None, 0 if last else 1, dst,
+                                  _p(out0) if last else None, B, Z, Y, X, stream))
+            src, dst = dst, dst + layer
+        self._acts = x, acts
         return out0
 
     def backward(self, dy, dims, work):
@@ -341,16 +342,19 @@ class Net:
         n = B * Z * Y * X
         L, stream = ps.lib(), self.stream()
         nsplit = work.numel() // (27 * C * C + C)
-        dx = list(torch.empty((2, n * C), dtype=torch.bfloat16, device="cuda"))
-        g = dy
+        dx = torch.empty((2, n * C), dtype=torch.bfloat16, device="cuda")
+        layer = n * C * 2  # bytes
+        x, acts = self._acts
+        act = [_p(x)] + [_p(acts) + l * layer for l in range(LAYERS - 1)]  # of each layer's input
+        g, part, spare = _p(dy), _p(work), [_p(dx), _p(dx) + layer]
         for l in range(LAYERS - 1, -1, -1):
-            _ok(L.PSWarmStartWeightGrad(_p(self._acts[l]), _p(g), _p(work), nsplit,
-                                        _p(self.grads[l]), _p(self.grads[LAYERS + l]),
-                                        B, Z, Y, X, stream))
+            _ok(L.PSWarmStartWeightGrad(act[l], g, part, nsplit, _p(self.grads[l]),
+                                        _p(self.grads[LAYERS + l]), B, Z, Y, X, stream))
             if l:
-                _ok(L.PSWarmStartConv(_p(g), _p(self.wb[l]), None, _p(self._acts[l]), 0,
-                                      _p(dx[l % 2]), None, B, Z, Y, X, stream))
-                g = dx[l % 2]
+                to = spare[l % 2]
+                _ok(L.PSWarmStartConv(g, _p(self.wb[l]), None, act[l], 0, to, None, B, Z, Y, X,
+                                      stream))
+                g = to
 
     def adam(self, lr, b1=0.9, b2=0.999, eps=1e-8):
         self.step += 1
