@@ -19,7 +19,7 @@
 // one does not otherwise take the other's until it is idle).  Himeno's comes
 // first: its items are the longer ones, and CTAs of it that found their places
 // taken would make the tail (48 grids up to 320 x 320 x 512 161.7 GLUPS, 155.7 with
-// the 7-point family first).
+// the 7-point family first, in turn on one box; other boxes gave 157 to 163).
 // In each kernel the last warp is a producer that fills the ring on into the
 // CTA's next item, and consumer warps release stages one by one.
 // Bound: the Himeno family HBM (216 of the 24-problem batch's 256 us a step), the
