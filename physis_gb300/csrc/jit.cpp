@@ -564,14 +564,20 @@ struct GridUse {
   int r[3] = {0, 0, 0};          // halo widths
 };
 
-std::vector<GridUse> grid_uses(const JitKernel &k) {
+// One per parameter; *elsewhere: some PSGridEmit names what is no grid parameter (a
+// helper function's own), so any of them may be emitted.
+std::vector<GridUse> grid_uses(const JitKernel &k, bool *elsewhere) {
   std::vector<GridUse> uses(k.params.size());
+  *elsewhere = false;
   const std::string &src = k.source;
   const std::regex emit_re("\\bPSGridEmit(?:Utype)?\\s*\\(\\s*(\\w+)");
   for (auto it = std::sregex_iterator(src.begin(), src.end(), emit_re);
-       it != std::sregex_iterator(); ++it)
+       it != std::sregex_iterator(); ++it) {
+    bool ours = false;
     for (size_t pi = 0; pi < uses.size(); ++pi)
-      if (k.params[pi].grid && k.params[pi].name == (*it)[1].str()) uses[pi].emitted = true;
+      if (k.params[pi].grid && k.params[pi].name == (*it)[1].str()) uses[pi].emitted = ours = true;
+    *elsewhere |= !ours;
+  }
   const std::regex get_re("\\bPSGridGet(Periodic)?\\s*\\(");
   for (auto it = std::sregex_iterator(src.begin(), src.end(), get_re);
        it != std::sregex_iterator(); ++it) {
@@ -651,7 +657,7 @@ void no_stages(JitKernel *k) {
 // start: plain (two coefficients 300 x 20 x 400 50, staged 79), also for one grid
 // read three or more planes away (a star of radius 4, 61 and 160; 187 and 704
 // above, 299 and 2041 plain).
-void choose_form(JitKernel *k, const std::vector<GridUse> &uses) {
+void choose_form(JitKernel *k, const std::vector<GridUse> &uses, bool emits_elsewhere) {
   int grids = 0, left = 0, rz = 0;
   bool wide = false, left_off = false;
   for (size_t pi = 0; pi < uses.size(); ++pi) {
@@ -688,6 +694,8 @@ void choose_form(JitKernel *k, const std::vector<GridUse> &uses) {
     k->min_ctas = 3;
     return;
   }
+  // a cell that is read after it was emitted has to show what was emitted
+  if (emits_elsewhere) return no_stages(k);
   for (size_t pi = 0; pi < uses.size(); ++pi) {
     bool staged = false;
     for (const JitStage &st : k->stages) staged |= st.param == (int)pi;
@@ -707,10 +715,11 @@ void choose_form(JitKernel *k, const std::vector<GridUse> &uses) {
 void choose_stages(JitKernel *k) {
   no_stages(k);
   if (k->nd != 3) return;
-  const std::vector<GridUse> uses = grid_uses(*k);
+  bool elsewhere = false;
+  const std::vector<GridUse> uses = grid_uses(*k, &elsewhere);
   for (size_t pi = 0; pi < uses.size(); ++pi)
     if (uses[pi].off_centre) add_stage(k, pi, uses[pi]);
-  if (!k->stages.empty()) choose_form(k, uses);
+  if (!k->stages.empty()) choose_form(k, uses, elsewhere);
 }
 
 std::string tiled_entry_source(const JitKernel &k) {

@@ -74,6 +74,35 @@ def test_tiled_form_gives_the_plain_bits(rt, monkeypatch, name, dtype):
             assert np.array_equal(got[0].view(np.uint8), other.view(np.uint8)), shape
 
 
+def test_read_after_an_emit_in_a_helper(rt, monkeypatch):
+    # k is read at the cell only and emitted under another name: its second read
+    # sees what was emitted, on both entries
+    k = ps.stencil_function("""
+void put(PSGrid3DFloat g, float v) { PSGridEmit(g, v); }
+void f(const int x, const int y, const int z, PSGrid3DFloat u, PSGrid3DFloat k,
+       PSGrid3DFloat out) {
+  float a = PSGridGet(k, x, y, z) + PSGridGet(u, x + 1, y, z) + PSGridGet(u, x, y, z - 1);
+  put(k, a);
+  PSGridEmit(out, 2.0f * PSGridGet(k, x, y, z));
+}
+""", "f")
+    shape = (9, 18, 67)
+    nz, ny, nx = shape
+    rng = np.random.default_rng(9)
+    u, v = (rng.random(shape, dtype=np.float32) for _ in range(2))
+    a = (v[1:-1, 1:-1, 1:-1] + u[1:-1, 1:-1, 2:]) + u[:-2, 1:-1, 1:-1]
+    for env in ("0", "1"):
+        monkeypatch.setenv("PS_FUNCTION_TILED", env)
+        grids = [ps.Grid(shape) for _ in range(3)]
+        for g, w in zip(grids, (u, v, np.zeros_like(u))):
+            g.copyin(w)
+        ps.stencil_run([ps.stencil_map(k, ps.domain(1, nx - 1, 1, ny - 1, 1, nz - 1), grids)])
+        assert np.array_equal(grids[2].copyout()[1:-1, 1:-1, 1:-1], np.float32(2) * a)
+        assert np.array_equal(grids[1].copyout()[1:-1, 1:-1, 1:-1], a)
+        for g in grids:
+            g.free()
+
+
 @pytest.mark.parametrize("name", ["four coefficients", "nine grids"])
 def test_large_domains_choose_for_themselves(rt, monkeypatch, name):
     # 4.5 M cells: past the line under which these run the plain entry
