@@ -1876,8 +1876,10 @@ void PSFinalize(void) {
   g_batches.clear();
   for (psg::JitKernel &k : rt->funcs) psg::jit_unload(&k);
   psg::nn_set_error_word(nullptr);
-  cudaFreeHost(rt->host_err);
   cudaFree(rt->partials);
+  // after a free of device memory, which waits for kernels on the callers' streams
+  // that may still write the error word
+  cudaFreeHost(rt->host_err);
   cudaFree(rt->ticket);
   cudaFree(rt->res_packets);
   for (int i = 0; i < kNumEvents; ++i) cudaEventDestroy(rt->events[i]);
