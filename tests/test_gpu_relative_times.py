@@ -110,3 +110,18 @@ def test_points_in_random_order(rt):
     for g in grids:
         g.free()
     assert t[1] < 9 * t[0]  # 5; 19 where loads held for later were spilled
+
+
+def test_function_of_one_plane(rt):
+    src = """void scale1(const int x, const int y, const int z, PSGrid3DFloat u, PSGrid3DFloat o,
+             float c) { PSGridEmit(o, c * PSGridGet(u, x, y, z)); }"""
+    fn = ps.stencil_function(src, "scale1")
+    t = []
+    for nz in (1, 4):
+        shape = (nz, 1, 5000000)
+        grids = _grids(shape, 2)
+        t.append(_time(_sweeps(fn, ps.full_domain(shape), grids, [0.5]), 4))
+        for g in grids:
+            g.free()
+    # 0.50; as many CTAs each, and 0.95 where their start took most of the time
+    assert t[0] < 0.7 * t[1]
