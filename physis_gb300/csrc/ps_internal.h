@@ -105,6 +105,7 @@ struct Temporal7Args {
   int k;
   bool fma;        // contract each multiply-add (else bit-exact to k plain steps)
   bool overlap;
+  bool first;      // a sweep or a call ahead of it, not a pass
 };
 int temporal7_max_k(int esz);
 size_t temporal7_smem_bytes(int esz, const MarchConfig &cfg, int k);

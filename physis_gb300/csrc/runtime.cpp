@@ -700,14 +700,15 @@ bool launch_map(const Map &m, bool want_gosa) {
   return launch_s7(m, view(m.grids[0]), view(m.grids[1]));
 }
 
-// One temporal pass: out = k steps of map m's stencil applied to in.
-bool launch_t7(const Map &m, const GridView &in, const GridView &out, int k) {
+// One temporal pass (first: of a run): out = k steps of map m's stencil applied to in.
+bool launch_t7(const Map &m, const GridView &in, const GridView &out, int k, bool first) {
   psg::Temporal7Args a{};
   a.in = in;
   a.out = out;
   a.k = k;
   a.fma = rt->fma;
   a.overlap = rt->overlap;
+  a.first = first;
   for (int i = 0; i < 7; ++i) a.coef[i] = m.scalars[i];
   const MarchConfig cfg = m.has_plan ? m.plan.tshape : rt->tshapes[shape_slot(m.kernel)];
   const int vec = 16 / in.esz;
@@ -776,7 +777,7 @@ bool run_temporal(const Map &a, int iter) {
   // the previous step also ends up in memory.
   while (total - 1 - t >= 2) {
     const int kk = std::min(k, total - 1 - t);
-    if (!launch_t7(a, cur, oth, kk)) return false;
+    if (!launch_t7(a, cur, oth, kk, t == 0)) return false;
     std::swap(cur, oth);
     t += kk;
   }

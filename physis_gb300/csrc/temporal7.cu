@@ -325,7 +325,7 @@ t7_kernel(const __grid_constant__ CUtensorMap tin, const TParams<T> p) {
 
 template <typename T, int RY, int K, bool FMA>
 cudaError_t launch_k(TParams<T> p, const MarchConfig &cfg, const CUtensorMap *tin,
-                     int sm_count, bool overlap, cudaStream_t st) {
+                     int sm_count, bool overlap, bool first, cudaStream_t st) {
   constexpr int VEC = 16 / (int)sizeof(T);
   constexpr int TXO = 30 * VEC;
   const int tye = cfg.warps * cfg.rows;
@@ -353,29 +353,34 @@ cudaError_t launch_k(TParams<T> p, const MarchConfig &cfg, const CUtensorMap *ti
   int64_t grid = resident;
   if (grid > p.items) grid = p.items;
   p.early = grid == resident;
+  // A double pass is bound by the FP64 pipes.  If it leaves places free, its CTAs are
+  // spread evenly only when they find the GPU empty, not when a sweep lets them in
+  // where its first CTAs end (12 steps in five and four passes, us, the first
+  // overlapping and not: 100 x 66 x 40 k 2 604 and 518, k 3 536 and 492; 80 x 90 x 100 k 2 627 and 541).
+  if (sizeof(T) == 8 && first && !p.early) overlap = false;
   return launch_kernel(kern, (unsigned)grid, dim3(32, cfg.warps, 1), smem, st, overlap, *tin, p);
 }
 
 template <typename T, int RY, bool FMA>
 cudaError_t launch_rows(const TParams<T> &p, const MarchConfig &cfg, const CUtensorMap *tin,
-                        int sm_count, bool overlap, cudaStream_t st) {
+                        int sm_count, bool overlap, bool first, cudaStream_t st) {
   constexpr int VEC = 16 / (int)sizeof(T);
-  if (p.k <= 2) return launch_k<T, RY, 2, FMA>(p, cfg, tin, sm_count, overlap, st);
-  if (p.k <= 3) return launch_k<T, RY, 3, FMA>(p, cfg, tin, sm_count, overlap, st);
+  if (p.k <= 2) return launch_k<T, RY, 2, FMA>(p, cfg, tin, sm_count, overlap, first, st);
+  if (p.k <= 3) return launch_k<T, RY, 3, FMA>(p, cfg, tin, sm_count, overlap, first, st);
   if constexpr (VEC >= 4) {
-    if (p.k <= 4) return launch_k<T, RY, 4, FMA>(p, cfg, tin, sm_count, overlap, st);
-    if (p.k <= 5) return launch_k<T, RY, 5, FMA>(p, cfg, tin, sm_count, overlap, st);
+    if (p.k <= 4) return launch_k<T, RY, 4, FMA>(p, cfg, tin, sm_count, overlap, first, st);
+    if (p.k <= 5) return launch_k<T, RY, 5, FMA>(p, cfg, tin, sm_count, overlap, first, st);
   }
   return cudaErrorInvalidValue;
 }
 
 template <typename T, bool FMA>
 cudaError_t launch_shape(const TParams<T> &p, const MarchConfig &cfg, const CUtensorMap *tin,
-                         int sm_count, bool overlap, cudaStream_t st) {
+                         int sm_count, bool overlap, bool first, cudaStream_t st) {
   switch (cfg.rows) {
-    case 1: return launch_rows<T, 1, FMA>(p, cfg, tin, sm_count, overlap, st);
-    case 2: return launch_rows<T, 2, FMA>(p, cfg, tin, sm_count, overlap, st);
-    case 4: return launch_rows<T, 4, FMA>(p, cfg, tin, sm_count, overlap, st);
+    case 1: return launch_rows<T, 1, FMA>(p, cfg, tin, sm_count, overlap, first, st);
+    case 2: return launch_rows<T, 2, FMA>(p, cfg, tin, sm_count, overlap, first, st);
+    case 4: return launch_rows<T, 4, FMA>(p, cfg, tin, sm_count, overlap, first, st);
   }
   return cudaErrorInvalidConfiguration;
 }
@@ -402,8 +407,8 @@ cudaError_t launch_t(const Temporal7Args &a, const MarchConfig &cfg, const CUten
   p.err = dev_err;
   if (cfg.warps < 1 || cfg.warps > 8 || cfg.ns < 2 || cfg.ns > 16)
     return cudaErrorInvalidConfiguration;
-  return a.fma ? launch_shape<T, true>(p, cfg, tin, sm_count, a.overlap, st)
-               : launch_shape<T, false>(p, cfg, tin, sm_count, a.overlap, st);
+  return a.fma ? launch_shape<T, true>(p, cfg, tin, sm_count, a.overlap, a.first, st)
+               : launch_shape<T, false>(p, cfg, tin, sm_count, a.overlap, a.first, st);
 }
 
 }  // namespace
